@@ -27,6 +27,8 @@
 #include "decode_gemv.cuh"
 #include "dispatch.cuh"
 #include "ep_window.cuh"
+#include "exact_dense.cuh"
+#include "host_stage.h"
 #include "misc_kernels.cuh"
 #include "prefill_gemm.cuh"
 #include "pair_gemm.cuh"
@@ -36,6 +38,7 @@
 using namespace apus;
 
 constexpr int ROUTER_SMALL_MAX_T = 64;
+constexpr size_t DENSE_PARTS = 4;
 
 /* ------------------------------------------------------------------------ */
 /* context                                                                   */
@@ -44,6 +47,7 @@ constexpr int ROUTER_SMALL_MAX_T = 64;
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
+    float wmin = 0.0f, wmax = 0.0f;   /* smallest nonzero and largest magnitude */
 };
 
 struct Arena {
@@ -88,6 +92,7 @@ struct Ctx {
     uint64_t bytes_resident = 0, bytes_uploaded = 0, launches = 0;
     Arena ws;      /* block workspace */
     Arena io;      /* host-pointer staging */
+    HostStage hs;  /* page-locked side of the host-pointer copies */
     int *d_status = nullptr;
     unsigned int *d_scratch_u32 = nullptr;
     unsigned int *d_router_counters = nullptr;   /* [ROUTER_SMALL_MAX_T], self-resetting */
@@ -112,6 +117,9 @@ struct Ctx {
     long host_split_t = 4096;    /* APUS_CUDA_HOST_SPLIT_T: from this many tokens (0: never) */
     cudaStream_t s_in = nullptr, s_out = nullptr;
     cudaEvent_t ev_io[5] = {};   /* start, in[2], done[2] */
+    /* dense products of many rows run in parts beside each other */
+    cudaStream_t s_part[DENSE_PARTS] = {};
+    cudaEvent_t ev_part = nullptr;
     /* ordering of calls that arrive on different streams */
     cudaStream_t cur_stream = nullptr, last_stream = nullptr;
     cudaEvent_t last_ev = nullptr;
@@ -381,6 +389,7 @@ extern "C" void apus_cuda_disable(void) {
     for (auto &kv : c->layers) layer_free(kv.second);
     arena_free(c->ws);
     arena_free(c->io);
+    c->hs.release();
     if (c->last_ev) cudaEventDestroy(c->last_ev);
     if (c->d_status) cudaFree(c->d_status);
     if (c->d_router_counters) cudaFree(c->d_router_counters);
@@ -397,6 +406,9 @@ extern "C" void apus_cuda_disable(void) {
     if (c->s_out) cudaStreamDestroy(c->s_out);
     for (auto &e : c->ev_io)
         if (e) cudaEventDestroy(e);
+    for (auto &p : c->s_part)
+        if (p) cudaStreamDestroy(p);
+    if (c->ev_part) cudaEventDestroy(c->ev_part);
     g_ctx = nullptr;
     delete c;
 }
@@ -419,10 +431,23 @@ extern "C" const char *apus_cuda_last_error(void) { return g_err; }
 /* per-matmul entry points (host pointers)                                   */
 /* ------------------------------------------------------------------------ */
 
-static void *weight_buf(Ctx *c, const void *ptr, size_t bytes) {
+/* magnitude range of n BF16 values on the device (set-up: synchronises) */
+static int bf16_range(Ctx *c, const uint16_t *d, size_t n, float *lo, float *hi) {
+    unsigned int v[2] = {0x7f800000u, 0u};
+    CU_OK(cudaMemcpyAsync(c->d_scratch_u32, v, sizeof v, cudaMemcpyHostToDevice, c->stream));
+    bf16_range_kernel<<<c->sm_count * 4, 256, 0, c->stream>>>(d, n, c->d_scratch_u32);
+    CU_OK(cudaGetLastError());
+    CU_OK(cudaMemcpyAsync(v, c->d_scratch_u32, sizeof v, cudaMemcpyDeviceToHost, c->stream));
+    CU_OK(cudaStreamSynchronize(c->stream));
+    memcpy(lo, &v[0], 4);
+    memcpy(hi, &v[1], 4);
+    return 0;
+}
+
+static const DevBuf *weight_buf(Ctx *c, const void *ptr, size_t bytes) {
     auto it = c->wcache.find(ptr);
     if (it != c->wcache.end()) {
-        if (it->second.bytes >= bytes) return it->second.ptr;
+        if (it->second.bytes >= bytes) return &it->second;
         /* same key, larger view: replace the copy */
         cudaFree(it->second.ptr);
         c->bytes_resident -= it->second.bytes;
@@ -438,15 +463,87 @@ static void *weight_buf(Ctx *c, const void *ptr, size_t bytes) {
         cudaGetLastError();
         return nullptr;
     }
-    if (cudaMemcpy(d, ptr, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+    DevBuf b{d, bytes};
+    if (cudaMemcpy(d, ptr, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+        bf16_range(c, (const uint16_t *)d, bytes / 2, &b.wmin, &b.wmax)) {
         fail("weight upload failed");
         cudaFree(d);
         return nullptr;
     }
     c->bytes_resident += bytes;
     c->bytes_uploaded += bytes;
-    c->wcache.emplace(ptr, DevBuf{d, bytes});
-    return d;
+    return &c->wcache.emplace(ptr, b).first->second;
+}
+
+/* Launches the exact-order product that fits the shape.
+ *  - up to ER_MAX_M rows: weights streamed row by row, one chain per lane.  As
+ *    few warps per CTA as still put a CTA on every SM (a lane's chain takes the
+ *    same time however many run beside it), at most eight;
+ *  - more rows: by outputs per SM.  A wide warp tile widens fewer operands per
+ *    multiply-add but leaves SMs idle when there are few outputs (M 64, O 1024:
+ *    28 us with 2 x 32 per warp, 41 with 8 x 32; M 221, O 949: 68 us with 8 x 32,
+ *    53 with 8 x 64; M 512, O 1024: 86 us with 8 x 64, 74 with 8 x 128);
+ *  - K not a multiple of 8: rows are not made of aligned 16-byte pieces, the
+ *    plain kernel.
+ * M_all: rows of the whole call when a.M is one of the parts it runs in. */
+static int launch_exact(Ctx *c, const ExactArgs &a, int M_all, cudaStream_t st) {
+    const size_t optin = (size_t)c->smem_optin;
+    auto allow = [&](const void *kern, size_t smem) {
+        return smem <= 40 * 1024 ||        /* 48 KB with the static part */
+               cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)smem) == cudaSuccess;
+    };
+    if (a.K % 8 == 0 && a.M <= ER_MAX_M && exact_rows_smem(a.M, a.K, 1) <= optin) {
+        const long groups = (a.O + 31) / 32;
+        int warps = (int)((groups + c->sm_count - 1) / c->sm_count);
+        warps = warps < 1 ? 1 : (warps > 8 ? 8 : warps);
+        while (exact_rows_smem(a.M, a.K, warps) > optin) warps--;
+        long grid = (groups + warps - 1) / warps;
+        if (grid > c->sm_count) grid = c->sm_count;
+        const size_t smem = exact_rows_smem(a.M, a.K, warps);
+        const bool few = warps <= ER_FEW_WARPS;
+        void (*kern)(ExactArgs) =
+            a.M == 1   ? (few ? exact_rows_kernel<1, true> : exact_rows_kernel<1, false>)
+            : a.M == 2 ? (few ? exact_rows_kernel<2, true> : exact_rows_kernel<2, false>)
+            : a.M == 3 ? (few ? exact_rows_kernel<3, true> : exact_rows_kernel<3, false>)
+                       : (few ? exact_rows_kernel<4, true> : exact_rows_kernel<4, false>);
+        if (!allow((const void *)kern, smem)) return fail("exact rows: shared memory");
+        kern<<<(unsigned)grid, warps * 32, smem, st>>>(a);
+    } else if (a.K % 8 == 0) {
+        const long per_sm = (long)M_all * a.O / c->sm_count;
+        auto launch = [&](auto tile, void (*kern)(ExactArgs)) -> int {
+            using Tile = decltype(tile);
+            const long ot = (a.O + Tile::O - 1) / Tile::O,
+                       all = ((long)M_all + Tile::M - 1) / Tile::M * ot;
+            /* one wave: a CTA asks for more than half of an SM's shared memory, so
+             * that the parts of a call spread over the SMs instead of doubling up */
+            size_t smem = Tile::SMEM;
+            if (M_all > a.M && all <= c->sm_count && smem < optin / 2 + 1024)
+                smem = optin / 2 + 1024;
+            if (!allow((const void *)kern, smem)) return fail("exact tile: shared memory");
+            kern<<<dim3((unsigned)((a.M + Tile::M - 1) / Tile::M),
+                        (unsigned)(ot < 65535 ? ot : 65535)),
+                   Tile::THREADS, smem, st>>>(a);
+            return 0;
+        };
+        const int rc = per_sm <= 512    ? launch(ExactTile<2, 1>(), exact_tile_kernel<2, 1>)
+                       : per_sm <= 1024 ? launch(ExactTile<4, 1>(), exact_tile_kernel<4, 1>)
+                       : per_sm <= 2048 ? launch(ExactTile<8, 2>(), exact_tile_kernel<8, 2>)
+                                        : launch(ExactTile<8, 4>(), exact_tile_kernel<8, 4>);
+        if (rc) return 1;
+    } else {
+        const long total = (long)a.M * a.O;
+        int blocks = (int)((total + 127) / 128);
+        if (blocks > c->sm_count * 16) blocks = c->sm_count * 16;
+        if (a.f32_out)
+            exact_matvec_f32_kernel<<<blocks, 128, 0, st>>>(a.w, a.x, (float *)a.y, a.O,
+                                                                   a.K);
+        else
+            exact_gemm_kernel<<<blocks, 128, 0, st>>>(a.w, a.x, (uint16_t *)a.y, a.M, a.O,
+                                                             a.K);
+    }
+    LAUNCHED();
+    return 0;
 }
 
 static int dense_op(const uint16_t *w, const uint16_t *x, void *y, size_t M,
@@ -458,26 +555,75 @@ static int dense_op(const uint16_t *w, const uint16_t *x, void *y, size_t M,
     c->last_block_launches = 0;
     Ordered ord(c, c->stream);
     if (ord.rc) return 1;
-    const uint16_t *dw = (const uint16_t *)weight_buf(c, w, O * K * 2);
-    if (!dw) return 1;
-    size_t xb = M * K * 2, yb = M * O * (f32_out ? 4 : 2);
+    const DevBuf *wb = weight_buf(c, w, O * K * 2);
+    if (!wb) return 1;
+    const size_t xb = M * K * 2, yb = M * O * (f32_out ? 4 : 2);
     if (arena_reserve(c->io, xb + yb + 1024)) return 1;
     c->io.reset();
+    ExactArgs a;
+    a.w = (const uint16_t *)wb->ptr;
+    a.wmin = wb->wmin;
+    a.wmax = wb->wmax;
     uint16_t *dx = (uint16_t *)c->io.take(xb);
+    a.x = dx;
     void *dy = c->io.take(yb);
-    CU_OK(cudaMemcpyAsync(dx, x, xb, cudaMemcpyHostToDevice, c->stream));
-    long total = (long)(M * O);
-    int blocks = (int)((total + 127) / 128);
-    if (blocks > c->sm_count * 16) blocks = c->sm_count * 16;
-    if (f32_out)
-        exact_matvec_f32_kernel<<<blocks, 128, 0, c->stream>>>(
-            dw, dx, (float *)dy, (long)O, (int)K);
-    else
-        exact_gemm_kernel<<<blocks, 128, 0, c->stream>>>(
-            dw, dx, (uint16_t *)dy, (long)M, (long)O, (int)K);
-    LAUNCHED();
-    CU_OK(cudaMemcpyAsync(y, dy, yb, cudaMemcpyDeviceToHost, c->stream));
-    CU_OK(cudaStreamSynchronize(c->stream));
+    a.M = (int)M;
+    a.O = (long)O;
+    a.K = (int)K;
+    a.f32_out = f32_out ? 1 : 0;
+    /* Many rows: the call is cut into parts on streams of their own, so that the
+     * rows of one part travel while another computes.  A part fills only its share
+     * of the SMs; the parts' kernels run beside each other. */
+    const size_t parts = K % 8 == 0 && M >= DENSE_PARTS * 64 && xb >= (512u << 10) ? DENSE_PARTS : 1;
+    /* A small result, or one row of any size the slots hold, is stored straight
+     * into page-locked memory by the kernel: one operation less between the last
+     * chain and the caller.  (Several large rows go over PCIe as 64-byte stores
+     * of many tiles at once: 4 x slower than the copy engine.) */
+    const bool direct =
+        parts == 1 && yb <= (M == 1 ? HostStage::SLOTS * HostStage::SLOT_BYTES : 64u << 10);
+    if (direct) CU_OK(c->hs.init());
+    if (parts == 1) {
+        CU_OK(c->hs.upload(dx, x, xb, c->stream));
+        a.y = direct ? (void *)c->hs.out_dev : dy;
+        if (launch_exact(c, a, (int)M, c->stream)) return 1;
+        if (direct) {
+            CU_OK(cudaStreamSynchronize(c->stream));
+            host_copy(y, c->hs.out, yb);
+        } else {
+            CU_OK(c->hs.download(y, dy, yb, c->stream));
+            CU_OK(cudaStreamSynchronize(c->stream));
+        }
+        return 0;
+    }
+    for (size_t p = 0; p < parts; p++)
+        if (!c->s_part[p])
+            CU_OK(cudaStreamCreateWithFlags(&c->s_part[p], cudaStreamNonBlocking));
+    if (!c->ev_part) CU_OK(cudaEventCreateWithFlags(&c->ev_part, cudaEventDisableTiming));
+    CU_OK(cudaEventRecord(c->ev_part, c->stream));       /* earlier work owns dx, dy */
+    const size_t row = yb / M;                            /* bytes of a result row */
+    auto first = [&](size_t p) { return p >= parts ? M : M / 64 * p / parts * 64; };
+    static_assert(DENSE_PARTS <= (size_t)HostStage::SLOTS, "a download slot per part");
+    const bool slots = first(parts) - first(parts - 1) <= HostStage::SLOT_BYTES / row &&
+                       first(1) <= HostStage::SLOT_BYTES / row && !HostStage::page_locked(y);
+    for (size_t p = 0; p < parts; p++) {
+        const size_t r0 = first(p), n = first(p + 1) - r0;
+        CU_OK(cudaStreamWaitEvent(c->s_part[p], c->ev_part, 0));
+        CU_OK(c->hs.upload(dx + r0 * K, x + r0 * K, n * K * 2, c->s_part[p]));
+        a.x = dx + r0 * K;
+        a.y = (char *)dy + r0 * row;
+        a.M = (int)n;
+        if (launch_exact(c, a, (int)M, c->s_part[p])) return 1;
+        if (slots) CU_OK(c->hs.download_begin((int)p, a.y, n * row, c->s_part[p]));
+    }
+    for (size_t p = 0; p < parts; p++) {
+        const size_t r0 = first(p), n = first(p + 1) - r0;
+        char *dst = (char *)y + r0 * row;
+        if (slots)
+            CU_OK(c->hs.download_end((int)p, dst, n * row));
+        else
+            CU_OK(c->hs.download(dst, (char *)dy + r0 * row, n * row, c->s_part[p]));
+    }
+    for (size_t p = 0; p < parts; p++) CU_OK(cudaStreamSynchronize(c->s_part[p]));
     return 0;
 }
 

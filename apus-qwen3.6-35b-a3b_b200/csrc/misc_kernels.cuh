@@ -11,8 +11,9 @@ namespace apus {
 
 /* One fp32 chain per output, k strictly ascending, product and sum each
  * rounded once (c/bf16.h:285-294).  The product of two BF16 values is exact
- * in fp32 unless it underflows, so the literal multiply-then-add is kept here
- * (these hooks are launch- and PCIe-bound; chain latency is what it is). */
+ * in fp32 unless it underflows; the literal multiply-then-add is kept here.  This
+ * form serves rows that are not made of aligned 16-byte pieces (K % 8 != 0); the
+ * others run exact_dense.cuh. */
 __device__ __forceinline__ float exact_dot(const uint16_t *__restrict__ wrow,
                                            const uint16_t *__restrict__ xrow,
                                            int K) {

@@ -31,6 +31,30 @@ def test_hook_gemm_bitwise(gpu, orc, M):
     assert np.array_equal(gpu.bf16_gemm(w, x), orc.gemm(w, x))
 
 
+@pytest.mark.parametrize("M,O,K", [
+    (1, 31, 8), (1, 33, 64), (2, 32, 72), (3, 5000, 136), (4, 95, 2048),   # rows per lane
+    (5, 64, 8), (16, 65, 40), (17, 63, 96), (9, 130, 2048),                # 8-row tiles
+    (50, 2300, 72), (51, 4000, 136), (300, 1000, 104),                     # 16 and 32 rows
+    (129, 2560, 512), (513, 1500, 520)])                                   # 32 rows, in parts
+@pytest.mark.parametrize("scale", ["plain", "underflow", "overflow"])
+def test_hook_exact_order_kernels(gpu, orc, M, O, K, scale):
+    """Each kernel of the exact-order product at the edges of its tiles, with
+    products that are exact in fp32 (fused chain) and with products that
+    underflow or overflow (literal chain): bit for bit the anchor."""
+    rng = np.random.default_rng(M * 131 + O * 7 + K)
+    f = {"plain": 1.0, "underflow": 1e-20, "overflow": 1e19}[scale]
+    w, x = rng_codes(rng, (O, K), 0.5 * f), rng_codes(rng, (M, K), f)
+    exp = orc.gemm(w, x)
+    got = gpu.bf16_gemm(w, x)
+    nan = np.isnan(f32(exp))
+    assert np.array_equal(np.isnan(f32(got)), nan)
+    assert np.array_equal(got[~nan], exp[~nan])
+    if M == 1:
+        assert np.array_equal(gpu.bf16_gemv(w, x[0])[~nan[0]], exp[0][~nan[0]])
+        assert np.array_equal(gpu.bf16_matvec_f32(w, x[0]), orc.matvec_f32(w, x[0]),
+                              equal_nan=True)
+
+
 def test_hook_zero_dims_and_counters(gpu):
     assert gpu.lib.apus_cuda_bf16_gemv(None, None, None, 0, 8) != 0
     assert gpu.lib.apus_cuda_bf16_gemm(None, None, None, 1, 0, 8) != 0
