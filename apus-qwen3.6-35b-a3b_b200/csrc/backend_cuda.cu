@@ -76,6 +76,7 @@ struct ApusCudaLayer {
              *sh_gate = nullptr;
     float wmin = 0.0f;          /* smallest nonzero |rtr_w| (0 = unknown) */
     float wmin_gate = 0.0f;     /* the same for the shared-gate row */
+    float wmax = 0.0f, wmax_gate = 0.0f;   /* largest magnitudes */
     float *d_wnorm = nullptr;   /* [E + 1] router row norms (rounded up), [E] = max */
     size_t bytes = 0;
     PrefillMaps *maps = nullptr; /* tensor maps for the tcgen05 path */
@@ -102,8 +103,9 @@ struct Ctx {
     int decode_max_t = 4;        /* above this the tcgen05 grouped GEMM runs */
     int fused_max_t = 4;         /* up to this the one-kernel decode path runs */
     /* scratch of the fused decode kernel */
-    float *d_df_logits = nullptr;
-    uint16_t *d_df_sgl = nullptr, *d_df_act = nullptr, *d_df_sa = nullptr;
+    uint32_t *d_df_codes = nullptr;              /* [DF_MAX_T][1025] */
+    uint16_t *d_df_chains = nullptr;             /* [DF_MAX_T * 1025] */
+    uint16_t *d_df_act = nullptr, *d_df_sa = nullptr;
     unsigned int *d_df_sync = nullptr;
     unsigned long long *d_df_timeline = nullptr;   /* [sm_count][DF_MARKS] */
     bool df_timeline_valid = false;
@@ -215,8 +217,8 @@ static int ctx_init() {
     CU_OK(cudaMemset(c->d_rc_stats, 0, 64));
     c->fused_max_t = (int)env_long("APUS_CUDA_FUSED_MAX_T", DF_MAX_T);
     if (c->fused_max_t > DF_MAX_T) c->fused_max_t = DF_MAX_T;
-    CU_OK(cudaMalloc(&c->d_df_logits, (size_t)DF_MAX_T * 1024 * sizeof(float)));
-    CU_OK(cudaMalloc(&c->d_df_sgl, 64));
+    CU_OK(cudaMalloc(&c->d_df_codes, (size_t)DF_MAX_T * 1025 * sizeof(uint32_t)));
+    CU_OK(cudaMalloc(&c->d_df_chains, (size_t)DF_MAX_T * 1025 * sizeof(uint16_t)));
     CU_OK(cudaMalloc(&c->d_df_sync, 64));
     CU_OK(cudaMemset(c->d_df_sync, 0, 64));
     CU_OK(cudaMalloc(&c->d_df_timeline,
@@ -394,8 +396,8 @@ extern "C" void apus_cuda_disable(void) {
     if (c->d_status) cudaFree(c->d_status);
     if (c->d_router_counters) cudaFree(c->d_router_counters);
     if (c->d_rc_stats) cudaFree(c->d_rc_stats);
-    if (c->d_df_logits) cudaFree(c->d_df_logits);
-    if (c->d_df_sgl) cudaFree(c->d_df_sgl);
+    if (c->d_df_codes) cudaFree(c->d_df_codes);
+    if (c->d_df_chains) cudaFree(c->d_df_chains);
     if (c->d_df_sync) cudaFree(c->d_df_sync);
     if (c->d_df_timeline) cudaFree(c->d_df_timeline);
     if (c->d_df_act) cudaFree(c->d_df_act);
@@ -866,8 +868,8 @@ static int min_nonzero(Ctx *c, const uint16_t *d, size_t n, float *out,
  * (error bound of the fast logits) */
 static int layer_router_stats(Ctx *c, ApusCudaLayer *L) {
     const size_t E = L->cfg.experts, H = L->cfg.hidden;
-    if (min_nonzero(c, L->rtr_w, E * H, &L->wmin, c->stream) ||
-        min_nonzero(c, L->sh_gate, H, &L->wmin_gate, c->stream))
+    if (bf16_range(c, L->rtr_w, E * H, &L->wmin, &L->wmax) ||
+        bf16_range(c, L->sh_gate, H, &L->wmin_gate, &L->wmax_gate))
         return 1;
     if (!L->d_wnorm) CU_OK(cudaMalloc(&L->d_wnorm, (E + 1) * sizeof(float)));
     CU_OK(cudaMemsetAsync(L->d_wnorm, 0, (E + 1) * sizeof(float), c->stream));
@@ -1393,16 +1395,12 @@ static int run_fused_decode(Ctx *c, ApusCudaLayer *L, const uint16_t *d_ln2,
               TK = (int)cfg.top_k;
     if (fused_scratch(c, cfg)) return 1;
     FusedArgs a;
-    memset(&a, 0, sizeof a);
+    memset((void *)&a, 0, sizeof a);
     a.T = T; a.H = H; a.I = I; a.Is = Is; a.E = E; a.TK = TK;
-    a.stages = 3;
-    size_t smem = decode_fused_smem(T, H, I, Is, E, TK, 3);
-    if (smem > (size_t)c->smem_optin) {
-        a.stages = 2;
-        smem = decode_fused_smem(T, H, I, Is, E, TK, 2);
-    }
-    a.wmin = L->wmin;
-    a.wmin_gate = L->wmin_gate;
+    a.L = FusedLayout(T, H, I, Is, E, TK, c->sm_count);
+    const size_t smem = (size_t)a.L.total;
+    a.wmin = L->wmin; a.wmax = L->wmax;
+    a.wmin_gate = L->wmin_gate; a.wmax_gate = L->wmax_gate;
     a.x = d_ln2;
     if (rz) {
         a.res = rz->res;
@@ -1411,7 +1409,7 @@ static int run_fused_decode(Ctx *c, ApusCudaLayer *L, const uint16_t *d_ln2,
     }
     a.rtr_w = L->rtr_w; a.exp_gu = L->exp_gu; a.exp_d = L->exp_d;
     a.sh_g = L->sh_g; a.sh_u = L->sh_u; a.sh_d = L->sh_d; a.sh_gate = L->sh_gate;
-    a.logits_ws = c->d_df_logits; a.sgl_ws = c->d_df_sgl;
+    a.code_ws = c->d_df_codes; a.chain_ws = c->d_df_chains;
     a.act_ws = c->d_df_act; a.sa_ws = c->d_df_sa; a.sync = c->d_df_sync;
     a.out = d_out;
     a.idx_out = tr ? tr->rtr_idx : nullptr;
@@ -1420,13 +1418,13 @@ static int run_fused_decode(Ctx *c, ApusCudaLayer *L, const uint16_t *d_ln2,
     a.tr_shared = tr ? tr->moe_shared : nullptr;
     a.tr_out = tr ? tr->moe_out : nullptr;
     a.status = c->d_status;
+    a.stats = c->d_rc_stats;
     a.timeline = c->stage_timing ? c->d_df_timeline : nullptr;
     c->df_timeline_valid = c->stage_timing;
     static size_t set_smem = 0;
     if (smem > set_smem) {
         CU_OK(cudaFuncSetAttribute(decode_fused_kernel,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         set_smem = smem;
     }
     cudaLaunchConfig_t cfgl = {};
@@ -1446,14 +1444,39 @@ static int run_fused_decode(Ctx *c, ApusCudaLayer *L, const uint16_t *d_ln2,
 
 static bool fused_supported(Ctx *c, const ApusCudaMoeCfg &cfg, size_t T) {
     if ((int)T > c->fused_max_t || T * cfg.top_k > DF_MAX_A) return false;
-    if (cfg.experts > 1024 || cfg.hidden / 8 > 2 * (size_t)c->sm_count) return false;
-    if (cfg.moe_inter * 2 > DF_STAGE_BYTES / 8 || cfg.shared_inter * 2 > DF_STAGE_BYTES / 8)
-        return false;                      /* eight down rows per stage */
-    if (cfg.hidden * 4 > DF_STAGE_BYTES) return false;   /* a gate+up row pair */
-    size_t smem = decode_fused_smem((int)T, (int)cfg.hidden, (int)cfg.moe_inter,
-                                    (int)cfg.shared_inter, (int)cfg.experts,
-                                    (int)cfg.top_k, 2);
-    return smem <= (size_t)c->smem_optin;
+    if (cfg.experts > 1024 || cfg.hidden % 16 || cfg.moe_inter % 16 || cfg.shared_inter % 16)
+        return false;                                      /* whole k steps of the MMA */
+    if (cfg.hidden > DF_CW * DF_KS * 16 || cfg.moe_inter > DF_MAX_K_DOWN ||
+        cfg.shared_inter > DF_MAX_K_DOWN)
+        return false;                                      /* fragments in registers */
+    if ((cfg.hidden + c->sm_count - 1) / c->sm_count > DF_MAX_COLS || c->sm_count > (int)DF_ROUND)
+        return false;
+    const FusedLayout L((int)T, (int)cfg.hidden, (int)cfg.moe_inter, (int)cfg.shared_inter,
+                        (int)cfg.experts, (int)cfg.top_k, c->sm_count);
+    return (size_t)L.total + DF_STATIC_SMEM <= (size_t)c->smem_optin;
+}
+
+/* rows of whole 16-byte pieces: one warp per row without the sequential chain;
+ * others: the plain kernel */
+static int launch_rmsnorm(Ctx *c, const uint16_t *x, const uint16_t *w, uint16_t *y, int T, int N,
+                          cudaStream_t st) {
+    const size_t rows = (size_t)RN_WARPS * LaneRow(N).bytes();
+    if (N % 8 == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) == 0 &&
+        rows <= 40 * 1024) {
+        launch_k(rmsnorm_rows_kernel, dim3((T + RN_WARPS - 1) / RN_WARPS), dim3(RN_WARPS * 32),
+                 rows, st, x, w, y, T, N, LaneRow(N));
+        LAUNCHED();
+        return 0;
+    }
+    const size_t smem = 4 * (size_t)N * sizeof(float);
+    if (smem > 48 * 1024) {
+        if (smem > (size_t)c->smem_optin) return fail("rmsnorm: N too large");
+        CU_OK(cudaFuncSetAttribute(rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)smem));
+    }
+    rmsnorm_kernel<<<(unsigned)((T + 3) / 4), 128, smem, st>>>(x, w, y, T, N);
+    LAUNCHED();
+    return 0;
 }
 
 static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
@@ -1482,15 +1505,7 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
     if (rz) {
         uint16_t *ln = (uint16_t *)c->ws.take(T * cfg.hidden * 2);
         if (!ln) return fail("workspace arena too small");
-        const size_t smem = 4 * cfg.hidden * sizeof(float);
-        if (smem > 48 * 1024) {
-            if (smem > (size_t)c->smem_optin) return fail("rmsnorm: hidden too large");
-            CU_OK(cudaFuncSetAttribute(rmsnorm_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        }
-        rmsnorm_kernel<<<(unsigned)((T + 3) / 4), 128, smem, st>>>(rz->res, rz->ln_w, ln, (int)T,
-                                                                   (int)cfg.hidden);
-        LAUNCHED();
+        if (launch_rmsnorm(c, rz->res, rz->ln_w, ln, (int)T, (int)cfg.hidden, st)) return 1;
         d_ln2 = ln;
     }
     const int Ti = (int)T, E = (int)cfg.experts, H = (int)cfg.hidden,
@@ -2513,17 +2528,7 @@ extern "C" int apus_cuda_rmsnorm_dev(const uint16_t *d_x, const uint16_t *d_w,
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     if (ctx_init()) return 1;
     cudaStream_t st = (cudaStream_t)stream;
-    size_t smem = 4 * N * sizeof(float);
-    if (smem > 48 * 1024) {
-        if (smem > (size_t)g_ctx->smem_optin) return fail("rmsnorm: N too large");
-        CU_OK(cudaFuncSetAttribute(rmsnorm_kernel,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
-    }
-    rmsnorm_kernel<<<(unsigned)((T + 3) / 4), 128, smem, st>>>(d_x, d_w, d_y,
-                                                               (int)T, (int)N);
-    LAUNCHED();
-    return 0;
+    return launch_rmsnorm(g_ctx, d_x, d_w, d_y, (int)T, (int)N, st);
 }
 
 template <int M>

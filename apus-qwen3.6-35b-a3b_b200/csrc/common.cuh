@@ -166,6 +166,11 @@ __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+/* 16 bytes global -> shared, asynchronously, past L1 */
+__device__ __forceinline__ void cp_async16_to(uint32_t dst_smem, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+
 /* 16-byte read-only global load */
 __device__ __forceinline__ uint4 ldg16(const void *p) {
     return __ldg(reinterpret_cast<const uint4 *>(p));

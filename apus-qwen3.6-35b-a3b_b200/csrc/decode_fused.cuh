@@ -1,73 +1,139 @@
 /*
- * decode_fused.cuh — the whole MoE block for one to four tokens in ONE
- * cooperative kernel (c/layer.h:333-370 end to end): router chains, softmax /
- * top-k, the routed and shared experts' gate/up rows with SwiGLU, one grid-wide
- * barrier, the down rows, and the weighted combine + shared gate + add.
+ * decode_fused.cuh — the whole MoE block for one to eight tokens in ONE
+ * cooperative kernel (c/layer.h:333-370 end to end, and through
+ * apus_cuda_moe_layer_dev the norm before and the residual add after,
+ * c/layer.h:386-388): router, softmax / top-k, the routed and shared experts'
+ * gate/up rows with SwiGLU, one grid-wide barrier, the down rows, and the weighted
+ * combine + shared gate + add.
  *
- * At this size the block is a 57 MB weight stream that should take ~9 us, and
- * every kernel boundary, dependent global round trip and idle SM shows.  So:
+ * At one token the block is a 57 MB weight stream that should take 9 us; what it
+ * takes instead is dependent latencies, so the kernel is built around those:
  *
- *  - one launch; 148 persistent CTAs (one per SM), 8 warps each;
- *  - the first ceil((E+1)/8) CTAs walk the exact router chains (eight rows per
- *    CTA, one lane per (row, token), rows pulled in by bulk copies) while all
- *    the others already stream and reduce their share of the shared expert's
- *    gate/up rows, which do not depend on routing;
- *  - the logits meet in global memory behind a release/acquire counter; every
- *    CTA then runs the (cheap, bit-exact) softmax/top-k itself instead of
- *    waiting for a second broadcast;
- *  - expert rows arrive through per-warp rings of cp.async.bulk copies (no
- *    multicast); each CTA owns a contiguous slice of the flattened (expert,
- *    row) space;
+ *  - one launch; one CTA per SM; sixteen compute warps and one helper warp;
+ *  - no sequential chain on the path (exact_sum.cuh): the norm's sum of squares by
+ *    parity functions, the router's logits as intervals that nearly always pin
+ *    their BF16 code.  The experts whose rank the intervals decide are streamed at
+ *    once; the helper warps walk the few chains that are left (one token needs one
+ *    in five times) beside the stream, since only the order and the weights of the
+ *    selected experts can still depend on them.  Only when the SET is open does
+ *    everyone wait for the chains.  (A chain for every logit, then softmax over
+ *    all of them, put 21 of 47 us in front of the first expert weight.)
+ *  - selection looks at BF16 logits, not at probabilities: exp and the division
+ *    keep their order whenever the logits near the top differ by 2^-18 or more,
+ *    which is checked; otherwise the engine's softmax runs on exact logits;
+ *  - weight rows are multiplied by mma.sync m16n8k16 with the tokens as the eight
+ *    columns, so eight tokens cost the instructions of one (scalar multiply-adds
+ *    held the gate/up phase at 27 us for 15 us of bytes at three tokens).  Each
+ *    warp owns a sixteenth of K: it fetches exactly what it multiplies, into a
+ *    ring of its own (cp.async), and keeps its token fragments in registers; the
+ *    sixteen partial sums of a row meet in shared memory;
+ *  - the ring never drains between phases: shared gate/up rows are requested
+ *    before anything is known, down rows as soon as the last gate/up row has been,
+ *    i.e. before the grid barrier they come after;
  *  - the down phase gives each CTA a slice of the output columns across ALL
- *    selected experts, so the combine is local and no second barrier is
- *    needed; its first weight copies are issued before the barrier wait.
+ *    selected experts, so the combine is local and no second barrier is needed.
  *
- * CTAs wait on one another (router counter, barrier), which is only legal
- * because the launch is cooperative (all CTAs co-resident).  Every wait is
+ * CTAs wait on one another (router counter, chain counter, barrier), which is only
+ * legal because the launch is cooperative (all CTAs co-resident).  Every wait is
  * bounded: on a timeout the CTA records a status code and drains to the exit.
- * The counters are reset by the last CTA to leave, so the kernel can be
- * replayed from a CUDA graph.
+ * The counters only ever grow, the two that count CTAs by DF_ROUND per launch (CTA 0
+ * adds what the others leave to it), so that a CTA finds its launch's target in the
+ * value it reads at its start, nobody has to reset anything on the way out, and the
+ * kernel can be replayed from a CUDA graph.
  */
 #pragma once
 #include <climits>
 
 #include "common.cuh"
 #include "decode_gemv.cuh"
+#include "exact_dense.cuh"
+#include "exact_sum.cuh"
 #include "router.cuh"
 
 namespace apus {
 
-constexpr int DF_THREADS = 256;
-constexpr int DF_WARPS = 8;
-constexpr int DF_MAX_T = 4;
-constexpr int DF_MAX_A = 32;            /* T * top_k */
-constexpr int DF_STAGE_BYTES = 8192;    /* a gate+up row pair, or 8 down rows */
+constexpr int DF_CW = 16;               /* compute warps */
+constexpr int DF_THREADS = (DF_CW + 1) * 32;
+constexpr int DF_MAX_T = 8;
+constexpr int DF_MAX_A = 64;            /* T * top_k */
+constexpr int DF_ROWS = 16;             /* weight rows of a tile: 8 gate + 8 up, or down rows */
+constexpr int DF_PAIRS = DF_ROWS / 2;
+constexpr int DF_KS = 8;                /* 16-wide k steps of a tile, at most */
+constexpr int DF_MAX_K_DOWN = 4 * DF_KS * 16;   /* half of it is at most two tiles */
+constexpr int DF_DEPTH = 2;             /* tiles of a warp's ring */
+constexpr int DF_STATIC_SMEM = 1920;    /* the static tables (with them the full-size layer at
+                                         * eight tokens fills an SM to the byte) */
+constexpr int DF_MAX_COLS = 16;         /* output columns of a CTA, at most */
+
+/* ---- shared memory ------------------------------------------------------------ */
+struct FusedLayout {
+    int per;                 /* gate/up: k steps per warp */
+    int pitch;               /* bytes of a tile row */
+    int slot;                /* bytes of a ring slot */
+    LaneRow lr;
+    int xrow;                /* bytes of a token row (LaneRow) */
+    int act_pitch, sact_pitch;
+    int rrows;               /* router rows of a CTA, at most */
+    int off_x, off_rr, off_code, off_key, off_tmask, off_amb, off_act, off_sact, off_red, total;
+    FusedLayout() = default;
+    FusedLayout(int T, int H, int I, int Is, int E, int TK, int G) {
+        const int A = T * TK;
+        per = (H / 16 + DF_CW - 1) / DF_CW;
+        pitch = DF_KS * 32 + 16;
+        slot = DF_ROWS * pitch;
+        lr = LaneRow(H);
+        xrow = lr.bytes();
+        act_pitch = I * 2 + 16;
+        sact_pitch = Is * 2 + 16;
+        rrows = (E + 1 + G - 1) / G;
+        int p = DF_CW * DF_DEPTH * slot;
+        /* tokens, router rows, logits, their keys, open pairs; later the activations */
+        off_x = p;
+        off_rr = off_x + T * xrow;
+        off_code = off_rr + rrows * xrow;
+        off_key = off_code + T * (E + 1) * 4;
+        off_tmask = off_key + T * E * 4;
+        off_amb = off_tmask + 1024;
+        const int end1 = off_amb + T * (E + 1) * 2;
+        off_act = p;
+        off_sact = off_act + A * act_pitch;
+        const int end2 = off_sact + T * sact_pitch;
+        p = ((end1 > end2 ? end1 : end2) + 127) & ~127;
+        /* partial sums of a tile [2][warps][rows][8]; before them the norm's gains,
+         * after them the down outputs [2 halves][A + T][columns] */
+        off_red = p;
+        const int r1 = 2 * DF_CW * DF_ROWS * 8 * 4, r2 = 2 * (A + T) * DF_MAX_COLS * 4;
+        total = p + (r1 > r2 ? r1 : r2);
+    }
+};
 
 struct FusedArgs {
-    int T, H, I, Is, E, TK, stages;
-    float wmin, wmin_gate;              /* smallest nonzero |w|: router, shared-gate row */
+    int T, H, I, Is, E, TK;
+    float wmin, wmax;                   /* smallest nonzero and largest |w|: router matrix */
+    float wmin_gate, wmax_gate;         /* ... shared-gate row */
     const uint16_t *x;                  /* [T, H] block input; or, with res set, unused */
-    /* the two steps either side of the block folded in (c/layer.h:386,388):
-     * res [T,H] is the residual stream, the block input is rmsnorm(res, 1 + ln_w)
-     * (c/attn.h:175-186, every CTA computes it for itself: 4 KB per token and
-     * one sequential chain per token, no exchange), and res_out = rnd(res + moe_out) */
+    /* the two steps either side of the block folded in: res [T,H] is the residual
+     * stream, the block input is rmsnorm(res, 1 + ln_w) (every CTA computes it for
+     * itself: 4 KB per token, no exchange), and res_out = rnd(res + moe_out) */
     const uint16_t *res, *ln_w;
     uint16_t *res_out;
     const uint16_t *rtr_w, *exp_gu, *exp_d, *sh_g, *sh_u, *sh_d, *sh_gate;
     /* global scratch owned by the backend */
-    float *logits_ws;                   /* [DF_MAX_T][E] */
-    uint16_t *sgl_ws;                   /* [DF_MAX_T] */
+    uint32_t *code_ws;                  /* [DF_MAX_T][E + 1] logit code intervals */
+    uint16_t *chain_ws;                 /* [DF_MAX_T * (E + 1)] codes of the walked chains */
     uint16_t *act_ws;                   /* [DF_MAX_A][I] */
     uint16_t *sa_ws;                    /* [DF_MAX_T][Is] */
-    unsigned int *sync;                 /* [0] router done, [1] barrier, [2] exits */
+    unsigned int *sync;                 /* [0] router, [1] barrier, [2] chains */
     /* outputs */
     uint16_t *out;                      /* [T, H] */
     int32_t *idx_out;                   /* [T, TK] (optional) */
     uint16_t *w_out;                    /* [T, TK] (optional) */
     uint16_t *tr_routed, *tr_shared, *tr_out;
     int *status;
+    unsigned int *stats;                /* [0] += chains walked */
     /* optional phase timeline: [grid][DF_MARKS] global-timer nanoseconds */
     unsigned long long *timeline;
+    FusedLayout L;
 };
 constexpr int DF_MARKS = 8;
 __device__ __forceinline__ void df_mark(const FusedArgs &a, int k) {
@@ -86,692 +152,802 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
 __device__ __forceinline__ void red_release_add(unsigned int *p, unsigned int v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-/* thread 0 of a CTA: wait until *p >= target; false on timeout */
-__device__ __forceinline__ bool spin_until(const unsigned int *p,
-                                           unsigned int target) {
+constexpr unsigned DF_ROUND = 256;      /* >= the number of CTAs, a power of two */
+/* the value a round counter reaches when every CTA of this launch has arrived; v was
+ * read before this CTA arrived */
+__device__ __forceinline__ unsigned int round_target(unsigned int v) {
+    return (v & ~(DF_ROUND - 1)) + DF_ROUND;
+}
+__device__ __forceinline__ void round_arrive(unsigned int *p) {
+    red_release_add(p, blockIdx.x == 0 ? DF_ROUND - gridDim.x + 1u : 1u);
+}
+/* one thread: wait until *p has reached the target (modulo 2^32); false on timeout */
+__device__ __forceinline__ bool spin_until(const unsigned int *p, unsigned int target) {
     for (uint32_t i = 0; i < (1u << 21); i++) {
-        if (ld_acquire(p) >= target) return true;
-        if (i > 32) __nanosleep(40);
+        if ((int)(ld_acquire(p) - target) >= 0) return true;
+        if (i > 64) __nanosleep(40);
     }
     return false;
 }
-
-/* butterfly-reduce N independent values at once (the shuffles of different
- * values overlap; a value-at-a-time reduction would serialise 5 shuffle
- * latencies per value) */
-template <int N>
-__device__ __forceinline__ void warp_sum_n(float (&v)[N]) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int i = 0; i < N; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+__device__ __forceinline__ void df_bar_compute() {
+    asm volatile("bar.sync 1, %0;" ::"n"(DF_CW * 32) : "memory");
+}
+/* the helper warp has finished with the token rows and the logits */
+__device__ __forceinline__ void df_bar_helper_arrive() {
+    asm volatile("bar.arrive 2, %0;" ::"n"(DF_THREADS) : "memory");
+}
+__device__ __forceinline__ void df_bar_helper_wait() {
+    asm volatile("bar.sync 2, %0;" ::"n"(DF_THREADS) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+/* D[16 x 8] += A[16 x 16] B[16 x 8], BF16 in, fp32 accumulate */
+__device__ __forceinline__ void mma_16x8(float (&c)[4], const uint32_t (&a)[4], uint32_t b_lo,
+                                         uint32_t b_hi) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, "
+        "{%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b_lo), "r"(b_hi));
 }
 
-/* eight weight rows (contiguous, K each) against NT selected activation rows */
-template <int NT>
-__device__ __forceinline__ void df_down8(const uint16_t *ws, const uint16_t *src,
-                                         const int *rows, int K, int lane,
-                                         float (&acc)[8 * 4]) {
-    float a[8 * NT];
+/* Order-preserving 16-bit key of a BF16 code (-0 counts as +0). */
+__device__ __forceinline__ uint32_t code_key(uint32_t code) {
+    code &= 0xffffu;
+    if (code == 0x8000u) code = 0;
+    return code ^ ((code & 0x8000u) ? 0xffffu : 0x8000u);
+}
+
+/* One exact chain by one lane, both rows LaneRows in shared memory. */
+template <bool FMA>
+__device__ __forceinline__ float df_chain(const unsigned char *w, const unsigned char *x,
+                                          const LaneRow lr) {
+    float acc = 0.0f;
+#pragma unroll 1
+    for (int l = 0; l < lr.nl; l++, w += lr.pitch, x += lr.pitch) {
+#pragma unroll 2
+        for (int c = 0; c < lr.nu; c++) {
+            float wf[8], xf[8];
+            unpack8(*reinterpret_cast<const uint4 *>(w + c * 16), wf);
+            unpack8(*reinterpret_cast<const uint4 *>(x + c * 16), xf);
 #pragma unroll
-    for (int i = 0; i < 8 * NT; i++) a[i] = 0.f;
-    for (int k = lane * 8; k < K; k += 256) {
-        float xf[NT][8];
-#pragma unroll
-        for (int n = 0; n < NT; n++)
-            unpack8(*reinterpret_cast<const uint4 *>(src + (size_t)rows[n] * K + k),
-                    xf[n]);
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-            float wf[8];
-            unpack8(*reinterpret_cast<const uint4 *>(ws + (size_t)r * K + k), wf);
-#pragma unroll
-            for (int n = 0; n < NT; n++)
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    a[r * NT + n] = fmaf(wf[j], xf[n][j], a[r * NT + n]);
+            for (int j = 0; j < 8; j++)
+                acc = FMA ? __fmaf_rn(wf[j], xf[j], acc)
+                          : __fadd_rn(acc, __fmul_rn(wf[j], xf[j]));
         }
     }
-    warp_sum_n<8 * NT>(a);
-#pragma unroll
-    for (int r = 0; r < 8; r++)
-#pragma unroll
-        for (int n = 0; n < NT; n++) acc[r * 4 + n] = a[r * NT + n];
+    return acc;
 }
 
-/* gate and up rows against NT selected token rows; reduced */
-template <int NT>
-__device__ __forceinline__ void df_gate_up(const uint16_t *gs, const uint16_t *us,
-                                           const uint16_t *xs, int stride,
-                                           const int *rows, int K, int lane,
-                                           float (&ag)[4], float (&au)[4]) {
-    float a[2 * NT];
-#pragma unroll
-    for (int i = 0; i < 2 * NT; i++) a[i] = 0.f;
-    for (int k = lane * 8; k < K; k += 256) {
-        float gf[8], uf[8];
-        unpack8(*reinterpret_cast<const uint4 *>(gs + k), gf);
-        unpack8(*reinterpret_cast<const uint4 *>(us + k), uf);
-#pragma unroll
-        for (int n = 0; n < NT; n++) {
-            float xf[8];
-            unpack8(*reinterpret_cast<const uint4 *>(xs + (size_t)rows[n] * stride + k),
-                    xf);
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                a[n] = fmaf(gf[j], xf[j], a[n]);
-                a[NT + n] = fmaf(uf[j], xf[j], a[NT + n]);
-            }
-        }
-    }
-    warp_sum_n<2 * NT>(a);
-#pragma unroll
-    for (int n = 0; n < NT; n++) {
-        ag[n] = a[n];
-        au[n] = a[NT + n];
-    }
-}
-__device__ __forceinline__ void df_gate_up_n(int nt, const uint16_t *gs,
-                                             const uint16_t *us, const uint16_t *xs,
-                                             int stride, const int *rows, int K,
-                                             int lane, float (&ag)[4],
-                                             float (&au)[4]) {
-    switch (nt) {
-        case 1: df_gate_up<1>(gs, us, xs, stride, rows, K, lane, ag, au); break;
-        case 2: df_gate_up<2>(gs, us, xs, stride, rows, K, lane, ag, au); break;
-        case 3: df_gate_up<3>(gs, us, xs, stride, rows, K, lane, ag, au); break;
-        default: df_gate_up<4>(gs, us, xs, stride, rows, K, lane, ag, au); break;
-    }
-}
-__device__ __forceinline__ void df_down8_n(int nt, const uint16_t *ws,
-                                           const uint16_t *src, const int *rows,
-                                           int K, int lane, float (&acc)[32]) {
-    switch (nt) {
-        case 1: df_down8<1>(ws, src, rows, K, lane, acc); break;
-        case 2: df_down8<2>(ws, src, rows, K, lane, acc); break;
-        case 3: df_down8<3>(ws, src, rows, K, lane, acc); break;
-        default: df_down8<4>(ws, src, rows, K, lane, acc); break;
-    }
-}
-
-
-/* xs[t][:] = rmsnorm(res[t][:], 1 + ln_w) for t < T, bit for bit the engine's
- * (c/attn.h:175-186): the sum of squares is one ascending fp32 chain (lane 0 of
- * warp t walks it over the row staged in shared memory, operands converted on
- * the fly: the dependent add is the critical path), then y = rnd((x*rs)*(1+w)).
- * All threads call it; ends with a CTA barrier. */
-__device__ __forceinline__ void df_rmsnorm_to_smem(const FusedArgs &a, uint16_t *xs) {
-    const int T = a.T, H = a.H;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int c = tid; c < T * (H / 8); c += DF_THREADS)
-        reinterpret_cast<uint4 *>(xs)[c] = ldg16(a.res + (size_t)c * 8);
-    __syncthreads();
-    if (warp < T) {
-        uint16_t *row = xs + (size_t)warp * H;
-        /* the gains are asked for before the chain starts, so that their trip
-         * from L2 hides behind it: 16 bytes a lane and round, H / 256 rounds */
-        const int nj = H / 256;
-        const bool vec = H % 256 == 0 && nj <= 8;
-        uint4 lw[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-            lw[j] = (vec && a.ln_w && j < nj) ? ldg16(a.ln_w + (size_t)(lane + 32 * j) * 8)
-                                              : make_uint4(0, 0, 0, 0);
-        float ss = 0.0f;
-        if (lane == 0) {
-            const uint4 *r4 = reinterpret_cast<const uint4 *>(row);
-            /* four rows of eight ahead: the shared-memory loads and the squares
-             * stay off the chain of dependent adds */
-#pragma unroll 4
-            for (int i = 0; i < H / 8; i++) {
-                const uint4 v = r4[i];
-                const float f[8] = {bf16lo(v.x), bf16hi(v.x), bf16lo(v.y), bf16hi(v.y),
-                                    bf16lo(v.z), bf16hi(v.z), bf16lo(v.w), bf16hi(v.w)};
-                float q[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++) q[j] = __fmul_rn(f[j], f[j]);
-#pragma unroll
-                for (int j = 0; j < 8; j++) ss = __fadd_rn(ss, q[j]);
-            }
-        }
-        ss = __shfl_sync(0xffffffffu, ss, 0);
-        const float rs =
-            __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)H), 1e-6f)));
-        if (vec) {
-            uint4 *r4 = reinterpret_cast<uint4 *>(row);
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                if (j < nj) {
-                    const uint4 v = r4[lane + 32 * j];
-                    const uint32_t xw[4] = {v.x, v.y, v.z, v.w};
-                    const uint32_t gw[4] = {lw[j].x, lw[j].y, lw[j].z, lw[j].w};
-                    uint32_t o[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const float g0 = __fadd_rn(1.0f, bf16lo(gw[q])),
-                                    g1 = __fadd_rn(1.0f, bf16hi(gw[q]));
-                        const float y0 = __fmul_rn(__fmul_rn(bf16lo(xw[q]), rs), g0),
-                                    y1 = __fmul_rn(__fmul_rn(bf16hi(xw[q]), rs), g1);
-                        o[q] = (uint32_t)bf16_bits(y0) | ((uint32_t)bf16_bits(y1) << 16);
-                    }
-                    r4[lane + 32 * j] = make_uint4(o[0], o[1], o[2], o[3]);
-                }
-            }
-        } else {
-            for (int i = lane; i < H; i += 32) {
-                const float g = __fadd_rn(1.0f, a.ln_w ? bf16_f32(__ldg(a.ln_w + i)) : 0.0f);
-                row[i] = bf16_bits(__fmul_rn(__fmul_rn(bf16_f32(row[i]), rs), g));
-            }
-        }
-    }
-    __syncthreads();
-}
-
-/* A warp's private ring of bulk copies.  issue() is called by lane 0 only. */
-struct WarpRing {
-    unsigned char *base;     /* stages * DF_STAGE_BYTES */
-    uint64_t *bars;
-    int stages;
-    int issued, consumed;
-    __device__ __forceinline__ void issue(const void *src0, uint32_t b0,
-                                          const void *src1, uint32_t b1) {
-        const int s = issued % stages;
-        unsigned char *dst = base + (size_t)s * DF_STAGE_BYTES;
-        mbar_expect_tx(&bars[s], b0 + b1);
-        bulk_g2s(dst, src0, b0, &bars[s]);
-        if (b1) bulk_g2s(dst + b0, src1, b1, &bars[s]);
-    }
-    __device__ __forceinline__ bool wait() {
-        const int s = consumed % stages;
-        return mbar_wait(&bars[s], (uint32_t)(consumed / stages) & 1u);
-    }
-    __device__ __forceinline__ const unsigned char *cur() const {
-        return base + (size_t)(consumed % stages) * DF_STAGE_BYTES;
-    }
-};
-
-/*
- * Dynamic shared memory:
- *   ring   [DF_WARPS][stages][8 KB]      (router CTAs first use it for their
- *                                          eight rows and the fp32 tokens)
- *   xs     uint16 [T][H]                  tokens (phase A/B); then
- *          uint16 [A][I] + [T][Is]        activations (phase C)   (union)
- *   ps     float  [T][E]                  logits -> probabilities
- *   ytab   uint16 [A + T][16]             down outputs of this CTA's columns
- *   small tables and barriers
- */
 __global__ void __launch_bounds__(DF_THREADS, 1)
-decode_fused_kernel(FusedArgs a) {
-    pdl_enter();
+decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     extern __shared__ __align__(128) unsigned char df_smem[];
     const int T = a.T, H = a.H, I = a.I, Is = a.Is, E = a.E, TK = a.TK;
-    const int A = T * TK;
-    const int G = gridDim.x;
+    const int A = T * TK, G = gridDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
-    unsigned char *ring_all = df_smem;
-    const size_t ring_bytes = (size_t)DF_WARPS * a.stages * DF_STAGE_BYTES;
-    const size_t un_bytes_x = (size_t)T * H * 2;
-    const size_t un_bytes_a = ((size_t)A * I + (size_t)T * Is) * 2;
-    const size_t un_bytes = un_bytes_x > un_bytes_a ? un_bytes_x : un_bytes_a;
-    uint16_t *xs = reinterpret_cast<uint16_t *>(df_smem + ring_bytes);
-    float *ps = reinterpret_cast<float *>(df_smem + ring_bytes + ((un_bytes + 127) & ~(size_t)127));
-    uint16_t *ytab = reinterpret_cast<uint16_t *>(ps + (size_t)T * E);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(
-        (reinterpret_cast<uintptr_t>(ytab + (size_t)(DF_MAX_A + DF_MAX_T) * 16) + 7) & ~(uintptr_t)7);
-    uint64_t *rbar = bars + DF_WARPS * 3;          /* router rows barrier */
-    __shared__ int s_idx[DF_MAX_A];
+    const FusedLayout &L = a.L;
+    const LaneRow lr = L.lr;
+    unsigned char *xs = df_smem + L.off_x, *rr = df_smem + L.off_rr;
+    uint32_t *codes = reinterpret_cast<uint32_t *>(df_smem + L.off_code);   /* [T][E + 1] */
+    uint32_t *keys = reinterpret_cast<uint32_t *>(df_smem + L.off_key);     /* [T][E] */
+    uint16_t *amb = reinterpret_cast<uint16_t *>(df_smem + L.off_amb);      /* t << 11 | e */
+    unsigned char *act = df_smem + L.off_act, *sact = df_smem + L.off_sact;
+    uint32_t *s_tmask = reinterpret_cast<uint32_t *>(df_smem + L.off_tmask);   /* [256]: tokens of
+                                                        * each expert, a byte each */
+    float *red = reinterpret_cast<float *>(df_smem + L.off_red);
+    __shared__ int s_sel[DF_MAX_A];                /* selected experts, in provisional order */
+    __shared__ int s_idx[DF_MAX_A], s_row[DF_MAX_A];   /* final order; down output of each */
     __shared__ uint16_t s_w[DF_MAX_A];
-    __shared__ uint16_t s_sgl[DF_MAX_T];
-    __shared__ int s_uexp[DF_MAX_A];               /* unique experts */
-    __shared__ unsigned int s_umask[DF_MAX_A];     /* assignments of each */
+    __shared__ float s_gate[DF_MAX_T], s_sum[DF_MAX_T], s_rs[DF_MAX_T];
+    __shared__ unsigned int s_xlo[DF_MAX_T], s_xhi[DF_MAX_T];
+    __shared__ int s_namb[DF_MAX_T], s_full[DF_MAX_T], s_open;
+    __shared__ int s_wu[DF_CW], s_wa[DF_CW];       /* per warp: experts, assignments before it */
+    __shared__ int s_uexp[DF_MAX_A], s_ubase[DF_MAX_A];
+    __shared__ uint8_t s_umask[DF_MAX_A];
     __shared__ int s_U;
-    __shared__ int s_dead;
-    __shared__ unsigned int s_xmin;
-
-    if (tid == 0) {
-        for (int i = 0; i < DF_WARPS * 3; i++) mbar_init(&bars[i], 1);
-        mbar_init(rbar, 1);
-        mbar_fence_init();
-        s_dead = 0;
-        s_xmin = 0x7f800000u;
-    }
-    __syncthreads();
-
-    WarpRing ring;
-    ring.base = ring_all + (size_t)warp * a.stages * DF_STAGE_BYTES;
-    ring.bars = bars + warp * 3;
-    ring.stages = a.stages;
-    ring.issued = 0;
-    ring.consumed = 0;
+    __shared__ volatile int s_dead;
+    __shared__ unsigned int s_chain0;              /* chain counter before this launch */
 
     df_mark(a, 0);                          /* start */
-    const int nR = (E + 1 + 7) / 8;        /* router CTAs */
-    const bool is_router = (int)blockIdx.x < nR;
-    const uint32_t rowb = (uint32_t)H * 2u;
+    /* ---- this CTA's shares ---- */
+    const int r_first = blockIdx.x, n_rr = r_first <= E ? (E - r_first) / G + 1 : 0;
+    const int sh_lo = (int)((long)Is * blockIdx.x / G),
+              sh_n = (int)((long)Is * (blockIdx.x + 1) / G) - sh_lo;
+    const int nS = (sh_n + DF_PAIRS - 1) / DF_PAIRS;   /* shared gate/up tiles */
+    const int h_lo = (int)((long)H * blockIdx.x / G);
+    const int ncols = (int)((long)H * (blockIdx.x + 1) / G) - h_lo;
+    /* routed gate/up pairs and tiles, distinct experts: known after the selection */
+    int gu_lo = 0, gu_n = 0, nR = 0, U = 0;
 
-    /* ---------------- router chains (first nR CTAs) ---------------- */
-    if (is_router) {
-        const int r0 = blockIdx.x * 8;
-        const int nrows = min(8, E + 1 - r0);
-        const int pitch = H * 2 + 16;
-        unsigned char *rows_s = ring_all;
-        float *xf = reinterpret_cast<float *>(ring_all + 8 * pitch);
-        const int xpitch = H + 8;        /* floats: tokens on different banks */
-        if (tid == 0) {
-            mbar_expect_tx(rbar, (uint32_t)nrows * rowb);
-            for (int r = 0; r < nrows; r++) {
-                const uint16_t *src = (r0 + r == E) ? a.sh_gate
-                                                    : a.rtr_w + (size_t)(r0 + r) * H;
-                bulk_g2s(rows_s + (size_t)r * pitch, src, rowb, rbar);
-            }
-        }
-        unsigned int xmin = 0x7f800000u;
-        /* with the norm folded in, the block input is computed here (every CTA
-         * does, the router CTAs first of all: their chains start from it) */
-        if (a.res) df_rmsnorm_to_smem(a, xs);
-        for (int c = tid; c < T * (H / 8); c += DF_THREADS) {
-            const uint4 v = a.res ? reinterpret_cast<const uint4 *>(xs)[c]
-                                  : ldg16(a.x + (size_t)c * 8);
-            const uint32_t wds[4] = {v.x, v.y, v.z, v.w};
-            const int tt = c / (H / 8), cc = c - tt * (H / 8);
-            float4 *d = reinterpret_cast<float4 *>(xf + (size_t)tt * xpitch + cc * 8);
-            d[0] = make_float4(bf16lo(v.x), bf16hi(v.x), bf16lo(v.y), bf16hi(v.y));
-            d[1] = make_float4(bf16lo(v.z), bf16hi(v.z), bf16lo(v.w), bf16hi(v.w));
+    /* ---- tokens, router rows and gains: requested first of all ---- */
+    const int cph = H / 8;
+    const uint4 *xsrc = reinterpret_cast<const uint4 *>(a.res ? a.res : a.x);
+    auto rsrc = [&](int c) {
+        const int r = c / cph, e = r_first + r * G;
+        return (e == E ? a.sh_gate : a.rtr_w + (size_t)e * H) + (size_t)(c - r * cph) * 8;
+    };
+    uint4 rv = make_uint4(0, 0, 0, 0), xv = rv;
+    if (tid < T * cph) xv = __ldcg(xsrc + tid);
+    if (tid < n_rr * cph) rv = ldg16(rsrc(tid));
+    uint4 gv = make_uint4(0, 0, 0, 0);       /* gain offsets; H / 8 <= the thread count */
+    if (a.res && a.ln_w && tid < cph) gv = ldg16(a.ln_w + tid * 8);
+    uint4 *gains = reinterpret_cast<uint4 *>(red);   /* the partial sums come later */
+
+    /* ---- ring of this warp ---- */
+    const uint32_t ring = smem_u32(df_smem + (size_t)warp * DF_DEPTH * L.slot);
+    const int ks_lo = min(warp * L.per, H / 16), nks = min(L.per, H / 16 - ks_lo);
+    /* fetch: a lane takes the same 16 bytes of every other row where a row slice is
+     * 256 bytes (gate rows by the lower lanes, up rows by the upper ones) */
+    const uint32_t f_dst = (uint32_t)((lane >> 4) * L.pitch + (lane & 15) * 16);
+    const size_t f_col = (size_t)ks_lo * 16 + (lane & 15) * 8;
+    const uint16_t *f_src = ((lane >> 4) ? a.sh_u : a.sh_g) + (size_t)sh_lo * H + f_col;
+    int f_left = 1 << 30;                   /* pairs of the expert from f_src on */
+    auto pair_row = [&](bool sh, int pi, int up) {   /* row `up` (0 gate, 1 up) of pair pi */
+        if (sh) return (up ? a.sh_u : a.sh_g) + (size_t)(sh_lo + pi) * H;
+        const int it = gu_lo + pi, u = it / I;
+        return a.exp_gu + ((size_t)s_uexp[u] * 2 * I + (size_t)(it - u * I + (up ? I : 0))) * H;
+    };
+    auto fetch_pairs = [&](uint32_t slot, bool sh, int p0, int np) {
+        if (nks == DF_KS && np == DF_PAIRS && f_left >= DF_PAIRS) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                unsigned int lo = (wds[q] << 16) & 0x7fffffffu;
-                unsigned int hi = wds[q] & 0x7fff0000u;
-                if (lo != 0 && lo < xmin) xmin = lo;
-                if (hi != 0 && hi < xmin) xmin = hi;
+            for (int q = 0; q < DF_PAIRS; q++)
+                cp_async16_to(slot + f_dst + (uint32_t)(2 * q * L.pitch), f_src + (size_t)q * H);
+        } else if (nks > 0) {
+            /* ragged: the slice is narrower, or the tile ends or changes expert */
+            const int cpr = nks * 2;
+#pragma unroll 1
+            for (int c = lane; c < 2 * np * cpr; c += 32) {
+                const int r = c / cpr, ch = c - r * cpr;
+                cp_async16_to(slot + (uint32_t)(r * L.pitch + ch * 16),
+                              pair_row(sh, p0 + (r >> 1), r & 1) + ks_lo * 16 + ch * 8);
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            xmin = min(xmin, __shfl_xor_sync(0xffffffffu, xmin, o));
-        if (lane == 0) atomicMin(&s_xmin, xmin);
-        __syncthreads();
-        /* the fused form is exact while the smallest product is a normal
-         * number; the shared-gate row has its own smallest weight */
-        const double xmn = (double)__uint_as_float(s_xmin);
-        const bool use_fma = (a.wmin > 0.0f) && ((double)a.wmin * xmn >= 7.52316384526264e-37);
-        const bool use_fma_gate =
-            (a.wmin_gate > 0.0f) && ((double)a.wmin_gate * xmn >= 7.52316384526264e-37);
-        const bool arrived = mbar_wait(rbar, 0);      /* every warp waits */
-        if (!arrived) {
-            set_status(a.status, ST_MBAR_TIMEOUT);
-            s_dead = 1;
-        }
-        if (warp == 0) {
-            const int r = lane / T, t = lane - r * T;
-            if (arrived && r < nrows) {
-                const uint16_t *wrow =
-                    reinterpret_cast<const uint16_t *>(rows_s + (size_t)r * pitch);
-                const bool fma_row = (r0 + r != E) ? use_fma : use_fma_gate;
-                const float acc =
-                    fma_row ? small_chain<true>(wrow, xf + (size_t)t * xpitch, H)
-                            : small_chain<false>(wrow, xf + (size_t)t * xpitch, H);
-                const uint16_t code = bf16_bits(acc);
-                if (r0 + r == E)
-                    a.sgl_ws[t] = code;
-                else
-                    a.logits_ws[(size_t)t * E + r0 + r] = bf16_f32(code);
-            }
-            __syncwarp();
-            if (lane == 0) {
-                __threadfence();
-                red_release_add(&a.sync[0], 1u);
-            }
-        }
-        fence_proxy_async();  /* generic writes above, bulk copies next */
-        __syncthreads();      /* the ring region is free again */
-    }
-
-    df_mark(a, 1);                          /* router chains done (router CTAs) */
-    /* ---------------- phase A: tokens to shared; shared gate/up ---------------- */
-    if (a.res) {
-        if (!is_router) df_rmsnorm_to_smem(a, xs);    /* router CTAs hold it already */
-    } else {
-        for (int c = tid; c < T * (H / 8); c += DF_THREADS)
-            reinterpret_cast<uint4 *>(xs)[c] = ldg16(a.x + (size_t)c * 8);
-    }
-    __syncthreads();
-    {
-        /* The shared expert's rows go to the CTAs that have no router chains to
-         * walk (they would otherwise idle until the logits arrive); a router CTA
-         * that also took a share reached the selection 2-3 us after everyone
-         * else and held up the grid barrier by as much. */
-        const bool spare = G > nR;
-        const int Gs = spare ? G - nR : G, bs = spare ? (int)blockIdx.x - nR : (int)blockIdx.x;
-        const int lo = bs < 0 ? 0 : (int)((long)Is * bs / Gs);
-        const int hi = bs < 0 ? 0 : (int)((long)Is * (bs + 1) / Gs);
-        const int n_my = (lo + warp < hi) ? (hi - lo - warp + DF_WARPS - 1) / DF_WARPS : 0;
-        if (lane == 0)
-            for (; ring.issued < n_my && ring.issued < a.stages; ring.issued++) {
-                const int row = lo + warp + ring.issued * DF_WARPS;
-                ring.issue(a.sh_g + (size_t)row * H, rowb, a.sh_u + (size_t)row * H, rowb);
-            }
-        ring.issued = min(n_my, a.stages);
-        const int rows[4] = {0, 1, 2, 3};
-        for (int j = 0; j < n_my; j++) {
-            const bool ok = !s_dead && ring.wait();
-            if (!ok && !s_dead) {
-                set_status(a.status, ST_MBAR_TIMEOUT);
-                s_dead = 1;
-            }
-            const int row = lo + warp + j * DF_WARPS;
-            if (ok) {
-                const uint16_t *gs = reinterpret_cast<const uint16_t *>(ring.cur());
-                float ag[4] = {0, 0, 0, 0}, au[4] = {0, 0, 0, 0};
-                df_gate_up_n(T, gs, gs + H, xs, H, rows, H, lane, ag, au);
-                if (lane < T) {
-                    float g = 0.f, u = 0.f;
-#pragma unroll
-                    for (int n = 0; n < 4; n++)
-                        if (lane == n) { g = ag[n]; u = au[n]; }
-                    a.sa_ws[(size_t)lane * Is + row] =
-                        silu_mul_bits(bf16_round(g), bf16_round(u));
-                }
-            }
-            __syncwarp();
-            ring.consumed++;
-            if (!s_dead && ring.issued < n_my) {
-                if (lane == 0) {
-                    const int r2 = lo + warp + ring.issued * DF_WARPS;
-                    ring.issue(a.sh_g + (size_t)r2 * H, rowb, a.sh_u + (size_t)r2 * H, rowb);
-                }
-                ring.issued++;
-            }
-        }
-    }
-
-    df_mark(a, 2);                          /* shared gate/up done */
-    /* ---------------- routing result ---------------- */
-    if (tid == 0 && !s_dead) {
-        if (!spin_until(&a.sync[0], (unsigned)nR)) {
-            set_status(a.status, ST_SCHED_TIMEOUT);
-            s_dead = 1;
-        }
-    }
-    __syncthreads();
-    if (!s_dead) {
-        for (int i = tid; i < T * E; i += DF_THREADS) ps[i] = __ldcg(&a.logits_ws[i]);
-        if (tid < T) s_sgl[tid] = __ldcg(&a.sgl_ws[tid]);
-    }
-    __syncthreads();
-    __shared__ int s_scratch[32];
-    if (T == 1 && E <= DF_THREADS && TK <= 16) {
-        /* one token: the whole CTA shares the softmax / selection */
-        if (!s_dead)               /* uniform: s_dead is read after a barrier */
-            router_softmax_topk_cta256(ps, E, TK, s_scratch, s_idx, s_w);
-    } else if (!s_dead && warp < T) {
-        router_softmax_topk(ps + (size_t)warp * E, E, TK, lane, s_idx + warp * TK,
-                            s_w + warp * TK);
-    }
-    __syncthreads();
-    if (blockIdx.x == 0 && tid < A) {
-        if (a.idx_out) a.idx_out[tid] = s_idx[tid];
-        if (a.w_out) a.w_out[tid] = s_w[tid];
-    }
-    /* unique experts and who uses them (A <= 32: one warp) */
-    if (warp == 0) {
-        const int e = lane < A ? s_idx[lane] : -1 - lane;
-        const unsigned peers = __match_any_sync(0xffffffffu, e);
-        const bool leader = lane < A && (__ffs(peers) - 1) == lane;
-        const unsigned leaders = __ballot_sync(0xffffffffu, leader);
-        if (leader) {
-            const int u = __popc(leaders & ((1u << lane) - 1u));
-            s_uexp[u] = e;
-            s_umask[u] = peers;
-        }
-        if (lane == 0) s_U = __popc(leaders);
-    }
-    __syncthreads();
-    const int U = s_dead ? 0 : s_U;
-
-    df_mark(a, 3);                          /* logits seen, softmax/top-k done */
-    /* ---------------- phase B: routed gate/up ---------------- */
-    {
-        const long N = (long)U * I;
-        const long lo = N * blockIdx.x / G, hi = N * (blockIdx.x + 1) / G;
-        const long first = lo + warp;
-        const int n_my = first < hi ? (int)((hi - first + DF_WARPS - 1) / DF_WARPS) : 0;
-        ring.issued = ring.consumed;            /* ring is drained */
-        const int base_c = ring.consumed;
-        auto item_src = [&](int j, const uint16_t *&g, const uint16_t *&u) {
-            const long it = first + (long)j * DF_WARPS;
-            const int uu = (int)(it / I), row = (int)(it - (long)uu * I);
-            const uint16_t *b = a.exp_gu + (size_t)s_uexp[uu] * 2 * I * H;
-            g = b + (size_t)row * H;
-            u = b + (size_t)(I + row) * H;
-        };
-        int issued_j = 0;
-        if (lane == 0)
-            for (; issued_j < n_my && issued_j < a.stages; issued_j++) {
-                const uint16_t *g, *u;
-                item_src(issued_j, g, u);
-                ring.issue(g, rowb, u, rowb);
-                ring.issued++;
-            }
-        issued_j = min(n_my, a.stages);
-        ring.issued = base_c + issued_j;
-        for (int j = 0; j < n_my; j++) {
-            const bool ok = !s_dead && ring.wait();
-            if (!ok && !s_dead) {
-                set_status(a.status, ST_MBAR_TIMEOUT);
-                s_dead = 1;
-            }
-            if (ok) {
-                const long it = first + (long)j * DF_WARPS;
-                const int uu = (int)(it / I), row = (int)(it - (long)uu * I);
-                unsigned m = s_umask[uu];
-                int rows[4] = {0, 0, 0, 0}, asg[4] = {0, 0, 0, 0}, nt = 0;
-                while (m && nt < 4) {
-                    const int aidx = __ffs(m) - 1;
-                    m &= m - 1;
-                    asg[nt] = aidx;
-                    rows[nt] = aidx / TK;
-                    nt++;
-                }
-                const uint16_t *gs = reinterpret_cast<const uint16_t *>(ring.cur());
-                float ag[4] = {0, 0, 0, 0}, au[4] = {0, 0, 0, 0};
-                df_gate_up_n(nt, gs, gs + H, xs, H, rows, H, lane, ag, au);
-                if (lane < nt) {
-                    float g = 0.f, u = 0.f;
-                    int an = 0;
-#pragma unroll
-                    for (int n = 0; n < 4; n++)
-                        if (lane == n) { g = ag[n]; u = au[n]; an = asg[n]; }
-                    a.act_ws[(size_t)an * I + row] =
-                        silu_act_bits(bf16_round(g), bf16_round(u));
-                }
-            }
-            __syncwarp();
-            ring.consumed++;
-            if (!s_dead && issued_j < n_my) {
-                if (lane == 0) {
-                    const uint16_t *g, *u;
-                    item_src(issued_j, g, u);
-                    ring.issue(g, rowb, u, rowb);
-                }
-                issued_j++;
-                ring.issued++;
-            }
-        }
-    }
-
-    df_mark(a, 4);                          /* routed gate/up done */
-    /* ---------------- phase C set-up: first down copies, then the barrier ------- */
-    const int HB = H / 8;
-    const int b_lo = (int)((long)HB * blockIdx.x / G);
-    const int b_hi = (int)((long)HB * (blockIdx.x + 1) / G);
-    const int nb = b_hi - b_lo;                    /* 8-row blocks of this CTA (<= 2) */
-    const int n_items = (U + 1) * nb;              /* expert-major, block-minor */
-    const int n_my_c = warp < n_items ? (n_items - warp + DF_WARPS - 1) / DF_WARPS : 0;
-    auto down_src = [&](int j, const uint16_t *&src, uint32_t &bytes) {
-        const int it = warp + j * DF_WARPS;
-        const int uu = it / nb, b = b_lo + (it - uu * nb);
-        if (uu == U) {
-            src = a.sh_d + (size_t)b * 8 * Is;
-            bytes = (uint32_t)(8 * Is * 2);
-        } else {
-            src = a.exp_d + ((size_t)s_uexp[uu] * H + (size_t)b * 8) * I;
-            bytes = (uint32_t)(8 * I * 2);
+        f_src += (size_t)DF_PAIRS * H;
+        f_left -= DF_PAIRS;
+        if (!sh && f_left <= 0 && p0 + DF_PAIRS < gu_n) {      /* the next tile's expert */
+            const int it = gu_lo + p0 + DF_PAIRS, u = it / I;
+            f_src = pair_row(false, p0 + DF_PAIRS, lane >> 4) + f_col;
+            f_left = (u + 1) * I - it;
         }
     };
-    int issued_c = 0;
-    {
-        const int base_c = ring.consumed;
-        if (lane == 0 && !s_dead)
-            for (; issued_c < n_my_c && issued_c < a.stages; issued_c++) {
-                const uint16_t *src;
-                uint32_t bytes;
-                down_src(issued_c, src, bytes);
-                ring.issued = base_c + issued_c;
-                ring.issue(src, bytes, nullptr, 0);
+    /* Down: warp w takes (item, half of K) = w, w + 16, ...; items are the distinct
+     * experts and, last, the shared expert.  A unit is one or two tiles of at most
+     * 128 k, all of this CTA's columns high. */
+    struct DownUnit {
+        const uint16_t *src;
+        int K, k0, nk;                      /* first k step, k steps */
+    };
+    auto down_unit = [&](int j) {
+        const int v = j * DF_CW + warp, item = v >> 1;
+        DownUnit d;
+        d.K = item == U ? Is : I;
+        const int half = (d.K / 16 + 1) / 2;
+        d.k0 = (v & 1) * half;
+        d.nk = min(half, d.K / 16 - d.k0);
+        d.src = (item == U ? a.sh_d : a.exp_d + (size_t)s_uexp[item] * H * I) +
+                (size_t)h_lo * d.K + d.k0 * 16;
+        return d;
+    };
+    auto fetch_down = [&](uint32_t slot, const DownUnit &d, int ks0) {
+        const int cpr = 2 * min(DF_KS, d.nk - ks0);
+        const uint16_t *src = d.src + ks0 * 16;
+        if (cpr == 16) {
+            src += (size_t)(lane >> 4) * d.K + (lane & 15) * 8;
+#pragma unroll
+            for (int q = 0; q < DF_ROWS / 2; q++)
+                if (2 * q + (lane >> 4) < ncols)
+                    cp_async16_to(slot + f_dst + (uint32_t)(2 * q * L.pitch),
+                                  src + (size_t)(2 * q) * d.K);
+        } else {
+#pragma unroll 1
+            for (int c = lane; c < ncols * cpr; c += 32) {
+                const int r = c / cpr, ch = c - r * cpr;
+                cp_async16_to(slot + (uint32_t)(r * L.pitch + ch * 16),
+                              src + (size_t)r * d.K + ch * 8);
             }
-        issued_c = s_dead ? 0 : min(n_my_c, a.stages);
-        ring.issued = base_c + issued_c;
+        }
+    };
+    int i_tile = 0, i_slot = 0;             /* next gate/up tile of the phase, next slot */
+    int i_unit = 0, i_ks = 0, n_unit = 0;   /* next down unit and k step in it */
+    bool i_sh = true;
+    /* requests this warp's next tile if it is known; one commit group per call, so
+     * that a fixed number of groups stays ahead of the tile in use */
+    auto issue = [&]() {
+        const uint32_t slot = ring + (uint32_t)(i_slot * L.slot);
+        bool some = true;
+        if (i_tile < (i_sh ? nS : nR)) {
+            const int p0 = i_tile++ * DF_PAIRS;
+            fetch_pairs(slot, i_sh, p0, min(DF_PAIRS, (i_sh ? sh_n : gu_n) - p0));
+        } else if (i_unit < n_unit) {
+            const DownUnit d = down_unit(i_unit);
+            fetch_down(slot, d, i_ks);
+            i_ks += DF_KS;
+            if (i_ks >= d.nk) {
+                i_ks = 0;
+                i_unit++;
+            }
+        } else {
+            some = false;
+        }
+        if (some && ++i_slot == DF_DEPTH) i_slot = 0;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (warp < DF_CW)
+#pragma unroll 1
+        for (int j = 0; j < DF_DEPTH; j++) issue();   /* constants: nothing to wait for */
+
+    unsigned int sync_at[2] = {0, 0};
+    if (tid == 0) {
+        s_dead = 0;
+        s_open = 0;
+        s_U = 0;
+        sync_at[0] = round_target(ld_acquire(&a.sync[0]));
+        sync_at[1] = round_target(ld_acquire(&a.sync[1]));
+        s_chain0 = ld_acquire(&a.sync[2]);
+    }
+    if (tid < DF_MAX_T) {
+        s_xlo[tid] = 0x7f800000u;
+        s_xhi[tid] = 0;
+    }
+    if (tid < cph) gains[tid] = gv;
+#pragma unroll 1
+    for (int c = tid, t = tid / cph; c < T * cph; c += DF_THREADS, t = c / cph) {
+        if (c != tid) xv = __ldcg(xsrc + c);
+        *reinterpret_cast<uint4 *>(xs + t * L.xrow + lr.at(c - t * cph)) = xv;
+    }
+#pragma unroll 1
+    for (int c = tid, r = tid / cph; c < n_rr * cph; c += DF_THREADS, r = c / cph) {
+        if (c != tid) rv = ldg16(rsrc(c));
+        *reinterpret_cast<uint4 *>(rr + r * L.xrow + lr.at(c - r * cph)) = rv;
     }
     __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        red_release_add(&a.sync[1], 1u);
-        if (!s_dead && !spin_until(&a.sync[1], (unsigned)G)) {
+    /* Norm (bit for bit the engine's) and the range of the tokens' values: warps t
+     * and 8 + t have a half of token t each, where its lane chunks can be halved. */
+    {
+        const int t = warp & 7, part = warp >> 3, parts = lr.nu % 2 == 0 ? 2 : 1;
+        if (t < T && part < parts) {
+            unsigned char *row = xs + t * L.xrow;
+            float rs = 1.0f;
+            auto meet = [&] { asm volatile("bar.sync %0, 64;" ::"r"(3 + t) : "memory"); };
+            if (a.res) {
+                const float ss = exact_sumsq(row, lr, lane, part, parts, &s_sum[t], meet);
+                if (part) s_rs[t] = norm_scale(ss, H);
+                if (parts == 2) {
+                    meet();
+                    rs = s_rs[t];
+                } else {
+                    rs = norm_scale(ss, H);
+                }
+            }
+            unsigned int lo = 0x7f800000u, hi = 0;
+#pragma unroll 1
+            for (int c = part * 32 + lane; c < cph; c += 32 * parts) {
+                uint4 *p = reinterpret_cast<uint4 *>(row + lr.at(c));
+                uint4 v = *p;
+                if (a.res) *p = v = norm8(v, gains[c], rs);
+                fold_range8(v, lo, hi);
+            }
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            if (lane == 0) {
+                atomicMin(&s_xlo[t], lo);
+                atomicMax(&s_xhi[t], hi);
+            }
+        }
+    }
+    __syncthreads();
+
+    /* ---- router logits of this CTA's rows ---- */
+    if (warp < DF_CW)
+        for (int p = warp; p < n_rr * T; p += DF_CW) {
+            const int r = p / T, t = p - r * T, e = r_first + r * G;
+            const bool exact =
+                e == E ? products_exact(a.wmin_gate, a.wmax_gate, s_xlo[t], s_xhi[t])
+                       : products_exact(a.wmin, a.wmax, s_xlo[t], s_xhi[t]);
+            const uint32_t v = exact ? certified_logit(rr + r * L.xrow, xs + t * L.xrow, lr, lane)
+                                     : CODE_UNKNOWN;
+            if (lane == 0) a.code_ws[(size_t)t * (E + 1) + e] = v;
+        }
+    __syncthreads();
+    if (tid == 0) round_arrive(&a.sync[0]);          /* cumulative over the barrier */
+    df_mark(a, 1);                          /* own logits published */
+
+    /* ---- token fragments of this warp's k slice (all tokens are columns) ---- */
+    uint32_t bf[DF_KS][2];
+    {
+        const int t = lane >> 2, q = (lane & 3) * 2;
+#pragma unroll
+        for (int s = 0; s < DF_KS; s++) {
+            bf[s][0] = bf[s][1] = 0;
+            if (warp < DF_CW && s < nks && t < T) {
+                const unsigned char *row = xs + t * L.xrow;
+                const int c = (ks_lo + s) * 2;
+                bf[s][0] = *reinterpret_cast<const uint32_t *>(row + lr.at(c) + q * 2);
+                bf[s][1] = *reinterpret_cast<const uint32_t *>(row + lr.at(c + 1) + q * 2);
+            }
+        }
+    }
+    int c_slot = 0;
+    /* where ldmatrix finds this lane's row of the tile in use: matrices are (rows
+     * 0-7, k 0-7), (rows 8-15, k 0-7), (rows 0-7, k 8-15), (rows 8-15, k 8-15) */
+    const uint32_t m_off = (uint32_t)((lane & 15) * L.pitch + (lane >> 4) * 16);
+    auto next_tile = [&]() {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DF_DEPTH - 1) : "memory");
+        __syncwarp();
+        const uint32_t t = ring + (uint32_t)(c_slot * L.slot) + m_off;
+        if (++c_slot == DF_DEPTH) c_slot = 0;
+        return t;
+    };
+    /* gate/up tiles [0, n): the warps' partial sums meet in shared memory, four
+     * warps in turn finish a tile while the others go on */
+    auto run_tiles = [&](int n, bool sh) {
+#pragma unroll 1
+        for (int j = 0; j < n; j++) {
+            float *buf = red + (j & 1) * (DF_CW * DF_ROWS * 8);
+            const uint32_t t = next_tile();
+            float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int s = 0; s < DF_KS; s++)
+                if (s < nks) {
+                    uint32_t r[4];
+                    ldmatrix_x4(r, t + (uint32_t)(s * 32));
+                    mma_16x8((s & 1) ? c1 : c0, r, bf[s][0], bf[s][1]);
+                }
+            float *dst = buf + (warp * DF_ROWS + (lane >> 2)) * 8 + (lane & 3) * 2;
+            *reinterpret_cast<float2 *>(dst) = make_float2(c0[0] + c1[0], c0[1] + c1[1]);
+            *reinterpret_cast<float2 *>(dst + 64) = make_float2(c0[2] + c1[2], c0[3] + c1[3]);
+            __syncwarp();                       /* the slot is read out */
+            issue();
+            df_bar_compute();
+            if ((warp >> 2) == (j & 3)) {
+                /* thread = row (2p gate, 2p + 1 up) x column */
+                const int i = (warp & 3) * 32 + lane, col = i & 7, pi = j * DF_PAIRS + (i >> 4);
+                float v = 0.0f;
+#pragma unroll
+                for (int w = 0; w < DF_CW; w++) v += buf[w * (DF_ROWS * 8) + i];
+                const float up = __shfl_xor_sync(0xffffffffu, v, 8);
+                if (!(i & 8) && pi < (sh ? sh_n : gu_n)) {
+                    const float g = bf16_round(v), u = bf16_round(up);
+                    if (sh) {
+                        if (col < T)
+                            a.sa_ws[(size_t)col * Is + sh_lo + pi] = silu_mul_bits(g, u);
+                    } else {
+                        const int it = gu_lo + pi, uu = it / I;
+                        const unsigned m = s_umask[uu];
+                        if ((m >> col) & 1u)
+                            a.act_ws[(size_t)(s_ubase[uu] + __popc(m & ((1u << col) - 1u))) * I +
+                                     (it - uu * I)] = silu_act_bits(g, u);
+                    }
+                }
+            }
+        }
+    };
+    if (warp < DF_CW) run_tiles(nS, true);
+    df_mark(a, 2);                          /* shared gate/up done */
+    /* ---- routing ---- */
+    if (tid == 0 && !spin_until(&a.sync[0], sync_at[0])) {
+        set_status(a.status, ST_SCHED_TIMEOUT);
+        s_dead = 1;
+    }
+    if (tid < 256) s_tmask[tid] = 0;
+    __syncthreads();
+    bool dead = s_dead != 0;
+#pragma unroll 1
+    for (int i = tid; i < T * (E + 1); i += DF_THREADS)
+        codes[i] = dead ? 0u : __ldcg(&a.code_ws[i]);
+    __syncthreads();
+    /* Selection of token t by one warp: the TK experts with the largest low codes
+     * (lowest index first on ties).  Anything else whose high code reaches the
+     * TK-th low code may belong there instead. */
+    auto select = [&](int t, bool first) {
+        const uint32_t *cd = codes + t * (E + 1);
+        /* keys: low code, then lowest index first; all different.  Up to 256 experts
+         * they stay in registers. */
+        constexpr int R = 8;
+        uint32_t *kd = keys + t * E, kr[R], best = 0, kth = 0;
+        const bool regs = E <= 32 * R;
+        auto key_of = [&](int e) { return (code_key(cd[e]) << 16) | (0xffffu - (uint32_t)e); };
+        if (regs) {
+#pragma unroll
+            for (int i = 0; i < R; i++) {
+                kr[i] = lane + 32 * i < E ? key_of(lane + 32 * i) : 0u;
+                best = max(best, kr[i]);
+            }
+        } else {
+#pragma unroll 1
+            for (int e = lane; e < E; e += 32) best = max(best, kd[e] = key_of(e));
+        }
+#pragma unroll 1
+        for (int i = 0; i < TK; i++) {
+            kth = __reduce_max_sync(0xffffffffu, best);
+            if (lane == 0) s_sel[t * TK + i] = (int)(0xffffu - (kth & 0xffffu));
+            if (regs) {
+                best = 0;
+#pragma unroll
+                for (int j = 0; j < R; j++)
+                    if (kr[j] < kth) best = max(best, kr[j]);
+            } else if (best == kth) {                    /* this lane's next one */
+                best = 0;
+                for (int e = lane; e < E; e += 32)
+                    if (kd[e] < kth) best = max(best, kd[e]);
+            }
+        }
+        /* does code order decide?  (see the head of this file) */
+        const uint32_t kkey = kth >> 16;
+        bool open = false, odd = false, any = false;
+        float top = -INFINITY;
+        uint32_t reach = 0;                              /* bit i: expert lane + 32 i competes */
+        if (regs) {
+#pragma unroll
+            for (int i = 0; i < R; i++)
+                if (lane + 32 * i < E && code_key(cd[lane + 32 * i] >> 16) >= kkey)
+                    reach |= 1u << i;
+        } else {
+            for (int e = lane, i = 0; e < E; e += 32, i++)
+                if (code_key(cd[e] >> 16) >= kkey) reach |= 1u << i;
+        }
+        for (; reach; reach &= reach - 1) {
+            const int e = lane + 32 * (__ffs(reach) - 1);
+            const uint32_t v = cd[e];
+            const bool known = code_known(v);
+            any |= !known;
+            if (!known && key_of(e) < kth) open = true;  /* not among the chosen */
+            const float lo = bf16lo(v), hi = bf16hi(v);
+            const bool zero = known && (v & 0x7fffu) == 0;
+            const bool plain = fabsf(lo) >= 9.765625e-4f && fabsf(hi) >= 9.765625e-4f &&
+                               (lo < 0.0f) == (hi < 0.0f) && fabsf(hi) <= 32.0f;
+            if (!plain && !(zero && code_key(v) != kkey)) odd = true;
+            top = fmaxf(top, hi);
+        }
+        __syncwarp();
+        /* order-preserving integer of a float, for the integer reduction */
+        const int ti = __float_as_int(top);
+        const int tm = __reduce_max_sync(0xffffffffu, ti >= 0 ? ti : ti ^ 0x7fffffff);
+        top = __int_as_float(tm >= 0 ? tm : tm ^ 0x7fffffff);
+        const uint32_t kc = kkey ^ ((kkey & 0x8000u) ? 0x8000u : 0xffffu);
+        if (!(__uint_as_float(kc << 16) - top >= -80.0f)) odd = true;
+        odd = __any_sync(0xffffffffu, odd);
+        open = __any_sync(0xffffffffu, open);
+        any = __any_sync(0xffffffffu, any) || odd || !code_known(cd[E]);
+        if (first) {
+            /* logits that need their chain: competitors whose code is open (all of
+             * them if probabilities have to decide), and the shared gate */
+            int n = 0;
+            if (any)
+#pragma unroll 1
+                for (int e0 = 0; e0 <= E; e0 += 32) {
+                    const int e = e0 + lane;
+                    const bool need = e <= E && !code_known(cd[e]) &&
+                                      (odd || e == E || code_key(cd[e] >> 16) >= kkey);
+                    n += __popc(__ballot_sync(0xffffffffu, need));
+                }
+            if (lane == 0) {
+                s_namb[t] = n;
+                s_full[t] = odd;
+                if (open || odd) s_open = 1;
+            }
+        }
+        return kkey;
+    };
+    uint32_t kkey = 0;
+    if (warp < T && !dead) kkey = select(warp, true);
+    __syncthreads();
+    int n_amb = 0;
+    if (!dead)
+        for (int t = 0; t < T; t++) n_amb += s_namb[t];
+    if (n_amb > 0) {
+        if (warp < T) {
+            /* the same list in every CTA: by token, then by expert */
+            int at = 0;
+            for (int t = 0; t < warp; t++) at += s_namb[t];
+            const uint32_t *cd = codes + warp * (E + 1);
+            for (int e0 = 0; e0 <= E; e0 += 32) {
+                const int e = e0 + lane;
+                const bool need = e <= E && !code_known(cd[e]) &&
+                                  (s_full[warp] || e == E || code_key(cd[e] >> 16) >= kkey);
+                const unsigned m = __ballot_sync(0xffffffffu, need);
+                if (need) amb[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)((warp << 11) | e);
+                at += __popc(m);
+            }
+        }
+        __syncthreads();
+    }
+    const bool open = s_open != 0;           /* the set itself waits for the chains */
+    /* Pair i of the list is CTA i % G's.  Its helper warp brings the weight rows
+     * into the place of the router rows (under the expert stream a row read piece
+     * by piece would wait an L2 round trip per piece), as many at a time as fit. */
+    auto walk_chains = [&]() {
+        if ((int)blockIdx.x >= n_amb) return;
+        const int room = min(L.rrows, 32);
+        for (int i0 = blockIdx.x; i0 < n_amb; i0 += room * G) {
+            for (int q = 0; q < room && i0 + q * G < n_amb; q++) {
+                const int e = amb[i0 + q * G] & 0x7ff;
+                const uint16_t *w = e == E ? a.sh_gate : a.rtr_w + (size_t)e * H;
+                for (int c = lane; c < H / 8; c += 32)
+                    cp_async16_to(smem_u32(rr + q * L.xrow + lr.at(c)), w + c * 8);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();
+            const int i = i0 + lane * G;
+            if (lane < room && i < n_amb) {
+                const int t = amb[i] >> 11, e = amb[i] & 0x7ff;
+                const bool fma =
+                    e == E ? products_exact(a.wmin_gate, a.wmax_gate, s_xlo[t], s_xhi[t])
+                           : products_exact(a.wmin, a.wmax, s_xlo[t], s_xhi[t]);
+                const unsigned char *wr = rr + lane * L.xrow, *xr = xs + t * L.xrow;
+                const float z = fma ? df_chain<true>(wr, xr, lr) : df_chain<false>(wr, xr, lr);
+                a.chain_ws[i] = bf16_bits(z);
+            }
+            __syncwarp();
+        }
+        if (lane == 0) {
+            if (a.stats && blockIdx.x == 0) atomicAdd(&a.stats[0], (unsigned)n_amb);
+            red_release_add(&a.sync[2], 1u);
+        }
+    };
+    const unsigned chain_target = s_chain0 + (unsigned)min(n_amb, G);
+    if (open) {
+        if (warp == DF_CW) walk_chains();
+        if (tid == 0 && !spin_until(&a.sync[2], chain_target)) {
             set_status(a.status, ST_SCHED_TIMEOUT);
             s_dead = 1;
         }
-    }
-    __syncthreads();
-
-    df_mark(a, 5);                          /* barrier passed */
-    /* activations of every assignment, and the shared activations */
-    uint16_t *as = xs;
-    uint16_t *sas = xs + (size_t)A * I;
-    if (!s_dead) {
-        for (int c = tid; c < A * (I / 8); c += DF_THREADS)
-            reinterpret_cast<uint4 *>(as)[c] =
-                __ldcg(reinterpret_cast<const uint4 *>(a.act_ws) + c);
-        for (int c = tid; c < T * (Is / 8); c += DF_THREADS)
-            reinterpret_cast<uint4 *>(sas)[c] =
-                __ldcg(reinterpret_cast<const uint4 *>(a.sa_ws) + c);
-    }
-    __syncthreads();
-
-    /* ---------------- phase C: down rows of this CTA's columns ---------------- */
-    for (int j = 0; j < n_my_c; j++) {
-        const bool ok = !s_dead && j < issued_c && ring.wait();
-        if (!ok && !s_dead) {
-            set_status(a.status, ST_MBAR_TIMEOUT);
-            s_dead = 1;
+        __syncthreads();
+        dead = s_dead != 0;
+        for (int i = tid; i < n_amb && !dead; i += DF_THREADS) {
+            const uint32_t c = __ldcg(&a.chain_ws[i]);
+            codes[(amb[i] >> 11) * (E + 1) + (amb[i] & 0x7ff)] = c | (c << 16);
         }
-        if (ok) {
-            const int it = warp + j * DF_WARPS;
-            const int uu = it / nb, bl = it - uu * nb;
-            const uint16_t *ws = reinterpret_cast<const uint16_t *>(ring.cur());
-            int rows[4] = {0, 1, 2, 3}, nt, K;
-            const uint16_t *src;
-            int slot0;                          /* ytab row of rows[0] ... */
-            int slots[4] = {0, 0, 0, 0};
-            if (uu == U) {
-                nt = T; K = Is; src = sas;
-                for (int n = 0; n < 4; n++) slots[n] = DF_MAX_A + n;
+        __syncthreads();
+        if (warp < T && !dead) {
+            if (s_full[warp]) {
+                /* the engine's softmax and selection on exact logits */
+                float *p = reinterpret_cast<float *>(keys + warp * E);
+                for (int e = lane; e < E; e += 32) p[e] = bf16lo(codes[warp * (E + 1) + e]);
+                __syncwarp();
+                router_softmax_topk(p, E, TK, lane, s_idx + warp * TK, s_w + warp * TK);
+                __syncwarp();
+                for (int i = lane; i < TK; i += 32) s_sel[warp * TK + i] = s_idx[warp * TK + i];
             } else {
-                unsigned m = s_umask[uu];
-                nt = 0; K = I; src = as;
-                while (m && nt < 4) {
-                    const int aidx = __ffs(m) - 1;
-                    m &= m - 1;
-                    rows[nt] = aidx;
-                    slots[nt] = aidx;
-                    nt++;
+                select(warp, false);
+            }
+        }
+        __syncthreads();
+    }
+    /* ---- the distinct experts, ascending, and who uses them ---- */
+    if (tid < A && !dead)
+        atomicOr(&s_tmask[s_sel[tid] >> 2], (1u << (tid / TK)) << ((s_sel[tid] & 3) * 8));
+    __syncthreads();
+    if (warp < DF_CW) {
+        /* warp w looks at experts 64 w .. 64 w + 63 */
+        unsigned m0 = 0, m1 = 0;
+        const int e0 = warp * 64 + lane, e1 = e0 + 32;
+        const unsigned b0 = (s_tmask[e0 >> 2] >> ((e0 & 3) * 8)) & 0xffu,
+                       b1 = (s_tmask[e1 >> 2] >> ((e1 & 3) * 8)) & 0xffu;
+        m0 = __ballot_sync(0xffffffffu, b0 != 0);
+        m1 = __ballot_sync(0xffffffffu, b1 != 0);
+        int c0 = __popc(b0), c1 = __popc(b1), i0 = c0, i1 = c1;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v0 = __shfl_up_sync(0xffffffffu, i0, d),
+                      v1 = __shfl_up_sync(0xffffffffu, i1, d);
+            if (lane >= d) { i0 += v0; i1 += v1; }
+        }
+        const int t0 = __shfl_sync(0xffffffffu, i0, 31), t1 = __shfl_sync(0xffffffffu, i1, 31);
+        if (lane == 0) {
+            s_wu[warp] = __popc(m0) + __popc(m1);
+            s_wa[warp] = t0 + t1;
+        }
+        df_bar_compute();
+        int ub = 0, ab = 0;
+        const int nw = (E + 63) / 64;
+        for (int w = 0; w < min(warp, nw); w++) {
+            ub += s_wu[w];
+            ab += s_wa[w];
+        }
+        const unsigned below = (1u << lane) - 1u;
+        if (b0) {
+            const int u = ub + __popc(m0 & below);
+            s_uexp[u] = e0; s_umask[u] = (uint8_t)b0; s_ubase[u] = ab + i0 - c0;
+        }
+        if (b1) {
+            const int u = ub + __popc(m0) + __popc(m1 & below);
+            s_uexp[u] = e1; s_umask[u] = (uint8_t)b1; s_ubase[u] = ab + t0 + i1 - c1;
+        }
+        if (warp == nw - 1 && lane == 0) s_U = ub + s_wu[warp];
+    }
+    __syncthreads();
+    U = dead ? 0 : s_U;
+    df_mark(a, 3);                          /* selection known */
+
+    if (warp == DF_CW) {
+        /* ---- helper warp: chains, final order, weights, shared gate ---- */
+        if (!open && n_amb > 0) {
+            walk_chains();
+            bool ok = true;
+            if (lane == 0) ok = spin_until(&a.sync[2], chain_target);
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+            if (!ok) set_status(a.status, ST_SCHED_TIMEOUT);
+            for (int i = lane; i < n_amb && ok; i += 32) {
+                const uint32_t c = __ldcg(&a.chain_ws[i]);
+                codes[(amb[i] >> 11) * (E + 1) + (amb[i] & 0x7ff)] = c | (c << 16);
+            }
+            __syncwarp();
+        }
+        for (int t = 0; t < T && !dead; t++) {
+            if (!s_full[t]) {
+                /* lane i holds selected expert i: its rank, then the weights
+                 * q_i / sum q in rank order (the softmax denominator cancels) */
+                const bool on = lane < TK;
+                const int e = on ? s_sel[t * TK + lane] : 0;
+                const uint32_t c = codes[t * (E + 1) + e] & 0xffffu;
+                const uint32_t key = on ? (code_key(c) << 16) | (0xffffu - (uint32_t)e) : 0u;
+                int rank = 0;
+                for (int i = 0; i < TK; i++) rank += __shfl_sync(0xffffffffu, key, i) > key;
+                const uint32_t top = __reduce_max_sync(0xffffffffu, key) >> 16;
+                const float m =
+                    __uint_as_float((top ^ ((top & 0x8000u) ? 0x8000u : 0xffffu)) << 16);
+                const float q = on ? (float)exp((double)__fsub_rn(bf16lo(c), m)) : 0.0f;
+                float sw = 0.0f;
+                for (int i = 0; i < TK; i++) {
+                    const int src = __ffs(__ballot_sync(0xffffffffu, on && rank == i)) - 1;
+                    sw = __fadd_rn(sw, __shfl_sync(0xffffffffu, q, src));
+                }
+                if (on) {
+                    s_idx[t * TK + rank] = e;
+                    s_w[t * TK + rank] = bf16_bits(__fdiv_rn(q, sw));
                 }
             }
-            (void)slot0;
-            float acc[32];
-            df_down8_n(nt, ws, src, rows, K, lane, acc);
-            if (lane < nt) {
-                int sl = 0;
-#pragma unroll
-                for (int n = 0; n < 4; n++)
-                    if (lane == n) sl = slots[n];
-                uint32_t pk[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float v0 = 0.f, v1 = 0.f;
-#pragma unroll
-                    for (int n = 0; n < 4; n++)
-                        if (lane == n) {
-                            v0 = acc[(2 * q) * 4 + n];
-                            v1 = acc[(2 * q + 1) * 4 + n];
-                        }
-                    pk[q] = pack_bf16(v0, v1);
-                }
-                *reinterpret_cast<uint4 *>(ytab + sl * 16 + bl * 8) =
-                    make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            if (lane == 0)
+                s_gate[t] = bf16_round(sigmoid_f32(bf16lo(codes[t * (E + 1) + E])));
+        }
+        __syncwarp();
+        /* where the down output of each slot will be */
+        for (int i = lane; i < A && !dead; i += 32) {
+            const int t = i / TK, e = s_idx[i];
+            int lo = 0, hi = U - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (s_uexp[mid] < e) lo = mid + 1; else hi = mid;
+            }
+            s_row[i] = s_ubase[lo] + __popc(s_umask[lo] & ((1u << t) - 1u));
+            if (blockIdx.x == 0) {
+                if (a.idx_out) a.idx_out[i] = e;
+                if (a.w_out) a.w_out[i] = s_w[i];
             }
         }
         __syncwarp();
-        ring.consumed++;
-        if (!s_dead && issued_c < n_my_c) {
-            if (lane == 0) {
-                const uint16_t *src;
-                uint32_t bytes;
-                down_src(issued_c, src, bytes);
-                ring.issue(src, bytes, nullptr, 0);
-            }
-            issued_c++;
-            ring.issued++;
+        df_bar_helper_arrive();
+        return;
+    }
+
+    /* ---- routed gate/up ---- */
+    if (!dead) {
+        gu_lo = (int)((long)U * I * blockIdx.x / G);
+        gu_n = (int)((long)U * I * (blockIdx.x + 1) / G) - gu_lo;
+        nR = (gu_n + DF_PAIRS - 1) / DF_PAIRS;
+        const int units = 2 * (U + 1);
+        n_unit = warp < units ? (units - warp + DF_CW - 1) / DF_CW : 0;
+        if (gu_n > 0) {
+            f_src = pair_row(false, 0, lane >> 4) + f_col;
+            f_left = (gu_lo / I + 1) * I - gu_lo;
         }
     }
-    __syncthreads();
+    i_tile = 0;
+    i_sh = false;
+#pragma unroll 1
+    for (int j = 0; j < DF_DEPTH; j++) issue();
+    run_tiles(nR, false);
+    df_mark(a, 4);                      /* routed gate/up done */
+    df_bar_compute();
+    if (tid == 0) {
+        round_arrive(&a.sync[1]);
+        if (!spin_until(&a.sync[1], sync_at[1])) {
+            set_status(a.status, ST_SCHED_TIMEOUT);
+            s_dead = 1;
+        }
+    }
+    df_bar_helper_wait();               /* token rows and logits make room */
+    dead = s_dead != 0;
+    df_mark(a, 5);                      /* barrier passed */
+    {
+        /* routed activations, then the shared ones: four pieces requested before
+         * the first is stored */
+        const int ci = I / 8, cs = Is / 8, na = A * ci, n = na + T * cs;
+#pragma unroll 1
+        for (int c0 = tid; c0 < n; c0 += 4 * DF_CW * 32) {
+            uint4 v[4];
+            uint32_t dst[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int c = c0 + q * DF_CW * 32;
+                if (c < n) {
+                    const bool sh = c >= na;
+                    const int k = sh ? c - na : c, w = sh ? cs : ci, r = k / w;
+                    v[q] = __ldcg(reinterpret_cast<const uint4 *>(sh ? a.sa_ws : a.act_ws) + k);
+                    dst[q] = (uint32_t)((sh ? L.off_sact + r * L.sact_pitch
+                                            : L.off_act + r * L.act_pitch) + (k - r * w) * 16);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (c0 + q * DF_CW * 32 < n) *reinterpret_cast<uint4 *>(df_smem + dst[q]) = v[q];
+        }
+    }
+    df_bar_compute();
+    /* ---- down rows of this CTA's columns ---- */
+#pragma unroll 1
+    for (int j = 0; j < n_unit; j++) {
+        const DownUnit d = down_unit(j);
+        const int v = j * DF_CW + warp, item = v >> 1;
+        const bool sh = item == U;
+        const int cnt = sh ? T : __popc(s_umask[item]), row0 = sh ? 0 : s_ubase[item];
+        const int n = min(lane & 7, cnt - 1);            /* extra columns are not used */
+        uint32_t ba = (sh ? smem_u32(sact) + (uint32_t)(n * L.sact_pitch)
+                          : smem_u32(act) + (uint32_t)((row0 + n) * L.act_pitch)) +
+                      (uint32_t)(d.k0 * 32 + (lane >> 3) * 16);
+        float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+        for (int ks0 = 0; ks0 < d.nk; ks0 += DF_KS, ba += DF_KS * 32) {
+            const uint32_t t = next_tile();
+            const int nk = min(DF_KS, d.nk - ks0);
+#pragma unroll
+            for (int s = 0; s < DF_KS; s += 2)
+                if (s < nk) {
+                    uint32_t br[4], r[4];
+                    ldmatrix_x4(br, ba + (uint32_t)(s * 32));
+                    ldmatrix_x4(r, t + (uint32_t)(s * 32));
+                    mma_16x8(c0, r, br[0], br[1]);
+                    if (s + 1 < nk) {
+                        ldmatrix_x4(r, t + (uint32_t)(s * 32 + 32));
+                        mma_16x8(c1, r, br[2], br[3]);
+                    }
+                }
+            __syncwarp();
+            issue();
+        }
+        const int r = lane >> 2, col = (lane & 3) * 2;
+        float *dst = red + ((size_t)(v & 1) * (A + T) + (sh ? A : row0) + col) * DF_MAX_COLS + r;
+        if (col < cnt) {
+            dst[0] = c0[0] + c1[0];
+            dst[8] = c0[2] + c1[2];
+        }
+        if (col + 1 < cnt) {
+            dst[DF_MAX_COLS] = c0[1] + c1[1];
+            dst[DF_MAX_COLS + 8] = c0[3] + c1[3];
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    df_bar_compute();
+    df_mark(a, 6);                      /* down rows done */
 
-    df_mark(a, 6);                          /* down rows done */
-    /* ---------------- combine (c/layer.h:350,356-361), this CTA's columns ------- */
-    if (!s_dead && tid < T * nb * 8) {
-        const int t = tid / (nb * 8), hl = tid - t * (nb * 8);
+    /* ---- combine (c/layer.h:350,356-361), this CTA's columns ---- */
+    if (!dead && tid < T * ncols) {
+        const int t = tid / ncols, h = tid - t * ncols;
+        const float *y0 = red, *y1 = red + (size_t)(A + T) * DF_MAX_COLS;
         float acc = 0.0f;
-        for (int s = 0; s < TK; s++)
-            acc = __fadd_rn(acc, __fmul_rn(bf16_f32(s_w[t * TK + s]),
-                                           bf16_f32(ytab[(t * TK + s) * 16 + hl])));
+        for (int s = 0; s < TK; s++) {
+            const int o = s_row[t * TK + s] * DF_MAX_COLS + h;
+            acc = __fadd_rn(acc, __fmul_rn(bf16_f32(s_w[t * TK + s]), bf16_round(y0[o] + y1[o])));
+        }
         const float routed = bf16_round(acc);
-        const float sgat = bf16_round(sigmoid_f32(bf16_f32(s_sgl[t])));
-        const float shared =
-            bf16_round(__fmul_rn(bf16_f32(ytab[(DF_MAX_A + t) * 16 + hl]), sgat));
-        const uint16_t o = bf16_bits(__fadd_rn(routed, shared));
-        const size_t at = (size_t)t * H + (size_t)b_lo * 8 + hl;
-        if (a.out) a.out[at] = o;
+        const int o = (A + t) * DF_MAX_COLS + h;
+        const float shared = bf16_round(__fmul_rn(bf16_round(y0[o] + y1[o]), s_gate[t]));
+        const uint16_t v = bf16_bits(__fadd_rn(routed, shared));
+        const size_t at = (size_t)t * H + h_lo + h;
+        if (a.out) a.out[at] = v;
         if (a.res_out)                          /* c/layer.h:230-234,388 */
-            a.res_out[at] = bf16_bits(__fadd_rn(bf16_f32(__ldg(a.res + at)), bf16_f32(o)));
-        if (a.tr_out) a.tr_out[at] = o;
+            a.res_out[at] = bf16_bits(__fadd_rn(bf16_f32(a.res[at]), bf16_f32(v)));
+        if (a.tr_out) a.tr_out[at] = v;
         if (a.tr_routed) a.tr_routed[at] = bf16_bits(routed);
         if (a.tr_shared) a.tr_shared[at] = bf16_bits(shared);
     }
-
-    /* last CTA out resets the counters for the next launch */
-    __syncthreads();
-    df_mark(a, 7);                          /* combine done */
-    if (tid == 0) {
-        __threadfence();
-        const unsigned old = atomicAdd(&a.sync[2], 1u);
-        if (old == (unsigned)G - 1) {
-            a.sync[0] = 0;
-            a.sync[1] = 0;
-            __threadfence();
-            a.sync[2] = 0;
-        }
-    }
-}
-
-inline size_t decode_fused_smem(int T, int H, int I, int Is, int E, int TK,
-                                int stages) {
-    const size_t A = (size_t)T * TK;
-    size_t ring = (size_t)DF_WARPS * stages * DF_STAGE_BYTES;
-    size_t ux = (size_t)T * H * 2, ua = (A * I + (size_t)T * Is) * 2;
-    size_t un = ((ux > ua ? ux : ua) + 127) & ~(size_t)127;
-    size_t ps = (size_t)T * E * 4;
-    size_t yt = (size_t)(DF_MAX_A + DF_MAX_T) * 16 * 2;
-    return ring + un + ps + yt + (DF_WARPS * 3 + 1) * 8 + 64;
+    df_mark(a, 7);                      /* combine done */
 }
 
 }  // namespace apus

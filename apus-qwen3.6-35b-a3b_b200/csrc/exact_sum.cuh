@@ -1,0 +1,333 @@
+/*
+ * exact_sum.cuh — results of the engine's sequential fp32 sums without walking
+ * the whole chain.
+ *
+ * The engine's sums are chains of 2048 dependent fp32 adds (4.6 cycles each on
+ * this GPU: 4.8 us), and their last bits matter.  Two observations:
+ *
+ * 1. Sum of squares (RMSNorm, c/attn.h:175-186).  All terms are >= 0, so the sum
+ *    only grows, and while it stays inside one binade [2^k, 2^(k+1)) it is an
+ *    integer number of units u = 2^(k-23) to which every step adds an integer:
+ *    the term rounded to units, ties decided by whether the sum is even.  A step
+ *    is therefore a function of the sum's parity, such functions compose, and
+ *    composition is associative.  Each of 32 lanes finds the function of its 64
+ *    terms by adding them to the binade's smallest even and smallest odd sum, and
+ *    a segmented scan joins the lanes.  Only where the sum crosses into the next
+ *    binade (about six lanes, lane 0 among them) are the additions done one after
+ *    another.  Every run is verified (it must start and end inside the binade it
+ *    was composed for) and redone sequentially otherwise, so the result is the
+ *    chain's, bit for bit, whatever the data.
+ *
+ * 2. Router logits (c/moe.h:289-291) are rounded to BF16 before anything looks at
+ *    them.  With exact products, chain and true sum differ by at most
+ *    u * sum |partial sum| (each add errs by half an ulp of its result), so a
+ *    tree sum with that bound, evaluated from the data, usually pins the BF16
+ *    code (97-99 % of the logits that compete for the top-k at the real
+ *    dimensions); only the others need their chain.
+ */
+#pragma once
+#include "common.cuh"
+#include "decode_gemv.cuh"
+
+namespace apus {
+
+/* A row of H values as BF16 in shared memory, cut into nl lane chunks of nu 16-byte
+ * pieces, each followed by 16 bytes, so that 32 lanes reading 16 bytes of their
+ * chunks meet no bank conflict.  nl = the largest power of two <= 32 with 8 nl | H. */
+struct LaneRow {
+    int nl, nu, pitch;                /* lanes, 16-byte pieces per lane, bytes per chunk */
+    uint32_t inv;                     /* piece / nu == piece * inv >> 20 below 4096 pieces */
+    LaneRow() = default;
+    __host__ __device__ explicit LaneRow(int H) {
+        nl = 32;
+        while (nl > 1 && H % (8 * nl)) nl >>= 1;
+        nu = H / (8 * nl);
+        pitch = nu * 16 + 16;
+        inv = (1u << 20) / (uint32_t)(nu > 0 ? nu : 1) + 1;
+    }
+    __host__ __device__ int bytes() const { return nl * pitch; }
+    /* byte offset of piece c (values 8 c .. 8 c + 7) */
+    __device__ __forceinline__ int at(int c) const {
+        const int l = (int)(((uint32_t)c * inv) >> 20);
+        return l * 16 + c * 16;       /* l * pitch + (c - l * nu) * 16 */
+    }
+};
+
+/* what a run of additions does to a sum in units, by the parity it starts from */
+struct ParityFn {
+    int i0, i1;
+};
+__device__ __forceinline__ ParityFn compose(ParityFn f, ParityFn g) {
+    ParityFn r;
+    r.i0 = f.i0 + ((f.i0 & 1) ? g.i1 : g.i0);
+    r.i1 = f.i1 + ((f.i1 & 1) ? g.i0 : g.i1);
+    return r;
+}
+__device__ __forceinline__ int binade(float s) { return (int)(__float_as_uint(s) >> 23); }
+
+/* eight additions, as the engine does them */
+__device__ __forceinline__ float add8(float s, const float (&q)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) s = __fadd_rn(s, q[j]);
+    return s;
+}
+__device__ __forceinline__ void square8(const unsigned char *p, float (&q)[8]) {
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4 *>(p), f);
+#pragma unroll
+    for (int j = 0; j < 8; j++) q[j] = __fmul_rn(f[j], f[j]);
+}
+
+/* Sum of squares of a LaneRow; the chain's value in every lane.  One warp (parts
+ * == 1), or two with half of the row each (parts == 2, an even lr.nu): the second
+ * prepares everything while the first walks, then takes the sum over from
+ * `hand_over` in shared memory and goes on, `meet` being a barrier of the two.  The
+ * loops stay rolled: at one row per launch the code runs once, and unrolled it
+ * waits for its instructions. */
+template <typename Meet>
+__device__ __forceinline__ float exact_sumsq(const unsigned char *row, const LaneRow lr, int lane,
+                                             int part, int parts, float *hand_over, Meet meet) {
+    /* chunk of this lane: of lr.nl * parts chunks in row order */
+    const int per = lr.nu / parts, nl = lr.nl;           /* pieces of a chunk; lanes at work */
+    const bool active = lane < nl;
+    const int chunk = part * nl + (active ? lane : 0), l = chunk / parts;
+    const unsigned char *mine = row + l * lr.pitch + (chunk - l * parts) * per * 16;
+    const int nu = active ? per : 0;
+    /* where the sum will be, roughly: tree sums and a scan over the lanes */
+    auto rough = [&](const unsigned char *p) {
+        float t = 0.0f;
+#pragma unroll 1
+        for (int u = 0; u < nu; u++) {
+            float q[8];
+            square8(p + u * 16, q);
+            t += ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+        }
+        return t;
+    };
+    const float tot = rough(mine);
+    float before = 0.0f;
+    if (part) {                                          /* the first half's */
+        const int c0 = active ? lane : 0, l0 = c0 / parts;
+        before = warp_sum(rough(row + l0 * lr.pitch + (c0 - l0 * parts) * per * 16));
+    }
+    float incl = tot;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+    }
+    /* the binade this lane's terms are expected to be added in (key < 0: more than
+     * one, or unsure) and what they do there, found by adding them to the binade's
+     * smallest even and odd sum */
+    const int b0 = binade((before + (incl - tot)) * 0.9998f),
+              b1 = binade((before + incl) * 1.0002f);
+    const int key = active && b0 == b1 && b0 > 0 && b0 < 255 ? b0 : -1 - lane;
+    const float even = __uint_as_float((uint32_t)b0 << 23),
+                odd = __uint_as_float(((uint32_t)b0 << 23) + 1u);
+    float fe = even, fo = odd;
+#pragma unroll 1
+    for (int u = 0; u < nu; u++) {
+        float q[8];
+        square8(mine + u * 16, q);
+        fe = add8(fe, q);
+        fo = add8(fo, q);
+    }
+    ParityFn f;
+    f.i0 = __float_as_int(fe) - __float_as_int(even);
+    f.i1 = __float_as_int(fo) - __float_as_int(odd);
+    /* joined over runs of lanes in the same binade */
+    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || key != prev);
+    const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+#pragma unroll 1
+    for (int d = 1; d < 32; d <<= 1) {
+        ParityFn g;
+        g.i0 = __shfl_up_sync(0xffffffffu, f.i0, d);
+        g.i1 = __shfl_up_sync(0xffffffffu, f.i1, d);
+        if (lane - d >= head) f = compose(g, f);
+    }
+    float s = 0.0f;
+    if (part) {
+        meet();
+        s = *hand_over;
+    }
+    /* walk the runs in order; a run must start and end in its binade (then it never
+     * left it), otherwise its lanes add one by one */
+#pragma unroll 1
+    for (int cur = 0; cur < nl;) {
+        const unsigned rest = cur == 31 ? 0u : heads & (0xffffffffu << (cur + 1));
+        const int end = min(rest ? __ffs(rest) - 1 : 32, nl);
+        const int kb = __shfl_sync(0xffffffffu, key, cur);
+        if (kb >= 0) {
+            const int i0 = __shfl_sync(0xffffffffu, f.i0, end - 1),
+                      i1 = __shfl_sync(0xffffffffu, f.i1, end - 1);
+            const int bits = __float_as_int(s);
+            const float s2 = __int_as_float(bits + ((bits & 1) ? i1 : i0));
+            if (binade(s) == kb && binade(s2) == kb && s2 >= s) {
+                s = s2;
+                cur = end;
+                continue;
+            }
+        }
+#pragma unroll 1
+        for (; cur < end; cur++) {
+            if (lane == cur) {
+#pragma unroll 2
+                for (int u = 0; u < nu; u++) {
+                    float q[8];
+                    square8(mine + u * 16, q);
+                    s = add8(s, q);
+                }
+            }
+            s = __shfl_sync(0xffffffffu, s, cur);
+        }
+    }
+    if (parts == 2 && part == 0) {
+        if (lane == 0) *hand_over = s;
+        meet();
+    }
+    return s;
+}
+__device__ __forceinline__ float exact_sumsq(const unsigned char *row, const LaneRow lr,
+                                             int lane) {
+    return exact_sumsq(row, lr, lane, 0, 1, nullptr, [] {});
+}
+
+/* y = rnd((x * rs) * (1 + w)), eight values; w: the gain offsets */
+__device__ __forceinline__ uint4 norm8(const uint4 v, const uint4 g, float rs) {
+    const uint32_t xw[4] = {v.x, v.y, v.z, v.w}, gw[4] = {g.x, g.y, g.z, g.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const float g0 = __fadd_rn(1.0f, bf16lo(gw[q])), g1 = __fadd_rn(1.0f, bf16hi(gw[q]));
+        o[q] = pack_bf16_rn(__fmul_rn(__fmul_rn(bf16lo(xw[q]), rs), g0),
+                            __fmul_rn(__fmul_rn(bf16hi(xw[q]), rs), g1));
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ float norm_scale(float ss, int H) {
+    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)H), 1e-6f)));
+}
+
+/* RMSNorm with (1+w) gain (c/attn.h:175-186), rows of N % 8 == 0 values, 16-byte
+ * aligned; one warp per row.  Bound: the latency of one row for few rows, and
+ * instruction issue for many.  N 2048: 9.5 us for up to 64 rows (launch included;
+ * the sequential chain took 12.6), 30 us for 8192 (65). */
+constexpr int RN_WARPS = 4;
+__global__ void __launch_bounds__(RN_WARPS * 32)
+rmsnorm_rows_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ w,
+                    uint16_t *__restrict__ y, int T, int N, LaneRow lr) {
+    extern __shared__ __align__(16) unsigned char rn_smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = blockIdx.x * RN_WARPS + warp;
+    pdl_enter();
+    if (t >= T) return;
+    unsigned char *row = rn_smem + warp * lr.bytes();
+    const uint4 *src = reinterpret_cast<const uint4 *>(x + (size_t)t * N);
+    const uint4 *gsrc = reinterpret_cast<const uint4 *>(w);
+    constexpr int R = 8;                /* pieces a lane holds: rows of up to 2048 values */
+    uint4 g[R];
+    if (N <= R * 256) {
+        uint4 v[R];
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const int c = lane + 32 * i;
+            v[i] = c < N / 8 ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
+            g[i] = w && c < N / 8 ? __ldg(gsrc + c) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const int c = lane + 32 * i;
+            if (c < N / 8) *reinterpret_cast<uint4 *>(row + lr.at(c)) = v[i];
+        }
+    } else {
+        for (int c = lane; c < N / 8; c += 32)
+            *reinterpret_cast<uint4 *>(row + lr.at(c)) = __ldg(src + c);
+    }
+    __syncwarp();
+    const float rs = norm_scale(exact_sumsq(row, lr, lane), N);
+    uint4 *dst = reinterpret_cast<uint4 *>(y + (size_t)t * N);
+    if (N <= R * 256) {
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const int c = lane + 32 * i;
+            if (c < N / 8)
+                dst[c] = norm8(*reinterpret_cast<const uint4 *>(row + lr.at(c)), g[i], rs);
+        }
+    } else {
+        for (int c = lane; c < N / 8; c += 32)
+            dst[c] = norm8(*reinterpret_cast<const uint4 *>(row + lr.at(c)),
+                           w ? __ldg(gsrc + c) : make_uint4(0, 0, 0, 0), rs);
+    }
+}
+
+/* A logit as far as it is known: the BF16 codes between which the chain's rounded
+ * result must lie, low code in the low half.  Equal halves: known. */
+__device__ __forceinline__ bool code_known(uint32_t lohi) {
+    return (lohi & 0xffffu) == (lohi >> 16);
+}
+constexpr uint32_t CODE_UNKNOWN = 0x7f80ff80u;       /* [-inf, +inf] */
+
+/* One logit by a warp: w and x are LaneRows, every product exact (the caller has
+ * checked the operands' ranges).  The error terms, with u = 2^-24:
+ *   chain against true sum:  u * sum over its adds of |result|, and a result
+ *     inside a group of eight terms is at most |sum before the group| plus the
+ *     group's sum of magnitudes;
+ *   this sum against the true one:  3 u per group of eight (a tree of three
+ *     levels), then fp64.
+ * The factors below round both up (second-order terms, and the fp32 sums that the
+ * bound itself is built from). */
+__device__ __forceinline__ uint32_t certified_logit(const unsigned char *w,
+                                                    const unsigned char *x, const LaneRow lr,
+                                                    int lane) {
+    const bool active = lane < lr.nl;
+    const int nu = active ? lr.nu : 0;
+    const unsigned char *wp = w + (active ? lane : 0) * lr.pitch,
+                        *xp = x + (active ? lane : 0) * lr.pitch;
+    auto group = [&](int g, float &sum, float &mag) {
+        float wf[8], xf[8], p[8];
+        unpack8(*reinterpret_cast<const uint4 *>(wp + g * 16), wf);
+        unpack8(*reinterpret_cast<const uint4 *>(xp + g * 16), xf);
+#pragma unroll
+        for (int j = 0; j < 8; j++) p[j] = __fmul_rn(wf[j], xf[j]);
+        sum = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+        mag = ((fabsf(p[0]) + fabsf(p[1])) + (fabsf(p[2]) + fabsf(p[3]))) +
+              ((fabsf(p[4]) + fabsf(p[5])) + (fabsf(p[6]) + fabsf(p[7])));
+    };
+    float tot = 0.0f;
+    double dtot = 0.0;
+#pragma unroll 1
+    for (int g = 0; g < nu; g++) {
+        float s, m;
+        group(g, s, m);
+        tot += s;
+        dtot += (double)s;
+    }
+    float incl = tot;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+    }
+    float at = incl - tot, bound = 0.0f, mags = 0.0f;
+#pragma unroll 1
+    for (int g = 0; g < nu; g++) {
+        float s, m;
+        group(g, s, m);
+        bound += fabsf(at) + m;
+        mags += m;
+        at += s;
+    }
+    float e = 8.0f * bound + 4.0f * mags;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+        dtot += __shfl_xor_sync(0xffffffffu, dtot, o);
+    }
+    const double err = (double)e * (1.05 * 5.9604644775390625e-8);
+    const float lo = __double2float_rd(dtot - err), hi = __double2float_ru(dtot + err);
+    if (!(lo <= hi)) return CODE_UNKNOWN;             /* NaN */
+    return (uint32_t)bf16_bits(lo) | ((uint32_t)bf16_bits(hi) << 16);
+}
+
+}  // namespace apus

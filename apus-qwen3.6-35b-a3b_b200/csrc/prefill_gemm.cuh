@@ -321,7 +321,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
     /* The next kernel may be scheduled now.  This kernel's own wait for the
      * previous one comes after the prologue below (barriers, TMEM), which
      * touches nothing the previous kernel writes. */
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (MODE != 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr bool GATE_UP = MODE == 0;
     constexpr int STAGES = PG_STAGES;
     constexpr int BN = MODE == 1 ? PG_BN_DN : PG_BN_GU;
@@ -369,6 +369,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
     /* the down kernel of an overlapped pair does not wait for the whole gate_up
      * kernel: its producer waits per expert instead */
     if (!(MODE == 1 && p.done)) asm volatile("griddepcontrol.wait;" ::: "memory");
+    /* the router's second kernel reads the tokens before its own wait, so it may not
+     * start before what wrote them is complete */
+    if (MODE == 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int n_tiles = MODE == 2 ? p.dense_ntiles : *p.n_tiles;
     const int num_kb = p.K / PG_BK;
 

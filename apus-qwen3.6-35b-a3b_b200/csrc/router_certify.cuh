@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(RC_THREADS, 2)
 router_certify_kernel(CertifyArgs a) {
     /* the next kernel may be scheduled; this kernel's own wait for the fast-logit
      * GEMM comes after the tokens are staged (they are the GEMM's input, complete
-     * before it started) */
+     * before it lets this kernel start) */
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(16) unsigned char rc_smem[];
     const int T = a.T, E = a.E, K = a.K;

@@ -97,6 +97,39 @@ def test_block_one_kernel_path(gpu, orc, be, synth, qwen_weights, cfgname, T):
         check_block(got, orc.moe_block(cfg, W, x), f"{cfgname} T={T}")
 
 
+@pytest.mark.parametrize("T,H,E,I,Is,TK", [
+    (5, 2048, 256, 512, 512, 8), (8, 2048, 256, 512, 512, 8), (7, 208, 37, 48, 16, 3),
+    (8, 1040, 300, 272, 144, 8), (3, 512, 1024, 128, 256, 2), (8, 16, 8, 16, 16, 8),
+    (1, 128, 16, 32, 32, 1)])
+@pytest.mark.parametrize("case", ["plain", "tied_rows", "tiny_logits", "opposite", "underflow"])
+def test_block_one_kernel_edges(gpu, orc, be, synth, T, H, E, I, Is, TK, case):
+    """The one-kernel path at the edges of its tiles (k slices, columns, expert
+    changes inside a tile) and of its routing: logits tied with their neighbours,
+    logits so small that probabilities decide, sums that cancel (wide intervals: the
+    chains run), products that underflow (every chain runs)."""
+    cfg = dict(hidden=H, experts=E, moe_inter=I, shared_inter=Is, top_k=TK)
+    # gate and up of unit variance at most: outputs stay below 4, where one BF16 step
+    # (2^-6), the difference two summation orders may show, is below MAX_ABS
+    W = synth.host_weights(be, cfg, seed=700 + T + E, sigma=min(0.06, 0.9 / H ** 0.5))
+    x = synth.host_x(be, T, H, seed=700 + T)
+    rtr = W["rtr_w"]
+    if case == "tied_rows":
+        rtr[1::2] = rtr[0::2][:rtr[1::2].shape[0]]
+    elif case == "tiny_logits":
+        rtr[:] = synth.f32_to_bf16(synth.bf16_to_f32(rtr) * 2.0 ** -14)
+    elif case == "opposite":
+        rtr[:, 1::2] = rtr[:, 0::2] ^ 0x8000
+        x[:, 1::2] = x[:, 0::2]
+    elif case == "underflow":
+        rtr[:] = synth.f32_to_bf16(synth.bf16_to_f32(rtr) * 1e-36)
+    before = gpu.router_exact_chains()
+    got = gpu.moe_block(cfg, W, x)
+    assert gpu.last_block_launches() == 1 and gpu.last_block_status() == 0
+    check_block(got, orc.moe_block(cfg, W, x), f"{case} T={T}")
+    if case == "underflow":
+        assert gpu.router_exact_chains() - before >= T * E
+
+
 def test_block_batched_equals_per_token(gpu, be, synth):
     """tests/m9c of the reference: the batched body equals the per-token body.
     Here: selected ids are identical and outputs agree to BF16 tolerance when

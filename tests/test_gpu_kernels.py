@@ -270,6 +270,32 @@ def test_rmsnorm_and_residual_add_bitwise(gpu, orc, be, synth, T, N):
     assert np.array_equal(d_y.cpu().numpy().view(np.uint16), orc.resadd(x, b))
 
 
+@pytest.mark.parametrize("N", [8, 128, 256, 768, 2048, 2560])
+def test_rmsnorm_sum_without_the_chain(gpu, orc, N):
+    """The sum of squares composed from parity functions against the sequential
+    chain, bit for bit, on rows made to go wrong: ties in every add, sums that sit
+    on a binade's edge, one value that jumps several binades, descending and
+    ascending magnitudes, zeros, subnormal squares, an overflow."""
+    import torch
+    rng = np.random.default_rng(N)
+    rows = [rng.normal(0, s, N) for s in (1.0, 1e-3, 30.0, 1e-18)]
+    rows += [np.ones(N), np.full(N, 1.5), np.full(N, 1.0 + 2 ** -7), np.zeros(N)]
+    rows += [np.where(np.arange(N) == N // 2, 1e4, rng.normal(0, 1, N)),
+             np.where(np.arange(N) == N - 1, 3e3, rng.normal(0, 1e-2, N)),
+             np.exp2(np.linspace(6, -12, N)), np.exp2(np.linspace(-12, 6, N)),
+             rng.integers(1, 4, N) * 0.5, np.where(np.arange(N) % 64 == 0, 8.0, 0.0),
+             np.full(N, 1e20), np.sign(rng.normal(0, 1, N)) * 181.0]
+    rows += [rng.normal(0, 2.0 ** rng.integers(-3, 4), N) for _ in range(40)]
+    u = np.asarray(rows, np.float32).view(np.uint32).astype(np.uint64)
+    x = ((u + 0x7fff + ((u >> 16) & 1)) >> 16).astype(np.uint16)
+    d_x = torch.from_numpy(x.view(np.int16)).cuda()
+    d_y = torch.empty_like(d_x)
+    gpu.rmsnorm_dev(d_x.data_ptr(), None, d_y.data_ptr(), len(rows), N,
+                    stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert np.array_equal(d_y.cpu().numpy().view(np.uint16), orc.rmsnorm(x, None))
+
+
 # ---- the dense weight stream on device pointers --------------------------------
 
 @pytest.mark.parametrize("M,O,K", [(1, 4096, 2048), (3, 1000, 512), (8, 777, 256),
