@@ -39,6 +39,10 @@ using namespace apus;
 
 constexpr int ROUTER_SMALL_MAX_T = 64;
 constexpr size_t DENSE_PARTS = 4;
+/* behind the status word: the result of a small host-pointer block call, so that one
+ * copy brings both back */
+constexpr size_t STATUS_BYTES = 256, SMALL_OUT_MAX = 64 << 10;
+constexpr int HOST_PARTS = 3;
 
 /* ------------------------------------------------------------------------ */
 /* context                                                                   */
@@ -118,7 +122,7 @@ struct Ctx {
      * upload and the first half's download beside the other half's kernels */
     long host_split_t = 4096;    /* APUS_CUDA_HOST_SPLIT_T: from this many tokens (0: never) */
     cudaStream_t s_in = nullptr, s_out = nullptr;
-    cudaEvent_t ev_io[5] = {};   /* start, in[2], done[2] */
+    cudaEvent_t ev_io[1 + 2 * HOST_PARTS] = {};   /* start, in[], done[] */
     /* dense products of many rows run in parts beside each other */
     cudaStream_t s_part[DENSE_PARTS] = {};
     cudaEvent_t ev_part = nullptr;
@@ -202,8 +206,8 @@ static int ctx_init() {
         c->sm_count = (int)env_long("APUS_CUDA_SMS", 0);
     c->smem_optin = (int)prop.sharedMemPerBlockOptin;
     CU_OK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-    CU_OK(cudaMalloc(&c->d_status, 256));
-    CU_OK(cudaMemset(c->d_status, 0, 256));
+    CU_OK(cudaMalloc(&c->d_status, STATUS_BYTES + SMALL_OUT_MAX));
+    CU_OK(cudaMemset(c->d_status, 0, STATUS_BYTES));
     c->d_scratch_u32 = reinterpret_cast<unsigned int *>(c->d_status) + 16;
     CU_OK(cudaMalloc(&c->d_router_counters, ROUTER_SMALL_MAX_T * 4));
     CU_OK(cudaMemset(c->d_router_counters, 0, ROUTER_SMALL_MAX_T * 4));
@@ -1574,6 +1578,20 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
     return 0;
 }
 
+/* the block on device pointers, inside an ordered section */
+static int block_locked(ApusCudaLayer *layer, const uint16_t *d_ln2, uint16_t *d_out, size_t T,
+                        const ApusCudaMoeTrace *d_tr, cudaStream_t st) {
+    if (layer->maps == nullptr && prefill_supported(layer->cfg) &&
+        (int)T > g_ctx->decode_max_t) {
+        layer->maps = prefill_maps_create(layer->cfg, layer->exp_gu,
+                                          layer->exp_d, layer->sh_g,
+                                          layer->sh_u, layer->sh_d,
+                                          layer->e_end - layer->e_begin);
+        if (!layer->maps) return fail("%s", prefill_last_error());
+    }
+    return block_dev_locked(layer, d_ln2, d_out, T, d_tr, st);
+}
+
 extern "C" int apus_cuda_moe_block_dev(ApusCudaLayer *layer,
                                        const uint16_t *d_ln2, uint16_t *d_out,
                                        size_t T, const ApusCudaMoeTrace *d_tr,
@@ -1585,15 +1603,7 @@ extern "C" int apus_cuda_moe_block_dev(ApusCudaLayer *layer,
     cudaStream_t st = (cudaStream_t)stream;
     Ordered ord(g_ctx, st);
     if (ord.rc) return 1;
-    if (layer->maps == nullptr && prefill_supported(layer->cfg) &&
-        (int)T > g_ctx->decode_max_t) {
-        layer->maps = prefill_maps_create(layer->cfg, layer->exp_gu,
-                                          layer->exp_d, layer->sh_g,
-                                          layer->sh_u, layer->sh_d,
-                                          layer->e_end - layer->e_begin);
-        if (!layer->maps) return fail("%s", prefill_last_error());
-    }
-    return block_dev_locked(layer, d_ln2, d_out, T, d_tr, st);
+    return block_locked(layer, d_ln2, d_out, T, d_tr, st);
 }
 
 static int layer_dev(ApusCudaLayer *layer, const uint16_t *d_res, const uint16_t *d_ln_w,
@@ -1787,6 +1797,25 @@ extern "C" int apus_cuda_moe_block(const ApusCudaMoeCfg *cfg,
     c->io.reset();
     uint16_t *dx = (uint16_t *)c->io.take(T * H * 2);
     uint16_t *dout = (uint16_t *)c->io.take(T * H * 2);
+    const char *const st_at = (const char *)c->d_status;
+    auto status_ok = [&](int st) -> int {
+        if (!st) return 0;
+        cudaMemset(c->d_status, 0, 4);
+        return fail("moe_block: device status %d (a bounded wait gave up or "
+                    "an index was out of range)", st);
+    };
+    /* a handful of tokens: result and status word come back in one copy */
+    if (!tr && T * H * 2 <= SMALL_OUT_MAX) {
+        CU_OK(c->hs.upload(dx, ln2, T * H * 2, c->stream));
+        if (block_locked(L, dx, (uint16_t *)(st_at + STATUS_BYTES), T, nullptr, c->stream))
+            return 1;
+        CU_OK(c->hs.download_begin(0, st_at, STATUS_BYTES + T * H * 2, c->stream));
+        CU_OK(cudaEventSynchronize(c->hs.eout[0]));
+        int st;
+        memcpy(&st, c->hs.out, 4);
+        memcpy(moe_out, c->hs.out + STATUS_BYTES, T * H * 2);
+        return status_ok(st);
+    }
     ApusCudaMoeTrace dtr;
     memset(&dtr, 0, sizeof dtr);
     if (tr) {
@@ -1798,21 +1827,18 @@ extern "C" int apus_cuda_moe_block(const ApusCudaMoeCfg *cfg,
     /* rows [r0, r0 + n) of the call: upload on s_up, block on the library's
      * stream, download on s_dn (all three the same stream for a small call) */
     auto download = [&](size_t r0, size_t n, cudaStream_t s_dn) -> int {
-        CU_OK(cudaMemcpyAsync(moe_out + r0 * H, dout + r0 * H, n * H * 2,
-                              cudaMemcpyDeviceToHost, s_dn));
+        CU_OK(c->hs.download(moe_out + r0 * H, dout + r0 * H, n * H * 2, s_dn));
         if (!tr) return 0;
         if (tr->rtr_idx)
-            CU_OK(cudaMemcpyAsync(tr->rtr_idx + r0 * TK, dtr.rtr_idx + r0 * TK, n * TK * 4,
-                                  cudaMemcpyDeviceToHost, s_dn));
+            CU_OK(c->hs.download(tr->rtr_idx + r0 * TK, dtr.rtr_idx + r0 * TK, n * TK * 4, s_dn));
         if (tr->rtr_w)
-            CU_OK(cudaMemcpyAsync(tr->rtr_w + r0 * TK, dtr.rtr_w + r0 * TK, n * TK * 2,
-                                  cudaMemcpyDeviceToHost, s_dn));
+            CU_OK(c->hs.download(tr->rtr_w + r0 * TK, dtr.rtr_w + r0 * TK, n * TK * 2, s_dn));
         if (tr->moe_routed)
-            CU_OK(cudaMemcpyAsync(tr->moe_routed + r0 * H, dtr.moe_routed + r0 * H,
-                                  n * H * 2, cudaMemcpyDeviceToHost, s_dn));
+            CU_OK(c->hs.download(tr->moe_routed + r0 * H, dtr.moe_routed + r0 * H, n * H * 2,
+                                 s_dn));
         if (tr->moe_shared)
-            CU_OK(cudaMemcpyAsync(tr->moe_shared + r0 * H, dtr.moe_shared + r0 * H,
-                                  n * H * 2, cudaMemcpyDeviceToHost, s_dn));
+            CU_OK(c->hs.download(tr->moe_shared + r0 * H, dtr.moe_shared + r0 * H, n * H * 2,
+                                 s_dn));
         return 0;
     };
     auto part_trace = [&](size_t r0) {
@@ -1825,52 +1851,48 @@ extern "C" int apus_cuda_moe_block(const ApusCudaMoeCfg *cfg,
     };
     const bool split = c->host_split_t > 0 && T >= (size_t)c->host_split_t;
     if (!split) {
-        CU_OK(cudaMemcpyAsync(dx, ln2, T * H * 2, cudaMemcpyHostToDevice, c->stream));
-        if (apus_cuda_moe_block_dev(L, dx, dout, T, tr ? &dtr : nullptr, c->stream))
-            return 1;
+        CU_OK(c->hs.upload(dx, ln2, T * H * 2, c->stream));
+        if (block_locked(L, dx, dout, T, tr ? &dtr : nullptr, c->stream)) return 1;
         if (download(0, T, c->stream)) return 1;
     } else {
-        /* A token's result does not depend on which other tokens share the call,
-         * so two half calls give the same bits; the PCIe copies of one half run
-         * beside the kernels of the other. */
+        /* A token's result does not depend on which other tokens share the call, so
+         * a call in parts gives the same bits; the PCIe copies of one part run
+         * beside the kernels of another.  A part costs a pass over the weights
+         * (~250 us) and saves the travel of its rows (~0.08 us a row and way): two
+         * halves from 4096 rows, a short first and last part from 6144. */
         if (!c->s_in) {
             CU_OK(cudaStreamCreateWithFlags(&c->s_in, cudaStreamNonBlocking));
             CU_OK(cudaStreamCreateWithFlags(&c->s_out, cudaStreamNonBlocking));
             for (auto &e : c->ev_io) CU_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
-        const size_t r1 = T / 2, cut[3] = {0, r1, T};
+        const int parts = T >= 6144 ? 3 : 2;
+        const size_t edge = parts == 3 ? T / 5 : T / 2;
+        const size_t cut[HOST_PARTS + 1] = {0, edge, parts == 3 ? T - edge : T, T};
         CU_OK(cudaEventRecord(c->ev_io[0], c->stream));       /* earlier work owns dx, dout */
         CU_OK(cudaStreamWaitEvent(c->s_in, c->ev_io[0], 0));
         CU_OK(cudaStreamWaitEvent(c->s_out, c->ev_io[0], 0));
-        for (int k = 0; k < 2; k++) {
-            CU_OK(cudaMemcpyAsync(dx + cut[k] * H, ln2 + cut[k] * H,
-                                  (cut[k + 1] - cut[k]) * H * 2, cudaMemcpyHostToDevice,
-                                  c->s_in));
-            CU_OK(cudaEventRecord(c->ev_io[1 + k], c->s_in));
-        }
-        for (int k = 0; k < 2; k++) {
+        for (int k = 0; k < parts; k++) {
             const size_t r0 = cut[k], n = cut[k + 1] - cut[k];
+            CU_OK(c->hs.upload(dx + r0 * H, ln2 + r0 * H, n * H * 2, c->s_in));
+            CU_OK(cudaEventRecord(c->ev_io[1 + k], c->s_in));
             CU_OK(cudaStreamWaitEvent(c->stream, c->ev_io[1 + k], 0));
             ApusCudaMoeTrace tk = part_trace(r0);
-            if (apus_cuda_moe_block_dev(L, dx + r0 * H, dout + r0 * H, n, tr ? &tk : nullptr,
-                                        c->stream))
+            if (block_locked(L, dx + r0 * H, dout + r0 * H, n, tr ? &tk : nullptr, c->stream))
                 return 1;
-            CU_OK(cudaEventRecord(c->ev_io[3 + k], c->stream));
-            CU_OK(cudaStreamWaitEvent(c->s_out, c->ev_io[3 + k], 0));
-            if (download(r0, n, c->s_out)) return 1;
+            CU_OK(cudaEventRecord(c->ev_io[1 + HOST_PARTS + k], c->stream));
+        }
+        for (int k = 0; k < parts; k++) {
+            CU_OK(cudaStreamWaitEvent(c->s_out, c->ev_io[1 + HOST_PARTS + k], 0));
+            if (download(cut[k], cut[k + 1] - cut[k], c->s_out)) return 1;
         }
         CU_OK(cudaStreamSynchronize(c->s_out));
     }
-    int st = 0;
-    CU_OK(cudaMemcpyAsync(&st, c->d_status, 4, cudaMemcpyDeviceToHost, c->stream));
+    CU_OK(c->hs.download_begin(0, st_at, 4, c->stream));
     CU_OK(cudaStreamSynchronize(c->stream));
+    int st;
+    memcpy(&st, c->hs.out, 4);
     if (tr && tr->moe_out) memcpy(tr->moe_out, moe_out, T * H * 2);
-    if (st) {
-        cudaMemset(c->d_status, 0, 4);
-        return fail("moe_block: device status %d (a bounded wait gave up or "
-                    "an index was out of range)", st);
-    }
-    return 0;
+    return status_ok(st);
 }
 
 
