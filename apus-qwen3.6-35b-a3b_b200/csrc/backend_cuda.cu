@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "decode_fused.cuh"
 #include "router_certify.cuh"
+#include "router_select.cuh"
 #include "decode_gemv.cuh"
 #include "dispatch.cuh"
 #include "ep_window.cuh"
@@ -81,7 +82,9 @@ struct ApusCudaLayer {
     float wmin = 0.0f;          /* smallest nonzero |rtr_w| (0 = unknown) */
     float wmin_gate = 0.0f;     /* the same for the shared-gate row */
     float wmax = 0.0f, wmax_gate = 0.0f;   /* largest magnitudes */
-    float *d_wnorm = nullptr;   /* [E + 1] router row norms (rounded up), [E] = max */
+    float *d_wnorm = nullptr;   /* [E + 1] router row norms (rounded up), [E] = max; behind
+                                 * them the shared-gate row's, twice */
+    float wnorm_gate = 0.0f;
     size_t bytes = 0;
     PrefillMaps *maps = nullptr; /* tensor maps for the tcgen05 path */
 };
@@ -671,7 +674,8 @@ static int launch_router_tt(Ctx *c, const uint16_t *dx, const uint16_t *dwr,
 /* optional inputs of the certified many-token path */
 struct RouterAux {
     const float *wnorm;     /* [E + 1] row norms of the router matrix */
-    float wmin_extra;       /* smallest nonzero |extra_row| */
+    float wmax;             /* largest |w| */
+    float wmin_extra, wmax_extra, wnorm_extra;   /* the same of extra_row */
     float *approx_ws;       /* fp32 workspace, at least T*E*4 bytes */
     size_t approx_bytes;    /* its size: up to four [T, E] slabs are used */
 };
@@ -688,7 +692,7 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
     if (c->router_certify && aux && aux->wnorm && aux->approx_ws && dlogits &&
         T > ROUTER_SMALL_MAX_T && E % PG_BM == 0 && K % 256 == 0 &&
         (((uintptr_t)dwr | (uintptr_t)dx | (uintptr_t)extra_row) & 15) == 0 &&
-        router_certify_smem(E, K) <= (size_t)c->smem_optin) {
+        router_certify_smem(E, K, 6) * RC_WARPS + 2048 <= (size_t)c->smem_optin) {
         int ksplit = dense_logits_ksplit(c->sm_count, T, E, K);
         while (ksplit > 1 && (size_t)ksplit * T * E * 4 > aux->approx_bytes) ksplit /= 2;
         if (run_dense_logits(c->sm_count, c->smem_optin, dwr, dx, T, E, K, ksplit,
@@ -697,40 +701,52 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
             return fail("%s", prefill_last_error());
         c->launches++;
         CertifyArgs ca;
-        memset(&ca, 0, sizeof ca);
+        memset((void *)&ca, 0, sizeof ca);
         ca.approx = aux->approx_ws;
         ca.nslab = ksplit;
         ca.x = dx;
         ca.w = dwr;
         ca.extra_row = extra_row;
         ca.wnorm = aux->wnorm;
+        ca.wnorm_extra = aux->wnorm_extra;
         ca.T = T; ca.E = E; ca.K = K; ca.topk = topk;
         ca.wmin = wmin;
+        ca.wmax = aux->wmax;
         ca.wmin_extra = aux->wmin_extra;
+        ca.wmax_extra = aux->wmax_extra;
         /* the sequential chain errs by at most (K-1)u times the sum of the
          * term magnitudes; the tensor cores are granted eight times that */
         ca.cbound = 9.1f * (float)K * 5.9604645e-8f;   /* = debug_fast_logits' *cbound */
-        ca.logits = nullptr;        /* nobody reads the merged logits */
         ca.idx_out = didx;
         ca.w_out = dw;
         ca.extra_out = extra_out;
         ca.status = c->d_status;
         ca.stats = c->d_rc_stats;
-        const size_t smem = router_certify_smem(E, K);
+        ca.lr = LaneRow(K);
+        /* one warp per token.  Too few tokens to fill the SMs: deep rings, which hide
+         * the rows' latency where a full SM hides it behind other warps. */
+        const int warps = T <= c->sm_count ? 1 : RC_WARPS;
+        const bool deep = T <= 6 * c->sm_count && K == 2048 && E <= 256;
+        void (*kern)(CertifyArgs) = E > 256     ? router_certify_kernel<32, 0, 2>
+                                    : deep      ? router_certify_kernel<8, 8, 6>
+                                    : K == 2048 ? router_certify_kernel<8, 8, 2>
+                                                : router_certify_kernel<8, 0, 2>;
+        const size_t smem = router_certify_smem(E, K, deep ? 6 : 2) * warps;
+        const size_t most = router_certify_smem(E, K, 6) * RC_WARPS;
         static size_t set_smem = 0;
-        if (smem > set_smem) {
-            CU_OK(cudaFuncSetAttribute(router_certify_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
-            set_smem = smem;
+        if (most > set_smem) {
+            for (auto k : {router_certify_kernel<32, 0, 2>, router_certify_kernel<8, 8, 6>,
+                           router_certify_kernel<8, 8, 2>, router_certify_kernel<8, 0, 2>})
+                CU_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)most));
+            set_smem = most;
         }
-        launch_k(router_certify_kernel, dim3((T + RC_TT - 1) / RC_TT), dim3(RC_THREADS),
-                 smem, st, ca);
+        launch_k(kern, dim3((T + warps - 1) / warps), dim3(warps * 32), smem, st, ca);
         LAUNCHED();
         return 0;
     }
-    /* few tokens: rows spread over many small CTAs, everything in flight at
-     * once (latency path) */
+    /* few tokens, every exact logit: rows spread over many small CTAs, everything in
+     * flight at once (latency path) */
     if (T <= ROUTER_SMALL_MAX_T && (K & 7) == 0 &&
         (((uintptr_t)dwr | (uintptr_t)extra_row) & 15) == 0) {
         const int rows = E + (extra_row ? 1 : 0);
@@ -875,11 +891,15 @@ static int layer_router_stats(Ctx *c, ApusCudaLayer *L) {
     if (bf16_range(c, L->rtr_w, E * H, &L->wmin, &L->wmax) ||
         bf16_range(c, L->sh_gate, H, &L->wmin_gate, &L->wmax_gate))
         return 1;
-    if (!L->d_wnorm) CU_OK(cudaMalloc(&L->d_wnorm, (E + 1) * sizeof(float)));
-    CU_OK(cudaMemsetAsync(L->d_wnorm, 0, (E + 1) * sizeof(float), c->stream));
+    if (!L->d_wnorm) CU_OK(cudaMalloc(&L->d_wnorm, (E + 3) * sizeof(float)));
+    CU_OK(cudaMemsetAsync(L->d_wnorm, 0, (E + 3) * sizeof(float), c->stream));
     row_norm_kernel<<<(unsigned)((E * 32 + 255) / 256), 256, 0, c->stream>>>(
         L->rtr_w, (int)E, (int)H, L->d_wnorm);
     LAUNCHED();
+    row_norm_kernel<<<1, 32, 0, c->stream>>>(L->sh_gate, 1, (int)H, L->d_wnorm + E + 1);
+    LAUNCHED();
+    CU_OK(cudaMemcpyAsync(&L->wnorm_gate, L->d_wnorm + E + 1, 4, cudaMemcpyDeviceToHost,
+                          c->stream));
     CU_OK(cudaStreamSynchronize(c->stream));
     return 0;
 }
@@ -1405,6 +1425,8 @@ static int run_fused_decode(Ctx *c, ApusCudaLayer *L, const uint16_t *d_ln2,
     const size_t smem = (size_t)a.L.total;
     a.wmin = L->wmin; a.wmax = L->wmax;
     a.wmin_gate = L->wmin_gate; a.wmax_gate = L->wmax_gate;
+    a.wnorm = L->d_wnorm;
+    a.wnorm_gate = L->wnorm_gate;
     a.x = d_ln2;
     if (rz) {
         a.res = rz->res;
@@ -1517,7 +1539,7 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
     c->n_ev = 0;
     stage_mark(c, -1, st);
     /* the fast logits live in the combine buffer, which is written much later */
-    RouterAux aux = {L->d_wnorm, L->wmin_gate, reinterpret_cast<float *>(b.eo),
+    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate, L->wnorm_gate, reinterpret_cast<float *>(b.eo),
                      (size_t)Ti * TK * H * 2};
     if (launch_router(c, d_ln2, L->rtr_w, Ti, E, H, TK, L->wmin, b.idx, b.rw,
                       b.logits, L->sh_gate, b.sgl, st,
@@ -1952,7 +1974,7 @@ extern "C" int apus_cuda_ep_route_dev(ApusCudaLayer *L, const uint16_t *d_x,
     if (arena_reserve(c->ws, T * E * 18 + 8192)) return 1;
     c->ws.reset();
     uint16_t *logits = (uint16_t *)c->ws.take(T * E * 2);
-    RouterAux aux = {L->d_wnorm, L->wmin_gate, (float *)c->ws.take(T * E * 16),
+    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate, L->wnorm_gate, (float *)c->ws.take(T * E * 16),
                      T * E * 16};
     return launch_router(c, d_x, L->rtr_w, (int)T, (int)E, (int)L->cfg.hidden,
                          (int)L->cfg.top_k, L->wmin, d_idx, d_w, logits,
@@ -2512,7 +2534,7 @@ extern "C" int apus_cuda_route_dev(ApusCudaLayer *L, const uint16_t *d_x,
     if (arena_reserve(c->ws, T * E * 18 + 8192)) return 1;
     c->ws.reset();
     uint16_t *logits = (uint16_t *)c->ws.take(T * E * 2);
-    RouterAux aux = {L->d_wnorm, 0.0f, (float *)c->ws.take(T * E * 16), T * E * 16};
+    RouterAux aux = {L->d_wnorm, L->wmax, 0.0f, 0.0f, 0.0f, (float *)c->ws.take(T * E * 16), T * E * 16};
     return launch_router(c, d_x, L->rtr_w, (int)T, (int)E, (int)L->cfg.hidden,
                          (int)L->cfg.top_k, L->wmin, d_idx, d_w, logits, nullptr,
                          nullptr, st, &aux);

@@ -18,9 +18,7 @@
  *    selected experts can still depend on them.  Only when the SET is open does
  *    everyone wait for the chains.  (A chain for every logit, then softmax over
  *    all of them, put 21 of 47 us in front of the first expert weight.)
- *  - selection looks at BF16 logits, not at probabilities: exp and the division
- *    keep their order whenever the logits near the top differ by 2^-18 or more,
- *    which is checked; otherwise the engine's softmax runs on exact logits;
+ *  - selection looks at BF16 logits, not at probabilities (router_select.cuh);
  *  - weight rows are multiplied by mma.sync m16n8k16 with the tokens as the eight
  *    columns, so eight tokens cost the instructions of one (scalar multiply-adds
  *    held the gate/up phase at 27 us for 15 us of bytes at three tokens).  Each
@@ -48,7 +46,7 @@
 #include "decode_gemv.cuh"
 #include "exact_dense.cuh"
 #include "exact_sum.cuh"
-#include "router.cuh"
+#include "router_select.cuh"
 
 namespace apus {
 
@@ -74,7 +72,7 @@ struct FusedLayout {
     int xrow;                /* bytes of a token row (LaneRow) */
     int act_pitch, sact_pitch;
     int rrows;               /* router rows of a CTA, at most */
-    int off_x, off_rr, off_code, off_key, off_tmask, off_amb, off_act, off_sact, off_red, total;
+    int off_x, off_rr, off_code, off_tmask, off_amb, off_act, off_sact, off_red, total;
     FusedLayout() = default;
     FusedLayout(int T, int H, int I, int Is, int E, int TK, int G) {
         const int A = T * TK;
@@ -87,12 +85,11 @@ struct FusedLayout {
         sact_pitch = Is * 2 + 16;
         rrows = (E + 1 + G - 1) / G;
         int p = DF_CW * DF_DEPTH * slot;
-        /* tokens, router rows, logits, their keys, open pairs; later the activations */
+        /* tokens, router rows, logits, open pairs; later the activations */
         off_x = p;
         off_rr = off_x + T * xrow;
-        off_code = off_rr + rrows * xrow;
-        off_key = off_code + T * (E + 1) * 4;
-        off_tmask = off_key + T * E * 4;
+        off_code = off_rr + (rrows * xrow > CH_BYTES ? rrows * xrow : CH_BYTES);
+        off_tmask = off_code + T * (E + 1) * 4;
         off_amb = off_tmask + 1024;
         const int end1 = off_amb + T * (E + 1) * 2;
         off_act = p;
@@ -111,6 +108,8 @@ struct FusedArgs {
     int T, H, I, Is, E, TK;
     float wmin, wmax;                   /* smallest nonzero and largest |w|: router matrix */
     float wmin_gate, wmax_gate;         /* ... shared-gate row */
+    const float *wnorm;                 /* [E] row norms, rounded up */
+    float wnorm_gate;
     const uint16_t *x;                  /* [T, H] block input; or, with res set, unused */
     /* the two steps either side of the block folded in: res [T,H] is the residual
      * stream, the block input is rmsnorm(res, 1 + ln_w) (every CTA computes it for
@@ -195,34 +194,6 @@ __device__ __forceinline__ void mma_16x8(float (&c)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b_lo), "r"(b_hi));
 }
 
-/* Order-preserving 16-bit key of a BF16 code (-0 counts as +0). */
-__device__ __forceinline__ uint32_t code_key(uint32_t code) {
-    code &= 0xffffu;
-    if (code == 0x8000u) code = 0;
-    return code ^ ((code & 0x8000u) ? 0xffffu : 0x8000u);
-}
-
-/* One exact chain by one lane, both rows LaneRows in shared memory. */
-template <bool FMA>
-__device__ __forceinline__ float df_chain(const unsigned char *w, const unsigned char *x,
-                                          const LaneRow lr) {
-    float acc = 0.0f;
-#pragma unroll 1
-    for (int l = 0; l < lr.nl; l++, w += lr.pitch, x += lr.pitch) {
-#pragma unroll 2
-        for (int c = 0; c < lr.nu; c++) {
-            float wf[8], xf[8];
-            unpack8(*reinterpret_cast<const uint4 *>(w + c * 16), wf);
-            unpack8(*reinterpret_cast<const uint4 *>(x + c * 16), xf);
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-                acc = FMA ? __fmaf_rn(wf[j], xf[j], acc)
-                          : __fadd_rn(acc, __fmul_rn(wf[j], xf[j]));
-        }
-    }
-    return acc;
-}
-
 __global__ void __launch_bounds__(DF_THREADS, 1)
 decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     extern __shared__ __align__(128) unsigned char df_smem[];
@@ -233,7 +204,6 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     const LaneRow lr = L.lr;
     unsigned char *xs = df_smem + L.off_x, *rr = df_smem + L.off_rr;
     uint32_t *codes = reinterpret_cast<uint32_t *>(df_smem + L.off_code);   /* [T][E + 1] */
-    uint32_t *keys = reinterpret_cast<uint32_t *>(df_smem + L.off_key);     /* [T][E] */
     uint16_t *amb = reinterpret_cast<uint16_t *>(df_smem + L.off_amb);      /* t << 11 | e */
     unsigned char *act = df_smem + L.off_act, *sact = df_smem + L.off_sact;
     uint32_t *s_tmask = reinterpret_cast<uint32_t *>(df_smem + L.off_tmask);   /* [256]: tokens of
@@ -242,7 +212,7 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     __shared__ int s_sel[DF_MAX_A];                /* selected experts, in provisional order */
     __shared__ int s_idx[DF_MAX_A], s_row[DF_MAX_A];   /* final order; down output of each */
     __shared__ uint16_t s_w[DF_MAX_A];
-    __shared__ float s_gate[DF_MAX_T], s_sum[DF_MAX_T], s_rs[DF_MAX_T];
+    __shared__ float s_gate[DF_MAX_T], s_sum[DF_MAX_T], s_rs[DF_MAX_T], s_sq[2][DF_MAX_T];
     __shared__ unsigned int s_xlo[DF_MAX_T], s_xhi[DF_MAX_T];
     __shared__ int s_namb[DF_MAX_T], s_full[DF_MAX_T], s_open;
     __shared__ int s_wu[DF_CW], s_wa[DF_CW];       /* per warp: experts, assignments before it */
@@ -424,16 +394,23 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
                 }
             }
             unsigned int lo = 0x7f800000u, hi = 0;
+            float sq = 0.0f;
 #pragma unroll 1
             for (int c = part * 32 + lane; c < cph; c += 32 * parts) {
                 uint4 *p = reinterpret_cast<uint4 *>(row + lr.at(c));
                 uint4 v = *p;
                 if (a.res) *p = v = norm8(v, gains[c], rs);
                 fold_range8(v, lo, hi);
+                float f[8];
+                unpack8(v, f);
+#pragma unroll
+                for (int j = 0; j < 8; j++) sq = fmaf(f[j], f[j], sq);
             }
+            sq = warp_sum(sq);
             lo = __reduce_min_sync(0xffffffffu, lo);
             hi = __reduce_max_sync(0xffffffffu, hi);
             if (lane == 0) {
+                s_sq[part][t] = sq;
                 atomicMin(&s_xlo[t], lo);
                 atomicMax(&s_xhi[t], hi);
             }
@@ -448,8 +425,11 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
             const bool exact =
                 e == E ? products_exact(a.wmin_gate, a.wmax_gate, s_xlo[t], s_xhi[t])
                        : products_exact(a.wmin, a.wmax, s_xlo[t], s_xhi[t]);
-            const uint32_t v = exact ? certified_logit(rr + r * L.xrow, xs + t * L.xrow, lr, lane)
-                                     : CODE_UNKNOWN;
+            uint32_t v = CODE_UNKNOWN;
+            if (exact)                       v = certified_logit(rr + r * L.xrow, xs + t * L.xrow, lr, lane,
+                                    (e == E ? a.wnorm_gate : __ldg(&a.wnorm[e])) *
+                                        norm_above(s_sq[0][t] +
+                                                       (lr.nu % 2 == 0 ? s_sq[1][t] : 0.0f), H));
             if (lane == 0) a.code_ws[(size_t)t * (E + 1) + e] = v;
         }
     __syncthreads();
@@ -540,101 +520,22 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     for (int i = tid; i < T * (E + 1); i += DF_THREADS)
         codes[i] = dead ? 0u : __ldcg(&a.code_ws[i]);
     __syncthreads();
-    /* Selection of token t by one warp: the TK experts with the largest low codes
-     * (lowest index first on ties).  Anything else whose high code reaches the
-     * TK-th low code may belong there instead. */
-    auto select = [&](int t, bool first) {
-        const uint32_t *cd = codes + t * (E + 1);
-        /* keys: low code, then lowest index first; all different.  Up to 256 experts
-         * they stay in registers. */
-        constexpr int R = 8;
-        uint32_t *kd = keys + t * E, kr[R], best = 0, kth = 0;
-        const bool regs = E <= 32 * R;
-        auto key_of = [&](int e) { return (code_key(cd[e]) << 16) | (0xffffu - (uint32_t)e); };
-        if (regs) {
-#pragma unroll
-            for (int i = 0; i < R; i++) {
-                kr[i] = lane + 32 * i < E ? key_of(lane + 32 * i) : 0u;
-                best = max(best, kr[i]);
-            }
-        } else {
-#pragma unroll 1
-            for (int e = lane; e < E; e += 32) best = max(best, kd[e] = key_of(e));
-        }
-#pragma unroll 1
-        for (int i = 0; i < TK; i++) {
-            kth = __reduce_max_sync(0xffffffffu, best);
-            if (lane == 0) s_sel[t * TK + i] = (int)(0xffffu - (kth & 0xffffu));
-            if (regs) {
-                best = 0;
-#pragma unroll
-                for (int j = 0; j < R; j++)
-                    if (kr[j] < kth) best = max(best, kr[j]);
-            } else if (best == kth) {                    /* this lane's next one */
-                best = 0;
-                for (int e = lane; e < E; e += 32)
-                    if (kd[e] < kth) best = max(best, kd[e]);
-            }
-        }
-        /* does code order decide?  (see the head of this file) */
-        const uint32_t kkey = kth >> 16;
-        bool open = false, odd = false, any = false;
-        float top = -INFINITY;
-        uint32_t reach = 0;                              /* bit i: expert lane + 32 i competes */
-        if (regs) {
-#pragma unroll
-            for (int i = 0; i < R; i++)
-                if (lane + 32 * i < E && code_key(cd[lane + 32 * i] >> 16) >= kkey)
-                    reach |= 1u << i;
-        } else {
-            for (int e = lane, i = 0; e < E; e += 32, i++)
-                if (code_key(cd[e] >> 16) >= kkey) reach |= 1u << i;
-        }
-        for (; reach; reach &= reach - 1) {
-            const int e = lane + 32 * (__ffs(reach) - 1);
-            const uint32_t v = cd[e];
-            const bool known = code_known(v);
-            any |= !known;
-            if (!known && key_of(e) < kth) open = true;  /* not among the chosen */
-            const float lo = bf16lo(v), hi = bf16hi(v);
-            const bool zero = known && (v & 0x7fffu) == 0;
-            const bool plain = fabsf(lo) >= 9.765625e-4f && fabsf(hi) >= 9.765625e-4f &&
-                               (lo < 0.0f) == (hi < 0.0f) && fabsf(hi) <= 32.0f;
-            if (!plain && !(zero && code_key(v) != kkey)) odd = true;
-            top = fmaxf(top, hi);
-        }
-        __syncwarp();
-        /* order-preserving integer of a float, for the integer reduction */
-        const int ti = __float_as_int(top);
-        const int tm = __reduce_max_sync(0xffffffffu, ti >= 0 ? ti : ti ^ 0x7fffffff);
-        top = __int_as_float(tm >= 0 ? tm : tm ^ 0x7fffffff);
-        const uint32_t kc = kkey ^ ((kkey & 0x8000u) ? 0x8000u : 0xffffu);
-        if (!(__uint_as_float(kc << 16) - top >= -80.0f)) odd = true;
-        odd = __any_sync(0xffffffffu, odd);
-        open = __any_sync(0xffffffffu, open);
-        any = __any_sync(0xffffffffu, any) || odd || !code_known(cd[E]);
-        if (first) {
-            /* logits that need their chain: competitors whose code is open (all of
-             * them if probabilities have to decide), and the shared gate */
-            int n = 0;
-            if (any)
-#pragma unroll 1
-                for (int e0 = 0; e0 <= E; e0 += 32) {
-                    const int e = e0 + lane;
-                    const bool need = e <= E && !code_known(cd[e]) &&
-                                      (odd || e == E || code_key(cd[e] >> 16) >= kkey);
-                    n += __popc(__ballot_sync(0xffffffffu, need));
-                }
-            if (lane == 0) {
-                s_namb[t] = n;
-                s_full[t] = odd;
-                if (open || odd) s_open = 1;
-            }
-        }
-        return kkey;
-    };
     uint32_t kkey = 0;
-    if (warp < T && !dead) kkey = select(warp, true);
+    if (warp < T && !dead) {
+        const uint32_t *cd = codes + warp * (E + 1);
+        const Choice c = rt_select(cd, E, TK, lane, s_sel + warp * TK);
+        kkey = c.kkey;
+        int n = 0;
+        if (c.any)
+#pragma unroll 1
+            for (int e0 = 0; e0 <= E; e0 += 32)
+                n += __popc(__ballot_sync(0xffffffffu, rt_needs(cd, e0 + lane, E, kkey, c.odd)));
+        if (lane == 0) {
+            s_namb[warp] = n;
+            s_full[warp] = c.odd;
+            if (c.open || c.odd) s_open = 1;
+        }
+    }
     __syncthreads();
     int n_amb = 0;
     if (!dead)
@@ -647,8 +548,7 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
             const uint32_t *cd = codes + warp * (E + 1);
             for (int e0 = 0; e0 <= E; e0 += 32) {
                 const int e = e0 + lane;
-                const bool need = e <= E && !code_known(cd[e]) &&
-                                  (s_full[warp] || e == E || code_key(cd[e] >> 16) >= kkey);
+                const bool need = rt_needs(cd, e, E, kkey, s_full[warp] != 0);
                 const unsigned m = __ballot_sync(0xffffffffu, need);
                 if (need) amb[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)((warp << 11) | e);
                 at += __popc(m);
@@ -657,33 +557,19 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
         __syncthreads();
     }
     const bool open = s_open != 0;           /* the set itself waits for the chains */
-    /* Pair i of the list is CTA i % G's.  Its helper warp brings the weight rows
-     * into the place of the router rows (under the expert stream a row read piece
-     * by piece would wait an L2 round trip per piece), as many at a time as fit. */
+    /* Pair i of the list is CTA i % G's; its helper warp walks it, the products in the
+     * place of the router rows. */
     auto walk_chains = [&]() {
         if ((int)blockIdx.x >= n_amb) return;
-        const int room = min(L.rrows, 32);
-        for (int i0 = blockIdx.x; i0 < n_amb; i0 += room * G) {
-            for (int q = 0; q < room && i0 + q * G < n_amb; q++) {
-                const int e = amb[i0 + q * G] & 0x7ff;
-                const uint16_t *w = e == E ? a.sh_gate : a.rtr_w + (size_t)e * H;
-                for (int c = lane; c < H / 8; c += 32)
-                    cp_async16_to(smem_u32(rr + q * L.xrow + lr.at(c)), w + c * 8);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncwarp();
-            const int i = i0 + lane * G;
-            if (lane < room && i < n_amb) {
-                const int t = amb[i] >> 11, e = amb[i] & 0x7ff;
-                const bool fma =
-                    e == E ? products_exact(a.wmin_gate, a.wmax_gate, s_xlo[t], s_xhi[t])
-                           : products_exact(a.wmin, a.wmax, s_xlo[t], s_xhi[t]);
-                const unsigned char *wr = rr + lane * L.xrow, *xr = xs + t * L.xrow;
-                const float z = fma ? df_chain<true>(wr, xr, lr) : df_chain<false>(wr, xr, lr);
-                a.chain_ws[i] = bf16_bits(z);
-            }
-            __syncwarp();
+        for (int i = blockIdx.x; i < n_amb; i += G) {
+            const int t = amb[i] >> 11, e = amb[i] & 0x7ff;
+            const uint16_t *w = e == E ? a.sh_gate : a.rtr_w + (size_t)e * H;
+            const unsigned char *xr = xs + t * L.xrow;
+            const float z = warp_chains<4>(
+                1, H, lane, reinterpret_cast<float *>(rr),
+                [&](int) { return w; },
+                [&](int p) { return *reinterpret_cast<const uint4 *>(xr + lr.at(p)); });
+            if (lane == 0) a.chain_ws[i] = bf16_bits(z);
         }
         if (lane == 0) {
             if (a.stats && blockIdx.x == 0) atomicAdd(&a.stats[0], (unsigned)n_amb);
@@ -707,14 +593,14 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
         if (warp < T && !dead) {
             if (s_full[warp]) {
                 /* the engine's softmax and selection on exact logits */
-                float *p = reinterpret_cast<float *>(keys + warp * E);
+                float *p = reinterpret_cast<float *>(codes + warp * (E + 1));
                 for (int e = lane; e < E; e += 32) p[e] = bf16lo(codes[warp * (E + 1) + e]);
                 __syncwarp();
                 router_softmax_topk(p, E, TK, lane, s_idx + warp * TK, s_w + warp * TK);
                 __syncwarp();
                 for (int i = lane; i < TK; i += 32) s_sel[warp * TK + i] = s_idx[warp * TK + i];
             } else {
-                select(warp, false);
+                rt_select(codes + warp * (E + 1), E, TK, lane, s_sel + warp * TK);
             }
         }
         __syncthreads();
@@ -780,29 +666,9 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
             __syncwarp();
         }
         for (int t = 0; t < T && !dead; t++) {
-            if (!s_full[t]) {
-                /* lane i holds selected expert i: its rank, then the weights
-                 * q_i / sum q in rank order (the softmax denominator cancels) */
-                const bool on = lane < TK;
-                const int e = on ? s_sel[t * TK + lane] : 0;
-                const uint32_t c = codes[t * (E + 1) + e] & 0xffffu;
-                const uint32_t key = on ? (code_key(c) << 16) | (0xffffu - (uint32_t)e) : 0u;
-                int rank = 0;
-                for (int i = 0; i < TK; i++) rank += __shfl_sync(0xffffffffu, key, i) > key;
-                const uint32_t top = __reduce_max_sync(0xffffffffu, key) >> 16;
-                const float m =
-                    __uint_as_float((top ^ ((top & 0x8000u) ? 0x8000u : 0xffffu)) << 16);
-                const float q = on ? (float)exp((double)__fsub_rn(bf16lo(c), m)) : 0.0f;
-                float sw = 0.0f;
-                for (int i = 0; i < TK; i++) {
-                    const int src = __ffs(__ballot_sync(0xffffffffu, on && rank == i)) - 1;
-                    sw = __fadd_rn(sw, __shfl_sync(0xffffffffu, q, src));
-                }
-                if (on) {
-                    s_idx[t * TK + rank] = e;
-                    s_w[t * TK + rank] = bf16_bits(__fdiv_rn(q, sw));
-                }
-            }
+            if (!s_full[t])
+                rt_weights(codes + t * (E + 1), s_sel + t * TK, TK, lane, s_idx + t * TK,
+                           s_w + t * TK);
             if (lane == 0)
                 s_gate[t] = bf16_round(sigmoid_f32(bf16lo(codes[t * (E + 1) + E])));
         }

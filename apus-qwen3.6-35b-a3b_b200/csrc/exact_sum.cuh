@@ -268,66 +268,57 @@ __device__ __forceinline__ bool code_known(uint32_t lohi) {
 }
 constexpr uint32_t CODE_UNKNOWN = 0x7f80ff80u;       /* [-inf, +inf] */
 
-/* One logit by a warp: w and x are LaneRows, every product exact (the caller has
- * checked the operands' ranges).  The error terms, with u = 2^-24:
- *   chain against true sum:  u * sum over its adds of |result|, and a result
- *     inside a group of eight terms is at most |sum before the group| plus the
- *     group's sum of magnitudes;
- *   this sum against the true one:  3 u per group of eight (a tree of three
- *     levels), then fp64.
- * The factors below round both up (second-order terms, and the fp32 sums that the
- * bound itself is built from). */
-__device__ __forceinline__ uint32_t certified_logit(const unsigned char *w,
-                                                    const unsigned char *x, const LaneRow lr,
-                                                    int lane) {
+/* At least the 2-norm of n values whose squares an fp32 sum (any order) gave as ss: the
+ * sum is within a relative n 2^-23 and, where squares underflow, n 2^-149. */
+__device__ __forceinline__ float norm_above(float ss, int n) {
+    return sqrtf(ss + (float)n * 1.4e-45f) * 1.001f;
+}
+
+/* The logit of one weight row and one token by a warp: LaneRows, every product exact
+ * (the caller has checked the operands' ranges).  A lane adds its terms in eights (two
+ * chains of four and their sum) onto a running sum; the lanes' sums are scanned.  The
+ * error terms, with u = 2^-24:
+ *   chain against true sum:  u * sum over its adds of |result|; a result inside an
+ *     eight is at most |sum before the lane| + |running sum before the eight| + the
+ *     eight's sum of magnitudes;
+ *   this sum against the true one:  4 u of the magnitudes, u |running sum| per eight,
+ *     u |lane sum| per level of the scan.
+ * The magnitudes of all eights together are at most cs = ||w|| ||x|| (Cauchy-Schwarz).
+ * The factors below round up (second-order terms, and the fp32 sums that the bound
+ * itself is built from). */
+__device__ __forceinline__ uint32_t certified_logit(const unsigned char *w, const unsigned char *x,
+                                                    const LaneRow lr, int lane, float cs) {
     const bool active = lane < lr.nl;
     const int nu = active ? lr.nu : 0;
     const unsigned char *wp = w + (active ? lane : 0) * lr.pitch,
                         *xp = x + (active ? lane : 0) * lr.pitch;
-    auto group = [&](int g, float &sum, float &mag) {
-        float wf[8], xf[8], p[8];
+    float run = 0.0f, e = 0.0f;
+#pragma unroll 2
+    for (int g = 0; g < nu; g++) {
+        float wf[8], xf[8];
         unpack8(*reinterpret_cast<const uint4 *>(wp + g * 16), wf);
         unpack8(*reinterpret_cast<const uint4 *>(xp + g * 16), xf);
+        float s0 = __fmul_rn(wf[0], xf[0]), s1 = __fmul_rn(wf[4], xf[4]);
 #pragma unroll
-        for (int j = 0; j < 8; j++) p[j] = __fmul_rn(wf[j], xf[j]);
-        sum = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
-        mag = ((fabsf(p[0]) + fabsf(p[1])) + (fabsf(p[2]) + fabsf(p[3]))) +
-              ((fabsf(p[4]) + fabsf(p[5])) + (fabsf(p[6]) + fabsf(p[7])));
-    };
-    float tot = 0.0f;
-    double dtot = 0.0;
-#pragma unroll 1
-    for (int g = 0; g < nu; g++) {
-        float s, m;
-        group(g, s, m);
-        tot += s;
-        dtot += (double)s;
+        for (int j = 1; j < 4; j++) {
+            s0 = __fmaf_rn(wf[j], xf[j], s0);
+            s1 = __fmaf_rn(wf[4 + j], xf[4 + j], s1);
+        }
+        e += fabsf(run);
+        run += s0 + s1;
     }
-    float incl = tot;
+    float sum = run;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const float v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += v;
+        const float v = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += v;
     }
-    float at = incl - tot, bound = 0.0f, mags = 0.0f;
-#pragma unroll 1
-    for (int g = 0; g < nu; g++) {
-        float s, m;
-        group(g, s, m);
-        bound += fabsf(at) + m;
-        mags += m;
-        at += s;
-    }
-    float e = 8.0f * bound + 4.0f * mags;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        e += __shfl_xor_sync(0xffffffffu, e, o);
-        dtot += __shfl_xor_sync(0xffffffffu, dtot, o);
-    }
-    const double err = (double)e * (1.05 * 5.9604644775390625e-8);
-    const float lo = __double2float_rd(dtot - err), hi = __double2float_ru(dtot + err);
-    if (!(lo <= hi)) return CODE_UNKNOWN;             /* NaN */
-    return (uint32_t)bf16_bits(lo) | ((uint32_t)bf16_bits(hi) << 16);
+    e = warp_sum(8.0f * nu * fabsf(sum - run) + 9.0f * e + 8.0f * fabsf(run));
+    const float tot = __shfl_sync(0xffffffffu, sum, 31),
+                err = (e + 12.0f * cs) * (1.05f * 5.9604645e-8f);
+    const float lo = __fadd_rd(tot, -err), hi = __fadd_ru(tot, err);
+    return lo <= hi ? (uint32_t)bf16_bits(lo) | ((uint32_t)bf16_bits(hi) << 16)
+                    : CODE_UNKNOWN;                              /* NaN */
 }
 
 }  // namespace apus

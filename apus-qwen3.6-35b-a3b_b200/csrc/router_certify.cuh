@@ -1,6 +1,6 @@
 /*
- * router_certify.cuh — exact expert selection at a fraction of the exact
- * router's cost (c/moe.h:321-371 decides with BF16-rounded logits whose every
+ * router_certify.cuh — exact expert selection for many tokens at a fraction of the
+ * exact router's cost (c/moe.h:321-371 decides with BF16-rounded logits whose every
  * bit depends on a 2048-step sequential fp32 chain per expert, c/moe.h:289-291).
  *
  * Only the top_k experts of a token matter, and an expert far below the
@@ -22,38 +22,34 @@
  *      other expert's exact rounded logit is strictly below those of top_k
  *      experts, whatever the rounding did: it cannot be selected;
  *   4. candidates (about top_k + 2 of 256 at the real dimensions) and the
- *      shared-gate row get their exact chain, one lane each; everything else
- *      keeps its rounded fast logit, which only enters the softmax
- *      denominator (and cancels in the renormalised weights);
- *   5. the kernel checks |a - z| <= B on every pair it evaluates exactly and
+ *      shared-gate row get an interval that nearly always pins the BF16 code of
+ *      their exact chain (exact_sum.cuh), the few that it does not and that matter
+ *      get the chain itself;
+ *   5. the kernel checks |a - z| <= B on every pair it evaluates and
  *      records ST_BOUND_VIOLATED if the assumption ever fails.
  *
- * The engine's softmax / top-k (router_softmax_topk, one warp per token) then
- * runs in the same kernel on the merged logits: ids are bit-exact by
- * construction, weights see exact logits for every selected expert.
+ * Selection and weights then follow from the codes (router_select.cuh).
+ *
+ * One warp per token from end to end.  Bound: instruction issue for many tokens
+ * (about 200 per candidate and warp), latency for few; so a lane keeps its 64 values
+ * of the token as fp32 in registers, the eights of a row are independent, and the
+ * lanes' partial results meet in shared memory, where one lane per candidate adds
+ * them up.  Candidate rows (4 KB each, from L2) arrive through a ring of D slots per
+ * warp.  (A chain per candidate, one per lane, took 33 us at 512 tokens, 55 at 1999
+ * and 148 at 8192.)
  */
 #pragma once
 #include <climits>
 
 #include "common.cuh"
 #include "decode_gemv.cuh"
-#include "router.cuh"
+#include "router_select.cuh"
 
 namespace apus {
 
-constexpr int RC_TT = 8;            /* tokens per CTA (6 with deeper prefetch measured the same) */
-constexpr int RC_THREADS = 256;      /* one warp per token in the first phase */
-constexpr int RC_XPAD = 4;          /* floats between token rows: rows on
-                                     * different bank groups */
-constexpr int RC_CW = 4;            /* warps that walk chains: 128 pairs in one round (8 tokens
-                                     * give 86 on average; a second round doubles the latency) */
-constexpr int RC_BLK = 32;          /* weights per staged row block */
-constexpr int RC_AHEAD = 2;         /* row blocks requested ahead of the one in use (4 ahead
-                                     * measured the same: the chain is bound by its
-                                     * dependent adds and shared-memory reads, ~12 cycles a
-                                     * step, not by the copies) */
-constexpr int RC_NBUF = RC_AHEAD + 1;
-constexpr int RC_WPITCH = RC_BLK * 2 + 16;   /* bytes per staged row block */
+constexpr int RC_WARPS = 2;         /* tokens of a CTA at most: a token with chains to walk takes
+                                     * twice as long as one without, and holds up its CTA's slot */
+constexpr int RC_MAX_E = 1024;
 constexpr int ST_BOUND_VIOLATED = 5;
 constexpr int RC_MAX_SLABS = 4;     /* K slices of the fast-logit GEMM */
 
@@ -63,15 +59,17 @@ struct CertifyArgs {
     const uint16_t *x, *w;          /* [T, K], [E, K] */
     const uint16_t *extra_row;      /* [K] shared-gate row (optional) */
     const float *wnorm;             /* [E + 1]: ||w_e||_2 rounded up; [E] = their max */
+    float wnorm_extra;              /* the same of extra_row */
     int T, E, K, topk;
-    float wmin, wmin_extra;         /* smallest nonzero |w| (0 = unknown) */
+    float wmin, wmax;               /* smallest nonzero and largest |w| (0: unknown) */
+    float wmin_extra, wmax_extra;
     float cbound;                   /* see above */
-    uint16_t *logits;               /* [T, E] merged BF16 logit codes out (optional) */
     int32_t *idx_out;               /* [T, topk] selection */
     uint16_t *w_out;                /* [T, topk] renormalised weights (optional) */
     uint16_t *extra_out;            /* [T] */
     int *status;
-    unsigned int *stats;            /* [0] += exact chains run (optional) */
+    unsigned int *stats;            /* [0] += logits resolved exactly (optional) */
+    LaneRow lr;
 };
 
 /* order-preserving integer key of a float (larger float -> larger int) */
@@ -79,330 +77,267 @@ __device__ __forceinline__ int rc_float_key(float f) {
     const int b = __float_as_int(f);
     return b >= 0 ? b : (b ^ 0x7fffffff);
 }
-
-/* Operands of RC_BLK steps of one exact chain: BF16 weights and fp32 tokens
- * from shared memory.  The chain is bound by instruction issue and by the
- * latency of the dependent add, so the tokens are kept converted (one shift or
- * mask per weight is all that remains beside the add) and the operands of the
- * next block are fetched while the current block's adds run. */
-struct RcOperands {
-    uint4 w[RC_BLK / 8];
-    float4 x[RC_BLK / 4];
-};
-__device__ __forceinline__ void rc_fetch(RcOperands &o, const unsigned char *__restrict__ w,
-                                         const float *__restrict__ x) {
+__device__ __forceinline__ float rc_approx(const CertifyArgs &a, int t, int e) {
+    float p[RC_MAX_SLABS];
 #pragma unroll
-    for (int c = 0; c < RC_BLK / 8; c++) {
-        o.w[c] = *reinterpret_cast<const uint4 *>(w + c * 16);
-        o.x[2 * c] = *reinterpret_cast<const float4 *>(x + c * 8);
-        o.x[2 * c + 1] = *reinterpret_cast<const float4 *>(x + c * 8 + 4);
-    }
-}
-template <bool FMA>
-__device__ __forceinline__ float rc_steps(const RcOperands &o, float acc) {
-#pragma unroll
-    for (int c = 0; c < RC_BLK / 8; c++) {
-        float wf[8];
-        unpack8(o.w[c], wf);
-        const float xf[8] = {o.x[2 * c].x,     o.x[2 * c].y,     o.x[2 * c].z,
-                             o.x[2 * c].w,     o.x[2 * c + 1].x, o.x[2 * c + 1].y,
-                             o.x[2 * c + 1].z, o.x[2 * c + 1].w};
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (FMA)
-                acc = __fmaf_rn(wf[j], xf[j], acc);
-            else
-                acc = __fadd_rn(acc, __fmul_rn(wf[j], xf[j]));
-        }
-    }
-    return acc;
-}
-__device__ __forceinline__ void cp_async16(void *dst_smem, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)),
-                 "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+    for (int sl = 0; sl < RC_MAX_SLABS; sl++)
+        p[sl] = sl < a.nslab ? __ldg(&a.approx[((size_t)sl * a.T + t) * a.E + e]) : 0.0f;
+    return (p[0] + p[1]) + (p[2] + p[3]);
 }
 
-/* One chain per lane over the warp's 32 staged rows (see the kernel's note).
- * rows[32]: the lanes' weight rows; wb: this warp's RC_NBUF buffers; x: this
- * lane's token in fp32.  Integer work issues at half the rate of the adds, so
- * the loop keeps running pointers instead of computing addresses. */
-template <bool FMA>
-__device__ __forceinline__ float rc_walk(const uint16_t *const *rows, unsigned char *wb,
-                                         const float *__restrict__ xr, int K, int lane) {
-    constexpr int LPR = RC_BLK / 8;            /* lanes per row in a copy instruction */
-    constexpr int RPI = 32 / LPR;              /* rows per copy instruction */
-    constexpr int NCP = 32 / RPI;              /* copy instructions per block */
-    constexpr size_t BUF = (size_t)32 * RC_WPITCH;
-    const int nblk = K / RC_BLK;
-    const uint16_t *src[NCP];
-#pragma unroll
-    for (int i = 0; i < NCP; i++) src[i] = rows[RPI * i + lane / LPR] + (lane % LPR) * 8;
-    unsigned char *const dst0 = wb + (size_t)(lane / LPR) * RC_WPITCH + (lane % LPR) * 16;
-    unsigned char *const wend = wb + RC_NBUF * BUF;
-    unsigned char *dst = dst0;                 /* where the next block goes */
-    auto issue = [&]() {
-#pragma unroll
-        for (int i = 0; i < NCP; i++) {
-            cp_async16(dst + (size_t)i * RPI * RC_WPITCH, src[i]);
-            src[i] += RC_BLK;
-        }
-        dst += BUF;
-        if (dst >= wend) dst -= RC_NBUF * BUF;
-    };
-    for (int b = 0; b < RC_AHEAD; b++) {
-        if (b < nblk) issue();
-        cp_async_commit();
-    }
-    const unsigned char *wl = wb + (size_t)lane * RC_WPITCH;   /* the block in use */
-    const unsigned char *const wlend = wl + RC_NBUF * BUF;
-    float z = 0.0f;
-#pragma unroll 1
-    for (int b = 0; b < nblk; b++) {
-        cp_async_wait<RC_AHEAD - 1>();     /* block b has landed (my copies) */
-        __syncwarp();                      /* ... and everyone else's; block b - 1 is
-                                            * read out everywhere, so its buffer can
-                                            * take block b + AHEAD */
-        if (b + RC_AHEAD < nblk) issue();
-        cp_async_commit();
-        RcOperands o;
-        rc_fetch(o, wl, xr);
-        z = rc_steps<FMA>(o, z);
-        wl += BUF;
-        if (wl >= wlend) wl -= RC_NBUF * BUF;
-        xr += RC_BLK;
-    }
-    return z;
+constexpr int RC_BATCH = 12;        /* candidates whose partial results meet at once */
+/* Dynamic shared memory, per warp: D row slots, partial sums, codes [E + 1],
+ * candidates [E + 1]. */
+inline size_t router_certify_smem(int E, int K, int slots) {
+    const size_t ring = (size_t)slots * LaneRow(K).bytes();   /* later the chains' products */
+    return (ring > CH_BYTES ? ring : CH_BYTES) + RC_BATCH * 33 * 2 * 4 +
+           (size_t)((E + 4) & ~3) * 4 + (size_t)((E + 8) & ~7) * 2;
 }
 
-/*
- * grid = ceil(T / RC_TT), block = RC_THREADS.  K % 256 == 0, E % 32 == 0,
- * E <= 1024.  Dynamic shared memory:
- *   xs    float  [RC_TT][K + RC_XPAD]   tokens
- *   af    float  [RC_TT][E]             fast logits
- *   pairs uint16 [RC_TT * (E + 1)]      (token << 11 | row); 16-bit so that TWO
- *                                        CTAs fit the SM's shared memory (one
- *                                        CTA per SM left the chain warps' idle
- *                                        phases uncovered: 7 waves of 22 us)
- *   wn    float  [E + 1]                row norms
- *   wbuf  [RC_CW][RC_NBUF][32][80 B]    staged weight blocks of the chain warps
- *
- * The chains: a warp takes 32 pairs, one per lane.  A lane reading its own
- * weight row 16 bytes at a time would cost the load unit one tag look-up per
- * lane and instruction; instead the warp copies each 32-weight block of its 32
- * rows into shared memory cooperatively (four lanes per row, cp.async, three
- * blocks in flight) and every lane then reads its row from there.
- */
-__global__ void __launch_bounds__(RC_THREADS, 2)
-router_certify_kernel(CertifyArgs a) {
+/* grid = ceil(T / warps); E % 32 == 0, K % 256 == 0.  R: experts per lane, at least
+ * E / 32; NU: 16-byte pieces of a lane's chunk that are kept in registers (K / 256),
+ * 0: any K, the token is read again for each candidate; D: ring slots. */
+template <int R, int NU, int D>
+__global__ void __launch_bounds__(RC_WARPS * 32, 16 / RC_WARPS)
+router_certify_kernel(const __grid_constant__ CertifyArgs a) {
     /* the next kernel may be scheduled; this kernel's own wait for the fast-logit
-     * GEMM comes after the tokens are staged (they are the GEMM's input, complete
+     * GEMM comes after the token is staged (it is the GEMM's input, complete
      * before it lets this kernel start) */
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(16) unsigned char rc_smem[];
-    const int T = a.T, E = a.E, K = a.K;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int t0 = blockIdx.x * RC_TT;
-    const int nt = min(RC_TT, T - t0);
-    const int xp = K + RC_XPAD;
-    float *xs = reinterpret_cast<float *>(rc_smem);
-    float *af = xs + (size_t)RC_TT * xp;
-    uint16_t *pairs = reinterpret_cast<uint16_t *>(af + (size_t)RC_TT * E);
-    float *wn = reinterpret_cast<float *>(
-        (reinterpret_cast<uintptr_t>(pairs + (size_t)RC_TT * (E + 1)) + 15) & ~(uintptr_t)15);
-    unsigned char *wbuf = reinterpret_cast<unsigned char *>(
-        (reinterpret_cast<uintptr_t>(wn + E + 1) + 15) & ~(uintptr_t)15);
-    __shared__ const uint16_t *s_rowptr[RC_CW][32];
-    __shared__ int s_npairs;
-    __shared__ unsigned int s_xmin;
-    __shared__ float s_xnorm[RC_TT];
+    __shared__ int s_sel[RC_WARPS][32];
+    const int E = a.E, K = a.K, TK = a.topk;
+    const LaneRow lr = a.lr;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int t = blockIdx.x * nw + warp;
+    const int row_bytes = lr.bytes(), ring_bytes = max(D * row_bytes, CH_BYTES);
+    const int cd_n = (E + 4) & ~3, cand_n = (E + 8) & ~7;
+    unsigned char *slots = rc_smem + (size_t)warp * ring_bytes;
+    float *part = reinterpret_cast<float *>(rc_smem + (size_t)nw * ring_bytes) +
+                  warp * (RC_BATCH * 33 * 2);
+    uint32_t *cd = reinterpret_cast<uint32_t *>(rc_smem + (size_t)nw * ring_bytes) +
+                   nw * (RC_BATCH * 33 * 2) + warp * cd_n;
+    uint16_t *cand = reinterpret_cast<uint16_t *>(rc_smem + (size_t)nw * ring_bytes +
+                                                  (size_t)nw * (RC_BATCH * 33 * 2 + cd_n) * 4) +
+                     warp * cand_n;
     auto mark = [&](int k) {
-        /* phase boundaries of CTA 0 (global timer, ns) for the profiling notes */
-        if (a.stats && blockIdx.x == 0 && tid == 0) {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            a.stats[2 + k] = (unsigned int)t;
+        /* phase boundaries of the first warp (global timer, ns) for the profiling notes */
+        if (a.stats && blockIdx.x == 0 && threadIdx.x == 0) {
+            unsigned long long tm;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(tm));
+            a.stats[2 + k] = (unsigned int)tm;
         }
     };
     mark(0);
-    if (tid == 0) {
-        s_npairs = 0;
-        s_xmin = 0x7f800000u;
-    }
-    for (int e = tid; e <= E; e += RC_THREADS) wn[e] = __ldg(&a.wnorm[e]);
-    __syncthreads();
-
-    /* ---- per token (one warp each, round robin): stage x, norm, fast logits,
-     *      the top_k-th of them, the candidates ---- */
-    for (int tl = warp; tl < nt; tl += RC_THREADS / 32) {
-        const int t = t0 + tl;
-        float ss[4] = {0.f, 0.f, 0.f, 0.f};
-        unsigned int xmin = 0x7f800000u;
-        /* every load of a batch is issued before the first is used */
-        for (int k0 = 0; k0 < K; k0 += 2048) {
-            uint4 xv[8];
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                const int k = k0 + c * 256 + lane * 8;
-                xv[c] = k < K ? ldg16(a.x + (size_t)t * K + k) : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                const int k = k0 + c * 256 + lane * 8;
-                if (k >= K) continue;
-                float f[8];
-                unpack8(xv[c], f);
-                float4 *d = reinterpret_cast<float4 *>(xs + (size_t)tl * xp + k);
-                d[0] = make_float4(f[0], f[1], f[2], f[3]);
-                d[1] = make_float4(f[4], f[5], f[6], f[7]);
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    ss[j & 3] = fmaf(f[j], f[j], ss[j & 3]);
-                    const unsigned int m = __float_as_uint(f[j]) & 0x7fffffffu;
-                    if (m != 0 && m < xmin) xmin = m;
-                }
-            }
-        }
-        float s2 = warp_sum((ss[0] + ss[1]) + (ss[2] + ss[3]));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            xmin = min(xmin, __shfl_xor_sync(0xffffffffu, xmin, o));
-        /* an upper bound of the norm: the fp32 sum of squares is within a
-         * relative K*2^-23 of the truth */
-        const float xnorm = sqrtf(s2) * 1.001f;
-        if (lane == 0) {
-            s_xnorm[tl] = xnorm;
-            atomicMin(&s_xmin, xmin);
-        }
+    if (t >= a.T) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        for (int e0 = 0; e0 < E; e0 += 256) {
-            float av[8];
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                const int e = e0 + c * 32 + lane;
-                float part[RC_MAX_SLABS];
-#pragma unroll
-                for (int sl = 0; sl < RC_MAX_SLABS; sl++)
-                    part[sl] = (e < E && sl < a.nslab)
-                                   ? __ldg(&a.approx[((size_t)sl * T + t) * E + e])
-                                   : 0.0f;
-                av[c] = (part[0] + part[1]) + (part[2] + part[3]);
-            }
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                const int e = e0 + c * 32 + lane;
-                if (e >= E) continue;
-                af[(size_t)tl * E + e] = av[c];
-                if (a.logits)
-                    a.logits[(size_t)t * E + e] = bf16_bits(av[c]);   /* unless replaced below */
-            }
-        }
-        __syncwarp();
-        /* top_k-th largest fast logit (with multiplicity) */
-        float a8 = 0.0f;
-        unsigned int taken = 0;              /* bit i: my entry lane + 32*i is out */
-        for (int i = 0; i < a.topk; i++) {
-            int bk = INT_MIN, be = 0x7fffffff;
-            for (int e = lane, j = 0; e < E; e += 32, j++) {
-                if ((taken >> j) & 1u) continue;
-                const int k = rc_float_key(af[(size_t)tl * E + e]);
-                if (k > bk) { bk = k; be = e; }
-            }
-            const int wk = __reduce_max_sync(0xffffffffu, bk);
-            const int we = (int)__reduce_min_sync(0xffffffffu,
-                                                  bk == wk ? (unsigned)be : 0x7fffffffu);
-            if (we < E) {
-                a8 = af[(size_t)tl * E + we];
-                if (lane == (we & 31)) taken |= 1u << (we >> 5);
-            }
-        }
-        const float cb = a.cbound * xnorm;
-        const float bmax = cb * wn[E];
-        /* one BF16 step at the magnitude of the values compared, rounded up */
-        const float spacing = (fabsf(a8) + bmax) * (1.0f / 64.0f) + 1e-30f;
-        const float thr = a8 - bmax - spacing;
-        for (int e0 = 0; e0 < E; e0 += 32) {
-            const int e = e0 + lane;
-            const float v = af[(size_t)tl * E + e];
-            const bool cand = v + cb * wn[e] >= thr;
-            const unsigned m = __ballot_sync(0xffffffffu, cand);
-            int base = 0;
-            if (lane == 0 && m) base = atomicAdd(&s_npairs, __popc(m));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (cand)
-                pairs[base + __popc(m & ((1u << lane) - 1u))] = (uint16_t)((tl << 11) | e);
-        }
-        if (a.extra_row && lane == 0)
-            pairs[atomicAdd(&s_npairs, 1)] = (uint16_t)((tl << 11) | E);
+        return;
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");   /* warps without a token */
-    __syncthreads();
+    /* ---- the token: norm, range of its values ---- */
+    const uint32_t slot0 = smem_u32(slots);
+    const unsigned char *x_lane = slots + lane * lr.pitch;
+    lane_row_fetch(slot0, a.x + (size_t)t * K, lr, K, lane);
+    cp_async_done();
+    __syncwarp();
+    unsigned long long xp[NU > 0 ? NU * 4 : 1];          /* pairs of values */
+    float ss = 0.0f;
+    unsigned int xlo = 0x7f800000u, xhi = 0;
+    auto square = [&](const uint4 v, float (&f)[8]) {
+        unpack8(v, f);
+        float q[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) q[j] = f[j] * f[j];
+        ss += ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+        fold_range8(v, xlo, xhi);
+    };
+    if (NU > 0) {
+#pragma unroll
+        for (int u = 0; u < NU; u++) {
+            float f[8];
+            square(*reinterpret_cast<const uint4 *>(x_lane + u * 16), f);
+#pragma unroll
+            for (int j = 0; j < 4; j++) xp[u * 4 + j] = pack_f32x2(f[2 * j], f[2 * j + 1]);
+        }
+    } else {
+        for (int u = 0; u < lr.nu; u++) {
+            float f[8];
+            square(*reinterpret_cast<const uint4 *>(x_lane + u * 16), f);
+        }
+    }
+    const float xnorm = norm_above(warp_sum(ss), K);
+    xlo = __reduce_min_sync(0xffffffffu, xlo);
+    xhi = __reduce_max_sync(0xffffffffu, xhi);
+    const bool ok = products_exact(a.wmin, a.wmax, xlo, xhi),
+               ok_extra = products_exact(a.wmin_extra, a.wmax_extra, xlo, xhi);
+    const float wn_max = __ldg(&a.wnorm[E]);
+    float av[R], wn[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) wn[i] = lane + 32 * i < E ? __ldg(&a.wnorm[lane + 32 * i]) : 0.0f;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    /* ---- fast logits, the top_k-th of them, the candidates ---- */
+#pragma unroll
+    for (int i = 0; i < R; i++) av[i] = lane + 32 * i < E ? rc_approx(a, t, lane + 32 * i) : 0.0f;
+    /* Keys of the values with their lowest bits replaced by the index: all different,
+     * and the top_k-th of them, those bits cleared, is at most the top_k-th value. */
+    constexpr unsigned IDX = R > 8 ? 1023u : 255u;
+    unsigned kr[R], best = 0, kth = 0;
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int e = lane + 32 * i;
+        kr[i] = e < E ? (((unsigned)rc_float_key(av[i]) ^ 0x80000000u) & ~IDX) | (unsigned)e : 0u;
+        best = max(best, kr[i]);
+    }
+#pragma unroll 1
+    for (int n = 0; n < TK; n++) {
+        kth = __reduce_max_sync(0xffffffffu, best);
+        best = 0;
+#pragma unroll
+        for (int i = 0; i < R; i++)
+            if (kr[i] < kth) best = max(best, kr[i]);
+    }
+    const int wk = (int)((kth & ~IDX) ^ 0x80000000u);
+    const float a8 = __int_as_float(wk >= 0 ? wk : wk ^ 0x7fffffff);
+    const float cb = a.cbound * xnorm;
+    const float bmax = cb * wn_max;
+    /* one BF16 step at the magnitude of the values compared, rounded up */
+    const float spacing = (fabsf(a8) + bmax) * (1.0f / 64.0f) + 1e-30f;
+    const float thr = a8 - bmax - spacing;
+    int n_cand = 0;
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int e = lane + 32 * i;
+        const bool in = e < E && av[i] + cb * wn[i] >= thr;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) cand[n_cand + __popc(m & ((1u << lane) - 1u))] = (uint16_t)e;
+        /* a candidate's fast logit waits in its code's place */
+        if (e < E) cd[e] = in ? __float_as_uint(av[i]) : CODE_NEVER;
+        n_cand += __popc(m);
+    }
+    if (lane == 0) {
+        if (a.extra_row) cand[n_cand] = (uint16_t)E;
+        cd[E] = a.extra_row ? 0u : CODE_NEVER;
+    }
+    const int n_eval = n_cand + (a.extra_row ? 1 : 0);
+    __syncwarp();
     mark(1);
 
-    /* ---- exact chains, one lane per pair ---- */
-    const int npairs = s_npairs;
-    const double xmn = (double)__uint_as_float(s_xmin);
-    const bool fma_ok = (a.wmin > 0.0f) && ((double)a.wmin * xmn >= 7.52316384526264e-37) &&
-                        (!a.extra_row || ((a.wmin_extra > 0.0f) &&
-                                          ((double)a.wmin_extra * xmn >= 7.52316384526264e-37)));
-    if (warp < RC_CW) {
-        unsigned char *wb = wbuf + (size_t)warp * RC_NBUF * 32 * RC_WPITCH;
-        for (int base = warp * 32; base < npairs; base += RC_CW * 32) {
-            const int p = base + lane;
-            const bool valid = p < npairs;
-            const int pr = pairs[valid ? p : base], tl = pr >> 11, e = pr & 0x7ff;
-            const uint16_t *wrow = (e == E) ? a.extra_row : a.w + (size_t)e * K;
-            __syncwarp();                     /* the previous round is done with these */
-            s_rowptr[warp][lane] = wrow;
+    /* ---- their intervals ---- */
+    auto row_of = [&](int e) { return e == E ? a.extra_row : a.w + (size_t)e * K; };
+    int f_slot = 0;
+    auto fetch = [&](int c) {
+        if (c < n_eval)
+            lane_row_fetch(slot0 + (uint32_t)(f_slot * row_bytes), row_of(cand[c]), lr, K, lane);
+        if (++f_slot == D) f_slot = 0;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const uint16_t *xg = a.x + (size_t)t * K + (size_t)lane * lr.nu * 8;   /* NU == 0 */
+#pragma unroll 1
+    for (int c = 0; c < D; c++) fetch(c);
+    int slot = 0;
+#pragma unroll 1
+    for (int c0 = 0; c0 < n_eval; c0 += RC_BATCH) {
+        const int n = min(RC_BATCH, n_eval - c0);
+#pragma unroll 1
+        for (int c = 0; c < n; c++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
             __syncwarp();
-            const float *xr = xs + (size_t)tl * xp;
-            /* the two forms are separate instantiations of the whole loop: a
-             * branch inside it would put both on the critical path */
-            const float z = fma_ok ? rc_walk<true>(s_rowptr[warp], wb, xr, K, lane)
-                                   : rc_walk<false>(s_rowptr[warp], wb, xr, K, lane);
-            if (valid) {
-                const int t = t0 + tl;
-                if (e == E) {
-                    a.extra_out[t] = bf16_bits(z);
-                } else {
-                    if (a.logits) a.logits[(size_t)t * E + e] = bf16_bits(z);
-                    const float bound = a.cbound * s_xnorm[tl] * wn[e];
-                    if (!(fabsf(z - af[(size_t)tl * E + e]) <= bound))
-                        set_status(a.status, ST_BOUND_VIOLATED);
-                    af[(size_t)tl * E + e] = bf16_round(z);    /* the exact logit */
+            const unsigned char *wl = slots + slot * row_bytes + lane * lr.pitch;
+            if (++slot == D) slot = 0;
+            float run = 0.0f, runs = 0.0f;
+            auto eight = [&](const uint4 v, const unsigned long long *f) {
+                float wf[8];
+                unpack8(v, wf);
+                unsigned long long q;                    /* even elements, odd elements */
+                asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(pack_f32x2(wf[0], wf[1])), "l"(f[0]));
+#pragma unroll
+                for (int j = 1; j < 4; j++)
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;"
+                        : "+l"(q) : "l"(pack_f32x2(wf[2 * j], wf[2 * j + 1])), "l"(f[j]));
+                runs += fabsf(run);
+                run += __uint_as_float((unsigned)q) + __uint_as_float((unsigned)(q >> 32));
+            };
+            if (NU > 0) {
+#pragma unroll
+                for (int u = 0; u < NU; u++)
+                    eight(*reinterpret_cast<const uint4 *>(wl + u * 16), xp + u * 4);
+            } else {
+#pragma unroll 1
+                for (int u = 0; u < lr.nu; u++) {
+                    float f[8];
+                    unsigned long long fp[4];
+                    unpack8(ldg16(xg + u * 8), f);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) fp[j] = pack_f32x2(f[2 * j], f[2 * j + 1]);
+                    eight(*reinterpret_cast<const uint4 *>(wl + u * 16), fp);
                 }
             }
+            part[c * 33 + lane] = run;
+            part[(RC_BATCH + c) * 33 + lane] = runs;
+            __syncwarp();                      /* the slot is read out */
+            fetch(c0 + c + D);
         }
-    }
-    if (a.stats && tid == 0) atomicAdd(&a.stats[0], (unsigned)npairs);
-
-    /* ---- softmax / top-k on the merged logits, one warp per token ---- */
-    __syncthreads();
-    mark(2);
-    if (a.stats && blockIdx.x == 0 && tid == 0) a.stats[6] = (unsigned)npairs;
-    for (int tl = warp; tl < nt; tl += RC_THREADS / 32) {
-        float *pt = af + (size_t)tl * E;
-        for (int e = lane; e < E; e += 32) pt[e] = bf16_round(pt[e]);
+        /* Lane c: the interval of candidate c.  Error terms as in exact_sum.cuh, the
+         * lanes' sums added in order: 8 nu |sum before the lane| (+ 1 for the add)
+         * and 8 (+ 1) |running sum| per eight, 8 (+ 4: two chains of four and their
+         * sum) of the magnitudes, which Cauchy-Schwarz bounds by the norms. */
+        if (lane < n) {
+            const int e = cand[c0 + lane];
+            const float wn_e = e == E ? a.wnorm_extra : __ldg(&a.wnorm[e]);
+            float s = 0.0f, starts = 0.0f, runs = 0.0f;
+#pragma unroll 8
+            for (int l = 0; l < 32; l++) {
+                starts += fabsf(s);
+                s += part[lane * 33 + l];
+                runs += part[(RC_BATCH + lane) * 33 + l];
+            }
+            const float err = (starts * (8.0f * lr.nu + 1.0f) + 9.0f * runs +
+                               12.0f * wn_e * xnorm) * (1.05f * 5.9604645e-8f);
+            if (e < E && !(fabsf(s - __uint_as_float(cd[e])) <= cb * wn_e))
+                set_status(a.status, ST_BOUND_VIOLATED);
+            const float lo = __fadd_rd(s, -err), hi = __fadd_ru(s, err);
+            cd[e] = (e == E ? ok_extra : ok) && lo <= hi
+                        ? (uint32_t)bf16_bits(lo) | ((uint32_t)bf16_bits(hi) << 16)
+                        : CODE_UNKNOWN;
+        }
         __syncwarp();
-        const int t = t0 + tl;
-        router_softmax_topk(pt, E, a.topk, lane, a.idx_out + (size_t)t * a.topk,
-                            a.w_out ? a.w_out + (size_t)t * a.topk : nullptr);
     }
-    __syncthreads();
-    mark(3);
-}
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
 
-inline size_t router_certify_smem(int E, int K) {
-    return (size_t)RC_TT * (K + RC_XPAD) * 4 + (size_t)RC_TT * E * 4 +
-           (size_t)RC_TT * (E + 1) * 2 + 16 + (size_t)(E + 1) * 4 + 16 +
-           (size_t)RC_CW * RC_NBUF * 32 * RC_WPITCH;
+    /* ---- selection; chains where an interval leaves something open ---- */
+    int *sel = s_sel[warp];
+    Choice ch = rt_select(cd, E, TK, lane, sel);
+    if (ch.any) {
+        resolve_chains(cd, cand, n_eval, E, K, ch.kkey, ch.odd, lane,
+                       reinterpret_cast<float *>(slots), row_of,
+                       [&](int p) { return ldg16(a.x + (size_t)t * K + p * 8); });
+        if (ch.open && !ch.odd) rt_select(cd, E, TK, lane, sel);
+        __syncwarp();
+    }
+    mark(2);
+    if (a.stats && lane == 0) {
+        atomicAdd(&a.stats[0], (unsigned)n_eval);
+        if (blockIdx.x == 0 && warp == 0) a.stats[6] = (unsigned)n_eval;
+    }
+    if (a.extra_row && lane == 0) a.extra_out[t] = (uint16_t)cd[E];
+    int32_t *idx = a.idx_out + (size_t)t * TK;
+    uint16_t *wo = a.w_out ? a.w_out + (size_t)t * TK : nullptr;
+    if (ch.odd) {
+        /* the engine's softmax on the exact logits of the candidates and the rounded
+         * fast ones of the rest, which only enter its denominator */
+        float *p = reinterpret_cast<float *>(cd);
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const int e = lane + 32 * i;
+            if (e < E) p[e] = cd[e] == CODE_NEVER ? bf16_round(av[i]) : bf16lo(cd[e]);
+        }
+        __syncwarp();
+        router_softmax_topk(p, E, TK, lane, idx, wo);
+    } else {
+        rt_weights(cd, sel, TK, lane, idx, wo);
+    }
+    mark(3);
 }
 
 /* ||w_e||_2 per row, rounded up; out[E] = the largest.  One warp per row. */
@@ -416,7 +351,7 @@ row_norm_kernel(const uint16_t *__restrict__ w, int E, int K, float *__restrict_
         ss = fmaf(v, v, ss);
     }
     ss = warp_sum(ss);
-    const float n = sqrtf(ss) * 1.001f;
+    const float n = norm_above(ss, K);
     if (lane == 0) {
         out[warp] = n;
         atomicMax(reinterpret_cast<unsigned int *>(out + E), __float_as_uint(n));

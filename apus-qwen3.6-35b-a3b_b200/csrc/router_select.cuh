@@ -1,0 +1,250 @@
+/*
+ * router_select.cuh — top-k selection on logit intervals (exact_sum.cuh), shared by
+ * the one-kernel decode path and the many-token router (c/moe.h:321-371).
+ *
+ * The engine takes the top-k of its softmax PROBABILITIES.  exp and the division keep
+ * the order of the BF16 logits whenever the logits near the top differ by 2^-18 or
+ * more: two different BF16 values of one sign and of magnitude >= 2^-10 do, and so
+ * does an exact zero from any of them; probabilities above exp(-80) do not
+ * underflow.  Where that cannot be shown (`odd`), the caller runs the engine's
+ * softmax on exact logits.
+ */
+#pragma once
+#include "common.cuh"
+#include "exact_dense.cuh"
+#include "exact_sum.cuh"
+#include "router.cuh"
+
+namespace apus {
+
+/* Order-preserving 16-bit key of a BF16 code (-0 counts as +0), and back. */
+__device__ __forceinline__ uint32_t code_key(uint32_t code) {
+    code &= 0xffffu;
+    if (code == 0x8000u) code = 0;
+    return code ^ ((code & 0x8000u) ? 0xffffu : 0x8000u);
+}
+__device__ __forceinline__ float key_value(uint32_t key) {
+    return __uint_as_float((key ^ ((key & 0x8000u) ? 0x8000u : 0xffffu)) << 16);
+}
+constexpr uint32_t CODE_NEVER = 0xff80ff80u;         /* known to be -inf: out of the race */
+
+struct Choice {
+    uint32_t kkey;       /* key of the top_k-th low code */
+    bool open;           /* the set depends on an interval */
+    bool odd;            /* code order may not decide */
+    bool any;            /* some competitor (or the shared gate) is not known */
+};
+/* One warp: sel[0 .. TK-1] = the TK experts with the largest low codes cd[0 .. E-1]
+ * (lowest index first on ties).  Anything else whose high code reaches the TK-th low
+ * code may belong there instead.  cd[E]: the shared gate's. */
+__device__ __forceinline__ Choice rt_select(const uint32_t *cd, int E, int TK, int lane,
+                                            int *sel) {
+    /* keys: low code, then lowest index first; all different.  Up to 256 experts
+     * they stay in registers. */
+    constexpr int R = 8;
+    uint32_t kr[R], best = 0, kth = 0;
+    const bool regs = E <= 32 * R;
+    auto key_of = [&](int e) { return (code_key(cd[e]) << 16) | (0xffffu - (uint32_t)e); };
+    if (regs) {
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            kr[i] = lane + 32 * i < E ? key_of(lane + 32 * i) : 0u;
+            best = max(best, kr[i]);
+        }
+    } else {
+#pragma unroll 1
+        for (int e = lane; e < E; e += 32) best = max(best, key_of(e));
+    }
+#pragma unroll 1
+    for (int i = 0; i < TK; i++) {
+        kth = __reduce_max_sync(0xffffffffu, best);
+        if (lane == 0) sel[i] = (int)(0xffffu - (kth & 0xffffu));
+        if (regs) {
+            best = 0;
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (kr[j] < kth) best = max(best, kr[j]);
+        } else if (best == kth) {                        /* this lane's next one */
+            best = 0;
+            for (int e = lane; e < E; e += 32) {
+                const uint32_t k = key_of(e);
+                if (k < kth) best = max(best, k);
+            }
+        }
+    }
+    Choice c;
+    c.kkey = kth >> 16;
+    bool open = false, odd = false, any = false;
+    float top = -INFINITY;
+    uint32_t reach = 0;                                  /* bit i: expert lane + 32 i competes */
+    if (regs) {
+#pragma unroll
+        for (int i = 0; i < R; i++)
+            if (lane + 32 * i < E && code_key(cd[lane + 32 * i] >> 16) >= c.kkey) reach |= 1u << i;
+    } else {
+        for (int e = lane, i = 0; e < E; e += 32, i++)
+            if (code_key(cd[e] >> 16) >= c.kkey) reach |= 1u << i;
+    }
+    for (; reach; reach &= reach - 1) {
+        const int e = lane + 32 * (__ffs(reach) - 1);
+        const uint32_t v = cd[e];
+        const bool known = code_known(v);
+        any |= !known;
+        if (!known && key_of(e) < kth) open = true;      /* not among the chosen */
+        const float lo = bf16lo(v), hi = bf16hi(v);
+        const bool zero = known && (v & 0x7fffu) == 0;
+        const bool plain = fabsf(lo) >= 9.765625e-4f && fabsf(hi) >= 9.765625e-4f &&
+                           (lo < 0.0f) == (hi < 0.0f) && fabsf(hi) <= 32.0f;
+        if (!plain && !(zero && code_key(v) != c.kkey)) odd = true;
+        top = fmaxf(top, hi);
+    }
+    __syncwarp();
+    /* order-preserving integer of a float, for the integer reduction */
+    const int ti = __float_as_int(top);
+    const int tm = __reduce_max_sync(0xffffffffu, ti >= 0 ? ti : ti ^ 0x7fffffff);
+    top = __int_as_float(tm >= 0 ? tm : tm ^ 0x7fffffff);
+    if (!(key_value(c.kkey) - top >= -80.0f)) odd = true;
+    c.odd = __any_sync(0xffffffffu, odd);
+    c.open = __any_sync(0xffffffffu, open);
+    c.any = __any_sync(0xffffffffu, any) || c.odd || !code_known(cd[E]);
+    return c;
+}
+/* the logits that need their chain: competitors whose code is open (all of them if
+ * probabilities have to decide), and the shared gate */
+__device__ __forceinline__ bool rt_needs(const uint32_t *cd, int e, int E, uint32_t kkey,
+                                         bool odd) {
+    return e <= E && !code_known(cd[e]) && (odd || e == E || code_key(cd[e] >> 16) >= kkey);
+}
+/* One warp, all codes of the selection known: its order and the renormalised weights
+ * q_i / sum q in that order (the softmax denominator cancels; c/moe.h:363-370). */
+__device__ __forceinline__ void rt_weights(const uint32_t *cd, const int *sel, int TK, int lane,
+                                           int32_t *idx_out, uint16_t *w_out) {
+    const bool on = lane < TK;
+    const int e = on ? sel[lane] : 0;
+    const uint32_t c = cd[e] & 0xffffu;
+    const uint32_t key = on ? (code_key(c) << 16) | (0xffffu - (uint32_t)e) : 0u;
+    int rank = 0;
+    for (int i = 0; i < TK; i++) rank += __shfl_sync(0xffffffffu, key, i) > key;
+    const float m = key_value(__reduce_max_sync(0xffffffffu, key) >> 16);
+    const float q = on ? (float)exp((double)__fsub_rn(bf16lo(c), m)) : 0.0f;
+    float sw = 0.0f;
+    for (int i = 0; i < TK; i++) {
+        const int src = __ffs(__ballot_sync(0xffffffffu, on && rank == i)) - 1;
+        sw = __fadd_rn(sw, __shfl_sync(0xffffffffu, q, src));
+    }
+    if (on) {
+        idx_out[rank] = e;
+        if (w_out) w_out[rank] = bf16_bits(__fdiv_rn(q, sw));
+    }
+}
+
+/* n <= G exact chains by one warp, chain c's result in lane c.  The dependent add per
+ * step is the floor (4.6 cycles: 4.8 us for 2048 steps), and a full SM is bound by
+ * issue: unpacking both operands in the chain's lane takes four slots a step for a
+ * handful of busy lanes.  So the warp first multiplies together, a lane eight products
+ * at a time, into G rows of 256 (256 elements of each chain, or 256 G of one), then a
+ * chain's lane only loads and adds, while the next segment's operands are under way.  A
+ * product rounded to fp32 and then added IS the engine's step, whether it is exact or
+ * not.
+ * wrow(c): weight row of chain c < n (called by all lanes together); xpiece(p): 16-byte
+ * piece p of the token; buf: CH_ROW * G floats of shared memory, 16-byte aligned. */
+constexpr int CH_ROW = 256 + 4;          /* the rows of eight lanes in different banks */
+constexpr int CH_CHAINS = 8;
+constexpr int CH_BYTES = CH_CHAINS * CH_ROW * 4;
+template <int G, typename WRow, typename XPiece>
+__device__ __forceinline__ float warp_chains(int n, int K, int lane, float *buf, WRow wrow,
+                                             XPiece xpiece) {
+    const bool one = n == 1;
+    const int seg = one ? 256 * G : 256;
+    uint4 wq[G], xq[G];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            if (!one && g >= n) break;
+            const uint16_t *w = wrow(one ? 0 : g);
+            const int k = k0 + (one ? g * 256 : 0) + lane * 8;
+            wq[g] = k < K ? ldg16(w + k) : make_uint4(0, 0, 0, 0);
+            if (one || g == 0) xq[g] = k < K ? xpiece(k / 8) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    float acc = 0.0f;
+    load(0);
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += seg) {
+        float xf[8];
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            if (!one && g >= n) break;
+            if (one || g == 0) unpack8(xq[g], xf);
+            float wf[8];
+            unpack8(wq[g], wf);
+            /* the first four of every eight, then the second four: consecutive lanes
+             * write consecutive pieces */
+            float4 *d = reinterpret_cast<float4 *>(buf + g * CH_ROW) + lane;
+            d[0] = make_float4(__fmul_rn(wf[0], xf[0]), __fmul_rn(wf[1], xf[1]),
+                               __fmul_rn(wf[2], xf[2]), __fmul_rn(wf[3], xf[3]));
+            d[32] = make_float4(__fmul_rn(wf[4], xf[4]), __fmul_rn(wf[5], xf[5]),
+                                __fmul_rn(wf[6], xf[6]), __fmul_rn(wf[7], xf[7]));
+        }
+        __syncwarp();
+        if (k0 + seg < K) load(k0 + seg);
+        if (lane < n) {
+#pragma unroll 1
+            for (int r = 0, left = min(seg, K - k0) / 8; left > 0; r++, left -= 32) {
+                const float4 *s = reinterpret_cast<const float4 *>(buf + (lane + r) * CH_ROW);
+                const int last = min(left, 32) - 1;
+                float4 a0 = s[0], b0 = s[32], a1 = s[min(1, last)], b1 = s[32 + min(1, last)];
+#pragma unroll 4
+                for (int i = 0; i <= last; i++) {        /* two eights (75 cycles) ahead */
+                    const float4 a = a0, b = b0;
+                    a0 = a1;
+                    b0 = b1;
+                    a1 = s[min(i + 2, last)];
+                    b1 = s[32 + min(i + 2, last)];
+                    acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, a.x), a.y), a.z), a.w);
+                    acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, b.x), b.y), b.z), b.w);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    return acc;
+}
+/* Resolves the logits that rt_needs names of list[0 .. n-1]: their codes become known.  row(e): weight row in global memory. */
+template <typename Row, typename XPiece>
+__device__ __forceinline__ int resolve_chains(uint32_t *cd, const uint16_t *list, int n, int E,
+                                              int K, uint32_t kkey, bool odd, int lane,
+                                              float *buf, Row row, XPiece xpiece) {
+    int chains = 0;
+#pragma unroll 1
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const int e = c0 + lane < n ? list[c0 + lane] : E + 1;
+        unsigned m = __ballot_sync(0xffffffffu, rt_needs(cd, e, E, kkey, odd));
+#pragma unroll 1
+        while (m) {
+            const int now = min(__popc(m), CH_CHAINS);
+            const int src = lane < now ? __fns(m, 0, lane + 1) : 0;
+            const int mine = __shfl_sync(0xffffffffu, e, src);
+            const float z = warp_chains<CH_CHAINS>(
+                now, K, lane, buf,
+                [&](int c) { return row(__shfl_sync(0xffffffffu, mine, c)); }, xpiece);
+            if (lane < now) cd[mine] = 0x10001u * bf16_bits(z);
+            __syncwarp();
+            chains += now;
+            m &= ~__reduce_or_sync(0xffffffffu, lane < now ? 1u << src : 0u);
+        }
+    }
+    return chains;
+}
+/* a row of global memory into a LaneRow, by one warp (asynchronously; the caller
+ * commits and waits) */
+__device__ __forceinline__ void lane_row_fetch(uint32_t dst, const uint16_t *src, const LaneRow lr,
+                                               int H, int lane) {
+    for (int c = lane; c < H / 8; c += 32) cp_async16_to(dst + (uint32_t)lr.at(c), src + c * 8);
+}
+__device__ __forceinline__ void cp_async_done() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+}  // namespace apus

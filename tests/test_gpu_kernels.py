@@ -227,6 +227,36 @@ def test_router_certified_selection_is_exact(gpu, orc, be, synth, T, case):
         assert chains <= 4 * cfg["top_k"] * T
 
 
+@pytest.mark.parametrize("T,E,K,kind", [
+    (148, 256, 2048, "bias"), (149, 256, 2048, "bias"),        # one token to a CTA, then two
+    (888, 256, 2048, "plain"), (889, 256, 2048, "bias"),       # deep rings, then shallow ones
+    (65, 1024, 256, "plain"), (66, 128, 768, "bias"), (67, 384, 2304, "plain"),
+    (65, 128, 512, "subnormal"), (65, 128, 512, "ties"), (65, 1024, 512, "zero")])
+def test_router_certified_kernel_edges(gpu, orc, be, synth, T, E, K, kind):
+    """The instances of the certifying kernel on both sides of the sizes that choose
+    between them; every logit on a chain of its own (products that round, ties of all
+    experts), more of them than one pass over the products takes, and tokens of zeros."""
+    cfg = dict(hidden=K, experts=E, moe_inter=128, shared_inter=128, top_k=8)
+    W = synth.host_weights(be, cfg, seed=T + K, sigma=0.05)
+    x = synth.host_x(be, T, K, seed=T + E)
+    rtr = W["rtr_w"]
+    if kind == "bias":               # selected logits small beside their terms
+        W, x = synth.apply_router_bias(W, x, synth.zipf_bias(cfg, seed=3))
+        rtr = W["rtr_w"]
+    elif kind == "subnormal":
+        x = synth.f32_to_bf16(synth.bf16_to_f32(x) * np.float32(2.0 ** -120))
+    elif kind == "ties":
+        rtr[:] = rtr[:1]
+    elif kind == "zero":
+        x[::2] = 0
+    idx, w = _route_dev(gpu, synth, cfg, W, x)
+    assert gpu.last_block_status() == 0
+    eidx, ew = orc.route_batch(x, rtr, cfg["top_k"])
+    assert np.array_equal(idx, eidx)
+    d = np.abs(w.astype(np.int32) - ew.astype(np.int32))
+    assert d.max() <= 1 and (d != 0).mean() <= 0.002
+
+
 def test_router_certified_can_be_switched_off(be, orc, synth, monkeypatch):
     monkeypatch.setenv("APUS_CUDA_ROUTER_CERTIFY", "0")
     be.enable()
