@@ -28,6 +28,7 @@
 #include "decode_gemv.cuh"
 #include "dispatch.cuh"
 #include "ep_window.cuh"
+#include "place.cuh"
 #include "exact_dense.cuh"
 #include "host_stage.h"
 #include "misc_kernels.cuh"
@@ -678,13 +679,16 @@ struct RouterAux {
     float wmin_extra, wmax_extra, wnorm_extra;   /* the same of extra_row */
     float *approx_ws;       /* fp32 workspace, at least T*E*4 bytes */
     size_t approx_bytes;    /* its size: up to four [T, E] slabs are used */
+    /* [ceil(T / PL_UNIT)][E]: the selections counted per unit of tokens (optional) */
+    int32_t *unit_hist = nullptr;
+    bool counted = false;   /* out: they were */
 };
 
 static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
                          int E, int K, int topk, float wmin, int32_t *didx,
                          uint16_t *dw, uint16_t *dlogits,
                          const uint16_t *extra_row, uint16_t *extra_out,
-                         cudaStream_t st, const RouterAux *aux = nullptr) {
+                         cudaStream_t st, RouterAux *aux = nullptr) {
     if (E < 1 || E > 1024 || topk < 1 || topk > 32 || topk > E || K < 1)
         return fail("router: unsupported E=%d topk=%d K=%d", E, topk, K);
     /* many tokens: fast logits on the tensor cores, exact chains only for the
@@ -696,8 +700,8 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         int ksplit = dense_logits_ksplit(c->sm_count, T, E, K);
         while (ksplit > 1 && (size_t)ksplit * T * E * 4 > aux->approx_bytes) ksplit /= 2;
         if (run_dense_logits(c->sm_count, c->smem_optin, dwr, dx, T, E, K, ksplit,
-                             aux->approx_ws, c->d_status, st,
-                             &c->last_block_launches))
+                             aux->approx_ws, c->d_status, st, &c->last_block_launches,
+                             aux->unit_hist, (T + PL_UNIT - 1) / PL_UNIT * E))
             return fail("%s", prefill_last_error());
         c->launches++;
         CertifyArgs ca;
@@ -720,6 +724,8 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         ca.idx_out = didx;
         ca.w_out = dw;
         ca.extra_out = extra_out;
+        ca.unit_hist = aux->unit_hist;
+        aux->counted = aux->unit_hist != nullptr;
         ca.status = c->d_status;
         ca.stats = c->d_rc_stats;
         ca.lr = LaneRow(K);
@@ -1539,8 +1545,9 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
     c->n_ev = 0;
     stage_mark(c, -1, st);
     /* the fast logits live in the combine buffer, which is written much later */
-    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate, L->wnorm_gate, reinterpret_cast<float *>(b.eo),
-                     (size_t)Ti * TK * H * 2};
+    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate, L->wnorm_gate,
+                     reinterpret_cast<float *>(b.eo), (size_t)Ti * TK * H * 2};
+    if (prefill && Ti > PL_UNIT) aux.unit_hist = b.unit_hist;
     if (launch_router(c, d_ln2, L->rtr_w, Ti, E, H, TK, L->wmin, b.idx, b.rw,
                       b.logits, L->sh_gate, b.sgl, st,
                       (size_t)E * 4 <= (size_t)TK * H * 2 ? &aux : nullptr))
@@ -1561,9 +1568,35 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
     TilePlan plan;
     memset(&plan, 0, sizeof plan);
     if (prefill && !pair) plan = prefill_tile_plan(cfg, Ti, true, Ti * TK, b.tiles);
-    if (launch_dispatch(c, b.idx, Ti * TK, E, b.d, b.unit_hist, st, DispatchKey{0, 1},
-                        prefill && !pair ? &plan : nullptr))
+    HybridPlan hplan;
+    /* sort, tile lists and permuted copy in one kernel, where the router has counted its
+     * selections or there are few enough to count again in every CTA */
+    const bool placed = prefill && (aux.counted || Ti <= PL_UNIT) &&
+                        (((uintptr_t)d_ln2) & 15) == 0 &&
+                        (!pair || (g_pp_gather == 0 &&
+                                   hybrid_plan(cfg, Ti, true, Ti * TK, b.tiles,
+                                               prefill_tiles_bytes_for(cfg, T * TK, T), &hplan)));
+    if (placed) {
+        PlaceArgs pa;
+        memset((void *)&pa, 0, sizeof pa);
+        pa.idx = b.idx;
+        pa.unit_hist = aux.counted ? b.unit_hist : nullptr;
+        pa.x = d_ln2;
+        pa.xg = !pair && prefill_direct(Ti * TK, Ti) ? nullptr : b.xg;
+        pa.perm = b.d.perm;
+        pa.T = Ti; pa.TK = TK; pa.E = E; pa.H = H;
+        pa.tb = place_tokens(Ti, TK, c->sm_count, pa.xg != nullptr);
+        pa.status = c->d_status;
+        const dim3 grid(1 + (Ti + pa.tb - 1) / pa.tb);
+        if (pair)
+            launch_k(place_kernel<HybridPlan>, grid, dim3(PL_THREADS), 0, st, pa, hplan);
+        else
+            launch_k(place_kernel<TilePlan>, grid, dim3(PL_THREADS), 0, st, pa, plan);
+        LAUNCHED();
+    } else if (launch_dispatch(c, b.idx, Ti * TK, E, b.d, b.unit_hist, st, DispatchKey{0, 1},
+                               prefill && !pair ? &plan : nullptr)) {
         return 1;
+    }
     stage_mark(c, APUS_CUDA_STAGE_DISPATCH, st);
     if (pair) {
         const int before = c->last_block_launches;
@@ -1571,7 +1604,7 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
         if (run_pair_experts(c->sm_count, c->smem_optin, L->maps, cfg, (int)L->e_begin,
                              d_ln2, Ti, Ti * TK, TK, true, b.d, b.xg, b.act, b.sa, b.eo,
                              b.sy, b.tiles, c->d_status, st, &c->last_block_launches,
-                             mark_cb))
+                             mark_cb, nullptr, placed ? &hplan : nullptr))
             return fail("%s", prefill_last_error());
         c->launches += (uint64_t)(c->last_block_launches - before);
     } else if (prefill) {
@@ -1581,7 +1614,7 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
                                 (int)L->e_begin, d_ln2, Ti, Ti * TK, TK, true, b.d,
                                 b.xg, b.act, b.sa, b.eo, b.sy, b.tiles,
                                 c->d_status, st, &c->last_block_launches,
-                                mark_cb, plan.on ? &plan : nullptr))
+                                mark_cb, plan.on ? &plan : nullptr, nullptr, placed))
             return fail("%s", prefill_last_error());
         c->launches += (uint64_t)(c->last_block_launches - before);
     } else {
@@ -1974,7 +2007,8 @@ extern "C" int apus_cuda_ep_route_dev(ApusCudaLayer *L, const uint16_t *d_x,
     if (arena_reserve(c->ws, T * E * 18 + 8192)) return 1;
     c->ws.reset();
     uint16_t *logits = (uint16_t *)c->ws.take(T * E * 2);
-    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate, L->wnorm_gate, (float *)c->ws.take(T * E * 16),
+    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate, L->wnorm_gate,
+                     (float *)c->ws.take(T * E * 16),
                      T * E * 16};
     return launch_router(c, d_x, L->rtr_w, (int)T, (int)E, (int)L->cfg.hidden,
                          (int)L->cfg.top_k, L->wmin, d_idx, d_w, logits,

@@ -628,7 +628,8 @@ inline TilePlan pair_tile_plan(const ApusCudaMoeCfg &c, int T, bool do_shared, i
  * to the pair kernels, a smaller remainder goes to the one-SM kernels of
  * prefill_gemm.cuh, whose MMA is exactly as wide as the rows it is given.
  * Four lists: pair gate_up / down (shared-expert tiles first), one-SM gate_up /
- * down (remainders only).  One CTA of 1024 threads, thread e = expert e. */
+ * down (remainders only).  One CTA of 1024 threads, thread e = expert e, which holds its
+ * row count and first sorted position. */
 struct HybridLists {
     int4 *pair_gu, *pair_dn, *solo_gu, *solo_dn;
     int *n_pair_gu, *n_pair_dn, *n_solo_gu, *n_solo_dn;
@@ -643,13 +644,9 @@ struct HybridPlan {
     HybridLists l;
 };
 
-__global__ void __launch_bounds__(1024)
-build_hybrid_tiles_kernel(const int32_t *__restrict__ counts,
-                          const int32_t *__restrict__ offsets, int E, HybridPlan hp) {
-    pdl_enter();
+__device__ __forceinline__ void build_hybrid_body(int cnt, int off, int E, const HybridPlan &hp) {
     __shared__ int wt[3][32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int cnt = tid < E ? counts[tid] : 0, off = tid < E ? offsets[tid] : 0;
     const int full = cnt / (2 * PP_BM), rem = cnt - full * 2 * PP_BM;
     const bool rem_pair = rem > 0 && rem >= hp.solo_below;   /* never a tile without rows */
     const int n_pair = full + (rem_pair ? 1 : 0);             /* 256-row chunks */
@@ -714,6 +711,14 @@ build_hybrid_tiles_kernel(const int32_t *__restrict__ counts,
         l.sched[0] = 0;
         l.sched[1] = 0;
     }
+}
+
+__global__ void __launch_bounds__(1024)
+build_hybrid_tiles_kernel(const int32_t *__restrict__ counts,
+                          const int32_t *__restrict__ offsets, int E, HybridPlan hp) {
+    pdl_enter();
+    const int tid = threadIdx.x;
+    build_hybrid_body(tid < E ? counts[tid] : 0, tid < E ? offsets[tid] : 0, E, hp);
 }
 
 /* xg rows of the one-SM lists only (the SM pairs fetch their rows themselves):
@@ -791,15 +796,16 @@ inline cudaError_t launch_pair(void (*kernel)(KArgs...), int grid, int threads, 
 }
 
 /* Routed + shared experts through the two-SM kernels.  Same contract as
- * run_prefill_experts; the tile lists come from build_tiles_kernel with
- * pair_tile_plan's shapes. */
+ * run_prefill_experts.  placed: tile lists and the permuted copy are made already
+ * (place.cuh). */
 inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
                             const ApusCudaMoeCfg &c, int e_begin, const uint16_t *x, int T,
                             int A, int TK, bool do_shared, const DispatchOut &d,
                             uint16_t *xg, uint16_t *act, uint16_t *sa, uint16_t *eo,
                             uint16_t *sy, void *tiles_ws, int *status, cudaStream_t st,
                             int *launches, void (*mark)(int stage),
-                            const PeerRows *peer = nullptr) {
+                            const PeerRows *peer = nullptr,
+                            const HybridPlan *placed = nullptr) {
     const int H = (int)c.hidden, I = (int)c.moe_inter, Is = (int)c.shared_inter,
               E = (int)c.experts;
     if (!maps) {
@@ -813,14 +819,18 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
         return 1;
     }
     HybridPlan plan;
-    if (!hybrid_plan(c, T, do_shared, A, tiles_ws,
-                     prefill_tiles_bytes_for(c, (size_t)A, (size_t)T), &plan)) {
-        snprintf(g_prefill_err, sizeof g_prefill_err, "tile workspace too small");
-        return 1;
+    if (placed) {
+        plan = *placed;
+    } else {
+        if (!hybrid_plan(c, T, do_shared, A, tiles_ws,
+                         prefill_tiles_bytes_for(c, (size_t)A, (size_t)T), &plan)) {
+            snprintf(g_prefill_err, sizeof g_prefill_err, "tile workspace too small");
+            return 1;
+        }
+        launch_k(build_hybrid_tiles_kernel, dim3(1), dim3(1024), 0, st,
+                 (const int32_t *)d.counts, (const int32_t *)d.offsets, E, plan);
+        (*launches)++;
     }
-    launch_k(build_hybrid_tiles_kernel, dim3(1), dim3(1024), 0, st,
-             (const int32_t *)d.counts, (const int32_t *)d.offsets, E, plan);
-    (*launches)++;
     const HybridLists tl = plan.l;
     const bool solo = plan.solo_below > 0 && A > 0;
     /* the one-SM kernels read the permuted copy, so it is made whenever they run */
@@ -834,7 +844,7 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
                  TK, xg);
         (*launches)++;
     }
-    if (A > 0 && !gather && !wgather) {
+    if (A > 0 && !gather && !wgather && !placed) {
         long total = (long)A * (H / 8);
         int blocks = (int)((total + 255) / 256);
         if (blocks > sm_count * 16) blocks = sm_count * 16;

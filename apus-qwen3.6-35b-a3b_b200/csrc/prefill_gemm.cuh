@@ -296,6 +296,8 @@ struct GemmParams {
     int dense_T, dense_mt, dense_ntiles, dense_ksplit;
     float *out_f32;        /* [dense_ksplit][dense_T, ld_f32]: one slab per K slice */
     int ld_f32;
+    int32_t *zero;         /* cleared on the way, for the kernel that follows (optional) */
+    int zero_n;
 };
 
 /* the tile with this index: from the list, or (MODE 2) generated: token tile
@@ -372,6 +374,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
     /* the router's second kernel reads the tokens before its own wait, so it may not
      * start before what wrote them is complete */
     if (MODE == 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (MODE == 2)
+        for (int i = blockIdx.x * PG_THREADS + tid; i < p.zero_n; i += gridDim.x * PG_THREADS)
+            p.zero[i] = 0;
     const int n_tiles = MODE == 2 ? p.dense_ntiles : *p.n_tiles;
     const int num_kb = p.K / PG_BK;
 
@@ -796,6 +801,11 @@ inline TilePlan prefill_tile_plan(const ApusCudaMoeCfg &c, int T, bool do_shared
     return p;
 }
 
+/* a handful of tokens: the gate_up kernel reads the block input itself */
+inline bool prefill_direct(int A, int T) {
+    return A > 0 && T <= 2 * PG_BN_MIN && g_pg_direct != 0;
+}
+
 /* Routed + shared experts through the tensor-core path.  x [T,H] is the block
  * input; d holds the dispatch results; xg/act/sa/eo/sy are workspace. */
 inline int run_prefill_experts(int sm_count, int smem_optin, PrefillMaps *maps,
@@ -807,7 +817,7 @@ inline int run_prefill_experts(int sm_count, int smem_optin, PrefillMaps *maps,
                                void *tiles_ws, int *status, cudaStream_t st,
                                int *launches, void (*mark)(int stage),
                                const TilePlan *built = nullptr,
-                               const PeerRows *peer = nullptr) {
+                               const PeerRows *peer = nullptr, bool placed = false) {
     const int H = (int)c.hidden, I = (int)c.moe_inter, Is = (int)c.shared_inter,
               E = (int)c.experts;
     if (!maps) {
@@ -820,7 +830,8 @@ inline int run_prefill_experts(int sm_count, int smem_optin, PrefillMaps *maps,
                  "grouped GEMM needs %d B shared memory", s1);
         return 1;
     }
-    /* tile lists: built by the dispatch kernel already, or here */
+    /* tile lists: built by the dispatch kernel already, or here.  placed: so is the
+     * permuted copy (place.cuh) */
     TilePlan plan = prefill_tile_plan(c, T, do_shared, A, tiles_ws);
     if (built) {
         plan = *built;
@@ -835,11 +846,10 @@ inline int run_prefill_experts(int sm_count, int smem_optin, PrefillMaps *maps,
     (void)m_gu; (void)m_gu_sh; (void)m_dn;
     const bool overlap = g_pg_overlap != 0;
     const int dynamic = g_pg_dynamic;
-    /* a handful of tokens: the gate_up kernel reads the block input itself */
-    const bool direct = A > 0 && T <= 2 * PG_BN_MIN && g_pg_direct != 0 && !peer;
+    const bool direct = prefill_direct(A, T) && !peer;
     const int box_gu = direct ? (T <= PG_BN_MIN ? PG_BN_MIN : 2 * PG_BN_MIN) : bn_gu;
     /* permuted activation rows */
-    if (A > 0 && !direct) {
+    if (A > 0 && !direct && !placed) {
         long total = (long)A * (H / 8);
         int blocks = (int)((total + 255) / 256);
         if (blocks > sm_count * 16) blocks = sm_count * 16;
@@ -940,7 +950,8 @@ inline int dense_logits_ksplit(int sm_count, int T, int E, int K) {
  * E % 128 == 0, K % 64 == 0. */
 inline int run_dense_logits(int sm_count, int smem_optin, const uint16_t *w,
                             const uint16_t *x, int T, int E, int K, int ksplit,
-                            float *out, int *status, cudaStream_t st, int *launches) {
+                            float *out, int *status, cudaStream_t st, int *launches,
+                            int32_t *zero = nullptr, int zero_n = 0) {
     PFN_encodeTiled_local enc = tensor_map_encoder();
     if (!enc) return 1;
     const int smem = PG_STAGES * 2 * PG_TILE_BYTES + 1024 + 256;
@@ -969,6 +980,8 @@ inline int run_dense_logits(int sm_count, int smem_optin, const uint16_t *w,
     p.dense_ntiles = ((T + PG_BN_GU - 1) / PG_BN_GU) * p.dense_mt * ksplit;
     p.out_f32 = out;
     p.ld_f32 = E;
+    p.zero = zero;
+    p.zero_n = zero ? zero_n : 0;
     p.status = status;
     const int grid = p.dense_ntiles < sm_count ? p.dense_ntiles : sm_count;
     launch_k(grouped_gemm_kernel<2>, dim3(grid), dim3(PG_THREADS), (size_t)smem, st,

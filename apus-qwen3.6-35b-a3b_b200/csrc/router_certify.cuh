@@ -67,6 +67,7 @@ struct CertifyArgs {
     int32_t *idx_out;               /* [T, topk] selection */
     uint16_t *w_out;                /* [T, topk] renormalised weights (optional) */
     uint16_t *extra_out;            /* [T] */
+    int32_t *unit_hist;             /* [T / 256][E] += the selection (optional, place.cuh) */
     int *status;
     unsigned int *stats;            /* [0] += logits resolved exactly (optional) */
     LaneRow lr;
@@ -336,6 +337,10 @@ router_certify_kernel(const __grid_constant__ CertifyArgs a) {
         router_softmax_topk(p, E, TK, lane, idx, wo);
     } else {
         rt_weights(cd, sel, TK, lane, idx, wo);
+    }
+    if (a.unit_hist) {
+        __syncwarp();
+        if (lane < TK) atomicAdd(&a.unit_hist[(size_t)(t / 256) * E + idx[lane]], 1);
     }
     mark(3);
 }
