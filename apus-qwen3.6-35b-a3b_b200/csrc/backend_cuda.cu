@@ -1585,13 +1585,13 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
         pa.xg = !pair && prefill_direct(Ti * TK, Ti) ? nullptr : b.xg;
         pa.perm = b.d.perm;
         pa.T = Ti; pa.TK = TK; pa.E = E; pa.H = H;
-        pa.tb = place_tokens(Ti, TK, c->sm_count, pa.xg != nullptr);
+        pa.tb = place_tokens(Ti, TK, c->sm_count * (pair ? 2 : 1), pa.xg != nullptr);
         pa.status = c->d_status;
         const dim3 grid(1 + (Ti + pa.tb - 1) / pa.tb);
         if (pair)
-            launch_k(place_kernel<HybridPlan>, grid, dim3(PL_THREADS), 0, st, pa, hplan);
+            launch_k(place_kernel<HybridPlan, 2>, grid, dim3(PL_THREADS), 0, st, pa, hplan);
         else
-            launch_k(place_kernel<TilePlan>, grid, dim3(PL_THREADS), 0, st, pa, plan);
+            launch_k(place_kernel<TilePlan, 1>, grid, dim3(PL_THREADS), 0, st, pa, plan);
         LAUNCHED();
     } else if (launch_dispatch(c, b.idx, Ti * TK, E, b.d, b.unit_hist, st, DispatchKey{0, 1},
                                prefill && !pair ? &plan : nullptr)) {

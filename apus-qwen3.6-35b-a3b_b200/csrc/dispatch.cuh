@@ -107,12 +107,11 @@ __device__ __forceinline__ void build_tiles_body(int cnt, int off, int E, int T,
     }
     if (lane == 31) { warp_tot[0][warp] = inc_a; warp_tot[1][warp] = inc_b; }
     __syncthreads();
-    int base_a = 0, total_a = 0, base_b = 0, total_b = 0;
-    for (int w = 0; w < 32; w++) {
-        if (w < warp) { base_a += warp_tot[0][w]; base_b += warp_tot[1][w]; }
-        total_a += warp_tot[0][w];
-        total_b += warp_tot[1][w];
-    }
+    const int wa = warp_tot[0][lane], wb = warp_tot[1][lane];
+    const int base_a = __reduce_add_sync(0xffffffffu, lane < warp ? wa : 0),
+              base_b = __reduce_add_sync(0xffffffffu, lane < warp ? wb : 0),
+              total_a = __reduce_add_sync(0xffffffffu, wa),
+              total_b = __reduce_add_sync(0xffffffffu, wb);
     const int first_a = base_a + inc_a - nt_a, first_b = base_b + inc_b - nt_b;
     /* The shared expert is dense over the tokens (always full-width tiles) and
      * its tiles come FIRST.  They are the expensive ones — wide MMAs fed from

@@ -664,12 +664,13 @@ __device__ __forceinline__ void build_hybrid_body(int cnt, int off, int E, const
     if (lane == 31)
         for (int q = 0; q < 3; q++) wt[q][warp] = inc[q];
     __syncthreads();
-    int base[3] = {0, 0, 0}, total[3] = {0, 0, 0};
-    for (int w = 0; w < 32; w++)
-        for (int q = 0; q < 3; q++) {
-            if (w < warp) base[q] += wt[q][w];
-            total[q] += wt[q][w];
-        }
+    int base[3], total[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const int v = wt[q][lane];
+        base[q] = __reduce_add_sync(0xffffffffu, lane < warp ? v : 0);
+        total[q] = __reduce_add_sync(0xffffffffu, v);
+    }
     const int first_p = base[0] + inc[0] - n_pair, first_sg = base[1] + inc[1] - n_sg,
               first_sd = base[2] + inc[2] - n_sd;
     const int nts = (hp.T + 2 * PP_BM - 1) / (2 * PP_BM);

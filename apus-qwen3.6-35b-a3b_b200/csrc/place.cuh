@@ -42,9 +42,10 @@ __device__ __forceinline__ void build_lists(int cnt, int off, int E, const Hybri
     build_hybrid_body(cnt, off, E, hp);
 }
 
-/* grid = 1 + ceil(T / tb); thread e speaks for expert e (E <= 1024) */
-template <typename Plan>
-__global__ void __launch_bounds__(PL_THREADS)
+/* grid = 1 + ceil(T / tb); thread e speaks for expert e (E <= 1024).  PER_SM: resident
+ * CTAs; two (and 32 registers) pay where the row writes dominate, not where the lists do. */
+template <typename Plan, int PER_SM>
+__global__ void __launch_bounds__(PL_THREADS, PER_SM)
 place_kernel(const __grid_constant__ PlaceArgs a, const __grid_constant__ Plan plan) {
     __shared__ int s_tot[PL_THREADS], s_bef[PL_THREADS];     /* [parts][E padded] */
     __shared__ int s_first[PL_THREADS];
@@ -107,8 +108,8 @@ place_kernel(const __grid_constant__ PlaceArgs a, const __grid_constant__ Plan p
     }
     if (lane == 31) s_warp[warp] = inc;
     __syncthreads();
-    int off = inc - total;
-    for (int w = 0; w < warp; w++) off += s_warp[w];
+    const int off =
+        inc - total + __reduce_add_sync(0xffffffffu, lane < warp ? s_warp[lane] : 0);
     if (lists) {
         build_lists(total, off, E, plan);
         return;
@@ -151,11 +152,10 @@ place_kernel(const __grid_constant__ PlaceArgs a, const __grid_constant__ Plan p
     }
 }
 
-/* tokens of a CTA: two CTAs per SM's worth of them; without a copy as few CTAs as
- * the rank loop allows */
-inline int place_tokens(int T, int TK, int sm_count, bool copy) {
-    const int most = PL_THREADS / TK;
-    const int want = copy ? (T + 2 * sm_count - 2) / (2 * sm_count - 1) : T;
+/* tokens of a CTA: all CTAs resident at once; without a copy as few CTAs as the rank
+ * loop allows */
+inline int place_tokens(int T, int TK, int ctas, bool copy) {
+    const int most = PL_THREADS / TK, want = copy ? (T + ctas - 2) / (ctas - 1) : T;
     return want < most ? want : most;
 }
 

@@ -130,6 +130,26 @@ def test_block_one_kernel_edges(gpu, orc, be, synth, T, H, E, I, Is, TK, case):
         assert gpu.router_exact_chains() - before >= T * E
 
 
+@pytest.mark.parametrize("T,E,TK,skew", [
+    (9, 128, 8, False), (65, 128, 1, True), (255, 128, 8, True), (256, 1024, 8, False),
+    (257, 128, 8, True), (513, 256, 3, False), (300, 128, 32, True),     # counted by the router
+    (301, 100, 5, False), (1030, 36, 8, True),         # another router: not counted
+    (3100, 128, 8, True)])                             # two-SM kernels' lists
+def test_block_placement_edges(gpu, orc, be, synth, T, E, TK, skew):
+    """Sort, tile lists and permuted copy in one kernel: around its unit of 256 tokens,
+    slots per token from one to 32, the most experts, remainders of every division, and
+    the three-pass form where the router does not count."""
+    H = 256
+    cfg = dict(hidden=H, experts=E, moe_inter=128, shared_inter=128, top_k=TK)
+    W = synth.host_weights(be, cfg, seed=T + E, sigma=0.9 / H ** 0.5)
+    x = synth.host_x(be, T, H, seed=T)
+    if skew:
+        W, x = synth.apply_router_bias(W, x, synth.zipf_bias(cfg, seed=5))
+    got = gpu.moe_block(cfg, W, x)
+    assert gpu.last_block_status() == 0
+    check_block(got, orc.moe_block(cfg, W, x), f"T={T} E={E} TK={TK}")
+
+
 def test_block_batched_equals_per_token(gpu, be, synth):
     """tests/m9c of the reference: the batched body equals the per-token body.
     Here: selected ids are identical and outputs agree to BF16 tolerance when
