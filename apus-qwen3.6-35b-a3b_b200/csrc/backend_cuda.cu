@@ -237,8 +237,7 @@ static int ctx_init() {
     g_pg_direct = (int)env_long("APUS_CUDA_GEMM_DIRECT", 1);
     g_pp_enable = (int)env_long("APUS_CUDA_PAIR", 1);
     g_pp_min_rows = (int)env_long("APUS_CUDA_PAIR_MIN_ROWS", 192);
-    g_pp_gather = (int)env_long("APUS_CUDA_PAIR_GATHER", 0);
-    g_pp_solo_below = (int)env_long("APUS_CUDA_PAIR_SOLO_BELOW", 160);
+    g_pp_swap_below = (int)env_long("APUS_CUDA_PAIR_SWAP_BELOW", 192);
     c->host_split_t = env_long("APUS_CUDA_HOST_SPLIT_T", 4096);
     g_ctx = c;
     return 0;
@@ -1568,14 +1567,13 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
     TilePlan plan;
     memset(&plan, 0, sizeof plan);
     if (prefill && !pair) plan = prefill_tile_plan(cfg, Ti, true, Ti * TK, b.tiles);
-    HybridPlan hplan;
+    PairPlan hplan;
     /* sort, tile lists and permuted copy in one kernel, where the router has counted its
      * selections or there are few enough to count again in every CTA */
     const bool placed = prefill && (aux.counted || Ti <= PL_UNIT) &&
                         (((uintptr_t)d_ln2) & 15) == 0 &&
-                        (!pair || (g_pp_gather == 0 &&
-                                   hybrid_plan(cfg, Ti, true, Ti * TK, b.tiles,
-                                               prefill_tiles_bytes_for(cfg, T * TK, T), &hplan)));
+                        (!pair || pair_plan(cfg, Ti, true, Ti * TK, b.tiles,
+                                            prefill_tiles_bytes_for(cfg, T * TK, T), &hplan));
     if (placed) {
         PlaceArgs pa;
         memset((void *)&pa, 0, sizeof pa);
@@ -1589,7 +1587,7 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
         pa.status = c->d_status;
         const dim3 grid(1 + (Ti + pa.tb - 1) / pa.tb);
         if (pair)
-            launch_k(place_kernel<HybridPlan, 2>, grid, dim3(PL_THREADS), 0, st, pa, hplan);
+            launch_k(place_kernel<PairPlan, 2>, grid, dim3(PL_THREADS), 0, st, pa, hplan);
         else
             launch_k(place_kernel<TilePlan, 1>, grid, dim3(PL_THREADS), 0, st, pa, plan);
         LAUNCHED();

@@ -15,33 +15,42 @@
  * 16 KB of weights for 128 x 256 outputs: two thirds of the bytes per flop of
  * the one-SM kernel, and an expert with up to 256 rows reads its weights once.
  *
- *   gate_up:  N = 128 gate rows (CTA 0's half) | the 128 matching up rows
- *             (CTA 1's half), so every thread finds g and u of the same
- *             (token, i) in its own TMEM lane:
+ *   gate_up:  a CTA's half is 64 gate rows and the 64 matching up rows, so every
+ *             thread finds g and u of the same (token, i) in its own TMEM lane:
  *             act = rnd(rnd(silu(rnd g)) * rnd u)   routed  (c/moe.h:387-395)
  *             sa  = rnd(silu(rnd g) * rnd u)        shared  (c/moe.h:438-445)
  *   down:     N = 256 output columns h0..h0+255 (128 per CTA);
  *             y = rnd(D) stored at row perm[r] of the flat assignment-ordered
  *             buffer (the engine's eo, c/layer.h:618) or row t of sy.
  *
- * A thread owns one token row, so its outputs are contiguous: 16-byte stores.
+ * That MMA costs the same however few of its 256 rows are tokens.  So an expert's last
+ * rows, or all of them where they are few, are multiplied the other way round: the
+ * weights are M and the token rows N (a multiple of 32), which costs what the rows
+ * cost.  In that orientation g and u of a pair (token, i) sit 64 lanes apart; the
+ * epilogue warps hand u over through shared memory.  Rows behind full chunks are taken
+ * right after those, while the expert's weights are in L2; half of the pairs start with
+ * the few-row experts, half end with them, so that these, bound by memory, run beside
+ * tiles bound by the tensor cores.  (Both ran in the one-SM kernels before, after the
+ * pair kernel: weights of experts with a remainder were fetched twice.  As a second MMA
+ * beside the chunk's own, the remainder took both accumulators, and the wait for the
+ * epilogue cost more than the extra tile.)
  *
- * The kernel is bound by the bytes an SM can take in from L2 (about 38 bytes
- * per clock measured), so a tile's rows are split evenly between the two CTAs
- * and each CTA fetches a token box just tall enough for its share (32, 64, 96
- * or 128 rows): an expert with 100 rows costs each CTA 16 KB of weights and
- * 8 KB of tokens per k-block instead of 32 KB.  (The MMA always spans 256
- * rows; rows past a CTA's share hold stale data whose results are not stored.)
+ * Bound: at 64 experts of 256 rows gate_up takes 98 us, its loads alone 87, MMAs and
+ * epilogue alone 68.  What held it back before (108) was the issuing lane: flag check,
+ * barrier, descriptors, 4 MMAs and commit took 900 cycles for 512 of tensor work; now
+ * the whole warp stays together and elects a lane (pg_elect).
+ *
+ * A CTA fetches a token box just tall enough for its share (32, 64, 96 or 128 rows).
+ * Rows past a CTA's share hold stale data whose results are not stored.
  *
  * One persistent cluster of two CTAs per SM pair, 10 warps per CTA: warp 0
  * issues TMA loads (no multicast: each CTA loads its own operands; the
  * completion bytes of both CTAs are counted on the leader's barrier), warp 1 of
  * the leader CTA issues the MMAs and both warps 1 own their CTA's 512 TMEM
- * columns (two accumulator stages), warps 2-9 drain the accumulators.  Stage
- * and accumulator hand-backs from the MMA to both CTAs are tcgen05.commit with
- * a cluster mask.  Every wait is bounded; a wait that runs out raises the
- * CTA's abort flag and records a status code, and every role falls through to
- * the common exit (cluster barrier, TMEM release).
+ * columns (two accumulators), warps 2-9 drain the accumulators.  Stage and accumulator hand-backs from the MMA to both CTAs are
+ * tcgen05.commit with a cluster mask.  Every wait is bounded; a wait that runs out
+ * raises the CTA's abort flag and records a status code, and every role falls through
+ * to the common exit (cluster barrier, TMEM release).
  */
 #pragma once
 #include <cuda.h>
@@ -61,20 +70,16 @@ constexpr int PP_STAGE_BYTES = 2 * PP_HALF_BYTES;    /* tokens | weights */
 constexpr int PP_STAGES = 6;
 constexpr int PP_EPI_WARPS = 8;
 constexpr int PP_THREADS = 64 + PP_EPI_WARPS * 32;
-/* gate_up only: six more warps that fetch the token rows themselves, so that no
- * permuted copy of the block input is needed */
-constexpr int PP_GATHER_WARPS = 6;    /* == PP_STAGES: warp w serves stage w */
-constexpr int PP_THREADS_GU = PP_THREADS + PP_GATHER_WARPS * 32;
 constexpr int PP_TMEM_COLS = 512;
 constexpr uint32_t PP_PEER_MASK = 0xFEFFFFFFu;      /* cluster address of CTA 0's copy */
 
-/* down with outputs stored into peers' memory: a 32-row x 128-byte staging tile
- * per epilogue warp, so that a row leaves as 128 contiguous bytes */
+/* Behind the stages and the barriers.  gate_up: u of 32 columns x 64 rows, per half of
+ * the epilogue warps.  down with outputs stored into peers' memory: a 32-row x 128-byte
+ * staging tile per epilogue warp, so that a row leaves as 128 contiguous bytes. */
+constexpr int PP_EXCH_BYTES = 2 * 32 * 64 * 2;
 constexpr int PP_STAGING_BYTES = PP_EPI_WARPS * 4096;
 inline int pp_smem_bytes(bool staging = false) {
-    /* after the stages and the barriers: the down epilogue's staging tiles, or
-     * the gate_up gather warps' token tables (6 x 128 ints) */
-    return PP_STAGES * PP_STAGE_BYTES + 1024 + 256 + (staging ? PP_STAGING_BYTES : 3072);
+    return PP_STAGES * PP_STAGE_BYTES + (staging ? PP_STAGING_BYTES : PP_EXCH_BYTES) + 1024 + 256;
 }
 
 /* token-side tensor maps: the same tensor with boxes of 32, 64, 96, 128 rows */
@@ -88,8 +93,9 @@ __host__ __device__ __forceinline__ int pp_rows_of(int c, int rank) {
 }
 
 struct PairParams {
-    const int4 *tiles;       /* {expert or E, n-tile, first row, rows <= 256} */
-    const int *n_tiles;
+    /* {expert or E, n-tile, first row, rows: up to 256, negative where they are N} */
+    const int4 *tiles, *few;           /* few: those of the few-row experts */
+    const int *n_tiles, *n_few;
     int K;
     int E, e_begin;
     int rows_per_expert;     /* weight rows per expert in the routed tensor */
@@ -102,17 +108,41 @@ struct PairParams {
     const unsigned long long *peer_dst;
     int peer_cap;
     int *status;
-    /* gate_up: token rows of the routed tiles fetched straight from the block
-     * input by index (row perm[p] / gather_tk), four rows per TMA instruction,
-     * instead of from a permuted copy */
-    int gather_tk;           /* 0: off */
-    /* gate_up: token rows fetched by the kernel's own gather warps with plain
-     * loads (row perm[p] / wgather_tk of x for a routed tile, row p for the shared
-     * expert) and written into the stage in the layout the TMA would have
-     * produced; the TMA producer then loads weights only.  0: off */
-    int wgather_tk;
-    const uint16_t *x;       /* [T, K] block input (wgather) */
 };
+
+/* The tiles of a pair: every npairs-th of both lists, the second one dealt from the
+ * other end (so that the same pairs do not get one more of both). */
+struct PairTiles {
+    const int4 *tiles, *few;
+    int pair, npairs, n_main, n_few;
+    bool few_first;
+    int4 ahead;
+    __device__ __forceinline__ PairTiles(const PairParams &p, int pair_, int npairs_)
+        : tiles(p.tiles), few(p.few), pair(pair_), npairs(npairs_) {
+        auto mine = [&](int n, int at) { return at < n ? (n - at + npairs - 1) / npairs : 0; };
+        n_main = mine(*p.n_tiles, pair);
+        n_few = mine(*p.n_few, npairs - 1 - pair);
+        few_first = pair >= npairs / 2;
+    }
+    __device__ __forceinline__ int n() const { return n_main + n_few; }
+    __device__ __forceinline__ int4 load(int k) const {
+        if (k >= n()) return make_int4(0, 0, 0, 0);
+        const bool f = few_first ? k < n_few : k >= n_main;
+        const int i = f == few_first ? k : k - (few_first ? n_few : n_main);
+        return __ldg(f ? &few[npairs - 1 - pair + i * npairs] : &tiles[pair + i * npairs]);
+    }
+    /* k-th tile (asked for in order): its rows as M or as N.  The next one's load is
+     * under way meanwhile. */
+    __device__ __forceinline__ int4 get(int k, int &rows_m, int &rows_n) {
+        const int4 t = k ? ahead : load(0);
+        ahead = load(k + 1);
+        rows_m = max(t.w, 0);
+        rows_n = max(-t.w, 0);
+        return t;
+    }
+};
+/* columns of the MMA that has the rows as N */
+__device__ __forceinline__ int pp_cols(int rows_n) { return (rows_n + 31) & ~31; }
 
 __device__ __forceinline__ uint32_t pp_cta_rank() {
     uint32_t r;
@@ -132,20 +162,6 @@ __device__ __forceinline__ void pp_tma_load(void *dst, const CUtensorMap *map, i
         "complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar) & PP_PEER_MASK), "r"(x),
         "r"(y)
-        : "memory");
-}
-/* Four arbitrary rows of a 2-D tensor (64 columns of each) into four consecutive
- * 128-byte rows of this CTA's shared memory; the tensor map's box is 64 x 1.
- * Completion bytes go to the leader CTA's barrier, as for pp_tma_load. */
-__device__ __forceinline__ void pp_tma_gather4(void *dst, const CUtensorMap *map, int x,
-                                               int r0, int r1, int r2, int r3,
-                                               uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::"
-        "complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(
-            smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar) & PP_PEER_MASK), "r"(x),
-        "r"(r0), "r"(r1), "r"(r2), "r"(r3)
         : "memory");
 }
 __device__ __forceinline__ void pp_tmem_alloc(uint32_t *holder, uint32_t cols) {
@@ -192,36 +208,6 @@ __device__ __forceinline__ void pp_arrive_leader(uint64_t *bar) {
         "}\n" ::"r"(smem_u32(bar))
         : "memory");
 }
-/* barrier wait that also acquires what the PEER CTA's threads wrote before
- * their (cluster-scope release) arrivals */
-__device__ __forceinline__ bool pp_try_wait_cluster(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool pp_wait_cluster(uint64_t *bar, uint32_t parity,
-                                                volatile int *abort_flag, int *status,
-                                                int code) {
-    if (*abort_flag) return false;
-    for (uint32_t i = 0; i < APUS_WAIT_LIMIT; i++) {
-        if (pp_try_wait_cluster(bar, parity)) return true;
-        if (i > 256) {
-            __nanosleep(32);
-            if (*abort_flag) return false;
-        }
-    }
-    *abort_flag = 1;
-    set_status(status, code);
-    return false;
-}
 /* kind::f16 instruction descriptor: D fp32, A/B BF16, both K-major, M x N */
 __device__ __forceinline__ uint32_t pp_idesc(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
@@ -238,33 +224,29 @@ __device__ __forceinline__ void st32(uint16_t *p, const uint32_t (&v)[8]) {
 
 /* MODE 0: gate_up + SwiGLU;  MODE 1: down */
 template <int MODE>
-__global__ void __launch_bounds__(MODE == 0 ? PP_THREADS_GU : PP_THREADS, 1)
+__global__ void __launch_bounds__(PP_THREADS, 1)
 pair_gemm_kernel(const __grid_constant__ PairMaps mapA,        /* xg | act   (tokens) */
                  const __grid_constant__ PairMaps mapAs,       /* x  | sa */
                  const __grid_constant__ CUtensorMap mapB,     /* routed weights */
                  const __grid_constant__ CUtensorMap mapBs,    /* shared g | d */
                  const __grid_constant__ CUtensorMap mapBs2,   /* shared u */
-                 const __grid_constant__ CUtensorMap mapG,     /* block input, 64 x 1 boxes */
                  PairParams p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    constexpr int STAGES = PP_STAGES;
     extern __shared__ unsigned char pp_smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(pp_smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)STAGES * PP_STAGE_BYTES);
-    uint64_t *full = bars, *empty = bars + STAGES;
-    uint64_t *tfull = bars + 2 * STAGES, *tempty = tfull + 2;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)PP_STAGES * PP_STAGE_BYTES);
+    unsigned char *behind = reinterpret_cast<unsigned char *>(bars) + 256;
+    uint64_t *full = bars, *empty = bars + PP_STAGES;
+    uint64_t *tfull = bars + 2 * PP_STAGES, *tempty = tfull + 2;
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(tempty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = pp_cta_rank();
-    const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     if (tid == 0) {
-        for (int s = 0; s < STAGES; s++) {
-            /* the producer's expect_tx arrival, plus the stage's gather warp of
-             * each CTA when they bring the token rows */
-            mbar_init(&full[s], 1 + (MODE == 0 && p.wgather_tk ? 2 : 0));
+        for (int s = 0; s < PP_STAGES; s++) {
+            mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
         for (int a = 0; a < 2; a++) {
@@ -282,251 +264,164 @@ pair_gemm_kernel(const __grid_constant__ PairMaps mapA,        /* xg | act   (to
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int n_tiles = *p.n_tiles;
-    const int num_kb = p.K / PP_BK;
+    PairTiles tiles(p, blockIdx.x >> 1, gridDim.x >> 1);
+    const int n_tiles = tiles.n(), num_kb = p.K / PP_BK;
 
     if (warp == 0) {
-        /* ---------------- TMA producer (both CTAs; the whole warp when the
-         *                  token rows are gathered by index) ---------------- */
-        uint32_t kiter = 0;
+        /* ---------------- TMA producer (both CTAs) ---------------- */
+        int s = 0;
+        uint32_t ph = 0;
         bool alive = true;
-        /* operand coordinates of a tile for this CTA */
-        struct Ops {
-            const CUtensorMap *ma, *mb;
-            int arow, brow, n_mine, n0, n1;
-            bool mine, shared;
-        };
-        auto ops_of = [&](const int4 t) -> Ops {
-            Ops o;
-            o.shared = t.x == p.E;
-            /* this CTA's share of the tile's rows and the box that covers it */
-            o.n0 = pp_rows_of(t.w, 0);
-            o.n1 = pp_rows_of(t.w, 1);
-            o.n_mine = rank ? o.n1 : o.n0;
-            const int hb_mine = (o.n_mine + 31) >> 5;
-            o.ma = o.shared ? &mapAs.m[hb_mine ? hb_mine - 1 : 0]
-                            : &mapA.m[hb_mine ? hb_mine - 1 : 0];
-            if (MODE == 0) {
-                o.mb = o.shared ? (rank ? &mapBs2 : &mapBs) : &mapB;
-                o.brow = (o.shared ? 0
-                                   : (t.x - p.e_begin) * p.rows_per_expert +
-                                         (rank ? p.up_off : 0)) +
-                         t.y * 128;
-            } else {
-                o.mb = o.shared ? &mapBs : &mapB;
-                o.brow = (o.shared ? 0 : (t.x - p.e_begin) * p.rows_per_expert) +
-                         t.y * PP_BN + (int)rank * 128;
-            }
-            o.arow = t.z + (rank ? o.n0 : 0);
-            /* a CTA without a row of the tile skips the token load */
-            o.mine = o.n_mine > 0;
-            return o;
-        };
-        for (int tile = pair; alive && tile < n_tiles; tile += npairs) {
-            const Ops o = ops_of(__ldg(&p.tiles[tile]));
-            const bool gath = MODE == 0 && p.gather_tk > 0 && !o.shared;
-            const bool wg = MODE == 0 && p.wgather_tk > 0;   /* rows come from the gather warps */
-            /* lane l fetches rows 4l .. 4l+3 of this CTA's share */
-            int g4[4] = {0, 0, 0, 0};
-            const int ng_mine = (o.n_mine + 3) >> 2;
-            if (gath && lane < ng_mine) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int rr = 4 * lane + j;
-                    if (rr < o.n_mine) g4[j] = __ldg(&p.perm[o.arow + rr]) / p.gather_tk;
-                }
-            }
-            const uint32_t bytes_all =
-                (uint32_t)(2 * PP_HALF_BYTES) +
-                (wg ? 0u : gath ? (uint32_t)(((o.n0 + 3) >> 2) + ((o.n1 + 3) >> 2)) * 4u * PP_BK * 2u
-                      : (uint32_t)(((o.n0 + 31) >> 5) + ((o.n1 + 31) >> 5)) * 32u * PP_BK * 2u);
-            for (int kb = 0; alive && kb < num_kb; kb++, kiter++) {
-                const int s = kiter % STAGES;
-                const uint32_t ph = (kiter / STAGES) & 1u;
-                int ok = 1;
-                if (lane == 0)
-                    ok = pg_wait(&empty[s], ph ^ 1u, abort_flag, p.status, ST_MBAR_TIMEOUT) ? 1 : 0;
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) {
+        for (int k = 0; alive && k < n_tiles; k++) {
+            int rows_m, rows_n;
+            const int4 t = tiles.get(k, rows_m, rows_n);
+            const bool shared = t.x == p.E;
+            const PairMaps &ma = shared ? mapAs : mapA;
+            /* this CTA's share of the rows, and the box that covers it */
+            const int r0 = rows_n ? pp_cols(rows_n) / 2 : pp_rows_of(rows_m, 0),
+                      r1 = rows_n ? r0 : rows_m - r0;
+            const int h0 = (r0 + 31) >> 5, h1 = (r1 + 31) >> 5, h = rank ? h1 : h0;
+            const int arow = t.z + (rank ? r0 : 0);
+            const CUtensorMap *map_a = &ma.m[h ? h - 1 : 0];
+            const CUtensorMap *mb = shared ? &mapBs : &mapB,
+                              *mb2 = shared ? &mapBs2 : &mapB;
+            const int wrow = shared ? 0 : (t.x - p.e_begin) * p.rows_per_expert;
+            const int brow = MODE == 0 ? wrow + t.y * 128 + (int)rank * 64
+                                       : wrow + t.y * PP_BN + (int)rank * 128;
+            const int brow2 = brow + (shared ? 0 : p.up_off);
+            const uint32_t bytes = (uint32_t)(2 * PP_HALF_BYTES) +
+                                   (uint32_t)(h0 + h1) * 32u * PP_BK * 2u;
+            for (int kb = 0; kb < num_kb; kb++) {
+                if (!pg_wait_warp(&empty[s], ph ^ 1u, abort_flag, p.status, ST_MBAR_TIMEOUT)) {
                     alive = false;
                     break;
                 }
                 unsigned char *st = smem + (size_t)s * PP_STAGE_BYTES;
-                if (lane == 0) {
-                    if (rank == 0) mbar_expect_tx(&full[s], bytes_all);
-                    if (!gath && !wg && o.mine)
-                        pp_tma_load(st, o.ma, kb * PP_BK, o.arow, &full[s]);
-                    pp_tma_load(st + PP_HALF_BYTES, o.mb, kb * PP_BK, o.brow, &full[s]);
+                if (pg_elect()) {
+                    if (rank == 0) mbar_expect_tx(&full[s], bytes);
+                    /* a CTA without a row of the tile skips the token load */
+                    if (h) pp_tma_load(st, map_a, kb * PP_BK, arow, &full[s]);
+                    pp_tma_load(st + PP_HALF_BYTES, mb, kb * PP_BK, brow, &full[s]);
+                    if (MODE == 0)
+                        pp_tma_load(st + PP_HALF_BYTES + PP_HALF_BYTES / 2, mb2, kb * PP_BK,
+                                    brow2, &full[s]);
                 }
-                if (gath && lane < ng_mine)
-                    pp_tma_gather4(st + (size_t)lane * 4 * PP_BK * 2, &mapG, kb * PP_BK, g4[0],
-                                   g4[1], g4[2], g4[3], &full[s]);
-                __syncwarp();
+                if (++s == PP_STAGES) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
         }
     } else if (warp == 1) {
         /* ---------------- MMA issuer (leader CTA only) ---------------- */
-        if (rank == 0 && lane == 0) {
-            uint32_t kiter = 0;
+        if (rank == 0) {
+            int s = 0;
+            uint32_t ph = 0;
             bool alive = true;
-            const uint32_t idesc = pp_idesc(2 * PP_BM, PP_BN);
-            int it = 0;
-            for (int tile = pair; alive && tile < n_tiles; tile += npairs, it++) {
-                const int acc = it & 1;
-                const uint32_t aph = (uint32_t)(it >> 1) & 1u;
-                if (!pg_wait(&tempty[acc], aph ^ 1u, abort_flag, p.status, ST_TMEM_TIMEOUT))
+            const uint64_t desc0 = umma_smem_desc(smem_u32(smem));   /* + offset / 16 */
+            for (int k = 0; k < n_tiles; k++) {
+                int rows_m, rows_n;
+                tiles.get(k, rows_m, rows_n);
+                const uint32_t idesc = pp_idesc(2 * PP_BM, rows_n ? pp_cols(rows_n) : PP_BN);
+                /* what is M and what is N of a stage */
+                const uint64_t off_m = rows_n ? PP_HALF_BYTES >> 4 : 0,
+                               off_n = rows_n ? 0 : PP_HALF_BYTES >> 4;
+                const uint32_t acc = (uint32_t)k & 1u, d = tmem_base + acc * 256u;
+                if (!pg_wait_warp(&tempty[acc], (((uint32_t)k >> 1) & 1u) ^ 1u, abort_flag,
+                                  p.status, ST_TMEM_TIMEOUT))
                     break;
                 tc_fence_after();
-                const uint32_t d0 = tmem_base + (uint32_t)acc * 256u;
-                for (int kb = 0; kb < num_kb; kb++, kiter++) {
-                    const int s = kiter % STAGES;
-                    const uint32_t ph = (kiter / STAGES) & 1u;
-                    if (!pp_wait_cluster(&full[s], ph, abort_flag, p.status, ST_MBAR_TIMEOUT)) {
+                for (int kb = 0; kb < num_kb; kb++) {
+                    if (!pg_wait_warp(&full[s], ph, abort_flag, p.status, ST_MBAR_TIMEOUT)) {
                         alive = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + (size_t)s * PP_STAGE_BYTES);
-                    const uint64_t da = umma_smem_desc(sa);
-                    const uint64_t db = umma_smem_desc(sa + PP_HALF_BYTES);
+                    const uint64_t at = desc0 + (uint64_t)(s * (PP_STAGE_BYTES >> 4)),
+                                   dm = at + off_m, dn = at + off_n;
+                    if (pg_elect()) {
 #pragma unroll
-                    for (int k = 0; k < PP_BK / 16; k++)
-                        pp_mma(d0, da + 2u * k, db + 2u * k, idesc, (kb | k) ? 1u : 0u);
-                    pp_commit_both(&empty[s]);       /* frees the stage in both CTAs */
-                }
-                if (alive) pp_commit_both(&tfull[acc]);
-            }
-        }
-    } else if (MODE == 0 && warp >= 2 + PP_EPI_WARPS) {
-        /* ---------------- gather warps (gate_up, both CTAs) ----------------
-         * Per k-block the CTA's 128 rows x 128 bytes are fetched as 16-byte
-         * units and land at (unit ^ (row & 7)) of their row — the 128-byte
-         * swizzle the MMA's descriptor expects.  Generic-proxy writes become
-         * visible to the tensor core through fence.proxy.async in the writer,
-         * before the warp's arrival on the leader CTA's full barrier. */
-        if (p.wgather_tk > 0) {
-            /* One warp per pipeline stage: warp w brings the rows of every
-             * PP_GATHER_WARPS-th k-block into stage w, so that a warp has one
-             * k-block of cp.async in flight at a time (fence.proxy.async waits
-             * for all of a thread's outstanding copies: issuing ahead within a
-             * thread buys nothing) while the CTA has six.  Eight lanes share a
-             * row (16 bytes each, one whole 128-byte line), four rows an
-             * instruction, 32 instructions a k-block. */
-            const int gw = warp - 2 - PP_EPI_WARPS, sub = lane >> 3, ch = lane & 7;
-            int *tok = reinterpret_cast<int *>(smem + (size_t)STAGES * PP_STAGE_BYTES + 256) +
-                       gw * PP_BM;
-            const int my_tiles = pair < n_tiles ? (n_tiles - pair + npairs - 1) / npairs : 0;
-            const uint32_t total = (uint32_t)my_tiles * (uint32_t)num_kb;
-            int cur = -1, n_mine = 0;
-            const uint32_t st0 = smem_u32(smem + (size_t)gw * PP_STAGE_BYTES);
-            for (uint32_t it = (uint32_t)gw; it < total; it += PP_GATHER_WARPS) {
-                const int tile_of = (int)(it / (uint32_t)num_kb),
-                          kb = (int)(it - (uint32_t)tile_of * (uint32_t)num_kb);
-                if (tile_of != cur) {
-                    cur = tile_of;
-                    const int4 t = __ldg(&p.tiles[pair + tile_of * npairs]);
-                    const int n0 = pp_rows_of(t.w, 0);
-                    n_mine = rank ? t.w - n0 : n0;
-                    __syncwarp();
-                    for (int g = lane; g < n_mine; g += 32) {
-                        const int r = t.z + (rank ? n0 : 0) + g;
-                        tok[g] = t.x == p.E ? r : __ldg(&p.perm[r]) / p.wgather_tk;
+                        for (int j = 0; j < PP_BK / 16; j++)
+                            pp_mma(d, dm + 2u * j, dn + 2u * j, idesc, (kb | j) ? 1u : 0u);
+                        pp_commit_both(&empty[s]);   /* frees the stage in both CTAs */
                     }
-                    __syncwarp();
+                    if (++s == PP_STAGES) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
-                const uint32_t ph = (it / STAGES) & 1u;
-                int ok = 1;
-                if (lane == 0)
-                    ok = pg_wait(&empty[gw], ph ^ 1u, abort_flag, p.status, ST_MBAR_TIMEOUT) ? 1
-                                                                                             : 0;
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) break;
-                const uint16_t *col = p.x + (size_t)kb * PP_BK + ch * 8;
-#pragma unroll 8
-                for (int j = 0; j < PP_BM / 4; j++) {
-                    const int g = j * 4 + sub;
-                    if (g < n_mine)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                         st0 + (uint32_t)(g * 128 + ((ch ^ (g & 7)) << 4))),
-                                     "l"(col + (size_t)tok[g] * p.K)
-                                     : "memory");
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) pp_arrive_leader(&full[gw]);
+                if (!alive) break;
+                if (pg_elect()) pp_commit_both(&tfull[acc]);
             }
         }
     } else {
         /* ---------------- epilogue (warps 2..9, both CTAs) ---------------- */
         const int q = warp & 3;                 /* TMEM lane quarter of this warp */
         const int half = (warp - 2) >> 2;       /* which columns of the tile */
-        const int rl = q * 32 + lane;           /* this thread's row among the CTA's rows */
-        int it = 0;
-        for (int tile = pair; tile < n_tiles; tile += npairs, it++) {
-            const int4 t = __ldg(&p.tiles[tile]);
+        const int rl = q * 32 + lane;           /* this thread's TMEM lane */
+        /* a warp that gave up goes on through the tiles without reading: the others may
+         * still meet it at the barriers below */
+        bool alive = true;
+        for (int k = 0; k < n_tiles; k++) {
+            int rows_m, rows_n;
+            const int4 t = tiles.get(k, rows_m, rows_n);
             const bool shared = t.x == p.E;
-            const int acc = it & 1;
-            const uint32_t aph = (uint32_t)(it >> 1) & 1u;
-            const int n_mine = pp_rows_of(t.w, (int)rank);
-            const int r = (rank ? pp_rows_of(t.w, 0) : 0) + rl;   /* row inside the tile */
-            const bool valid = rl < n_mine;
-            int orow = t.z + r;                 /* gate_up, and the shared expert */
-            if (MODE == 1 && !shared && valid) orow = __ldg(&p.perm[t.z + r]);
-            if (!pg_wait(&tfull[acc], aph, abort_flag, p.status, ST_TMEM_TIMEOUT)) break;
-            tc_fence_after();
-            const uint32_t taddr =
-                tmem_base + (uint32_t)acc * 256u + ((uint32_t)(q * 32) << 16);
             uint16_t *out = shared ? p.out_shared : p.out_routed;
             const int ld = shared ? p.ld_shared : p.ld_routed;
-            /* a warp whose rows are all past the tile's end has nothing to read */
-            const bool any = q * 32 < n_mine;
-            if (MODE == 0) {
-                for (int c0 = half * 64; any && c0 < half * 64 + 64; c0 += 32) {
-                    uint32_t g[32], u[32];
-                    tmem_ld32(taddr + (uint32_t)c0, g);
-                    tmem_ld32(taddr + 128u + (uint32_t)c0, u);
-                    tmem_ld_wait();
-                    if (valid) {
-                        uint16_t *dst = out + (size_t)orow * ld + t.y * 128 + c0;
+            const uint32_t acc = (uint32_t)k & 1u, aph = ((uint32_t)k >> 1) & 1u;
+            const uint32_t taddr = tmem_base + acc * 256u + ((uint32_t)(q * 32) << 16);
+            if (rows_m) {
+                /* ---- tokens as M: a thread owns a token row ---- */
+                const int n_mine = pp_rows_of(rows_m, (int)rank);
+                const bool valid = rl < n_mine;
+                int orow = t.z + (rank ? pp_rows_of(rows_m, 0) : 0) + rl;
+                if (MODE == 1 && !shared && valid) orow = __ldg(&p.perm[orow]);
+                alive = alive && pg_wait_warp(&tfull[acc], aph, abort_flag, p.status,
+                                              ST_TMEM_TIMEOUT);
+                tc_fence_after();
+                /* a warp whose rows are all past the tile's end has nothing to read */
+                const bool any = alive && q * 32 < n_mine;
+                if (MODE == 0) {
+                    /* columns of a CTA's half: 64 g, 64 u */
+                    for (int c0 = 0; any && c0 < 64; c0 += 32) {
+                        uint32_t g[32], u[32];
+                        tmem_ld32(taddr + (uint32_t)(half * 128 + c0), g);
+                        tmem_ld32(taddr + (uint32_t)(half * 128 + 64 + c0), u);
+                        tmem_ld_wait();
+                        if (valid) {
+                            uint16_t *dst = out + (size_t)orow * ld + t.y * 128 + half * 64 + c0;
 #pragma unroll
-                        for (int j = 0; j < 32; j += 16) {
-                            uint32_t pk[8];
+                            for (int j = 0; j < 32; j += 16) {
+                                uint32_t pk[8];
 #pragma unroll
-                            for (int h = 0; h < 8; h++) {
-                                float g0 = __uint_as_float(g[j + 2 * h]),
-                                      g1 = __uint_as_float(g[j + 2 * h + 1]),
-                                      u0 = __uint_as_float(u[j + 2 * h]),
-                                      u1 = __uint_as_float(u[j + 2 * h + 1]);
-                                bf16_round2(g0, g1);
-                                bf16_round2(u0, u1);
-                                pk[h] = shared ? silu_mul_pack2(g0, u0, g1, u1)
-                                               : silu_act_pack2(g0, u0, g1, u1);
+                                for (int h = 0; h < 8; h++) {
+                                    float g0 = __uint_as_float(g[j + 2 * h]),
+                                          g1 = __uint_as_float(g[j + 2 * h + 1]),
+                                          u0 = __uint_as_float(u[j + 2 * h]),
+                                          u1 = __uint_as_float(u[j + 2 * h + 1]);
+                                    bf16_round2(g0, g1);
+                                    bf16_round2(u0, u1);
+                                    pk[h] = shared ? silu_mul_pack2(g0, u0, g1, u1)
+                                                   : silu_act_pack2(g0, u0, g1, u1);
+                                }
+                                st32(dst + j, pk);
                             }
-                            st32(dst + j, pk);
                         }
                     }
-                }
-            } else {
-                /* the row's home: this GPU's buffer, or the source rank's */
-                uint16_t *out_row = out + (size_t)orow * ld;
-                if (p.peer_dst && !shared && valid) {
-                    const int s = orow / p.peer_cap;
-                    out_row = reinterpret_cast<uint16_t *>(__ldg(p.peer_dst + s)) +
-                              (size_t)(orow - s * p.peer_cap) * ld;
-                }
-                if (p.peer_dst && !shared) {
+                } else if (p.peer_dst && !shared) {
                     /* A thread owns a row, so a warp's store would touch 32 rows
                      * with 32 bytes each: fine for local memory, where L2 merges
                      * sectors, poor as NVLink packets.  The warp turns its 32 x 64
                      * chunk round in shared memory (16-byte units, XOR-swizzled by
                      * row) and stores it as 128 contiguous bytes per row, four
                      * rows an instruction. */
-                    unsigned char *stg = smem + (size_t)STAGES * PP_STAGE_BYTES + 256 +
-                                         (size_t)(warp - 2) * 4096;
-                    const unsigned long long my_row =
-                        valid ? (unsigned long long)reinterpret_cast<uintptr_t>(out_row) : 0ull;
+                    unsigned char *stg = behind + (size_t)(warp - 2) * 4096;
+                    unsigned long long my_row = 0;
+                    if (valid) {
+                        const int sr = orow / p.peer_cap;
+                        my_row = __ldg(p.peer_dst + sr) +
+                                 (unsigned long long)(orow - sr * p.peer_cap) * ld * 2ull;
+                    }
                     for (int c0 = half * 128; any && c0 < half * 128 + 128; c0 += 64) {
                         uint32_t v[32], v2[32];
                         tmem_ld32(taddr + (uint32_t)c0, v);
@@ -545,8 +440,8 @@ pair_gemm_kernel(const __grid_constant__ PairMaps mapA,        /* xg | act   (to
                         }
                         __syncwarp();
 #pragma unroll
-                        for (int it = 0; it < 8; it++) {
-                            const int rr = it * 4 + (lane >> 3), ch = lane & 7;
+                        for (int i = 0; i < 8; i++) {
+                            const int rr = i * 4 + (lane >> 3), ch = lane & 7;
                             const unsigned long long rp = __shfl_sync(0xffffffffu, my_row, rr);
                             const uint4 q4 = *reinterpret_cast<const uint4 *>(
                                 stg + rr * 128 + ((ch ^ (rr & 7)) << 4));
@@ -557,21 +452,95 @@ pair_gemm_kernel(const __grid_constant__ PairMaps mapA,        /* xg | act   (to
                         }
                         __syncwarp();
                     }
-                } else
-                for (int c0 = half * 128; any && c0 < half * 128 + 128; c0 += 32) {
+                } else {
+                    for (int c0 = half * 128; any && c0 < half * 128 + 128; c0 += 32) {
+                        uint32_t v[32];
+                        tmem_ld32(taddr + (uint32_t)c0, v);
+                        tmem_ld_wait();
+                        if (valid) {
+                            uint16_t *dst = out + (size_t)orow * ld + t.y * PP_BN + c0;
+#pragma unroll
+                            for (int j = 0; j < 32; j += 16) {
+                                uint32_t pk[8];
+#pragma unroll
+                                for (int h = 0; h < 8; h++)
+                                    pk[h] = pack_bf16_rn(__uint_as_float(v[j + 2 * h]),
+                                                         __uint_as_float(v[j + 2 * h + 1]));
+                                st32(dst + j, pk);
+                            }
+                        }
+                    }
+                }
+            } else {
+                /* ---- weights as M: a thread owns a weight row, a column is a token ---- */
+                alive = alive && pg_wait_warp(&tfull[acc], aph, abort_flag, p.status,
+                                              ST_TMEM_TIMEOUT);
+                tc_fence_after();
+                for (int c0 = half * 32; c0 < rows_n; c0 += 64) {
                     uint32_t v[32];
-                    tmem_ld32(taddr + (uint32_t)c0, v);
-                    tmem_ld_wait();
-                    if (valid) {
-                        uint16_t *dst = out_row + t.y * PP_BN + c0;
+                    if (alive) {
+                        tmem_ld32(taddr + (uint32_t)c0, v);
+                        tmem_ld_wait();
+                    }
+                    if (MODE == 0) {
+                        /* lanes 0..63: g of 64 rows, 64..127: u of the same */
+                        uint32_t *ex = reinterpret_cast<uint32_t *>(behind) + half * (16 * 64) +
+                                       (q & 1) * 32 + lane;
+                        if (alive && q >= 2) {
 #pragma unroll
-                        for (int j = 0; j < 32; j += 16) {
-                            uint32_t pk[8];
+                            for (int j = 0; j < 16; j++)
+                                ex[j * 64] = pack_bf16_rn(__uint_as_float(v[2 * j]),
+                                                          __uint_as_float(v[2 * j + 1]));
+                        }
+                        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+                        if (alive && q < 2) {
+                            uint16_t *dst = out + (size_t)(t.z + c0) * ld + t.y * 128 +
+                                            (int)rank * 64 + rl;
 #pragma unroll
-                            for (int h = 0; h < 8; h++)
-                                pk[h] = pack_bf16_rn(__uint_as_float(v[j + 2 * h]),
-                                                     __uint_as_float(v[j + 2 * h + 1]));
-                            st32(dst + j, pk);
+                            for (int j = 0; j < 16; j++) {
+                                const int n = c0 + 2 * j;
+                                if (n < rows_n) {
+                                    const uint32_t uu = ex[j * 64];
+                                    float g0 = __uint_as_float(v[2 * j]),
+                                          g1 = __uint_as_float(v[2 * j + 1]);
+                                    bf16_round2(g0, g1);
+                                    const uint32_t pk =
+                                        shared ? silu_mul_pack2(g0, bf16lo(uu), g1, bf16hi(uu))
+                                               : silu_act_pack2(g0, bf16lo(uu), g1, bf16hi(uu));
+                                    dst[(size_t)(2 * j) * ld] = (uint16_t)pk;
+                                    if (n + 1 < rows_n)
+                                        dst[(size_t)(2 * j + 1) * ld] = (uint16_t)(pk >> 16);
+                                }
+                            }
+                        }
+                        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+                    } else {
+                        /* output row of each of the 32 columns: one load per lane,
+                         * handed round by shuffle */
+                        unsigned long long my_row = 0;
+                        if (c0 + lane < rows_n) {
+                            int orow = t.z + c0 + lane;
+                            if (!shared) orow = __ldg(&p.perm[orow]);
+                            if (p.peer_dst && !shared) {
+                                const int sr = orow / p.peer_cap;
+                                my_row = __ldg(p.peer_dst + sr) +
+                                         (unsigned long long)(orow - sr * p.peer_cap) * ld * 2ull;
+                            } else {
+                                my_row = (unsigned long long)reinterpret_cast<uintptr_t>(
+                                    out + (size_t)orow * ld);
+                            }
+                        }
+                        const int col = t.y * PP_BN + (int)rank * 128 + rl;
+#pragma unroll
+                        for (int j = 0; j < 32; j += 2) {
+                            uint16_t *r0 = reinterpret_cast<uint16_t *>(
+                                (uintptr_t)__shfl_sync(0xffffffffu, my_row, j));
+                            uint16_t *r1 = reinterpret_cast<uint16_t *>(
+                                (uintptr_t)__shfl_sync(0xffffffffu, my_row, j + 1));
+                            const uint32_t pk = pack_bf16_rn(__uint_as_float(v[j]),
+                                                             __uint_as_float(v[j + 1]));
+                            if (alive && r0) r0[col] = (uint16_t)pk;
+                            if (alive && r1) r1[col] = (uint16_t)(pk >> 16);
                         }
                     }
                 }
@@ -595,183 +564,117 @@ pair_gemm_kernel(const __grid_constant__ PairMaps mapA,        /* xg | act   (to
 /* ---- host side ---------------------------------------------------------------- */
 inline int g_pp_enable = 1;          /* APUS_CUDA_PAIR=0: never take this path */
 inline int g_pp_min_rows = 192;      /* mean rows per resident expert from which it is taken */
-inline int g_pp_solo_below = 160;    /* APUS_CUDA_PAIR_SOLO_BELOW: see build_hybrid_tiles_kernel
-                                      * (0: every chunk to the pair kernels) */
-inline int g_pp_gather = 0;          /* APUS_CUDA_PAIR_GATHER: how gate_up gets its token rows.
-                                      * 0: permuted copy + TMA (fastest measured);
-                                      * 1: TMA gather4 from the block input (2.4x slower:
-                                      *    32 four-row requests per k-block);
-                                      * 2: the kernel's gather warps, cp.async into the
-                                      *    swizzled stage (gate_up 1.4x slower, no copy) */
+inline int g_pp_swap_below = 192;    /* APUS_CUDA_PAIR_SWAP_BELOW: see PairPlan */
 
 inline bool pair_supported(const ApusCudaMoeCfg &c, int sm_count, int smem_optin) {
     return g_pp_enable && prefill_supported(c) && c.hidden % PP_BN == 0 &&
            sm_count >= 2 && pp_smem_bytes() <= smem_optin;
 }
 
-/* tile shapes of this path for the common tile-list builder */
-inline TilePlan pair_tile_plan(const ApusCudaMoeCfg &c, int T, bool do_shared, int A,
-                               void *tiles_ws) {
-    TilePlan p = prefill_tile_plan(c, T, do_shared, A, tiles_ws);
-    p.m_gu = (int)c.moe_inter / 128;
-    p.m_gu_sh = (int)c.shared_inter / 128;
-    p.m_dn = (int)c.hidden / PP_BN;
-    p.bn_gu = p.bn_dn = p.bn_sh_gu = p.bn_sh_dn = 2 * PP_BM;
-    return p;
-}
-
-
-/* ---- tile lists for the two-SM path ------------------------------------------
- * The pair's MMA always spans 256 token rows, so a tile with few rows wastes
- * tensor work (and, under the power cap, clock).  An expert's rows are therefore
- * cut into chunks of 256; a last chunk of at least `solo_below` rows still goes
- * to the pair kernels, a smaller remainder goes to the one-SM kernels of
- * prefill_gemm.cuh, whose MMA is exactly as wide as the rows it is given.
- * Four lists: pair gate_up / down (shared-expert tiles first), one-SM gate_up /
- * down (remainders only).  One CTA of 1024 threads, thread e = expert e, which holds its
- * row count and first sorted position. */
-struct HybridLists {
-    int4 *pair_gu, *pair_dn, *solo_gu, *solo_dn;
-    int *n_pair_gu, *n_pair_dn, *n_solo_gu, *n_solo_dn;
-    int *sched;              /* two counters of the one-SM kernels' tile hand-out */
+/* ---- tile lists ---------------------------------------------------------------
+ * An expert's rows are cut into chunks of 256, one tile per chunk and 256 weight rows
+ * (128 gate, 128 up).  A remainder of fewer than `swap_below` rows is taken as N; behind
+ * full chunks it follows them in the list, without a full chunk it goes to the list of
+ * few-row experts.  Chunks of one expert are adjacent, so its weights come from HBM
+ * once and from L2 afterwards; the shared expert's (dense over the tokens) come first.
+ * One CTA of 1024 threads, thread e = expert e, which holds its row count and first
+ * sorted position. */
+struct PairLists {
+    int4 *gu, *dn, *few_gu, *few_dn;
+    int *n_gu, *n_dn, *n_few_gu, *n_few_dn;
 };
-struct HybridPlan {
+struct PairPlan {
     int T;                   /* tokens of the shared expert (0: none) */
-    int m_gu, m_gu_sh, m_dn; /* pair N-tiles: gate_up, shared gate_up, down */
-    int sm_gu, sm_dn;        /* one-SM weight-row tiles: gate_up, down */
-    int solo_bn_gu, solo_bn_dn;   /* token rows per one-SM tile */
-    int solo_below;          /* remainders below this many rows go to the one-SM kernels */
-    HybridLists l;
+    int m_gu, m_dn;          /* weight tiles per chunk: gate_up, down */
+    int swap_below;
+    PairLists l;
+};
+struct PairCut {
+    int chunks, few;                     /* of either list */
+    __device__ __forceinline__ PairCut(int cnt, int swap_below) {
+        few = cnt > 0 && cnt < swap_below;
+        chunks = few ? 0 : (cnt + 2 * PP_BM - 1) / (2 * PP_BM);
+    }
 };
 
-__device__ __forceinline__ void build_hybrid_body(int cnt, int off, int E, const HybridPlan &hp) {
-    __shared__ int wt[3][32];
+__device__ __forceinline__ void build_pair_body(int cnt, int off, int E, const PairPlan &pp) {
+    __shared__ int wt[2][32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int full = cnt / (2 * PP_BM), rem = cnt - full * 2 * PP_BM;
-    const bool rem_pair = rem > 0 && rem >= hp.solo_below;   /* never a tile without rows */
-    const int n_pair = full + (rem_pair ? 1 : 0);             /* 256-row chunks */
-    const int solo = rem_pair ? 0 : rem;                      /* rows for the one-SM kernels */
-    const int n_sg = (solo + hp.solo_bn_gu - 1) / hp.solo_bn_gu;
-    const int n_sd = (solo + hp.solo_bn_dn - 1) / hp.solo_bn_dn;
-    int inc[3] = {n_pair, n_sg, n_sd};
+    const PairCut cut(cnt, pp.swap_below), sh(pp.T, pp.swap_below);
+    int inc[2] = {cut.chunks, cut.few};
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1)
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
+        for (int q = 0; q < 2; q++) {
             const int v = __shfl_up_sync(0xffffffffu, inc[q], d);
             if (lane >= d) inc[q] += v;
         }
     if (lane == 31)
-        for (int q = 0; q < 3; q++) wt[q][warp] = inc[q];
+        for (int q = 0; q < 2; q++) wt[q][warp] = inc[q];
     __syncthreads();
-    int base[3], total[3];
+    int base[2], total[2];
 #pragma unroll
-    for (int q = 0; q < 3; q++) {
+    for (int q = 0; q < 2; q++) {
         const int v = wt[q][lane];
         base[q] = __reduce_add_sync(0xffffffffu, lane < warp ? v : 0);
         total[q] = __reduce_add_sync(0xffffffffu, v);
     }
-    const int first_p = base[0] + inc[0] - n_pair, first_sg = base[1] + inc[1] - n_sg,
-              first_sd = base[2] + inc[2] - n_sd;
-    const int nts = (hp.T + 2 * PP_BM - 1) / (2 * PP_BM);
-    const int sh_gu = nts * hp.m_gu_sh, sh_dn = nts * hp.m_dn;
-    const HybridLists &l = hp.l;
+    const PairLists &l = pp.l;
+    /* chunk n of `rows` rows that start at `o`: entry `at` of the list */
+    auto put = [&](int4 *gu, int4 *dn, int at, int e, int o, int rows, int n) {
+        const int left = min(rows - n * 2 * PP_BM, 2 * PP_BM),
+                  w = left < pp.swap_below ? -left : left;
+        for (int m = 0; m < pp.m_gu; m++)
+            gu[at * pp.m_gu + m] = make_int4(e, m, o + n * 2 * PP_BM, w);
+        for (int m = 0; m < pp.m_dn; m++)
+            dn[at * pp.m_dn + m] = make_int4(e, m, o + n * 2 * PP_BM, w);
+    };
     if (tid < E) {
-        for (int n = 0; n < n_pair; n++) {
-            const int rows = min(2 * PP_BM, cnt - n * 2 * PP_BM), r0 = off + n * 2 * PP_BM;
-            for (int m = 0; m < hp.m_gu; m++)
-                l.pair_gu[(size_t)sh_gu + (size_t)(first_p + n) * hp.m_gu + m] =
-                    make_int4(tid, m, r0, rows);
-            for (int m = 0; m < hp.m_dn; m++)
-                l.pair_dn[(size_t)sh_dn + (size_t)(first_p + n) * hp.m_dn + m] =
-                    make_int4(tid, m, r0, rows);
-        }
-        const int s0 = off + full * 2 * PP_BM;
-        for (int m = 0; m < hp.sm_gu; m++)
-            for (int n = 0; n < n_sg; n++)
-                l.solo_gu[(size_t)first_sg * hp.sm_gu + (size_t)m * n_sg + n] = make_int4(
-                    tid, m, s0 + n * hp.solo_bn_gu, min(hp.solo_bn_gu, solo - n * hp.solo_bn_gu));
-        for (int m = 0; m < hp.sm_dn; m++)
-            for (int n = 0; n < n_sd; n++)
-                l.solo_dn[(size_t)first_sd * hp.sm_dn + (size_t)m * n_sd + n] = make_int4(
-                    tid, m, s0 + n * hp.solo_bn_dn, min(hp.solo_bn_dn, solo - n * hp.solo_bn_dn));
+        const int first = sh.chunks + base[0] + inc[0] - cut.chunks;
+        for (int n = 0; n < cut.chunks; n++) put(l.gu, l.dn, first + n, tid, off, cnt, n);
+        if (cut.few) put(l.few_gu, l.few_dn, sh.few + base[1] + inc[1] - 1, tid, off, cnt, 0);
     }
-    for (int i = tid; i < sh_gu; i += blockDim.x) {
-        const int n = i / hp.m_gu_sh, m = i - n * hp.m_gu_sh;
-        l.pair_gu[i] = make_int4(E, m, n * 2 * PP_BM, min(2 * PP_BM, hp.T - n * 2 * PP_BM));
-    }
-    for (int i = tid; i < sh_dn; i += blockDim.x) {
-        const int n = i / hp.m_dn, m = i - n * hp.m_dn;
-        l.pair_dn[i] = make_int4(E, m, n * 2 * PP_BM, min(2 * PP_BM, hp.T - n * 2 * PP_BM));
-    }
+    for (int n = tid; n < sh.chunks; n += blockDim.x) put(l.gu, l.dn, n, E, 0, pp.T, n);
     if (tid == 0) {
-        *l.n_pair_gu = sh_gu + total[0] * hp.m_gu;
-        *l.n_pair_dn = sh_dn + total[0] * hp.m_dn;
-        *l.n_solo_gu = total[1] * hp.sm_gu;
-        *l.n_solo_dn = total[2] * hp.sm_dn;
-        l.sched[0] = 0;
-        l.sched[1] = 0;
+        if (sh.few) put(l.few_gu, l.few_dn, 0, E, 0, pp.T, 0);
+        *l.n_gu = (sh.chunks + total[0]) * pp.m_gu;
+        *l.n_dn = (sh.chunks + total[0]) * pp.m_dn;
+        *l.n_few_gu = (sh.few + total[1]) * pp.m_gu;
+        *l.n_few_dn = (sh.few + total[1]) * pp.m_dn;
     }
 }
 
 __global__ void __launch_bounds__(1024)
-build_hybrid_tiles_kernel(const int32_t *__restrict__ counts,
-                          const int32_t *__restrict__ offsets, int E, HybridPlan hp) {
+build_pair_tiles_kernel(const int32_t *__restrict__ counts,
+                        const int32_t *__restrict__ offsets, int E, PairPlan pp) {
     pdl_enter();
     const int tid = threadIdx.x;
-    build_hybrid_body(tid < E ? counts[tid] : 0, tid < E ? offsets[tid] : 0, E, hp);
-}
-
-/* xg rows of the one-SM lists only (the SM pairs fetch their rows themselves):
- * every gate_up tile of weight-row tile 0 names one run of rows. */
-__global__ void __launch_bounds__(256)
-gather_solo_rows_kernel(const uint16_t *__restrict__ x, const int32_t *__restrict__ perm,
-                        const int4 *__restrict__ tiles, const int *__restrict__ n_tiles, int H,
-                        int TK, uint16_t *__restrict__ xg) {
-    pdl_enter();
-    const int n = *n_tiles, c8 = H / 8;
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
-        const int4 t = tiles[i];
-        if (t.y != 0) continue;
-        for (int j = threadIdx.x; j < t.w * c8; j += blockDim.x) {
-            const int r = t.z + j / c8, c = j % c8;
-            const int tok = perm[r] / TK;
-            reinterpret_cast<uint4 *>(xg)[(size_t)r * c8 + c] =
-                ldg16(x + (size_t)tok * H + (size_t)c * 8);
-        }
-    }
+    build_pair_body(tid < E ? counts[tid] : 0, tid < E ? offsets[tid] : 0, E, pp);
 }
 
 /* list storage inside the block's tile workspace (prefill_tiles_bytes_for) */
-inline bool hybrid_plan(const ApusCudaMoeCfg &c, int T, bool do_shared, int A, void *ws,
-                        size_t ws_bytes, HybridPlan *out) {
-    const int H = (int)c.hidden, I = (int)c.moe_inter, Is = (int)c.shared_inter,
-              E = (int)c.experts;
-    HybridPlan p;
+inline bool pair_plan(const ApusCudaMoeCfg &c, int T, bool do_shared, int A, void *ws,
+                      size_t ws_bytes, PairPlan *out) {
+    const int E = (int)c.experts;
+    PairPlan p;
     memset(&p, 0, sizeof p);
     p.T = do_shared ? T : 0;
-    p.m_gu = I / 128;
-    p.m_gu_sh = Is / 128;
-    p.m_dn = H / PP_BN;
-    p.sm_gu = I / PG_BM;
-    p.sm_dn = H / PG_BM;
-    p.solo_bn_gu = PG_BN_GU;
-    p.solo_bn_dn = PG_BN_DN;
-    p.solo_below = g_pp_solo_below;
-    const size_t chunks = (size_t)A / (2 * PP_BM) + E + (size_t)T / (2 * PP_BM) + 1;
-    const size_t n_pg = chunks * (size_t)(p.m_gu > p.m_gu_sh ? p.m_gu : p.m_gu_sh),
-                 n_pd = chunks * p.m_dn, n_sg = (size_t)E * 2 * p.sm_gu,
-                 n_sd = (size_t)E * p.sm_dn;
-    if ((n_pg + n_pd + n_sg + n_sd) * sizeof(int4) + 64 > ws_bytes) return false;
-    p.l.pair_gu = reinterpret_cast<int4 *>(ws);
-    p.l.pair_dn = p.l.pair_gu + n_pg;
-    p.l.solo_gu = p.l.pair_dn + n_pd;
-    p.l.solo_dn = p.l.solo_gu + n_sg;
-    p.l.n_pair_gu = reinterpret_cast<int *>(p.l.solo_dn + n_sd);
-    p.l.n_pair_dn = p.l.n_pair_gu + 1;
-    p.l.n_solo_gu = p.l.n_pair_gu + 2;
-    p.l.n_solo_dn = p.l.n_pair_gu + 3;
-    p.l.sched = p.l.n_pair_gu + 4;
+    p.m_gu = (int)c.moe_inter / 128;
+    p.m_dn = (int)c.hidden / PP_BN;
+    p.swap_below = g_pp_swap_below < 2 * PP_BM ? g_pp_swap_below : 2 * PP_BM;
+    const size_t chunks = (size_t)A / (2 * PP_BM) + E + (size_t)T / (2 * PP_BM) + 1,
+                 few = (size_t)E + 1;
+    const size_t n_gu = chunks * p.m_gu, n_dn = chunks * p.m_dn, n_fg = few * p.m_gu,
+                 n_fd = few * p.m_dn;
+    if ((n_gu + n_dn + n_fg + n_fd) * sizeof(int4) + 64 > ws_bytes) return false;
+    p.l.gu = reinterpret_cast<int4 *>(ws);
+    p.l.dn = p.l.gu + n_gu;
+    p.l.few_gu = p.l.dn + n_dn;
+    p.l.few_dn = p.l.few_gu + n_fg;
+    p.l.n_gu = reinterpret_cast<int *>(p.l.few_dn + n_fd);
+    p.l.n_dn = p.l.n_gu + 1;
+    p.l.n_few_gu = p.l.n_gu + 2;
+    p.l.n_few_dn = p.l.n_gu + 3;
     *out = p;
     return true;
 }
@@ -805,8 +708,7 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
                             uint16_t *xg, uint16_t *act, uint16_t *sa, uint16_t *eo,
                             uint16_t *sy, void *tiles_ws, int *status, cudaStream_t st,
                             int *launches, void (*mark)(int stage),
-                            const PeerRows *peer = nullptr,
-                            const HybridPlan *placed = nullptr) {
+                            const PeerRows *peer = nullptr, const PairPlan *placed = nullptr) {
     const int H = (int)c.hidden, I = (int)c.moe_inter, Is = (int)c.shared_inter,
               E = (int)c.experts;
     if (!maps) {
@@ -819,33 +721,21 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
                  "two-SM grouped GEMM: %d B shared memory, shared_inter == moe_inter", smem);
         return 1;
     }
-    HybridPlan plan;
+    PairPlan plan;
     if (placed) {
         plan = *placed;
     } else {
-        if (!hybrid_plan(c, T, do_shared, A, tiles_ws,
-                         prefill_tiles_bytes_for(c, (size_t)A, (size_t)T), &plan)) {
+        if (!pair_plan(c, T, do_shared, A, tiles_ws,
+                       prefill_tiles_bytes_for(c, (size_t)A, (size_t)T), &plan)) {
             snprintf(g_prefill_err, sizeof g_prefill_err, "tile workspace too small");
             return 1;
         }
-        launch_k(build_hybrid_tiles_kernel, dim3(1), dim3(1024), 0, st,
+        launch_k(build_pair_tiles_kernel, dim3(1), dim3(1024), 0, st,
                  (const int32_t *)d.counts, (const int32_t *)d.offsets, E, plan);
         (*launches)++;
     }
-    const HybridLists tl = plan.l;
-    const bool solo = plan.solo_below > 0 && A > 0;
-    /* the one-SM kernels read the permuted copy, so it is made whenever they run */
-    const bool gather = g_pp_gather == 1 && !solo && !peer;
-    /* the SM pairs' gather warps read the block input themselves; a permuted
-     * copy is made of the one-SM lists' rows only */
-    const bool wgather = g_pp_gather == 2 && !peer && A > 0;
-    if (wgather && solo) {
-        launch_k(gather_solo_rows_kernel, dim3(sm_count * 4), dim3(256), 0, st, x,
-                 (const int32_t *)d.perm, (const int4 *)tl.solo_gu, (const int *)tl.n_solo_gu, H,
-                 TK, xg);
-        (*launches)++;
-    }
-    if (A > 0 && !gather && !wgather && !placed) {
+    const PairLists &tl = plan.l;
+    if (A > 0 && !placed) {
         long total = (long)A * (H / 8);
         int blocks = (int)((total + 255) / 256);
         if (blocks > sm_count * 16) blocks = sm_count * 16;
@@ -860,13 +750,11 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
     }
     if (mark) mark(APUS_CUDA_STAGE_GATHER);
     PairMaps m_xg, m_x, m_act, m_sa;
-    CUtensorMap m_g;
-    int bad = encode_2d(maps->encode, &m_g, x, (size_t)(T > 0 ? T : 1), H, 1);
+    int bad = 0;
     for (int h = 0; h < 4; h++) {
         const int box = 32 * (h + 1);
-        bad |= encode_2d(maps->encode, &m_xg.m[h],
-                         A > 0 && !gather ? (const void *)xg : (const void *)x,
-                         (size_t)(A > 0 && !gather ? A : (T > 0 ? T : 1)), H, box);
+        bad |= encode_2d(maps->encode, &m_xg.m[h], A > 0 ? (const void *)xg : (const void *)x,
+                         (size_t)(A > 0 ? A : (T > 0 ? T : 1)), H, box);
         bad |= encode_2d(maps->encode, &m_x.m[h], x, (size_t)(T > 0 ? T : 1), H, box);
         bad |= encode_2d(maps->encode, &m_act.m[h],
                          A > 0 ? (const void *)act : (const void *)sa, (size_t)(A > 0 ? A : 1),
@@ -881,14 +769,16 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
         cudaFuncSetAttribute(pair_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              smem);
         cudaFuncSetAttribute(pair_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             pp_smem_bytes(true) <= smem_optin ? pp_smem_bytes(true) : smem);
+                             smem);
         attr_set = true;
     }
     const int grid = sm_count & ~1;
     PairParams p1;
     memset(&p1, 0, sizeof p1);
-    p1.tiles = tl.pair_gu;
-    p1.n_tiles = tl.n_pair_gu;
+    p1.tiles = tl.gu;
+    p1.n_tiles = tl.n_gu;
+    p1.few = tl.few_gu;
+    p1.n_few = tl.n_few_gu;
     p1.K = H;
     p1.E = E;
     p1.e_begin = e_begin;
@@ -900,51 +790,15 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
     p1.ld_shared = Is;
     p1.perm = d.perm;
     p1.status = status;
-    /* the one-SM kernels for the small remainders */
-    CUtensorMap s_xg, s_act;
-    GemmParams g1;
-    memset(&g1, 0, sizeof g1);
-    if (solo) {
-        const int s1 = pg_smem_bytes(true);
-        if (encode_2d(maps->encode, &s_xg, xg, (size_t)A, H, PG_BN_GU) ||
-            encode_2d(maps->encode, &s_act, act, (size_t)A, I, PG_BN_DN))
-            return 1;
-        cudaFuncSetAttribute(grouped_gemm_kernel<0>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, s1);
-        cudaFuncSetAttribute(grouped_gemm_kernel<1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, s1);
-        g1.tiles = tl.solo_gu;
-        g1.n_tiles = tl.n_solo_gu;
-        g1.K = H;
-        g1.E = E;
-        g1.e_begin = e_begin;
-        g1.rows_per_expert = 2 * I;
-        g1.up_off = I;
-        g1.out_routed = act;
-        g1.out_shared = sa;
-        g1.ld_routed = I;
-        g1.ld_shared = Is;
-        g1.status = status;
-        g1.bn_rows = PG_BN_GU;
-        g1.perm = d.perm;
-        g1.sched = tl.sched;
-    }
-    p1.gather_tk = gather && A > 0 ? TK : 0;
-    p1.wgather_tk = wgather ? TK : 0;
-    p1.x = x;
-    launch_pair(pair_gemm_kernel<0>, grid, PP_THREADS_GU, (size_t)smem, st, m_xg, m_x, maps->w_gu, maps->sh_g,
-                maps->sh_u, m_g, p1);
+    launch_pair(pair_gemm_kernel<0>, grid, PP_THREADS, (size_t)smem, st, m_xg, m_x, maps->w_gu64,
+                maps->sh_g64, maps->sh_u64, p1);
     (*launches)++;
-    if (solo) {
-        launch_k(grouped_gemm_kernel<0>, dim3(sm_count), dim3(PG_THREADS),
-                 (size_t)pg_smem_bytes(true), st, maps->w_gu, maps->sh_g, maps->sh_u, s_xg,
-                 s_xg, g1);
-        (*launches)++;
-    }
     if (mark) mark(APUS_CUDA_STAGE_GATE_UP);
     PairParams p2 = p1;
-    p2.tiles = tl.pair_dn;
-    p2.n_tiles = tl.n_pair_dn;
+    p2.tiles = tl.dn;
+    p2.n_tiles = tl.n_dn;
+    p2.few = tl.few_dn;
+    p2.n_few = tl.n_few_dn;
     p2.K = I;
     p2.rows_per_expert = H;
     p2.up_off = 0;
@@ -952,33 +806,11 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
     p2.out_shared = sy;
     p2.ld_routed = H;
     p2.ld_shared = H;
-    p2.gather_tk = 0;
-    p2.wgather_tk = 0;
     p2.peer_dst = peer ? peer->dst : nullptr;
     p2.peer_cap = peer ? peer->cap : 0;
-    launch_pair(pair_gemm_kernel<1>, grid, PP_THREADS, (size_t)smem_dn, st, m_act, m_sa, maps->w_d, maps->sh_d,
-                maps->sh_d, m_g, p2);
+    launch_pair(pair_gemm_kernel<1>, grid, PP_THREADS, (size_t)smem_dn, st, m_act, m_sa,
+                maps->w_d, maps->sh_d, maps->sh_d, p2);
     (*launches)++;
-    if (solo) {
-        GemmParams g2 = g1;
-        g2.tiles = tl.solo_dn;
-        g2.n_tiles = tl.n_solo_dn;
-        g2.K = I;
-        g2.rows_per_expert = H;
-        g2.up_off = 0;
-        g2.out_routed = eo;
-        g2.out_shared = sy;
-        g2.ld_routed = H;
-        g2.ld_shared = H;
-        g2.bn_rows = PG_BN_DN;
-        g2.sched = tl.sched + 1;
-        g2.peer_dst = p2.peer_dst;
-        g2.peer_cap = p2.peer_cap;
-        launch_k(grouped_gemm_kernel<1>, dim3(sm_count), dim3(PG_THREADS),
-                 (size_t)pg_smem_bytes(false), st, maps->w_d, maps->sh_d, maps->sh_d, s_act,
-                 s_act, g2);
-        (*launches)++;
-    }
     if (mark) mark(APUS_CUDA_STAGE_DOWN);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -38,8 +38,8 @@ __device__ __forceinline__ void build_lists(int cnt, int off, int E, const TileP
     build_tiles_body(cnt, off, E, tp.T, tp.m_gu, tp.m_gu_sh, tp.m_dn, tp.bn_gu, tp.bn_dn,
                      tp.bn_sh_gu, tp.bn_sh_dn, tp.tl);
 }
-__device__ __forceinline__ void build_lists(int cnt, int off, int E, const HybridPlan &hp) {
-    build_hybrid_body(cnt, off, E, hp);
+__device__ __forceinline__ void build_lists(int cnt, int off, int E, const PairPlan &hp) {
+    build_pair_body(cnt, off, E, hp);
 }
 
 /* grid = 1 + ceil(T / tb); thread e speaks for expert e (E <= 1024).  PER_SM: resident

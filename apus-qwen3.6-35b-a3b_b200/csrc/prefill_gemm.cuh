@@ -170,6 +170,7 @@ __device__ __forceinline__ uint32_t umma_idesc(int n) {
 __device__ __forceinline__ bool pg_wait(uint64_t *bar, uint32_t parity,
                                         volatile int *abort_flag, int *status,
                                         int code) {
+    if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
     for (uint32_t i = 0; i < APUS_WAIT_LIMIT; i++) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -181,6 +182,27 @@ __device__ __forceinline__ bool pg_wait(uint64_t *bar, uint32_t parity,
     *abort_flag = 1;
     set_status(status, code);
     return false;
+}
+/* The same by a whole warp, with one answer. */
+__device__ __forceinline__ bool pg_wait_warp(uint64_t *bar, uint32_t parity,
+                                             volatile int *abort_flag, int *status, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, pg_wait(bar, parity, abort_flag, status, code)) != 0;
+}
+/* One lane of a converged warp.  The warps that issue copies and MMAs stay together and
+ * elect a lane for each batch of them, so that addresses and descriptors are computed in
+ * uniform registers, where those instructions want them: a lone lane's issue was what
+ * bound the two-SM kernel (about 900 cycles per 64-deep block, 512 of them MMA). */
+__device__ __forceinline__ bool pg_elect() {
+    uint32_t is;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(is));
+    return is != 0;
 }
 
 inline size_t prefill_max_ntiles(size_t A, size_t T, size_t E) {
@@ -675,6 +697,7 @@ typedef CUresult (*PFN_encodeTiled_local)(
 struct PrefillMaps {
     PFN_encodeTiled_local encode = nullptr;
     CUtensorMap w_gu, sh_g, sh_u, w_d, sh_d;
+    CUtensorMap w_gu64, sh_g64, sh_u64;      /* the same, boxes of 64 rows (pair_gemm.cuh) */
 };
 
 /* cuTensorMapEncodeTiled through the runtime's driver entry-point lookup (the
@@ -734,6 +757,10 @@ inline PrefillMaps *prefill_maps_create(const ApusCudaMoeCfg &c,
     m->encode = fn;
     const size_t H = c.hidden, I = c.moe_inter, Is = c.shared_inter;
     int bad = 0;
+    bad |= encode_2d(m->encode, &m->w_gu64, n_experts ? exp_gu : sh_g,
+                     n_experts ? n_experts * 2 * I : Is, H, 64);
+    bad |= encode_2d(m->encode, &m->sh_g64, sh_g, Is, H, 64);
+    bad |= encode_2d(m->encode, &m->sh_u64, sh_u, Is, H, 64);
     if (n_experts) {
         bad |= encode_2d(m->encode, &m->w_gu, exp_gu, n_experts * 2 * I, H);
         bad |= encode_2d(m->encode, &m->w_d, exp_d, n_experts * H, I);
