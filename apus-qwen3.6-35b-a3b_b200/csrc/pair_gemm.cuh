@@ -769,7 +769,7 @@ inline int run_pair_experts(int sm_count, int smem_optin, PrefillMaps *maps,
         cudaFuncSetAttribute(pair_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              smem);
         cudaFuncSetAttribute(pair_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem);
+                             pp_smem_bytes(true) <= smem_optin ? pp_smem_bytes(true) : smem);
         attr_set = true;
     }
     const int grid = sm_count & ~1;
