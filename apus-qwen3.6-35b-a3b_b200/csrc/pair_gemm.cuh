@@ -563,7 +563,10 @@ pair_gemm_kernel(const __grid_constant__ PairMaps mapA,        /* xg | act   (to
 
 /* ---- host side ---------------------------------------------------------------- */
 inline int g_pp_enable = 1;          /* APUS_CUDA_PAIR=0: never take this path */
-inline int g_pp_min_rows = 192;      /* mean rows per resident expert from which it is taken */
+inline int g_pp_min_rows = 104;      /* mean rows per resident expert from which it is taken:
+                                      * block at 94 rows 453 us against 434 of the one-SM
+                                      * kernels (skewed: 505 against 515), at 109 471
+                                      * against 475 (533, 550), at 156 554 against 609 */
 inline int g_pp_swap_below = 192;    /* APUS_CUDA_PAIR_SWAP_BELOW: see PairPlan */
 
 inline bool pair_supported(const ApusCudaMoeCfg &c, int sm_count, int smem_optin) {

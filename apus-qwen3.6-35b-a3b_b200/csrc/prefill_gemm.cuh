@@ -493,57 +493,52 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
         }
     } else if (warp == 1) {
         /* ---------------- MMA issuer ---------------- */
-        if (lane == 0) {
-            uint32_t kiter = 0;
-            bool alive = true;
-            for (int it = 0; alive; it++) {
-                const int qs = it % PG_TQ;
-                if (!pg_wait(&tqf[qs], (uint32_t)(it / PG_TQ) & 1u, abort_flag, p.status,
-                             ST_MBAR_TIMEOUT))
-                    break;
-                const int tile = tq[qs];
-                mbar_arrive(&tqe[qs]);
-                if (tile >= n_tiles) break;
-                const int4 t = pg_tile<MODE>(p, tile);
-                const int acc = it & 1;
-                const uint32_t aph = (uint32_t)(it >> 1) & 1u;
-                const int ncols = (MODE == 0 && p.direct_tk && t.x != p.E) ? p.direct_T : t.w;
-                const int n = ((ncols + 15) >> 4) << 4;
-                const uint32_t idesc = umma_idesc(n);
-                if (!pg_wait(&tempty[acc], aph ^ 1u, abort_flag, p.status,
-                             ST_TMEM_TIMEOUT)) {
+        uint32_t s = 0, ph = 0;
+        bool alive = true;
+        const uint64_t desc0 = umma_smem_desc(smem_u32(smem));   /* + offset / 16 */
+        for (int it = 0; alive; it++) {
+            const int qs = it % PG_TQ;
+            if (!pg_wait_warp(&tqf[qs], (uint32_t)(it / PG_TQ) & 1u, abort_flag, p.status,
+                              ST_MBAR_TIMEOUT))
+                break;
+            const int tile = tq[qs];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tqe[qs]);
+            if (tile >= n_tiles) break;
+            const int4 t = pg_tile<MODE>(p, tile);
+            const int acc = it & 1;
+            const uint32_t aph = (uint32_t)(it >> 1) & 1u;
+            const int ncols = (MODE == 0 && p.direct_tk && t.x != p.E) ? p.direct_T : t.w;
+            const uint32_t idesc = umma_idesc(((ncols + 15) >> 4) << 4);
+            if (!pg_wait_warp(&tempty[acc], aph ^ 1u, abort_flag, p.status, ST_TMEM_TIMEOUT))
+                break;
+            tc_fence_after();
+            const uint32_t d0 = tmem_base + (uint32_t)acc * 256u;
+            for (int kb = 0; kb < num_kb; kb++) {
+                if (!pg_wait_warp(&full[s], ph, abort_flag, p.status, ST_MBAR_TIMEOUT)) {
                     alive = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d0 = tmem_base + (uint32_t)acc * 256u;
-                for (int kb = 0; kb < num_kb; kb++, kiter++) {
-                    const int s = kiter % STAGES;
-                    const uint32_t ph = (kiter / STAGES) & 1u;
-                    if (!pg_wait(&full[s], ph, abort_flag, p.status,
-                                 ST_MBAR_TIMEOUT)) {
-                        alive = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + (size_t)s * STAGE_BYTES);
-                    const uint64_t da = umma_smem_desc(sa);
-                    const uint64_t db = umma_smem_desc(sa + B_OFF);
+                const uint64_t da = desc0 + (uint64_t)(s * (uint32_t)(STAGE_BYTES >> 4)),
+                               da2 = da + (PG_TILE_BYTES >> 4), db = da + (B_OFF >> 4);
+                if (pg_elect()) {
 #pragma unroll
                     for (int k = 0; k < PG_BK / 16; k++) {
                         const uint32_t accum = (kb | k) ? 1u : 0u;
                         /* +32 bytes per 16-element K step (encoded >> 4) */
                         umma_bf16(d0, da + 2u * k, db + 2u * k, idesc, accum);
-                        if (GATE_UP) {
-                            const uint64_t da2 = umma_smem_desc(sa + PG_TILE_BYTES);
-                            umma_bf16(d0 + 128u, da2 + 2u * k, db + 2u * k, idesc,
-                                      accum);
-                        }
+                        if (GATE_UP)
+                            umma_bf16(d0 + 128u, da2 + 2u * k, db + 2u * k, idesc, accum);
                     }
                     umma_commit(&empty[s]);    /* frees the stage when done */
                 }
-                if (alive) umma_commit(&tfull[acc]);
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
+            if (alive && pg_elect()) umma_commit(&tfull[acc]);
         }
     } else {
         /* ---------------- epilogue (warps 2..9) ---------------- */
