@@ -417,6 +417,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
             const bool dyn = MODE != 2 && p.sched != nullptr;
             const int kclaim = num_kb > PG_CLAIM_KB ? num_kb - PG_CLAIM_KB : 0;
             int tile = blockIdx.x;
+            int4 t_next = make_int4(0, 0, 0, 0);
             for (uint32_t qi = 0; alive; qi++) {
                 const int qs = qi % PG_TQ;
                 if (!pg_wait(&tqe[qs], ((qi / PG_TQ) & 1u) ^ 1u, abort_flag, p.status,
@@ -425,7 +426,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
                 tq[qs] = tile;
                 mbar_arrive(&tqf[qs]);
                 if (tile >= n_tiles) break;
-                const int4 t = pg_tile<MODE>(p, tile);
+                const int4 t = qi ? t_next : pg_tile<MODE>(p, tile);
                 const bool shared = MODE == 2 || t.x == p.E;
                 const int kb0 = MODE == 2 ? t.x * num_kb : 0;   /* K slice */
                 const CUtensorMap *ma = shared ? &mapAs : &mapA;
@@ -487,8 +488,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
                 int kb = 0;
                 for (; alive && kb <= kclaim; kb++) alive = request(kb);
                 if (dyn) claim = atomicAdd(p.sched, 1);
-                for (; alive && kb < num_kb; kb++) alive = request(kb);
+                for (; alive && kb < num_kb - 2; kb++) alive = request(kb);
                 tile = claim + (int)gridDim.x;
+                if (tile < n_tiles) t_next = pg_tile<MODE>(p, tile);   /* arrives meanwhile */
+                for (; alive && kb < num_kb; kb++) alive = request(kb);
             }
         }
     } else if (warp == 1) {
