@@ -2607,21 +2607,6 @@ extern "C" int apus_cuda_rmsnorm_dev(const uint16_t *d_x, const uint16_t *d_w,
     return launch_rmsnorm(g_ctx, d_x, d_w, d_y, (int)T, (int)N, st);
 }
 
-template <int M>
-static int launch_gemv_stream(Ctx *c, const uint16_t *w, const uint16_t *x, uint16_t *y,
-                              size_t O, size_t K, cudaStream_t st) {
-    const size_t smem = (size_t)M * K * sizeof(float);
-    if (smem > (size_t)c->smem_optin) return fail("gemv_dev: M * K too large");
-    if (smem > 48 * 1024)
-        CU_OK(cudaFuncSetAttribute(gemv_stream_kernel<M>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    size_t blocks = (O + 15) / 16;                 /* 8 warps x 2 rows per CTA pass */
-    const size_t cap = (size_t)c->sm_count * (smem > 64 * 1024 ? 1 : (smem > 24 * 1024 ? 3 : 6));
-    if (blocks > cap) blocks = cap;
-    gemv_stream_kernel<M><<<(unsigned)blocks, 256, smem, st>>>(w, x, y, (long)O, (int)K);
-    return 0;
-}
-
 extern "C" int apus_cuda_bf16_gemv_dev(const uint16_t *d_w, const uint16_t *d_x,
                                        uint16_t *d_y, size_t M, size_t O, size_t K,
                                        void *stream) {
@@ -2632,18 +2617,23 @@ extern "C" int apus_cuda_bf16_gemv_dev(const uint16_t *d_w, const uint16_t *d_x,
     if (ctx_init()) return 1;
     Ctx *c = g_ctx;
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = 1;
-    switch (M) {
-        case 1: rc = launch_gemv_stream<1>(c, d_w, d_x, d_y, O, K, st); break;
-        case 2: rc = launch_gemv_stream<2>(c, d_w, d_x, d_y, O, K, st); break;
-        case 3: rc = launch_gemv_stream<3>(c, d_w, d_x, d_y, O, K, st); break;
-        case 4: rc = launch_gemv_stream<4>(c, d_w, d_x, d_y, O, K, st); break;
-        case 5: rc = launch_gemv_stream<5>(c, d_w, d_x, d_y, O, K, st); break;
-        case 6: rc = launch_gemv_stream<6>(c, d_w, d_x, d_y, O, K, st); break;
-        case 7: rc = launch_gemv_stream<7>(c, d_w, d_x, d_y, O, K, st); break;
-        default: rc = launch_gemv_stream<8>(c, d_w, d_x, d_y, O, K, st); break;
+    /* as many warps as keep every SM busy, at most what fits beside x */
+    const size_t groups = (O + 15) / 16;
+    int warps = 8;
+    while (warps > 1 && (groups <= (size_t)c->sm_count * (warps / 2) ||
+                         gemv_stream_smem((int)M, (int)K, warps) > (size_t)c->smem_optin))
+        warps /= 2;
+    const size_t smem = gemv_stream_smem((int)M, (int)K, warps);
+    if (smem > (size_t)c->smem_optin) return fail("gemv_dev: M * K too large");
+    static size_t set_smem = 0;
+    if (smem > set_smem) {
+        CU_OK(cudaFuncSetAttribute(gemv_stream_kernel,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        set_smem = smem;
     }
-    if (rc) return 1;
+    const size_t want = (groups + warps - 1) / warps;
+    const unsigned grid = (unsigned)(want < (size_t)c->sm_count ? want : (size_t)c->sm_count);
+    gemv_stream_kernel<<<grid, warps * 32, smem, st>>>(d_w, d_x, d_y, (int)M, (long)O, (int)K);
     LAUNCHED();
     return 0;
 }

@@ -178,22 +178,6 @@ __device__ __forceinline__ void df_bar_helper_arrive() {
 __device__ __forceinline__ void df_bar_helper_wait() {
     asm volatile("bar.sync 2, %0;" ::"n"(DF_THREADS) : "memory");
 }
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr)
-                 : "memory");
-}
-/* D[16 x 8] += A[16 x 16] B[16 x 8], BF16 in, fp32 accumulate */
-__device__ __forceinline__ void mma_16x8(float (&c)[4], const uint32_t (&a)[4], uint32_t b_lo,
-                                         uint32_t b_hi) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, "
-        "{%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b_lo), "r"(b_hi));
-}
-
 __global__ void __launch_bounds__(DF_THREADS, 1)
 decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     extern __shared__ __align__(128) unsigned char df_smem[];

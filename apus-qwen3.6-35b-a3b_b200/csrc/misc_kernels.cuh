@@ -62,56 +62,112 @@ exact_matvec_f32_kernel(const uint16_t *__restrict__ w,
 
 /* y[m,o] = rnd(sum_k W[o,k] x[m,k]) as a weight STREAM (the engine's largest
  * dense product per token is the output head, 248320 x 2048 = 1 GB of weights,
- * c/model.h:667-688): device pointers, one warp per pair of weight rows, 16-byte
- * coalesced loads with eight in flight per lane, the M <= 8 activation rows in
- * shared memory as fp32, lane-strided fp32 partial sums closed by shuffles.
+ * c/model.h:667-688): device pointers, M <= 8 rows of x, K % 256 == 0.
+ *
+ * Bound: the weight stream.  A warp owns 16 weight rows at a time and copies 128 k of
+ * them per slot into a ring of its own (cp.async, whole 256-byte pieces of a row), four
+ * slots ahead; mma.sync m16n8k16 multiplies them with all rows of x at once (columns past
+ * M repeat the last row and are not stored), so eight rows cost what one does.  Scalar
+ * multiply-adds on rows loaded straight into registers took 179 us for one row and 783 for
+ * eight (O 248320, K 2048); this 174 and 182 (5.9 of 6.5 TB/s).
  * The summation order differs from the engine's sequential chain, so the result
- * agrees to BF16 tolerance, not bitwise; the exact-order form is
- * exact_gemm_kernel behind the host-pointer hooks. */
-template <int M>
+ * agrees to BF16 tolerance, not bitwise; the exact-order form is exact_dense.cuh
+ * behind the host-pointer hooks. */
+constexpr int GV_BK = 128;
+constexpr int GV_PITCH = GV_BK * 2 + 16;         /* ldmatrix rows in different banks */
+constexpr int GV_SLOT = 16 * GV_PITCH;
+constexpr int GV_STAGES = 5;
+inline size_t gemv_stream_smem(int M, int K, int warps) {
+    return (size_t)M * (2 * (size_t)K + 16) + (size_t)warps * GV_STAGES * GV_SLOT;
+}
+
 __global__ void __launch_bounds__(256)
 gemv_stream_kernel(const uint16_t *__restrict__ w, const uint16_t *__restrict__ x,
-                   uint16_t *__restrict__ y, long O, int K) {
-    extern __shared__ float gs_x[];          /* [M][K] */
-    for (int i = threadIdx.x; i < M * K; i += blockDim.x) gs_x[i] = bf16_f32(x[i]);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-    for (long o0 = warp * 2; o0 < O; o0 += nwarps * 2) {
-        const bool two = o0 + 1 < O;
-        const uint16_t *r0 = w + o0 * K, *r1 = w + (two ? o0 + 1 : o0) * K;
-        float a0[M], a1[M];
+                   uint16_t *__restrict__ y, int M, long O, int K) {
+    extern __shared__ __align__(16) unsigned char gv_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int x_pitch = 2 * K + 16;
+    const uint32_t ring = smem_u32(gv_smem) + (uint32_t)(M * x_pitch + warp * GV_STAGES * GV_SLOT);
+    /* Sixteen rows per warp and round, the warps side by side; what the last whole round
+     * leaves is dealt evenly, in pieces of fewer rows (those missing are not fetched, what
+     * lies in their place is not stored). */
+    const long nw = (long)gridDim.x * warps, id = (long)warp * gridDim.x + blockIdx.x;
+    const long rounds = O / (16 * nw), base = rounds * 16 * nw, left = O - base;
+    const long rest0 = base + left * id / nw, rest1 = base + left * (id + 1) / nw;
+    auto first = [&](long i) { return i < rounds ? (i * nw + id) * 16 : rest0; };
+    auto end = [&](long i) { return i < rounds ? (i * nw + id) * 16 + 16 : rest1; };
+    const long mine = rounds + (rest1 > rest0 ? 1 : 0);
+    const int nkb = K / GV_BK;
+    long i_i = 0;
+    int i_kb = 0, i_s = 0;
+    auto issue = [&]() {
+        if (i_i < mine) {
+            const long i_o = first(i_i), i_end = end(i_i);
+            const int c = lane & 15;
+            const uint32_t dst = ring + (uint32_t)(i_s * GV_SLOT + c * 16);
 #pragma unroll
-        for (int m = 0; m < M; m++) a0[m] = a1[m] = 0.0f;
-#pragma unroll 4
-        for (int k = lane * 8; k < K; k += 256) {
-            const uint4 v0 = ldg16(r0 + k), v1 = ldg16(r1 + k);
-            const float f0[8] = {bf16lo(v0.x), bf16hi(v0.x), bf16lo(v0.y), bf16hi(v0.y),
-                                 bf16lo(v0.z), bf16hi(v0.z), bf16lo(v0.w), bf16hi(v0.w)};
-            const float f1[8] = {bf16lo(v1.x), bf16hi(v1.x), bf16lo(v1.y), bf16hi(v1.y),
-                                 bf16lo(v1.z), bf16hi(v1.z), bf16lo(v1.w), bf16hi(v1.w)};
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                const float4 xa = *reinterpret_cast<const float4 *>(gs_x + (size_t)m * K + k);
-                const float4 xb = *reinterpret_cast<const float4 *>(gs_x + (size_t)m * K + k + 4);
-                const float xf[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    a0[m] = fmaf(f0[j], xf[j], a0[m]);
-                    a1[m] = fmaf(f1[j], xf[j], a1[m]);
-                }
+            for (int j = 0; j < 8; j++) {
+                const int r = j * 2 + (lane >> 4);
+                const long o = i_o + r;
+                if (o < i_end)
+                    cp_async16_to(dst + (uint32_t)(r * GV_PITCH),
+                                  w + o * K + i_kb * GV_BK + c * 8);
             }
+            if (++i_kb == nkb) {
+                i_kb = 0;
+                i_i++;
+            }
+            if (++i_s == GV_STAGES) i_s = 0;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int s = 0; s < GV_STAGES - 1; s++) issue();
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        for (int m = 0; m < M; m++)
+            for (int p = threadIdx.x; p < K / 8; p += blockDim.x)
+                *reinterpret_cast<uint4 *>(gv_smem + (size_t)m * x_pitch + p * 16) =
+                    ldg16(x + (size_t)m * K + p * 8);
+    } else {
+        for (int m = 0; m < M; m++)
+            for (int k = threadIdx.x; k < K; k += blockDim.x)
+                *reinterpret_cast<uint16_t *>(gv_smem + (size_t)m * x_pitch + k * 2) =
+                    x[(size_t)m * K + k];
+    }
+    __syncthreads();
+    /* ldmatrix: weights (rows 0-7, k 0-7), (rows 8-15, k 0-7), (rows 0-7, k 8-15), ..;
+     * x: eight k of the eight columns per matrix, 32 k at a time */
+    const uint32_t a_off = (uint32_t)((lane & 15) * GV_PITCH + (lane >> 4) * 16);
+    const uint32_t b_at = smem_u32(gv_smem) + (uint32_t)(min(lane & 7, M - 1) * x_pitch +
+                                                         (lane >> 3) * 16);
+    int s = 0;
+    for (long i = 0; i < mine; i++) {
+        const long o0 = first(i), o_end = end(i);
+        float c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
+#pragma unroll 1
+        for (int kb = 0; kb < nkb; kb++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(GV_STAGES - 2) : "memory");
+            __syncwarp();      /* everyone's pieces landed; the oldest slot is read out */
+            issue();
+            const uint32_t at = ring + (uint32_t)(s * GV_SLOT) + a_off;
+#pragma unroll
+            for (int k = 0; k < GV_BK; k += 32) {
+                uint32_t a0[4], a1[4], b[4];
+                ldmatrix_x4(b, b_at + (uint32_t)((kb * GV_BK + k) * 2));
+                ldmatrix_x4(a0, at + (uint32_t)(k * 2));
+                ldmatrix_x4(a1, at + (uint32_t)(k * 2 + 32));
+                mma_16x8(c0, a0, b[0], b[1]);
+                mma_16x8(c1, a1, b[2], b[3]);
+            }
+            if (++s == GV_STAGES) s = 0;
         }
 #pragma unroll
-        for (int m = 0; m < M; m++) {
-            const float s0 = warp_sum(a0[m]), s1 = warp_sum(a1[m]);
-            if (lane == 0) {
-                y[(size_t)m * O + o0] = bf16_bits(s0);
-                if (two) y[(size_t)m * O + o0 + 1] = bf16_bits(s1);
-            }
+        for (int q = 0; q < 4; q++) {
+            const long o = o0 + (lane >> 2) + (q >> 1) * 8;
+            const int m = (lane & 3) * 2 + (q & 1);
+            if (o < o_end && m < M) y[(size_t)m * O + o] = bf16_bits(c0[q] + c1[q]);
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 /* RMSNorm with (1+w) gain, single rounding (c/attn.h:175-186): the sum of

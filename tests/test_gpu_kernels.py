@@ -328,6 +328,31 @@ def test_rmsnorm_sum_without_the_chain(gpu, orc, N):
 
 # ---- the dense weight stream on device pointers --------------------------------
 
+@pytest.mark.parametrize("M,O,K,shift", [
+    (1, 15, 256, 0), (5, 16, 512, 0), (7, 17, 2304, 0), (8, 148 * 16, 256, 0),
+    (4, 148 * 16 * 8 + 5, 256, 0), (6, 148 * 16 * 8 * 2 - 1, 256, 0), (2, 31, 16384, 0),
+    (8, 40, 7168, 0), (3, 100, 512, 1)])
+def test_gemv_stream_edges(gpu, orc, M, O, K, shift):
+    """Whole rounds, remainders and fewer rows than warps; x beside a smaller ring; x that
+    is not 16-byte aligned.  Both sums are fp32 over K exact products: they differ by at
+    most 2 K 2^-24 of the sum of magnitudes, and each narrows to BF16 (2^-8)."""
+    import torch
+    rng = np.random.default_rng(M * 1000 + O)
+    w, x = rng_codes(rng, (O, K), 0.05), rng_codes(rng, (M, K), 1.0)
+    d_w = torch.from_numpy(w.view(np.int16)).cuda()
+    d_x = torch.zeros(M * K + 8, dtype=torch.int16, device="cuda")
+    d_x[shift:shift + M * K] = torch.from_numpy(x.view(np.int16)).cuda().reshape(-1)
+    d_y = torch.zeros((M + 1, O), dtype=torch.int16, device="cuda")
+    gpu.bf16_gemv_dev(d_w.data_ptr(), d_x.data_ptr() + 2 * shift, d_y.data_ptr(), M, O, K,
+                      stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    y = d_y.cpu().numpy().view(np.uint16)
+    got, exp = f32(y[:M]).astype(np.float64), f32(orc.gemm(w, x)).astype(np.float64)
+    mag = np.abs(f32(x).astype(np.float64)) @ np.abs(f32(w).astype(np.float64)).T
+    assert (np.abs(got - exp) <= 2 * K * 2.0 ** -24 * mag + np.abs(exp) * 2.0 ** -7).all()
+    assert not y[M].any()
+
+
 @pytest.mark.parametrize("M,O,K", [(1, 4096, 2048), (3, 1000, 512), (8, 777, 256),
                                    (1, 1, 256), (2, 33, 2048)])
 def test_gemv_stream_dev(gpu, orc, M, O, K):
