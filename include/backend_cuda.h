@@ -151,8 +151,9 @@ typedef struct {
  * apus_cuda_register_layer_slabs).  Synchronous: moe_out and the trace rows are complete on
  * return.  T == 0 writes nothing and succeeds, as the engine's loops over T do.
  * From APUS_CUDA_HOST_SPLIT_T tokens (default 4096; 0: never) the call runs as
- * two half calls whose PCIe copies overlap the other half's kernels: the same
- * bits, since a token's result does not depend on its neighbours.
+ * two half calls, from 6144 tokens as three (1/5, 3/5, 1/5), whose PCIe copies
+ * overlap the other parts' kernels: the same bits, since a token's result does not
+ * depend on its neighbours.
  * Returns 0, or nonzero with apus_cuda_last_error() set. */
 int apus_cuda_moe_block(const ApusCudaMoeCfg *c, const ApusCudaMoeW *w,
                         const uint16_t *ln2, uint16_t *moe_out, size_t T,
@@ -226,13 +227,13 @@ int apus_cuda_layer_load_slabs(ApusCudaLayer *layer, const char *container_dir,
  * device pointers (or NULL).  Enqueued on `stream` (a cudaStream_t; NULL is the
  * CUDA default stream, as everywhere in this header); does not synchronise.
  *
- * Path selection: T <= APUS_CUDA_FUSED_MAX_T (default and maximum 4) runs the
- * whole block as one cooperative kernel; larger T runs router -> dispatch ->
+ * Path selection: T <= APUS_CUDA_FUSED_MAX_T (default and maximum 8) runs the
+ * whole block as one cooperative kernel; larger T runs router -> placement ->
  * tcgen05 grouped GEMMs (gate/up, down) -> combine when the shape fits the MMA
  * tiles (H, I, Is multiples of 128, Is == I), else the grouped-GEMV kernels.
  * APUS_CUDA_DECODE_MAX_T (default 4) is the largest T that still takes the
  * grouped-GEMV kernels on a shape the GEMM supports.  From a mean of
- * APUS_CUDA_PAIR_MIN_ROWS (default 192) rows per expert on, and H a multiple of
+ * APUS_CUDA_PAIR_MIN_ROWS (default 104) rows per expert on, and H a multiple of
  * 256, the two GEMMs run with a pair of SMs per tile (cta_group::2: tokens
  * 256 per pair, each SM loading half of the weight tile); APUS_CUDA_PAIR=0
  * keeps the one-SM kernels.
@@ -304,22 +305,23 @@ enum {
 };
 int apus_cuda_stage_timing(int enable);
 int apus_cuda_last_stage_ms(float *ms, int cap);
-/* Diagnostic for the one-kernel path (T <= 4): with stage timing enabled each
+/* Diagnostic for the one-kernel path (T <= 8): with stage timing enabled each
  * CTA stamps the device's global timer (ns) at its eight phase boundaries;
  * this copies out[cta*8 + mark] for the last call and returns the number of
  * values written, or -1 if the last call did not take that path. */
 int apus_cuda_fused_timeline(unsigned long long *out, int cap);
 /* Diagnostic for the many-token router: it scores every expert with a fast
- * tensor-core product and walks the engine's exact sequential chain
- * (c/moe.h:289-291) only for the experts whose fast logit, widened by a proven
- * error bound, can still reach the top_k.  Returns how many exact chains have
- * run since enable (256 per token would be the plain exact router), -1 when
- * not enabled.  APUS_CUDA_ROUTER_CERTIFY=0 selects the plain exact router. */
+ * tensor-core product and resolves exactly (the code of the engine's sequential
+ * chain, c/moe.h:289-291, from an interval or from the chain itself) only the
+ * experts whose fast logit, widened by a proven error bound, can still reach the
+ * top_k.  Returns how many logits have been resolved since enable (256 per token
+ * would be the plain exact router; the one-kernel path counts the chains it walks),
+ * -1 when not enabled.  APUS_CUDA_ROUTER_CERTIFY=0 selects the plain exact router. */
 long apus_cuda_router_exact_chains(void);
 /* Diagnostic: phase boundaries of the many-token router's first CTA in its
- * last launch, out[0..3] = start, candidates known, exact chains done, end
- * (nanoseconds, low 32 bits of the device's global timer), out[4] = chains that
- * CTA walked.  Returns 0, or -1 when not enabled. */
+ * last launch, out[0..3] = start, candidates known, selection known, end
+ * (nanoseconds, low 32 bits of the device's global timer), out[4] = logits
+ * evaluated for its first token.  Returns 0, or -1 when not enabled. */
 int apus_cuda_router_timeline(unsigned int *out);
 /* Diagnostic for the same router (host pointers, synchronous): the fast
  * tensor-core logits of every (token, expert) pair, fast [T,E] fp32, summed
@@ -527,7 +529,7 @@ int apus_cuda_resadd_dev(const uint16_t *d_a, const uint16_t *d_b,
  * y [M,O], M <= 8, K a multiple of 256: the bandwidth-bound form of the
  * bf16_gemv / bf16_gemm hooks for resident weights and activations (the
  * output head is 248320 x 2048, 1 GB of weights per token, c/model.h:667-688).
- * fp32 accumulation in a lane-strided order, so the result agrees with the
+ * fp32 accumulation in tensor-core order, so the result agrees with the
  * engine's sequential chain to BF16 tolerance, not bitwise; callers that need
  * the chain's exact bits (the router) use the host-pointer entry points. */
 int apus_cuda_bf16_gemv_dev(const uint16_t *d_w, const uint16_t *d_x, uint16_t *d_y,
