@@ -49,13 +49,12 @@ FALLBACK_PEAKS = dict(hbm_gbs=6650.0, bf16_tflops=1590.0,
                       bf16_tflops_sustained=1400.0)
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the gate_up stage's
 # launches, keyed by (tokens, skewed router).  From an ncu capture of this
-# benchmark's own command on the build of commit 20ff240 (the GEMM kernels are
-# unchanged since); the launch-list summary under profiles/ holds the table.
+# benchmark's own command on the build of the commit named (what the one-SM kernel
+# moves has not changed since 20ff240).
 NCU_TRAFFIC = {
-    (8192, True): (1715.5e6, "ncu, commit 20ff240, bench.py --no-sub --no-cpu-baseline "
+    (8192, True): (1577.0e6, "ncu, commit 940827c, bench.py --no-sub --no-cpu-baseline "
                              "--sustain 0 --steps 2 --warmup 3 --no-graph: "
-                             "pair_gemm_kernel<0> 817.8 MB + grouped_gemm_kernel<0> "
-                             "897.7 MB per launch"),
+                             "pair_gemm_kernel<0> per launch"),
     (512, False): (1101.6e6, "ncu, commit 20ff240, bench.py --tokens 512 --uniform "
                              "--no-cpu-baseline --sustain 0 --steps 2 --warmup 3 "
                              "--no-graph: grouped_gemm_kernel<0> per launch"),
@@ -336,9 +335,7 @@ def measure_layer(env, layer, x_host, T, skew, steps, warmup, sustain_s,
     else:
         dom = max(("gate_up", "down"), key=lambda k: stage_ms.get(k, 0.0))
         two_sm = be.last_block_path() == 3
-        kname = (f"pair_gemm_kernel<{dom}> + grouped_gemm_kernel<{dom}> (the stage's "
-                 "two launches: 256-row chunks on SM pairs, the rest on single SMs)"
-                 if two_sm else f"grouped_gemm_kernel<{dom}>")
+        kname = f"pair_gemm_kernel<{dom}>" if two_sm else f"grouped_gemm_kernel<{dom}>"
         if dom == "gate_up":
             kbytes = (uniq + 1) * slab_gu + (A + T) * H * 2 + (A + T) * I * 2
             kflops = 2 * (A + T) * 2 * I * H
