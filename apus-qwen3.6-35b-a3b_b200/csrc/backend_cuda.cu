@@ -94,6 +94,7 @@ struct Ctx {
     int device = 0;
     int sm_count = 0;
     int smem_optin = 0;
+    size_t smem_sm = 0;
     cudaStream_t stream = nullptr;
     std::unordered_map<const void *, DevBuf> wcache;
     std::unordered_map<const void *, ApusCudaLayer *> layers;  /* host-ptr key */
@@ -209,6 +210,7 @@ static int ctx_init() {
     if (env_long("APUS_CUDA_SMS", 0) > 0 && env_long("APUS_CUDA_SMS", 0) < c->sm_count)
         c->sm_count = (int)env_long("APUS_CUDA_SMS", 0);
     c->smem_optin = (int)prop.sharedMemPerBlockOptin;
+    c->smem_sm = prop.sharedMemPerMultiprocessor;
     CU_OK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CU_OK(cudaMalloc(&c->d_status, STATUS_BYTES + SMALL_OUT_MAX));
     CU_OK(cudaMemset(c->d_status, 0, STATUS_BYTES));
@@ -755,22 +757,27 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
     if (T <= ROUTER_SMALL_MAX_T && (K & 7) == 0 &&
         (((uintptr_t)dwr | (uintptr_t)extra_row) & 15) == 0) {
         const int rows = E + (extra_row ? 1 : 0);
-        /* four tokens and one chain warp per CTA: two chain warps over eight
-         * tokens measured slower (33 against 24 us at 32 tokens) */
-        constexpr int tok = 4;
-        const size_t smem = router_small_smem(E, K, tok);
+        /* four tokens per CTA: two chain warps over eight measured slower (33 against
+         * 24 us at 32 tokens) */
+        const int groups = (T + ROUTER_SMALL_TOK - 1) / ROUTER_SMALL_TOK;
+        const size_t smem8 = router_small_smem(E, K, 8), smem16 = router_small_smem(E, K, 16);
+        const size_t slots = (size_t)c->sm_count * (c->smem_sm / (smem8 + 1280));
+        const bool wide = smem16 <= (size_t)c->smem_optin &&
+                          (size_t)((rows + 7) / 8) * groups > slots;
+        const size_t smem = wide ? smem16 : smem8;
         if (smem <= (size_t)c->smem_optin) {
-            static size_t set_smem = 48 * 1024;
-            auto kern = router_small_kernel<tok>;
-            if (smem > set_smem) {
+            static size_t set_smem[2] = {48 * 1024, 48 * 1024};
+            auto kern = wide ? router_small_kernel<16> : router_small_kernel<8>;
+            if (smem > set_smem[wide]) {
                 CU_OK(cudaFuncSetAttribute(
                     kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                set_smem = smem;
+                set_smem[wide] = smem;
             }
-            dim3 grid((rows + ROUTER_SMALL_ROWS - 1) / ROUTER_SMALL_ROWS, (T + tok - 1) / tok);
-            launch_k(kern, dim3(grid), dim3(ROUTER_SMALL_THREADS), smem, st, dx, dwr, T, E, K,
-                     topk, wmin, aux ? aux->wmin_extra : 0.0f, didx, dw, dlogits, extra_row,
-                     extra_out, c->d_router_logits, c->d_router_counters, c->d_status);
+            const int per = wide ? 16 : 8;
+            launch_k(kern, dim3((rows + per - 1) / per, groups), dim3(ROUTER_SMALL_THREADS), smem,
+                     st, dx, dwr, T, E, K, topk, wmin, aux ? aux->wmin_extra : 0.0f, didx, dw,
+                     dlogits, extra_row, extra_out, c->d_router_logits, c->d_router_counters,
+                     c->d_status);
             LAUNCHED();
             return 0;
         }

@@ -364,27 +364,28 @@ __device__ __forceinline__ float small_chain(const uint16_t *__restrict__ wrow,
 }
 
 /*
- * Latency path for few tokens.  grid = (ceil(rows / 8), ceil(T / TOK)), block
- * = 128: a CTA pulls eight router rows into shared memory with one bulk copy
+ * Latency path for few tokens.  grid = (ceil(rows / ROWS), ceil(T / 4)), block
+ * = 128: a CTA pulls ROWS router rows into shared memory with one bulk copy
  * each (all in flight at once, so the 1 MiB router matrix arrives spread over
- * 32 SMs instead of trickling through one) and stages TOK tokens as fp32;
- * the lanes of TOK/4 warps walk one exact chain each (lane = row * 4 + token),
- * and the BF16 logits go to global memory.  The CTA that arrives last for a
+ * many SMs instead of trickling through one) and stages four tokens as fp32;
+ * the lanes of ROWS/8 warps walk one exact chain each (lane = row * 4 + token),
+ * and the BF16 logits go to global memory.  ROWS is 8 while all CTAs are resident at
+ * once, three to an SM (up to 52 tokens here), and 16 above, two to an SM: a second
+ * wave costs a whole chain (61 tokens: 31 -> 24 us).  The CTA that arrives last for a
  * token (one atomic counter per token, which it resets for the next call) runs
  * that token's softmax / top-k on one of its warps.  No CTA ever waits on
  * another.  Requires K % 8 == 0 and a 16-byte-aligned router matrix.
- * Dynamic shared memory: 8 * (K*2 + 16) + TOK * ((K + 4) + E) * 4 bytes.
+ * Dynamic shared memory: ROWS * (K*2 + 16) + 4 * ((K + 4) + E) * 4 bytes.
  */
-constexpr int ROUTER_SMALL_ROWS = 8;
+constexpr int ROUTER_SMALL_TOK = 4;
 constexpr int ROUTER_SMALL_THREADS = 128;
 
-/* TOK tokens per CTA: 4 (one chain warp) or 8 (two, on different schedulers) */
-inline size_t router_small_smem(int E, int K, int tok) {
-    return (size_t)ROUTER_SMALL_ROWS * (K * 2 + 16) + (size_t)tok * (K + 4) * 4 +
-           (size_t)tok * E * 4;
+inline size_t router_small_smem(int E, int K, int rows) {
+    return (size_t)rows * (K * 2 + 16) + (size_t)ROUTER_SMALL_TOK * (K + 4) * 4 +
+           (size_t)ROUTER_SMALL_TOK * E * 4;
 }
 
-template <int ROUTER_SMALL_TOK>
+template <int ROUTER_SMALL_ROWS>
 __global__ void __launch_bounds__(ROUTER_SMALL_THREADS)
 router_small_kernel(const uint16_t *__restrict__ x,
                     const uint16_t *__restrict__ wr, int T, int E, int K,
@@ -453,14 +454,15 @@ router_small_kernel(const uint16_t *__restrict__ x,
         xmin = min(xmin, __shfl_xor_sync(0xffffffffu, xmin, o));
     if (lane == 0) atomicMin(&s_xmin, xmin);
     __syncthreads();
-    if (warp < ROUTER_SMALL_TOK / 4) {
+    constexpr int CHAIN_WARPS = ROUTER_SMALL_ROWS / 8;
+    if (warp < CHAIN_WARPS) {
         const double xmn = (double)__uint_as_float(s_xmin);
         const bool use_fma = (wmin > 0.0f) && ((double)wmin * xmn >= 7.52316384526264e-37);
         const bool use_fma_x =
             (wmin_extra > 0.0f) && ((double)wmin_extra * xmn >= 7.52316384526264e-37);
         const bool arrived = mbar_wait(&bar, 0);
         if (!arrived) set_status(status, ST_MBAR_TIMEOUT);
-        const int r = lane >> 2, tt = warp * 4 + (lane & 3);
+        const int r = warp * 8 + (lane >> 2), tt = lane & 3;
         if (arrived && r < nrows && tt < nt) {
             const uint16_t *wrow =
                 reinterpret_cast<const uint16_t *>(rows_s + (size_t)r * pitch);
@@ -480,9 +482,9 @@ router_small_kernel(const uint16_t *__restrict__ x,
         /* the last CTA of a token finishes that token */
         __threadfence();
         __syncwarp();
-        if (lane < 4 && warp * 4 + lane < nt)
-            s_last[warp * 4 + lane] =
-                atomicAdd(&counters[t0 + warp * 4 + lane], 1u) == gridDim.x - 1;
+        if (lane < nt &&
+            atomicAdd(&counters[t0 + lane], 1u) == gridDim.x * CHAIN_WARPS - 1)
+            s_last[lane] = 1;
     }
     __syncthreads();
     for (int tt = warp; tt < nt; tt += ROUTER_SMALL_THREADS / 32) {
