@@ -25,6 +25,7 @@
 #include "decode_fused.cuh"
 #include "router_certify.cuh"
 #include "router_select.cuh"
+#include "router_small.cuh"
 #include "decode_gemv.cuh"
 #include "dispatch.cuh"
 #include "ep_window.cuh"

@@ -257,6 +257,29 @@ def test_router_certified_kernel_edges(gpu, orc, be, synth, T, E, K, kind):
     assert d.max() <= 1 and (d != 0).mean() <= 0.002
 
 
+@pytest.mark.parametrize("T,E,K,topk", [
+    (9, 256, 2048, 8), (52, 256, 2048, 8), (53, 256, 2048, 8), (64, 257, 2048, 8),
+    (61, 300, 1032, 5), (64, 1024, 512, 32), (33, 37, 24, 1)])
+@pytest.mark.parametrize("case", ["plain", "tied_rows", "tiny_logits"])
+def test_router_few_tokens_edges(gpu, orc, be, synth, T, E, K, topk, case):
+    """The few-token router where a second wave of CTAs would begin, with remainders of
+    rows and tokens, and where code order may not decide."""
+    cfg = dict(hidden=K, experts=E, moe_inter=128, shared_inter=128, top_k=topk)
+    W = synth.host_weights(be, cfg, seed=T + K, sigma=0.05)
+    x = synth.host_x(be, T, K, seed=T + E)
+    rtr = W["rtr_w"]
+    if case == "tied_rows":
+        rtr[1::2] = rtr[0::2][:rtr[1::2].shape[0]]
+    elif case == "tiny_logits":
+        rtr[:] = synth.f32_to_bf16(synth.bf16_to_f32(rtr) * 2.0 ** -20)
+    idx, w = _route_dev(gpu, synth, cfg, W, x)
+    assert gpu.last_block_status() == 0
+    eidx, ew = orc.route_batch(x, rtr, topk)
+    assert np.array_equal(idx, eidx)
+    d = np.abs(w.astype(np.int32) - ew.astype(np.int32))
+    assert d.max() <= 1 and (d != 0).mean() <= 0.002
+
+
 def test_router_certified_can_be_switched_off(be, orc, synth, monkeypatch):
     monkeypatch.setenv("APUS_CUDA_ROUTER_CERTIFY", "0")
     be.enable()
