@@ -742,8 +742,11 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
                           : smem_u32(act) + (uint32_t)((row0 + n) * L.act_pitch)) +
                       (uint32_t)(d.k0 * 32 + (lane >> 3) * 16);
         float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+        /* a second half without a k step (16 values in all) is a turn and a slot of the
+         * ring like any other, as in issue() */
+        int ks0 = 0;
 #pragma unroll 1
-        for (int ks0 = 0; ks0 < d.nk; ks0 += DF_KS, ba += DF_KS * 32) {
+        do {
             const uint32_t t = next_tile();
             const int nk = min(DF_KS, d.nk - ks0);
 #pragma unroll
@@ -760,7 +763,9 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
                 }
             __syncwarp();
             issue();
-        }
+            ks0 += DF_KS;
+            ba += DF_KS * 32;
+        } while (ks0 < d.nk);
         const int r = lane >> 2, col = (lane & 3) * 2;
         float *dst = red + ((size_t)(v & 1) * (A + T) + (sh ? A : row0) + col) * DF_MAX_COLS + r;
         if (col < cnt) {

@@ -130,6 +130,21 @@ def test_block_one_kernel_edges(gpu, orc, be, synth, T, H, E, I, Is, TK, case):
         assert gpu.router_exact_chains() - before >= T * E
 
 
+@pytest.mark.parametrize("T,H,E,I,Is,TK", [
+    (1, 256, 64, 16, 32, 8), (1, 2048, 64, 16, 512, 8), (3, 208, 64, 16, 272, 8),
+    (8, 512, 64, 16, 32, 8), (8, 256, 256, 16, 512, 8), (1, 256, 64, 32, 16, 8)])
+def test_block_one_kernel_empty_halves(gpu, orc, be, synth, T, H, E, I, Is, TK):
+    """Down rows are taken in halves of K.  Sixteen values have no second half; with eight
+    distinct experts or more the same warp's next one (at last the shared expert's) does."""
+    cfg = dict(hidden=H, experts=E, moe_inter=I, shared_inter=Is, top_k=TK)
+    W = synth.host_weights(be, cfg, seed=40 + T, sigma=0.9 / H ** 0.5)
+    for seed in (50, 51):          # the second call finds the first one's ring contents
+        x = synth.host_x(be, T, H, seed=seed + T)
+        got = gpu.moe_block(cfg, W, x)
+        assert gpu.last_block_launches() == 1 and gpu.last_block_status() == 0
+        check_block(got, orc.moe_block(cfg, W, x), f"I={I} Is={Is} T={T}")
+
+
 @pytest.mark.parametrize("T,E,TK,skew", [
     (9, 128, 8, False), (65, 128, 1, True), (255, 128, 8, True), (256, 1024, 8, False),
     (257, 128, 8, True), (513, 256, 3, False), (300, 128, 32, True),     # counted by the router
