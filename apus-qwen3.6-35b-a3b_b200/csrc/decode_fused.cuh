@@ -749,17 +749,26 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
         do {
             const uint32_t t = next_tile();
             const int nk = min(DF_KS, d.nk - ks0);
+            /* mma.sync cuts off what its accumulator cannot hold: two steps on one that
+             * starts at zero, sums of those rounded to nearest.  Eight steps on one
+             * narrowed 1.02e-4 of the outputs to another BF16 value than 64-bit sums
+             * do (K 512), this 0.79e-4, as scalar multiply-adds did (0.78e-4).  The
+             * gate/up tiles end in a sum of sixteen warps and need no more than that
+             * (0.98e-4 of K 2048; scalar 1.04e-4). */
 #pragma unroll
             for (int s = 0; s < DF_KS; s += 2)
                 if (s < nk) {
                     uint32_t br[4], r[4];
+                    float p[4] = {0.f, 0.f, 0.f, 0.f};
                     ldmatrix_x4(br, ba + (uint32_t)(s * 32));
                     ldmatrix_x4(r, t + (uint32_t)(s * 32));
-                    mma_16x8(c0, r, br[0], br[1]);
+                    mma_16x8(p, r, br[0], br[1]);
                     if (s + 1 < nk) {
                         ldmatrix_x4(r, t + (uint32_t)(s * 32 + 32));
-                        mma_16x8(c1, r, br[2], br[3]);
+                        mma_16x8(p, r, br[2], br[3]);
                     }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) ((s & 2) ? c1 : c0)[q] += p[q];
                 }
             __syncwarp();
             issue();
