@@ -69,7 +69,11 @@ exact_matvec_f32_kernel(const uint16_t *__restrict__ w,
  * slots ahead; mma.sync m16n8k16 multiplies them with all rows of x at once (columns past
  * M repeat the last row and are not stored), so eight rows cost what one does.  Scalar
  * multiply-adds on rows loaded straight into registers took 179 us for one row and 783 for
- * eight (O 248320, K 2048); this 174 and 182 (5.9 of 6.5 TB/s).
+ * eight (O 248320, K 2048); this 176 and 183 (5.8 of 6.5 TB/s).
+ * mma.sync cuts off what its accumulator cannot hold, so two steps share one that starts
+ * at zero and the rest is a tree: at K 2048 1.0e-4 of the results narrow to another BF16
+ * value than 64-bit sums do, as in the scalar form (6e-4 with all 64 steps on one); at
+ * K 8192 1.1e-4 (scalar 1.7e-4, 23e-4).
  * The summation order differs from the engine's sequential chain, so the result
  * agrees to BF16 tolerance, not bitwise; the exact-order form is exact_dense.cuh
  * behind the host-pointer hooks. */
@@ -149,14 +153,26 @@ gemv_stream_kernel(const uint16_t *__restrict__ w, const uint16_t *__restrict__ 
             __syncwarp();      /* everyone's pieces landed; the oldest slot is read out */
             issue();
             const uint32_t at = ring + (uint32_t)(s * GV_SLOT) + a_off;
+            float p[4][4];
 #pragma unroll
-            for (int k = 0; k < GV_BK; k += 32) {
+            for (int j = 0; j < 4; j++) {
                 uint32_t a0[4], a1[4], b[4];
-                ldmatrix_x4(b, b_at + (uint32_t)((kb * GV_BK + k) * 2));
-                ldmatrix_x4(a0, at + (uint32_t)(k * 2));
-                ldmatrix_x4(a1, at + (uint32_t)(k * 2 + 32));
-                mma_16x8(c0, a0, b[0], b[1]);
-                mma_16x8(c1, a1, b[2], b[3]);
+#pragma unroll
+                for (int q = 0; q < 4; q++) p[j][q] = 0.0f;
+                ldmatrix_x4(b, b_at + (uint32_t)((kb * GV_BK + j * 32) * 2));
+                ldmatrix_x4(a0, at + (uint32_t)(j * 64));
+                ldmatrix_x4(a1, at + (uint32_t)(j * 64 + 32));
+                mma_16x8(p[j], a0, b[0], b[1]);
+                mma_16x8(p[j], a1, b[2], b[3]);
+            }
+            const bool fold = (kb & 3) == 3;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                c0[q] += (p[0][q] + p[1][q]) + (p[2][q] + p[3][q]);
+                if (fold) {
+                    c1[q] += c0[q];
+                    c0[q] = 0.0f;
+                }
             }
             if (++s == GV_STAGES) s = 0;
         }

@@ -376,6 +376,29 @@ def test_gemv_stream_edges(gpu, orc, M, O, K, shift):
     assert not y[M].any()
 
 
+@pytest.mark.parametrize("M,O,K,share", [(1, 65536, 2048, 0.97e-4), (8, 65536, 2048, 1.00e-4),
+                                          (4, 16384, 8192, 1.68e-4)])
+def test_gemv_stream_against_64_bit_sums(gpu, M, O, K, share):
+    """How often a result narrows to another BF16 value than its 64-bit sum does, against
+    `share`, what scalar multiply-adds in fp32 had there.  Bound: half as much again (six
+    standard deviations of the 150 and more events in the three passes)."""
+    import torch
+    wrong = n = 0
+    for seed in range(3 if M == 8 else 8):
+        gen = torch.Generator(device="cuda")
+        gen.manual_seed(seed)
+        w = (torch.randn(O, K, device="cuda", generator=gen) * 0.02).bfloat16()
+        x = torch.randn(M, K, device="cuda", generator=gen).bfloat16()
+        y = torch.empty((M, O), dtype=torch.bfloat16, device="cuda")
+        gpu.bf16_gemv_dev(w.data_ptr(), x.data_ptr(), y.data_ptr(), M, O, K,
+                          stream=torch.cuda.current_stream().cuda_stream)
+        exp = (x.double() @ w.double().T).contiguous().view(torch.int64)
+        exp = exp + ((1 << 44) - 1) + ((exp >> 45) & 1)          # one rounding to BF16
+        wrong += int((y.double() != (exp >> 45 << 45).view(torch.float64)).sum())
+        n += y.numel()
+    assert wrong <= 1.5 * share * n, wrong / n
+
+
 @pytest.mark.parametrize("M,O,K", [(1, 4096, 2048), (3, 1000, 512), (8, 777, 256),
                                    (1, 1, 256), (2, 33, 2048)])
 def test_gemv_stream_dev(gpu, orc, M, O, K):
