@@ -96,6 +96,7 @@ struct Ctx {
     int sm_count = 0;
     int smem_optin = 0;
     size_t smem_sm = 0;
+    std::unordered_map<const void *, size_t> static_smem;      /* of a kernel, once asked for */
     cudaStream_t stream = nullptr;
     std::unordered_map<const void *, DevBuf> wcache;
     std::unordered_map<const void *, ApusCudaLayer *> layers;  /* host-ptr key */
@@ -443,6 +444,21 @@ extern "C" const char *apus_cuda_last_error(void) { return g_err; }
 /* per-matmul entry points (host pointers)                                   */
 /* ------------------------------------------------------------------------ */
 
+/* dynamic shared memory that a CTA of this kernel can have beside its static tables */
+static size_t dynamic_smem_limit(Ctx *c, const void *kern) {
+    auto it = c->static_smem.find(kern);
+    if (it == c->static_smem.end()) {
+        cudaFuncAttributes at;
+        if (cudaFuncGetAttributes(&at, kern) != cudaSuccess) {
+            cudaGetLastError();
+            at.sharedSizeBytes = 4096;
+        }
+        it = c->static_smem.emplace(kern, at.sharedSizeBytes).first;
+    }
+    const size_t most = (size_t)c->smem_optin;
+    return it->second < most ? most - it->second : 0;
+}
+
 /* magnitude range of n BF16 values on the device (set-up: synchronises) */
 static int bf16_range(Ctx *c, const uint16_t *d, size_t n, float *lo, float *hi) {
     unsigned int v[2] = {0x7f800000u, 0u};
@@ -505,11 +521,13 @@ static int launch_exact(Ctx *c, const ExactArgs &a, int M_all, cudaStream_t st) 
                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)smem) == cudaSuccess;
     };
-    if (a.K % 8 == 0 && a.M <= ER_MAX_M && exact_rows_smem(a.M, a.K, 1) <= optin) {
+    /* (the instances of exact_rows_kernel have the same static tables) */
+    const size_t rows_most = dynamic_smem_limit(c, (const void *)exact_rows_kernel<1, true>);
+    if (a.K % 8 == 0 && a.M <= ER_MAX_M && exact_rows_smem(a.M, a.K, 1) <= rows_most) {
         const long groups = (a.O + 31) / 32;
         int warps = (int)((groups + c->sm_count - 1) / c->sm_count);
         warps = warps < 1 ? 1 : (warps > 8 ? 8 : warps);
-        while (exact_rows_smem(a.M, a.K, warps) > optin) warps--;
+        while (exact_rows_smem(a.M, a.K, warps) > rows_most) warps--;
         long grid = (groups + warps - 1) / warps;
         if (grid > c->sm_count) grid = c->sm_count;
         const size_t smem = exact_rows_smem(a.M, a.K, warps);
@@ -762,11 +780,14 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
          * 24 us at 32 tokens) */
         const int groups = (T + ROUTER_SMALL_TOK - 1) / ROUTER_SMALL_TOK;
         const size_t smem8 = router_small_smem(E, K, 8), smem16 = router_small_smem(E, K, 16);
-        const size_t slots = (size_t)c->sm_count * (c->smem_sm / (smem8 + 1280));
-        const bool wide = smem16 <= (size_t)c->smem_optin &&
-                          (size_t)((rows + 7) / 8) * groups > slots;
+        const size_t most8 = dynamic_smem_limit(c, (const void *)router_small_kernel<8>),
+                     most16 = dynamic_smem_limit(c, (const void *)router_small_kernel<16>);
+        /* resident at once: an SM also keeps 1 KB for each CTA */
+        const size_t slots = (size_t)c->sm_count *
+                             (c->smem_sm / (smem8 + ((size_t)c->smem_optin - most8) + 1024));
+        const bool wide = smem16 <= most16 && (size_t)((rows + 7) / 8) * groups > slots;
         const size_t smem = wide ? smem16 : smem8;
-        if (smem <= (size_t)c->smem_optin) {
+        if (smem <= (wide ? most16 : most8)) {
             static size_t set_smem[2] = {48 * 1024, 48 * 1024};
             auto kern = wide ? router_small_kernel<16> : router_small_kernel<8>;
             if (smem > set_smem[wide]) {
@@ -827,7 +848,7 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         return launch_router_tt<1>(c, dx, dwr, T, E, K, topk, wmin, didx, dw,
                                    dlogits, extra_row, extra_out, st);
     size_t smem8 = ((size_t)8 * K + (size_t)8 * E) * sizeof(float);
-    if (smem8 <= (size_t)c->smem_optin)
+    if (smem8 <= dynamic_smem_limit(c, (const void *)router_topk_kernel<8>))
         return launch_router_tt<8>(c, dx, dwr, T, E, K, topk, wmin, didx, dw,
                                    dlogits, extra_row, extra_out, st);
     return launch_router_tt<1>(c, dx, dwr, T, E, K, topk, wmin, didx, dw,
@@ -1492,7 +1513,8 @@ static bool fused_supported(Ctx *c, const ApusCudaMoeCfg &cfg, size_t T) {
         return false;
     const FusedLayout L((int)T, (int)cfg.hidden, (int)cfg.moe_inter, (int)cfg.shared_inter,
                         (int)cfg.experts, (int)cfg.top_k, c->sm_count);
-    return (size_t)L.total + DF_STATIC_SMEM <= (size_t)c->smem_optin;
+    /* (the full-size layer at eight tokens fills an SM to the byte) */
+    return (size_t)L.total <= dynamic_smem_limit(c, (const void *)decode_fused_kernel);
 }
 
 /* rows of whole 16-byte pieces: one warp per row without the sequential chain;

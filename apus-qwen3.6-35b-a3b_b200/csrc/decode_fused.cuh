@@ -59,8 +59,6 @@ constexpr int DF_PAIRS = DF_ROWS / 2;
 constexpr int DF_KS = 8;                /* 16-wide k steps of a tile, at most */
 constexpr int DF_MAX_K_DOWN = 4 * DF_KS * 16;   /* half of it is at most two tiles */
 constexpr int DF_DEPTH = 2;             /* tiles of a warp's ring */
-constexpr int DF_STATIC_SMEM = 1920;    /* the static tables (with them the full-size layer at
-                                         * eight tokens fills an SM to the byte) */
 constexpr int DF_MAX_COLS = 16;         /* output columns of a CTA, at most */
 
 /* ---- shared memory ------------------------------------------------------------ */

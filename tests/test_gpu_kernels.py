@@ -55,6 +55,17 @@ def test_hook_exact_order_kernels(gpu, orc, M, O, K, scale):
                               equal_nan=True)
 
 
+@pytest.mark.parametrize("M,O,K", [(4, 16000, 3008), (2, 14300, 6016)])
+def test_hook_rows_that_fill_shared_memory(gpu, orc, M, O, K):
+    """Rows of x and the rings of four warps are 232448 bytes here, all that a CTA may have,
+    static tables included: fewer warps have to be taken."""
+    rng = np.random.default_rng(K)
+    w = rng.integers(0x3c00, 0x3d80, (O, K), dtype=np.uint16) ^ \
+        (rng.integers(0, 2, (O, K), dtype=np.uint16) << 15)
+    x = rng_codes(rng, (M, K), 1.0)
+    assert np.array_equal(gpu.bf16_gemm(w, x), orc.gemm(w, x))
+
+
 def test_hook_zero_dims_and_counters(gpu):
     assert gpu.lib.apus_cuda_bf16_gemv(None, None, None, 0, 8) != 0
     assert gpu.lib.apus_cuda_bf16_gemm(None, None, None, 1, 0, 8) != 0
@@ -278,6 +289,21 @@ def test_router_few_tokens_edges(gpu, orc, be, synth, T, E, K, topk, case):
     assert np.array_equal(idx, eidx)
     d = np.abs(w.astype(np.int32) - ew.astype(np.int32))
     assert d.max() <= 1 and (d != 0).mean() <= 0.002
+
+
+@pytest.mark.parametrize("T,E,K,topk", [(64, 256, 4736, 8), (64, 256, 4744, 8),
+                                        (64, 256, 7104, 8), (64, 256, 7112, 8)])
+def test_router_few_tokens_at_the_shared_memory_limit(gpu, orc, be, synth, T, E, K, topk):
+    """The last sizes at which sixteen rows a CTA (4736) and eight (7104) fit beside the
+    static tables, and the first at which they fit only without those."""
+    cfg = dict(hidden=K, experts=E, moe_inter=8, shared_inter=8, top_k=topk)
+    W = synth.host_weights(be, cfg, seed=K, sigma=0.02)
+    x = synth.host_x(be, T, K, seed=T)
+    idx, w = _route_dev(gpu, synth, cfg, W, x)
+    assert gpu.last_block_status() == 0
+    eidx, ew = orc.route_batch(x, W["rtr_w"], topk)
+    assert np.array_equal(idx, eidx)
+    assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
 
 
 def test_router_certified_can_be_switched_off(be, orc, synth, monkeypatch):
