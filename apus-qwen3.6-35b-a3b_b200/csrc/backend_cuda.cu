@@ -492,8 +492,12 @@ static const DevBuf *weight_buf(Ctx *c, const void *ptr, size_t bytes) {
         return nullptr;
     }
     DevBuf b{d, bytes};
-    if (cudaMemcpy(d, ptr, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+    /* on the library's stream: the range kernel that follows reads what has arrived
+     * (cudaMemcpy may return before pageable memory is on the device, and orders
+     * nothing before a non-blocking stream) */
+    if (cudaMemcpyAsync(d, ptr, bytes, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
         bf16_range(c, (const uint16_t *)d, bytes / 2, &b.wmin, &b.wmax)) {
+        cudaStreamSynchronize(c->stream);      /* the copy may still be under way */
         fail("weight upload failed");
         cudaFree(d);
         return nullptr;
@@ -1081,13 +1085,20 @@ extern "C" int apus_cuda_layer_create(const ApusCudaMoeCfg *cfg,
         }
         L->bytes += bytes;
         if (it.src) {
-            if (cudaMemcpy(*it.dst, it.src, bytes, cudaMemcpyHostToDevice) !=
+            /* ordered before the kernels on this stream that look at the weights */
+            if (cudaMemcpyAsync(*it.dst, it.src, bytes, cudaMemcpyHostToDevice, c->stream) !=
                 cudaSuccess) {
+                cudaStreamSynchronize(c->stream);
                 layer_free(L);
                 return fail("layer weight upload failed");
             }
             c->bytes_uploaded += bytes;
         }
+    }
+    /* the caller's arrays are free again, and any stream may use the layer */
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
+        layer_free(L);
+        return fail("layer weight upload failed");
     }
     c->bytes_resident += L->bytes;
     L->maps = nullptr;
@@ -1148,7 +1159,8 @@ extern "C" int apus_cuda_layer_upload(ApusCudaLayer *L, int which,
     if (ctx_init()) return 1;
     /* set-up call: synchronous, whatever stream used the tensor before */
     CU_OK(cudaDeviceSynchronize());
-    CU_OK(cudaMemcpy(dst + first, src, n * 2, cudaMemcpyHostToDevice));
+    CU_OK(cudaMemcpyAsync(dst + first, src, n * 2, cudaMemcpyHostToDevice, g_ctx->stream));
+    CU_OK(cudaStreamSynchronize(g_ctx->stream));
     g_ctx->bytes_uploaded += n * 2;
     if (which == 1 || which == 7) return layer_router_stats(g_ctx, L);
     return 0;

@@ -66,6 +66,25 @@ def test_hook_rows_that_fill_shared_memory(gpu, orc, M, O, K):
     assert np.array_equal(gpu.bf16_gemm(w, x), orc.gemm(w, x))
 
 
+@pytest.mark.parametrize("mib", [1, 8, 32])
+def test_hook_range_of_a_weight_covers_its_end(gpu, orc, mib):
+    """The magnitude range that chooses between the fused and the literal chain is taken when
+    a weight becomes resident; the values that decide lie in the last row, which arrives
+    last.  (The rest of device memory holds ordinary values from the weight before.)"""
+    import torch
+    rng = np.random.default_rng(mib)
+    K, O = 512, mib * 1024
+    torch.full((mib << 20,), 0.5, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    x = rng_codes(rng, (5, K), 1e-20)
+    w = np.full((O, K), 0x3f00, np.uint16)
+    w[-1] = rng_codes(rng, (K,), 0.5e-20)
+    exp = orc.gemm(w, x)
+    assert np.array_equal(gpu.bf16_gemm(w, x), exp)
+    assert np.array_equal(gpu.bf16_gemv(w, x[0]), exp[0])
+
+
 def test_hook_zero_dims_and_counters(gpu):
     assert gpu.lib.apus_cuda_bf16_gemv(None, None, None, 0, 8) != 0
     assert gpu.lib.apus_cuda_bf16_gemm(None, None, None, 1, 0, 8) != 0
