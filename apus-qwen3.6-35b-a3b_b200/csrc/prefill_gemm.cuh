@@ -295,8 +295,9 @@ struct GemmParams {
      * kernel (programmatic dependent launch lets its CTAs start on SMs whose
      * gate_up CTA has run out of tiles) but, tile by tile, for done[expert] to
      * reach need[expert] * (epilogue warps).  The gate_up kernel never waits
-     * on the down kernel, and all of its CTAs are resident before the first
-     * down CTA can be, so the wait cannot hold up what it waits for. */
+     * on the down kernel, and all of its CTAs are resident and past their wait for
+     * the lists before the first down CTA can be, so the wait cannot hold up what
+     * it waits for. */
     int *done;
     const int *need;
     /* Tiles are handed out in list order by an atomic counter when `sched` is
@@ -342,10 +343,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
                     const __grid_constant__ CUtensorMap mapB,     /* xg | act */
                     const __grid_constant__ CUtensorMap mapBs,    /* x  | sa */
                     GemmParams p) {
-    /* The next kernel may be scheduled now.  This kernel's own wait for the
-     * previous one comes after the prologue below (barriers, TMEM), which
-     * touches nothing the previous kernel writes. */
-    if (MODE != 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    /* This kernel's wait for the previous one comes after the prologue below
+     * (barriers, TMEM), which touches nothing the previous kernel writes.  The kernel
+     * after the down kernel waits for it before it reads anything and may be
+     * scheduled now; the kernels after the other two may not (below). */
+    if (MODE == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr bool GATE_UP = MODE == 0;
     constexpr int STAGES = PG_STAGES;
     constexpr int BN = MODE == 1 ? PG_BN_DN : PG_BN_GU;
@@ -390,12 +392,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
-    /* the down kernel of an overlapped pair does not wait for the whole gate_up
-     * kernel: its producer waits per expert instead */
+    /* The down kernel of an overlapped pair does not wait for the whole gate_up
+     * kernel: its producer waits per expert instead.  What it reads besides (tile
+     * lists, counts, counters) comes from the kernels before gate_up, and no wait of
+     * its own covers those: it may not start before every gate_up CTA has seen them
+     * complete.  (gate_up let it start at once and relied on its own CTAs to leave no
+     * room for one on any SM, which a grid smaller than the GPU does not.)  Likewise
+     * the router's second kernel reads the tokens before its own wait. */
     if (!(MODE == 1 && p.done)) asm volatile("griddepcontrol.wait;" ::: "memory");
-    /* the router's second kernel reads the tokens before its own wait, so it may not
-     * start before what wrote them is complete */
-    if (MODE == 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (MODE != 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (MODE == 2)
         for (int i = blockIdx.x * PG_THREADS + tid; i < p.zero_n; i += gridDim.x * PG_THREADS)
             p.zero[i] = 0;
