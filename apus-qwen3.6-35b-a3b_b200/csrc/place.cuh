@@ -156,7 +156,8 @@ place_kernel(const __grid_constant__ PlaceArgs a, const __grid_constant__ Plan p
 /* tokens of a CTA: all CTAs resident at once; without a copy as few CTAs as the rank
  * loop allows */
 inline int place_tokens(int T, int TK, int ctas, bool copy) {
-    const int most = PL_THREADS / TK, want = copy ? (T + ctas - 2) / (ctas - 1) : T;
+    const int others = ctas > 1 ? ctas - 1 : 1;      /* beside the lists' (none waits for another) */
+    const int most = PL_THREADS / TK, want = copy ? (T + others - 1) / others : T;
     return want < most ? want : most;
 }
 

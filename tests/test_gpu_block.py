@@ -165,6 +165,24 @@ def test_block_placement_edges(gpu, orc, be, synth, T, E, TK, skew):
     check_block(got, orc.moe_block(cfg, W, x), f"T={T} E={E} TK={TK}")
 
 
+@pytest.mark.parametrize("sms", ["1", "2", "3"])
+@pytest.mark.parametrize("T", [9, 65, 300])
+def test_block_on_a_few_sms(be, orc, synth, monkeypatch, sms, T):
+    """APUS_CUDA_SMS: grids for fewer SMs than there are, down to one (the placement kernel
+    then has no CTA to spare for the copy; the expert kernels run side by side)."""
+    cfg = dict(hidden=512, experts=64, moe_inter=128, shared_inter=128, top_k=8)
+    W = synth.host_weights(be, cfg, seed=77, sigma=0.05)
+    x = synth.host_x(be, T, cfg["hidden"], seed=T)
+    monkeypatch.setenv("APUS_CUDA_SMS", sms)
+    be.enable()
+    try:
+        got = be.moe_block(cfg, W, x)
+        assert be.last_block_status() == 0
+        check_block(got, orc.moe_block(cfg, W, x), f"T={T} on {sms} SMs")
+    finally:
+        be.disable()
+
+
 def test_block_batched_equals_per_token(gpu, be, synth):
     """tests/m9c of the reference: the batched body equals the per-token body.
     Here: selected ids are identical and outputs agree to BF16 tolerance when
