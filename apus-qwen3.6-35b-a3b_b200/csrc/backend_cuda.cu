@@ -316,6 +316,26 @@ struct Ordered {
     ~Ordered() { order_end(c, st); }
 };
 
+/* An exit in the middle of a call on host buffers leaves nothing under way: neither
+ * copies from or to the caller's memory nor kernels on the call's device buffers. */
+struct DrainOnError {
+    Ctx *c;
+    bool armed = true;
+    explicit DrainOnError(Ctx *c_) : c(c_) {}
+    int done() {
+        armed = false;
+        return 0;
+    }
+    ~DrainOnError() {
+        if (!armed) return;
+        cudaStreamSynchronize(c->stream);
+        if (c->s_in) cudaStreamSynchronize(c->s_in);
+        if (c->s_out) cudaStreamSynchronize(c->s_out);
+        for (cudaStream_t p : c->s_part)
+            if (p) cudaStreamSynchronize(p);
+    }
+};
+
 #define LAUNCHED()                                                         \
     do {                                                                   \
         g_ctx->launches++;                                                 \
@@ -589,6 +609,7 @@ static int dense_op(const uint16_t *w, const uint16_t *x, void *y, size_t M,
     c->last_block_launches = 0;
     Ordered ord(c, c->stream);
     if (ord.rc) return 1;
+    DrainOnError drain(c);
     const DevBuf *wb = weight_buf(c, w, O * K * 2);
     if (!wb) return 1;
     const size_t xb = M * K * 2, yb = M * O * (f32_out ? 4 : 2);
@@ -627,7 +648,7 @@ static int dense_op(const uint16_t *w, const uint16_t *x, void *y, size_t M,
             CU_OK(c->hs.download(y, dy, yb, c->stream));
             CU_OK(cudaStreamSynchronize(c->stream));
         }
-        return 0;
+        return drain.done();
     }
     for (size_t p = 0; p < parts; p++)
         if (!c->s_part[p])
@@ -658,7 +679,7 @@ static int dense_op(const uint16_t *w, const uint16_t *x, void *y, size_t M,
             CU_OK(c->hs.download(dst, (char *)dy + r0 * row, n * row, c->s_part[p]));
     }
     for (size_t p = 0; p < parts; p++) CU_OK(cudaStreamSynchronize(c->s_part[p]));
-    return 0;
+    return drain.done();
 }
 
 extern "C" int apus_cuda_bf16_gemv(const uint16_t *w, const uint16_t *x,
@@ -1887,6 +1908,7 @@ extern "C" int apus_cuda_moe_block(const ApusCudaMoeCfg *cfg,
     const size_t H = cfg->hidden, TK = cfg->top_k;
     Ordered ord(c, c->stream);
     if (ord.rc) return 1;
+    DrainOnError drain(c);
     size_t need = 2 * T * H * 2 + T * TK * 6 + 3 * T * H * 2 + 8192;
     if (arena_reserve(c->io, need)) return 1;
     c->io.reset();
@@ -1894,7 +1916,7 @@ extern "C" int apus_cuda_moe_block(const ApusCudaMoeCfg *cfg,
     uint16_t *dout = (uint16_t *)c->io.take(T * H * 2);
     const char *const st_at = (const char *)c->d_status;
     auto status_ok = [&](int st) -> int {
-        if (!st) return 0;
+        if (!st) return drain.done();
         cudaMemset(c->d_status, 0, 4);
         return fail("moe_block: device status %d (a bounded wait gave up or "
                     "an index was out of range)", st);
@@ -1905,7 +1927,7 @@ extern "C" int apus_cuda_moe_block(const ApusCudaMoeCfg *cfg,
         if (block_locked(L, dx, (uint16_t *)(st_at + STATUS_BYTES), T, nullptr, c->stream))
             return 1;
         CU_OK(c->hs.download_begin(0, st_at, STATUS_BYTES + T * H * 2, c->stream));
-        CU_OK(cudaEventSynchronize(c->hs.eout[0]));
+        CU_OK(c->hs.out_wait(0));
         int st;
         memcpy(&st, c->hs.out, 4);
         memcpy(moe_out, c->hs.out + STATUS_BYTES, T * H * 2);
@@ -1984,6 +2006,7 @@ extern "C" int apus_cuda_moe_block(const ApusCudaMoeCfg *cfg,
     }
     CU_OK(c->hs.download_begin(0, st_at, 4, c->stream));
     CU_OK(cudaStreamSynchronize(c->stream));
+    CU_OK(c->hs.out_wait(0));
     int st;
     memcpy(&st, c->hs.out, 4);
     if (tr && tr->moe_out) memcpy(tr->moe_out, moe_out, T * H * 2);

@@ -45,6 +45,7 @@ struct HostStage {
     char *out_dev = nullptr;                 /* the same memory as the GPU addresses it */
     cudaEvent_t ein[SLOTS] = {}, eout[SLOTS] = {};
     unsigned n_in = 0;                       /* slots handed to uploads so far */
+    bool out_busy[SLOTS] = {};               /* a copy into the slot may be under way */
 
     cudaError_t init() {
         if (in) return cudaSuccess;
@@ -66,6 +67,7 @@ struct HostStage {
             if (ein[i]) cudaEventDestroy(ein[i]);
             if (eout[i]) cudaEventDestroy(eout[i]);
             ein[i] = eout[i] = nullptr;
+            out_busy[i] = false;
         }
         in = out = out_dev = nullptr;
         n_in = 0;
@@ -106,16 +108,25 @@ struct HostStage {
         return cudaSuccess;
     }
     /* The two halves of a download of at most SLOT_BYTES into pageable memory, for
-     * callers with more to enqueue in between; one at a time per slot. */
+     * callers with more to enqueue in between; one at a time per slot.  A slot that an
+     * abandoned call left with a copy under way (on whatever stream) is waited for. */
     cudaError_t download_begin(int slot, const void *src, size_t bytes, cudaStream_t st) {
         cudaError_t e = init();
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(out + (size_t)slot * SLOT_BYTES, src, bytes,
-                                cudaMemcpyDeviceToHost, st);
-        return e == cudaSuccess ? cudaEventRecord(eout[slot], st) : e;
+        if (e == cudaSuccess && out_busy[slot]) e = out_wait(slot);
+        if (e != cudaSuccess) return e;
+        e = cudaMemcpyAsync(out + (size_t)slot * SLOT_BYTES, src, bytes, cudaMemcpyDeviceToHost,
+                            st);
+        if (e != cudaSuccess) return e;
+        out_busy[slot] = true;
+        return cudaEventRecord(eout[slot], st);
+    }
+    cudaError_t out_wait(int slot) {
+        const cudaError_t e = cudaEventSynchronize(eout[slot]);
+        if (e == cudaSuccess) out_busy[slot] = false;
+        return e;
     }
     cudaError_t download_end(int slot, void *dst, size_t bytes) {
-        cudaError_t e = cudaEventSynchronize(eout[slot]);
+        const cudaError_t e = out_wait(slot);
         if (e == cudaSuccess) host_copy(dst, out + (size_t)slot * SLOT_BYTES, bytes);
         return e;
     }
@@ -129,19 +140,14 @@ struct HostStage {
         const size_t piece = piece_of(bytes), count = (bytes + piece - 1) / piece;
         auto len = [&](size_t i) { return i + 1 < count ? piece : bytes - i * piece; };
         auto issue = [&](size_t i) {
-            const int s = (int)(i % SLOTS);
-            cudaError_t r = cudaMemcpyAsync(out + (size_t)s * SLOT_BYTES,
-                                            (const char *)src + i * piece, len(i),
-                                            cudaMemcpyDeviceToHost, st);
-            return r == cudaSuccess ? cudaEventRecord(eout[s], st) : r;
+            return download_begin((int)(i % SLOTS), (const char *)src + i * piece, len(i), st);
         };
         for (size_t i = 0; i < count && i < SLOTS; i++)
             if ((e = issue(i)) != cudaSuccess) return e;
         for (size_t i = 0; i < count; i++) {
-            const int s = (int)(i % SLOTS);
-            if ((e = cudaEventSynchronize(eout[s])) != cudaSuccess) return e;
-            host_copy((char *)dst + i * piece, out + (size_t)s * SLOT_BYTES, len(i));
-            if (i + SLOTS < count && (e = issue(i + SLOTS)) != cudaSuccess) return e;
+            e = download_end((int)(i % SLOTS), (char *)dst + i * piece, len(i));
+            if (e == cudaSuccess && i + SLOTS < count) e = issue(i + SLOTS);
+            if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
     }
