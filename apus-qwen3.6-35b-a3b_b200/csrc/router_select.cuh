@@ -116,8 +116,13 @@ __device__ __forceinline__ bool rt_needs(const uint32_t *cd, int e, int E, uint3
     return e <= E && !code_known(cd[e]) && (odd || e == E || code_key(cd[e] >> 16) >= kkey);
 }
 /* One warp, all codes of the selection known: its order and the renormalised weights
- * q_i / sum q in that order (the softmax denominator cancels; c/moe.h:363-370). */
-__device__ __forceinline__ void rt_weights(const uint32_t *cd, const int *sel, int TK, int lane,
+ * q_i / sum q in that order (c/moe.h:363-370).  The engine divides by the softmax
+ * denominator S first, p_i = q_i / S, and S cancels only up to the rounding of the p_i and
+ * of their sum: the quotients are within (2 TK + 2) 2^-24 of each other, and their BF16
+ * codes can differ by a step where one of them lies that near a midpoint (5e-4 of the
+ * weights for TK 8; 1.5e-5 do differ).  Returned: some quotient does.
+ * A caller that knows every logit of the token runs the engine's steps then. */
+__device__ __forceinline__ bool rt_weights(const uint32_t *cd, const int *sel, int TK, int lane,
                                            int32_t *idx_out, uint16_t *w_out) {
     const bool on = lane < TK;
     const int e = on ? sel[lane] : 0;
@@ -132,10 +137,13 @@ __device__ __forceinline__ void rt_weights(const uint32_t *cd, const int *sel, i
         const int src = __ffs(__ballot_sync(0xffffffffu, on && rank == i)) - 1;
         sw = __fadd_rn(sw, __shfl_sync(0xffffffffu, q, src));
     }
+    const float w = on ? __fdiv_rn(q, sw) : 0.0f;
     if (on) {
         idx_out[rank] = e;
-        if (w_out) w_out[rank] = bf16_bits(__fdiv_rn(q, sw));
+        if (w_out) w_out[rank] = bf16_bits(w);
     }
+    const int off = (int)(__float_as_uint(w) & 0xffffu) - 0x8000;
+    return __any_sync(0xffffffffu, on && abs(off) <= 2 * TK + 2) != 0;
 }
 
 /* n <= G exact chains by one warp, chain c's result in lane c.  The dependent add per

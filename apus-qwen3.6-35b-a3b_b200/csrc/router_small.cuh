@@ -22,8 +22,8 @@ namespace apus {
  * token (one atomic counter per token, which it resets for the next call) runs
  * that token's softmax / top-k on one of its warps.  No CTA ever waits on
  * another.  It decides on the BF16 codes of the logits and only where code order may
- * not decide runs the engine's softmax (router_select.cuh; softmax for all took 2 us
- * more).  Requires K % 8 == 0 and a 16-byte-aligned router matrix.
+ * not decide, or a weight might narrow differently, runs the engine's softmax
+ * (router_select.cuh; softmax for all took 2 us more).  Requires K % 8 == 0 and a 16-byte-aligned router matrix.
  * Dynamic shared memory: ROWS * (K*2 + 16) + 4 * ((K + 4) + (E + 1)) * 4 bytes.
  */
 constexpr int ROUTER_SMALL_TOK = 4;
@@ -156,13 +156,13 @@ router_small_kernel(const uint16_t *__restrict__ x,
         int32_t *idx = idx_out + (size_t)t * topk;
         uint16_t *wo = w_out ? w_out + (size_t)t * topk : nullptr;
         const Choice c = rt_select(cd, E, topk, lane, s_sel[tt]);
-        if (c.odd || __any_sync(0xffffffffu, nan)) {
+        if (c.odd || __any_sync(0xffffffffu, nan) ||
+            (rt_weights(cd, s_sel[tt], topk, lane, idx, wo) && wo)) {
+            __syncwarp();
             float *p = reinterpret_cast<float *>(cd);
             for (int e = lane; e < E; e += 32) p[e] = bf16lo(cd[e]);
             __syncwarp();
             router_softmax_topk(p, E, topk, lane, idx, wo);
-        } else {
-            rt_weights(cd, s_sel[tt], topk, lane, idx, wo);
         }
     }
 }

@@ -325,6 +325,51 @@ def test_router_few_tokens_at_the_shared_memory_limit(gpu, orc, be, synth, T, E,
     assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
 
 
+def _weights_at_midpoints(orc, synth, E, topk, n):
+    """n logit vectors [n, E] (BF16 codes) whose weights differ between the engine's
+    (q_i / S) / sum(q / S) and q_i / sum(q), with the engine's result for them."""
+    rng = np.random.default_rng(E + topk)
+    found, want = [], []
+    while sum(len(v) for v in found) < n:
+        z = synth.f32_to_bf16(rng.normal(0, 1, (200000, E)).astype(np.float32))
+        v = f32(z)
+        q = np.exp((v - v.max(1, keepdims=True)).astype(np.float64)).astype(np.float32)
+        order = np.argsort(-v, axis=1, kind="stable")[:, :topk]
+        S = np.zeros(len(q), np.float32)
+        for e in range(E):
+            S = S + q[:, e]
+        qs = np.take_along_axis(q, order, 1)
+        ps = np.take_along_axis(q / S[:, None], order, 1)
+        sq, sp = np.zeros(len(q), np.float32), np.zeros(len(q), np.float32)
+        for i in range(topk):
+            sq, sp = sq + qs[:, i], sp + ps[:, i]
+        w = synth.f32_to_bf16(ps / sp[:, None])
+        diff = (w != synth.f32_to_bf16(qs / sq[:, None])).any(1)
+        found.append(z[diff])
+        want.append(w[diff])
+    return np.concatenate(found)[:n], np.concatenate(want)[:n]
+
+
+@pytest.mark.parametrize("E,topk", [(16, 8), (40, 3)])
+def test_router_few_tokens_weights_follow_the_engines_steps(gpu, orc, be, synth, E, topk):
+    """Weights that narrow differently when the softmax denominator is left out of the
+    quotient; the logits are written into a router matrix that one-hot tokens read."""
+    T = K = 64
+    z, w = _weights_at_midpoints(orc, synth, E, topk, T)
+    x = np.zeros((T, K), np.uint16)
+    x[np.arange(T), np.arange(T)] = 0x3f80
+    cfg = dict(hidden=K, experts=E, moe_inter=8, shared_inter=8, top_k=topk)
+    W = synth.host_weights(be, cfg, seed=1, sigma=0.05)
+    W["rtr_w"] = np.ascontiguousarray(z.T)
+    eidx, ew = orc.route_batch(x, W["rtr_w"], topk)
+    same = (ew == w).all(1)              # the rest: expf differs in a last bit
+    assert same.mean() > 0.8
+    for t0, n in ((0, 64), (0, 9), (30, 33)):
+        gidx, gw = _route_dev(gpu, synth, cfg, W, x[t0:t0 + n])
+        assert np.array_equal(gidx, eidx[t0:t0 + n])
+        assert np.array_equal(gw[same[t0:t0 + n]], ew[t0:t0 + n][same[t0:t0 + n]])
+
+
 def test_router_certified_can_be_switched_off(be, orc, synth, monkeypatch):
     monkeypatch.setenv("APUS_CUDA_ROUTER_CERTIFY", "0")
     be.enable()
