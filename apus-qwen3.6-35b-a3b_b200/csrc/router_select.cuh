@@ -4,10 +4,12 @@
  *
  * The engine takes the top-k of its softmax PROBABILITIES.  exp and the division keep
  * the order of the BF16 logits whenever the logits near the top differ by 2^-18 or
- * more: two different BF16 values of one sign and of magnitude >= 2^-10 do, and so
- * does an exact zero from any of them; probabilities above exp(-80) do not
- * underflow.  Where that cannot be shown (`odd`), the caller runs the engine's
- * softmax on exact logits.
+ * more: two different BF16 values do unless both are smaller than 2^-10 in magnitude
+ * (the spacing below 2^-10 is 2^-18, and 2^-10 itself is that far from the next smaller
+ * one); probabilities above exp(-80) do not underflow.  So one small competitor is in
+ * its place among the others, and what does not compete is below the top_k-th as long as
+ * that one is not small itself.  Where order cannot be shown (`odd`), the caller runs the
+ * engine's softmax on exact logits.
  */
 #pragma once
 #include "common.cuh"
@@ -75,6 +77,7 @@ __device__ __forceinline__ Choice rt_select(const uint32_t *cd, int E, int TK, i
     Choice c;
     c.kkey = kth >> 16;
     bool open = false, odd = false, any = false;
+    int small = 0, zeros = 0;                            /* below 2^-10: nonzero, zero */
     float top = -INFINITY;
     uint32_t reach = 0;                                  /* bit i: expert lane + 32 i competes */
     if (regs) {
@@ -92,10 +95,13 @@ __device__ __forceinline__ Choice rt_select(const uint32_t *cd, int E, int TK, i
         any |= !known;
         if (!known && key_of(e) < kth) open = true;      /* not among the chosen */
         const float lo = bf16lo(v), hi = bf16hi(v);
-        const bool zero = known && (v & 0x7fffu) == 0;
         const bool plain = fabsf(lo) >= 9.765625e-4f && fabsf(hi) >= 9.765625e-4f &&
-                           (lo < 0.0f) == (hi < 0.0f) && fabsf(hi) <= 32.0f;
-        if (!plain && !(zero && code_key(v) != c.kkey)) odd = true;
+                           (lo < 0.0f) == (hi < 0.0f);
+        if (!(fabsf(lo) <= 32.0f && fabsf(hi) <= 32.0f)) odd = true;      /* or a NaN */
+        if (known && (v & 0x7fffu) == 0)
+            zeros++;
+        else if (!plain)                                 /* an interval around zero counts */
+            small++;
         top = fmaxf(top, hi);
     }
     __syncwarp();
@@ -103,7 +109,12 @@ __device__ __forceinline__ Choice rt_select(const uint32_t *cd, int E, int TK, i
     const int ti = __float_as_int(top);
     const int tm = __reduce_max_sync(0xffffffffu, ti >= 0 ? ti : ti ^ 0x7fffffff);
     top = __int_as_float(tm >= 0 ? tm : tm ^ 0x7fffffff);
-    if (!(key_value(c.kkey) - top >= -80.0f)) odd = true;
+    const float kval = key_value(c.kkey);
+    if (!(kval - top >= -80.0f) || fabsf(kval) < 9.765625e-4f) odd = true;
+    /* equal zeros tie, as their probabilities do; beside another small one they may not */
+    small = (int)__reduce_add_sync(0xffffffffu, (unsigned)small);
+    zeros = (int)__reduce_add_sync(0xffffffffu, (unsigned)zeros);
+    if (small > 1 || (small > 0 && zeros > 0)) odd = true;
     c.odd = __any_sync(0xffffffffu, odd);
     c.open = __any_sync(0xffffffffu, open);
     c.any = __any_sync(0xffffffffu, any) || c.odd || !code_known(cd[E]);

@@ -370,6 +370,43 @@ def test_router_few_tokens_weights_follow_the_engines_steps(gpu, orc, be, synth,
         assert np.array_equal(gw[same[t0:t0 + n]], ew[t0:t0 + n][same[t0:t0 + n]])
 
 
+@pytest.mark.parametrize("path,T,E,K", [("few", 64, 48, 64), ("certified", 256, 128, 256),
+                                        ("one kernel", 8, 128, 128)])
+@pytest.mark.parametrize("seed", range(3))
+def test_router_small_logits_in_any_company(gpu, orc, be, synth, path, T, E, K, seed):
+    """Logits around 2^-10, below which two of them may have the same probability: one small
+    competitor among others, several, beside zeros of either sign, as the last one chosen and
+    right below it.  One-hot tokens read the logits from the router matrix."""
+    rng = np.random.default_rng(seed)
+    edge = 2.0 ** -10
+    small = [0.0, -0.0, edge, -edge, edge * (1 + 2 ** -7), edge * (1 - 2 ** -8), 2 ** -11,
+             -edge * (1 - 2 ** -8), 1e-5, 1.01e-5, -1e-5, 3e-20, -3e-20, 2e-38]
+    z = rng.normal(-1.0, 1.0, (T, E))
+    for t in range(T):
+        n, top = int(rng.integers(0, 8)), int(rng.integers(0, 9))
+        where = rng.permutation(E)
+        z[t] = np.where(z[t] > -0.01, z[t] - 3.0, z[t])          # all others below
+        z[t, where[:top]] = rng.uniform(0.01, 2.0, top)          # so many above
+        z[t, where[top:top + n]] = rng.choice(small, n)
+    z = synth.f32_to_bf16(z.astype(np.float32))
+    x = np.zeros((T, K), np.uint16)
+    x[np.arange(T), np.arange(T)] = 0x3f80
+    cfg = dict(hidden=K, experts=E, moe_inter=16, shared_inter=16, top_k=8)
+    W = synth.host_weights(be, cfg, seed=1, sigma=0.05)
+    W["rtr_w"] = np.zeros((E, K), np.uint16)
+    W["rtr_w"][:, :T] = z.T
+    eidx, ew = orc.route_batch(x, W["rtr_w"], 8)
+    if path == "one kernel":
+        got = gpu.moe_block(cfg, W, x)
+        assert gpu.last_block_path() == 0
+        gidx, gw = got["idx"], got["w"]
+    else:
+        gidx, gw = _route_dev(gpu, synth, cfg, W, x)
+    assert gpu.last_block_status() == 0
+    assert np.array_equal(gidx, eidx)
+    assert np.abs(gw.astype(np.int32) - ew.astype(np.int32)).max() <= 1
+
+
 def test_router_certified_can_be_switched_off(be, orc, synth, monkeypatch):
     monkeypatch.setenv("APUS_CUDA_ROUTER_CERTIFY", "0")
     be.enable()
