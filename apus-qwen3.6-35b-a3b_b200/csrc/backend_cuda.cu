@@ -774,20 +774,40 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         ca.status = c->d_status;
         ca.stats = c->d_rc_stats;
         ca.lr = LaneRow(K);
-        /* one warp per token.  Too few tokens to fill the SMs: deep rings, which hide
-         * the rows' latency where a full SM hides it behind other warps. */
+        /* One warp per token, two tokens a CTA where there are more tokens than SMs.  A
+         * warp's ring of rows hides their latency where other warps do not: the deepest
+         * with which all tokens still run at once, else two rows.  (1000 skewed tokens:
+         * 48 us with two, 41 with four; 1500: 57 and, with three, 49; 888: 44 and, with
+         * six, 40; where a second wave begins the deeper ring loses, 8192: 166 and 174.)
+         * Likewise the chains, one to a lane where all tokens run at once (512: 44 -> 37
+         * us, 2000: 62 -> 57, skewed), with the warp's help else (3000: 90 -> 83). */
         const int warps = T <= c->sm_count ? 1 : RC_WARPS;
-        const bool deep = T <= 6 * c->sm_count && K == 2048 && E <= 256;
-        void (*kern)(CertifyArgs) = E > 256     ? router_certify_kernel<32, 0, 2>
-                                    : deep      ? router_certify_kernel<8, 8, 6>
-                                    : K == 2048 ? router_certify_kernel<8, 8, 2>
-                                                : router_certify_kernel<8, 0, 2>;
-        const size_t smem = router_certify_smem(E, K, deep ? 6 : 2) * warps;
+        auto at_once = [&](int slots) {
+            return T <= c->sm_count * RC_WARPS *
+                            (int)(c->smem_sm / (router_certify_smem(E, K, slots) * RC_WARPS + 1280));
+        };
+        int ring = 2;
+        if (K == 2048 && E <= 256)
+            for (int d : {3, 4, 6})
+                if (at_once(d)) ring = d;
+        void (*kern)(CertifyArgs) = E > 256       ? router_certify_kernel<32, 0, 2, false>
+                                    : K != 2048   ? router_certify_kernel<8, 0, 2, false>
+                                    : ring == 6   ? router_certify_kernel<8, 8, 6, true>
+                                    : ring == 4   ? router_certify_kernel<8, 8, 4, true>
+                                    : ring == 3   ? router_certify_kernel<8, 8, 3, true>
+                                    : at_once(2)  ? router_certify_kernel<8, 8, 2, true>
+                                                  : router_certify_kernel<8, 8, 2, false>;
+        const size_t smem = router_certify_smem(E, K, ring) * warps;
         const size_t most = router_certify_smem(E, K, 6) * RC_WARPS;
         static size_t set_smem = 0;
         if (most > set_smem) {
-            for (auto k : {router_certify_kernel<32, 0, 2>, router_certify_kernel<8, 8, 6>,
-                           router_certify_kernel<8, 8, 2>, router_certify_kernel<8, 0, 2>})
+            for (auto k : {router_certify_kernel<32, 0, 2, false>,
+                           router_certify_kernel<8, 0, 2, false>,
+                           router_certify_kernel<8, 8, 2, false>,
+                           router_certify_kernel<8, 8, 2, true>,
+                           router_certify_kernel<8, 8, 3, true>,
+                           router_certify_kernel<8, 8, 4, true>,
+                           router_certify_kernel<8, 8, 6, true>})
                 CU_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)most));
             set_smem = most;

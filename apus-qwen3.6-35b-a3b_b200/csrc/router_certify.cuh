@@ -97,8 +97,9 @@ inline size_t router_certify_smem(int E, int K, int slots) {
 
 /* grid = ceil(T / warps); E % 32 == 0, K % 256 == 0.  R: experts per lane, at least
  * E / 32; NU: 16-byte pieces of a lane's chunk that are kept in registers (K / 256),
- * 0: any K, the token is read again for each candidate; D: ring slots. */
-template <int R, int NU, int D>
+ * 0: any K, the token is read again for each candidate; D: ring slots; LANES: chains one to
+ * a lane (lane_chain) and not with the warp's help (warp_chains). */
+template <int R, int NU, int D, bool LANES>
 __global__ void __launch_bounds__(RC_WARPS * 32, 16 / RC_WARPS)
 router_certify_kernel(const __grid_constant__ CertifyArgs a) {
     /* the next kernel may be scheduled; this kernel's own wait for the fast-logit
@@ -310,9 +311,22 @@ router_certify_kernel(const __grid_constant__ CertifyArgs a) {
     int *sel = s_sel[warp];
     Choice ch = rt_select(cd, E, TK, lane, sel);
     if (ch.any) {
-        resolve_chains(cd, cand, n_eval, E, K, ch.kkey, ch.odd, lane,
-                       reinterpret_cast<float *>(slots), row_of,
-                       [&](int p) { return ldg16(a.x + (size_t)t * K + p * 8); });
+        float *buf = reinterpret_cast<float *>(slots);
+        auto xpiece = [&](int p) { return ldg16(a.x + (size_t)t * K + p * 8); };
+        if (LANES) {
+            for (int p = lane; p < K / 8; p += 32) {     /* the token in fp32 */
+                float f[8];
+                unpack8(xpiece(p), f);
+                float4 *d = reinterpret_cast<float4 *>(buf + p * 8);
+                d[0] = make_float4(f[0], f[1], f[2], f[3]);
+                d[1] = make_float4(f[4], f[5], f[6], f[7]);
+            }
+            __syncwarp();
+            resolve_lanes(cd, cand, n_eval, E, K, ch.kkey, ch.odd, lane, buf,
+                          ok && (ok_extra || !a.extra_row), row_of);
+        } else {
+            resolve_chains(cd, cand, n_eval, E, K, ch.kkey, ch.odd, lane, buf, row_of, xpiece);
+        }
         if (ch.open && !ch.odd) rt_select(cd, E, TK, lane, sel);
         __syncwarp();
     }

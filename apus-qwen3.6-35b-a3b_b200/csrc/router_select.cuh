@@ -229,12 +229,60 @@ __device__ __forceinline__ float warp_chains(int n, int K, int lane, float *buf,
     }
     return acc;
 }
-/* Resolves the logits that rt_needs names of list[0 .. n-1]: their codes become known.  row(e): weight row in global memory. */
-template <typename Row, typename XPiece>
-__device__ __forceinline__ int resolve_chains(uint32_t *cd, const uint16_t *list, int n, int E,
+/* One chain per lane: weight row in global memory (16-byte pieces, sixteen of them under
+ * way), token in fp32 in shared memory; K % 128 == 0.  Eight steps are 37 cycles of
+ * dependent adds and 19 instructions for the warp, whatever its lanes are doing; no barrier
+ * on the way, and up to 32 chains at once.  The better form where the SM has issue slots to
+ * spare; warp_chains where it is full. */
+template <bool FMA>
+__device__ __forceinline__ float lane_chain(const uint16_t *w, const float *xs, int K) {
+    constexpr int AHEAD = 16;
+    uint4 q[AHEAD];
+#pragma unroll
+    for (int c = 0; c < AHEAD; c++) q[c] = ldg16(w + c * 8);
+    float acc = 0.0f;
+#pragma unroll 1
+    for (int k = 0; k < K; k += AHEAD * 8) {
+        const int next = k + AHEAD * 8 < K ? AHEAD * 8 : 0;
+        const float4 *x4 = reinterpret_cast<const float4 *>(xs + k);
+#pragma unroll
+        for (int c = 0; c < AHEAD; c++) {
+            float wf[8];
+            unpack8(q[c], wf);
+            q[c] = ldg16(w + k + next + c * 8);
+            const float4 a = x4[2 * c], b = x4[2 * c + 1];
+            const float xf[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc = exact_step<FMA>(wf[j], xf[j], acc);
+        }
+    }
+    return acc;
+}
+/* Both resolve the logits that rt_needs names of list[0 .. n-1]: their codes become known.
+ * row(e): weight row in global memory.  One chain to a lane; xs: the token in fp32, exact: no
+ * product rounds. */
+template <typename Row>
+__device__ __forceinline__ void resolve_lanes(uint32_t *cd, const uint16_t *list, int n, int E,
                                               int K, uint32_t kkey, bool odd, int lane,
-                                              float *buf, Row row, XPiece xpiece) {
-    int chains = 0;
+                                              const float *xs, bool exact, Row row) {
+#pragma unroll 1
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const int mine = c0 + lane < n ? list[c0 + lane] : E + 1;
+        const bool need = rt_needs(cd, mine, E, kkey, odd);
+        const unsigned m = __ballot_sync(0xffffffffu, need);
+        if (!m) continue;
+        /* the other lanes read along with the first */
+        const int first = __shfl_sync(0xffffffffu, mine, __ffs(m) - 1), e = need ? mine : first;
+        const float z = exact ? lane_chain<true>(row(e), xs, K) : lane_chain<false>(row(e), xs, K);
+        if (need) cd[e] = 0x10001u * bf16_bits(z);
+        __syncwarp();
+    }
+}
+/* The warp's help for up to CH_CHAINS at a time. */
+template <typename Row, typename XPiece>
+__device__ __forceinline__ void resolve_chains(uint32_t *cd, const uint16_t *list, int n, int E,
+                                               int K, uint32_t kkey, bool odd, int lane,
+                                               float *buf, Row row, XPiece xpiece) {
 #pragma unroll 1
     for (int c0 = 0; c0 < n; c0 += 32) {
         const int e = c0 + lane < n ? list[c0 + lane] : E + 1;
@@ -249,11 +297,9 @@ __device__ __forceinline__ int resolve_chains(uint32_t *cd, const uint16_t *list
                 [&](int c) { return row(__shfl_sync(0xffffffffu, mine, c)); }, xpiece);
             if (lane < now) cd[mine] = 0x10001u * bf16_bits(z);
             __syncwarp();
-            chains += now;
             m &= ~__reduce_or_sync(0xffffffffu, lane < now ? 1u << src : 0u);
         }
     }
-    return chains;
 }
 /* a row of global memory into a LaneRow, by one warp (asynchronously; the caller
  * commits and waits) */

@@ -325,6 +325,22 @@ def test_router_few_tokens_at_the_shared_memory_limit(gpu, orc, be, synth, T, E,
     assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
 
 
+@pytest.mark.parametrize("T", [1184, 1185, 1776, 1777, 2368, 2369])
+def test_router_certified_ring_and_chain_forms(gpu, orc, be, synth, T):
+    """Both sides of the token counts at which the ring of rows gets shallower (1184, 1776)
+    and the chains change their form (2368), with a router that leaves many logits open."""
+    cfg = dict(hidden=2048, experts=256, moe_inter=8, shared_inter=8, top_k=8)
+    W = synth.host_weights(be, cfg, seed=T, sigma=0.02)
+    x = synth.host_x(be, T, 2048, seed=T)
+    W, x = synth.apply_router_bias(W, x, synth.zipf_bias(cfg, seed=3, beta=0.27))
+    idx, w = _route_dev(gpu, synth, cfg, W, x)
+    assert gpu.last_block_status() == 0
+    eidx, ew = orc.route_batch(x, W["rtr_w"], 8)
+    assert np.array_equal(idx, eidx)
+    d = np.abs(w.astype(np.int32) - ew.astype(np.int32))
+    assert d.max() <= 1 and (d != 0).mean() <= 0.002
+
+
 def _weights_at_midpoints(orc, synth, E, topk, n):
     """n logit vectors [n, E] (BF16 codes) whose weights differ between the engine's
     (q_i / S) / sum(q / S) and q_i / sum(q), with the engine's result for them."""
