@@ -2702,13 +2702,19 @@ extern "C" int apus_cuda_bf16_gemv_dev(const uint16_t *d_w, const uint16_t *d_x,
     if (ctx_init()) return 1;
     Ctx *c = g_ctx;
     cudaStream_t st = (cudaStream_t)stream;
-    /* as many warps as keep every SM busy, at most what fits beside x */
-    const size_t groups = (O + 15) / 16;
-    int warps = 8;
-    while (warps > 1 && (groups <= (size_t)c->sm_count * (warps / 2) ||
-                         gemv_stream_smem((int)M, (int)K, warps) > (size_t)c->smem_optin))
-        warps /= 2;
-    const size_t smem = gemv_stream_smem((int)M, (int)K, warps);
+    /* Eight warps a CTA where that leaves no SM without one, at most what fits beside x;
+     * with fewer groups of sixteen rows than warps, several share a group, as long as each
+     * has its four slots to fill. */
+    const size_t groups = (O + 15) / 16, slots = K / GV_BK, sms = (size_t)c->sm_count;
+    int warps = 8, split = 1;
+    while (2 * split <= warps && 2 * split * groups <= sms * warps && 4 * (size_t)split <= slots)
+        split *= 2;
+    while (warps > split && groups * split <= sms * (warps / 2)) warps /= 2;
+    while (warps > 1 && gemv_stream_smem((int)M, (int)K, warps, split) > (size_t)c->smem_optin) {
+        warps = split > 1 ? warps / 2 : warps - 1;
+        if (split > warps) split = warps;
+    }
+    const size_t smem = gemv_stream_smem((int)M, (int)K, warps, split);
     if (smem > (size_t)c->smem_optin) return fail("gemv_dev: M * K too large");
     static size_t set_smem = 0;
     if (smem > set_smem) {
@@ -2716,9 +2722,10 @@ extern "C" int apus_cuda_bf16_gemv_dev(const uint16_t *d_w, const uint16_t *d_x,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         set_smem = smem;
     }
-    const size_t want = (groups + warps - 1) / warps;
-    const unsigned grid = (unsigned)(want < (size_t)c->sm_count ? want : (size_t)c->sm_count);
-    gemv_stream_kernel<<<grid, warps * 32, smem, st>>>(d_w, d_x, d_y, (int)M, (long)O, (int)K);
+    const size_t want = (groups * split + warps - 1) / warps;
+    const unsigned grid = (unsigned)(want < sms ? want : sms);
+    gemv_stream_kernel<<<grid, warps * 32, smem, st>>>(d_w, d_x, d_y, (int)M, (long)O, (int)K,
+                                                       split);
     LAUNCHED();
     return 0;
 }

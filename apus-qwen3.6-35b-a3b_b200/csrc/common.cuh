@@ -187,6 +187,16 @@ __device__ __forceinline__ void mma_16x8(float (&c)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b_lo), "r"(b_hi));
 }
 
+/* D = A B */
+__device__ __forceinline__ void mma_16x8_first(float (&d)[4], const uint32_t (&a)[4],
+                                               uint32_t b_lo, uint32_t b_hi) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, "
+        "{%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b_lo), "r"(b_hi), "f"(0.0f));
+}
+
 /* 16-byte read-only global load */
 __device__ __forceinline__ uint4 ldg16(const void *p) {
     return __ldg(reinterpret_cast<const uint4 *>(p));

@@ -68,8 +68,8 @@ exact_matvec_f32_kernel(const uint16_t *__restrict__ w,
  * them per slot into a ring of its own (cp.async, whole 256-byte pieces of a row), four
  * slots ahead; mma.sync m16n8k16 multiplies them with all rows of x at once (columns past
  * M repeat the last row and are not stored), so eight rows cost what one does.  Scalar
- * multiply-adds on rows loaded straight into registers took 179 us for one row and 783 for
- * eight (O 248320, K 2048); this 176 and 183 (5.8 of 6.5 TB/s).
+ * multiply-adds on rows loaded straight into registers took 174 us for one row and 780 for
+ * eight (O 248320, K 2048); this 174 and 182 (5.8 of 6.5 TB/s).
  * mma.sync cuts off what its accumulator cannot hold, so two steps share one that starts
  * at zero and the rest is a tree: at K 2048 1.0e-4 of the results narrow to another BF16
  * value than 64-bit sums do, as in the scalar form (6e-4 with all 64 steps on one); at
@@ -81,29 +81,39 @@ constexpr int GV_BK = 128;
 constexpr int GV_PITCH = GV_BK * 2 + 16;         /* ldmatrix rows in different banks */
 constexpr int GV_SLOT = 16 * GV_PITCH;
 constexpr int GV_STAGES = 5;
-inline size_t gemv_stream_smem(int M, int K, int warps) {
-    return (size_t)M * (2 * (size_t)K + 16) + (size_t)warps * GV_STAGES * GV_SLOT;
+/* Too few rows for all warps: `split` of them (a power of two) share sixteen rows, each
+ * with a part of K, and add up in shared memory; one warp alone is bound by the latency of
+ * its four slots (2048 rows of 2048: 8.4 us for one row of x and 12.3 for eight; shared 4.3
+ * and 6.3, the scalar form 4.5 and 19). */
+constexpr int GV_PART = 16 * 8 * 4;
+inline size_t gemv_stream_smem(int M, int K, int warps, int split) {
+    return (size_t)M * (2 * (size_t)K + 16) +
+           (size_t)warps * (GV_STAGES * GV_SLOT + (split > 1 ? GV_PART : 0));
 }
 
 __global__ void __launch_bounds__(256)
 gemv_stream_kernel(const uint16_t *__restrict__ w, const uint16_t *__restrict__ x,
-                   uint16_t *__restrict__ y, int M, long O, int K) {
+                   uint16_t *__restrict__ y, int M, long O, int K, int split) {
     extern __shared__ __align__(16) unsigned char gv_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int team = warp / split, part = warp - team * split, teams = warps / split;
     const int x_pitch = 2 * K + 16;
     const uint32_t ring = smem_u32(gv_smem) + (uint32_t)(M * x_pitch + warp * GV_STAGES * GV_SLOT);
-    /* Sixteen rows per warp and round, the warps side by side; what the last whole round
+    float *sums = reinterpret_cast<float *>(gv_smem + (size_t)M * x_pitch +
+                                            (size_t)warps * GV_STAGES * GV_SLOT) +
+                  (size_t)warp * (GV_PART / 4);
+    /* Sixteen rows per team and round, the teams side by side; what the last whole round
      * leaves is dealt evenly, in pieces of fewer rows (those missing are not fetched, what
      * lies in their place is not stored). */
-    const long nw = (long)gridDim.x * warps, id = (long)warp * gridDim.x + blockIdx.x;
+    const long nw = (long)gridDim.x * teams, id = (long)team * gridDim.x + blockIdx.x;
     const long rounds = O / (16 * nw), base = rounds * 16 * nw, left = O - base;
     const long rest0 = base + left * id / nw, rest1 = base + left * (id + 1) / nw;
     auto first = [&](long i) { return i < rounds ? (i * nw + id) * 16 : rest0; };
     auto end = [&](long i) { return i < rounds ? (i * nw + id) * 16 + 16 : rest1; };
     const long mine = rounds + (rest1 > rest0 ? 1 : 0);
-    const int nkb = K / GV_BK;
+    const int kb0 = K / GV_BK * part / split, kb1 = K / GV_BK * (part + 1) / split;
     long i_i = 0;
-    int i_kb = 0, i_s = 0;
+    int i_kb = kb0, i_s = 0;
     auto issue = [&]() {
         if (i_i < mine) {
             const long i_o = first(i_i), i_end = end(i_i);
@@ -117,8 +127,8 @@ gemv_stream_kernel(const uint16_t *__restrict__ w, const uint16_t *__restrict__ 
                     cp_async16_to(dst + (uint32_t)(r * GV_PITCH),
                                   w + o * K + i_kb * GV_BK + c * 8);
             }
-            if (++i_kb == nkb) {
-                i_kb = 0;
+            if (++i_kb == kb1) {
+                i_kb = kb0;
                 i_i++;
             }
             if (++i_s == GV_STAGES) i_s = 0;
@@ -148,23 +158,25 @@ gemv_stream_kernel(const uint16_t *__restrict__ w, const uint16_t *__restrict__ 
         const long o0 = first(i), o_end = end(i);
         float c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
 #pragma unroll 1
-        for (int kb = 0; kb < nkb; kb++) {
+        for (int kb = kb0; kb < kb1; kb++) {
             asm volatile("cp.async.wait_group %0;" ::"n"(GV_STAGES - 2) : "memory");
             __syncwarp();      /* everyone's pieces landed; the oldest slot is read out */
             issue();
             const uint32_t at = ring + (uint32_t)(s * GV_SLOT) + a_off;
+            /* everything is read before the first product, and no product waits for the one
+             * before it (the warp issues in order) */
+            uint32_t a0[4][4], a1[4][4], b[4][4];
             float p[4][4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                uint32_t a0[4], a1[4], b[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) p[j][q] = 0.0f;
-                ldmatrix_x4(b, b_at + (uint32_t)((kb * GV_BK + j * 32) * 2));
-                ldmatrix_x4(a0, at + (uint32_t)(j * 64));
-                ldmatrix_x4(a1, at + (uint32_t)(j * 64 + 32));
-                mma_16x8(p[j], a0, b[0], b[1]);
-                mma_16x8(p[j], a1, b[2], b[3]);
+                ldmatrix_x4(b[j], b_at + (uint32_t)((kb * GV_BK + j * 32) * 2));
+                ldmatrix_x4(a0[j], at + (uint32_t)(j * 64));
+                ldmatrix_x4(a1[j], at + (uint32_t)(j * 64 + 32));
             }
+#pragma unroll
+            for (int j = 0; j < 4; j++) mma_16x8_first(p[j], a0[j], b[j][0], b[j][1]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) mma_16x8(p[j], a1[j], b[j][2], b[j][3]);
             const bool fold = (kb & 3) == 3;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -177,10 +189,27 @@ gemv_stream_kernel(const uint16_t *__restrict__ w, const uint16_t *__restrict__ 
             if (++s == GV_STAGES) s = 0;
         }
 #pragma unroll
+        for (int q = 0; q < 4; q++) c0[q] += c1[q];
+        if (split > 1) {
+            *reinterpret_cast<float4 *>(sums + lane * 4) = make_float4(c0[0], c0[1], c0[2], c0[3]);
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(split * 32) : "memory");
+            if (part == 0)
+                for (int p = 1; p < split; p++) {
+                    const float4 v =
+                        *reinterpret_cast<const float4 *>(sums + p * (GV_PART / 4) + lane * 4);
+                    c0[0] += v.x;
+                    c0[1] += v.y;
+                    c0[2] += v.z;
+                    c0[3] += v.w;
+                }
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(split * 32) : "memory");
+            if (part) continue;
+        }
+#pragma unroll
         for (int q = 0; q < 4; q++) {
             const long o = o0 + (lane >> 2) + (q >> 1) * 8;
             const int m = (lane & 3) * 2 + (q & 1);
-            if (o < o_end && m < M) y[(size_t)m * O + o] = bf16_bits(c0[q] + c1[q]);
+            if (o < o_end && m < M) y[(size_t)m * O + o] = bf16_bits(c0[q]);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");

@@ -497,7 +497,11 @@ def test_rmsnorm_sum_without_the_chain(gpu, orc, N):
 @pytest.mark.parametrize("M,O,K,shift", [
     (1, 15, 256, 0), (5, 16, 512, 0), (7, 17, 2304, 0), (8, 148 * 16, 256, 0),
     (4, 148 * 16 * 8 + 5, 256, 0), (6, 148 * 16 * 8 * 2 - 1, 256, 0), (2, 31, 16384, 0),
-    (8, 40, 7168, 0), (3, 100, 512, 1)])
+    (8, 40, 7168, 0), (3, 100, 512, 1),
+    # warps that share sixteen rows: eight, four and two of them, K that they do not divide
+    (1, 148 * 16, 1280, 0), (3, 148 * 16 + 1, 2048, 0), (8, 148 * 32, 4096, 0),
+    (2, 148 * 32 + 9, 768, 1), (5, 148 * 64 - 3, 2304, 0), (1, 148 * 64 + 1, 512, 0),
+    (1, 9, 58112, 0), (8, 700, 7168, 0)])
 def test_gemv_stream_edges(gpu, orc, M, O, K, shift):
     """Whole rounds, remainders and fewer rows than warps; x beside a smaller ring; x that
     is not 16-byte aligned.  Both sums are fp32 over K exact products: they differ by at
