@@ -1570,12 +1570,16 @@ static bool fused_supported(Ctx *c, const ApusCudaMoeCfg &cfg, size_t T) {
     return (size_t)L.total <= dynamic_smem_limit(c, (const void *)decode_fused_kernel);
 }
 
-/* rows of whole 16-byte pieces: one warp per row without the sequential chain;
- * others: the plain kernel */
+/* Rows of whole 16-byte pieces in enough lane chunks: one warp per row without the
+ * sequential chain; others: the plain kernel.  N 1152 (16 chunks): 13.1 us at 2000 rows
+ * against 13.4; N 1088 (8): 8.4 against 10.3 at 512 rows, 17 against 13 at 2000; N 2040 (1):
+ * 29 against 14.5.  Short rows have little chain to save: N 256 at 8192 rows 13 us against
+ * 10, N 512 15.5 against 18.6. */
 static int launch_rmsnorm(Ctx *c, const uint16_t *x, const uint16_t *w, uint16_t *y, int T, int N,
                           cudaStream_t st) {
     const size_t rows = (size_t)RN_WARPS * LaneRow(N).bytes();
-    if (N % 8 == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) == 0 &&
+    const int chunks = LaneRow(N).nl;
+    if (N >= 512 && N % 8 == 0 && (chunks >= 16 || (chunks == 8 && T <= 4 * c->sm_count)) && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) == 0 &&
         rows <= 40 * 1024) {
         launch_k(rmsnorm_rows_kernel, dim3((T + RN_WARPS - 1) / RN_WARPS), dim3(RN_WARPS * 32),
                  rows, st, x, w, y, T, N, LaneRow(N));
