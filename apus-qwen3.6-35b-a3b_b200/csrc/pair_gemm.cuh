@@ -563,11 +563,16 @@ pair_gemm_kernel(const __grid_constant__ PairMaps mapA,        /* xg | act   (to
 
 /* ---- host side ---------------------------------------------------------------- */
 inline int g_pp_enable = 1;          /* APUS_CUDA_PAIR=0: never take this path */
-inline int g_pp_min_rows = 104;      /* mean rows per resident expert from which it is taken:
-                                      * block at 94 rows 453 us against 434 of the one-SM
-                                      * kernels (skewed: 505 against 515), at 109 471
-                                      * against 475 (533, 550), at 156 554 against 609 */
-inline int g_pp_swap_below = 192;    /* APUS_CUDA_PAIR_SWAP_BELOW: see PairPlan */
+/* Mean rows per resident expert from which it is taken.  us of the one-SM kernels against
+ * these, block, even router (experts alone): 112 rows 501, 519 (397, 404); 128 543, 539
+ * (431, 436); 144 615, 565 (488, 456); 160 672, 602.  Hidden 4096, width 768: 112 833, 825
+ * (514, 561); 128 865, 816 (560, 620); 160 1017, 894 (629, 587).  A skewed router gains
+ * earlier (112: 548, 522; 96: 493, 506). */
+inline int g_pp_min_rows = 136;
+/* Last chunks of fewer rows are taken as N (APUS_CUDA_PAIR_SWAP_BELOW).  8192 skewed tokens:
+ * never 912 us, below 64 911, 128 896, 160 891, 192 869, 224 860, 256 (always) 886; 144 rows
+ * an expert, skewed: 655, 589, 571, 618, 603, 586, 625. */
+inline int g_pp_swap_below = 192;
 
 inline bool pair_supported(const ApusCudaMoeCfg &c, int sm_count, int smem_optin) {
     return g_pp_enable && prefill_supported(c) && c.hidden % PP_BN == 0 &&
