@@ -629,7 +629,8 @@ static int dense_op(const uint16_t *w, const uint16_t *x, void *y, size_t M,
     /* Many rows: the call is cut into parts on streams of their own, so that the
      * rows of one part travel while another computes.  A part fills only its share
      * of the SMs; the parts' kernels run beside each other. */
-    const size_t parts = K % 8 == 0 && M >= DENSE_PARTS * 64 && xb >= (512u << 10) ? DENSE_PARTS : 1;
+    const bool cut = K % 8 == 0 && M >= DENSE_PARTS * 64 && xb >= (512u << 10);
+    const size_t parts = cut ? DENSE_PARTS : 1;
     /* A small result, or one row of any size the slots hold, is stored straight
      * into page-locked memory by the kernel: one operation less between the last
      * chain and the caller.  (Several large rows go over PCIe as 64-byte stores
@@ -1579,8 +1580,9 @@ static int launch_rmsnorm(Ctx *c, const uint16_t *x, const uint16_t *w, uint16_t
                           cudaStream_t st) {
     const size_t rows = (size_t)RN_WARPS * LaneRow(N).bytes();
     const int chunks = LaneRow(N).nl;
-    if (N >= 512 && N % 8 == 0 && (chunks >= 16 || (chunks == 8 && T <= 4 * c->sm_count)) && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) == 0 &&
-        rows <= 40 * 1024) {
+    const bool enough = chunks >= 16 || (chunks == 8 && T <= 4 * c->sm_count);
+    if (N >= 512 && N % 8 == 0 && enough && rows <= 40 * 1024 &&
+        (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) == 0) {
         launch_k(rmsnorm_rows_kernel, dim3((T + RN_WARPS - 1) / RN_WARPS), dim3(RN_WARPS * 32),
                  rows, st, x, w, y, T, N, LaneRow(N));
         LAUNCHED();

@@ -408,10 +408,12 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
                 e == E ? products_exact(a.wmin_gate, a.wmax_gate, s_xlo[t], s_xhi[t])
                        : products_exact(a.wmin, a.wmax, s_xlo[t], s_xhi[t]);
             uint32_t v = CODE_UNKNOWN;
-            if (exact)                       v = certified_logit(rr + r * L.xrow, xs + t * L.xrow, lr, lane,
-                                    (e == E ? a.wnorm_gate : __ldg(&a.wnorm[e])) *
-                                        norm_above(s_sq[0][t] +
-                                                       (lr.nu % 2 == 0 ? s_sq[1][t] : 0.0f), H));
+            if (exact) {
+                const float sq = s_sq[0][t] + (lr.nu % 2 == 0 ? s_sq[1][t] : 0.0f),
+                            wn = e == E ? a.wnorm_gate : __ldg(&a.wnorm[e]);
+                v = certified_logit(rr + r * L.xrow, xs + t * L.xrow, lr, lane,
+                                    wn * norm_above(sq, H));
+            }
             if (lane == 0) a.code_ws[(size_t)t * (E + 1) + e] = v;
         }
     __syncthreads();

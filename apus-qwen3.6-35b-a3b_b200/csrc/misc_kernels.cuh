@@ -18,24 +18,8 @@ __device__ __forceinline__ float exact_dot(const uint16_t *__restrict__ wrow,
                                            const uint16_t *__restrict__ xrow,
                                            int K) {
     float acc = 0.0f;
-    int k = 0;
-    if ((K & 7) == 0 && ((((uintptr_t)wrow) | ((uintptr_t)xrow)) & 15) == 0) {
-        for (; k < K; k += 8) {
-            uint4 wv = ldg16(wrow + k), xv = ldg16(xrow + k);
-            acc = __fadd_rn(acc, __fmul_rn(bf16lo(wv.x), bf16lo(xv.x)));
-            acc = __fadd_rn(acc, __fmul_rn(bf16hi(wv.x), bf16hi(xv.x)));
-            acc = __fadd_rn(acc, __fmul_rn(bf16lo(wv.y), bf16lo(xv.y)));
-            acc = __fadd_rn(acc, __fmul_rn(bf16hi(wv.y), bf16hi(xv.y)));
-            acc = __fadd_rn(acc, __fmul_rn(bf16lo(wv.z), bf16lo(xv.z)));
-            acc = __fadd_rn(acc, __fmul_rn(bf16hi(wv.z), bf16hi(xv.z)));
-            acc = __fadd_rn(acc, __fmul_rn(bf16lo(wv.w), bf16lo(xv.w)));
-            acc = __fadd_rn(acc, __fmul_rn(bf16hi(wv.w), bf16hi(xv.w)));
-        }
-    } else {
-        for (; k < K; k++)
-            acc = __fadd_rn(acc, __fmul_rn(bf16_f32(__ldg(wrow + k)),
-                                           bf16_f32(__ldg(xrow + k))));
-    }
+    for (int k = 0; k < K; k++)
+        acc = __fadd_rn(acc, __fmul_rn(bf16_f32(__ldg(wrow + k)), bf16_f32(__ldg(xrow + k))));
     return acc;
 }
 

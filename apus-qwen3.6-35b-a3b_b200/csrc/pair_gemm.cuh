@@ -47,10 +47,10 @@
  * issues TMA loads (no multicast: each CTA loads its own operands; the
  * completion bytes of both CTAs are counted on the leader's barrier), warp 1 of
  * the leader CTA issues the MMAs and both warps 1 own their CTA's 512 TMEM
- * columns (two accumulators), warps 2-9 drain the accumulators.  Stage and accumulator hand-backs from the MMA to both CTAs are
- * tcgen05.commit with a cluster mask.  Every wait is bounded; a wait that runs out
- * raises the CTA's abort flag and records a status code, and every role falls through
- * to the common exit (cluster barrier, TMEM release).
+ * columns (two accumulators), warps 2-9 drain the accumulators.  Stage and accumulator
+ * hand-backs from the MMA to both CTAs are tcgen05.commit with a cluster mask.  Every
+ * wait is bounded; a wait that runs out raises the CTA's abort flag and records a status
+ * code, and every role falls through to the common exit (cluster barrier, TMEM release).
  */
 #pragma once
 #include <cuda.h>

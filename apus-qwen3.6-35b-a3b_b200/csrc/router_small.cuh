@@ -23,7 +23,8 @@ namespace apus {
  * that token's softmax / top-k on one of its warps.  No CTA ever waits on
  * another.  It decides on the BF16 codes of the logits and only where code order may
  * not decide, or a weight might narrow differently, runs the engine's softmax
- * (router_select.cuh; softmax for all took 2 us more).  Requires K % 8 == 0 and a 16-byte-aligned router matrix.
+ * (router_select.cuh; softmax for all took 2 us more).  Requires K % 8 == 0 and a
+ * 16-byte-aligned router matrix.
  * Dynamic shared memory: ROWS * (K*2 + 16) + 4 * ((K + 4) + (E + 1)) * 4 bytes.
  */
 constexpr int ROUTER_SMALL_TOK = 4;
