@@ -337,15 +337,14 @@ def test_block_few_tokens_without_gathered_rows(be, orc, synth, qwen_weights, T,
 @pytest.mark.parametrize("T,E,TK,skew", [(300, 8, 4, False), (257, 8, 4, False),
                                          (1000, 8, 4, False), (1500, 16, 8, True),
                                          (129, 4, 4, False)])
-@pytest.mark.parametrize("gather", ["0", "1", "2"])
-def test_block_two_sm_gemm_path(be, orc, synth, monkeypatch, T, E, TK, skew, gather):
+@pytest.mark.parametrize("swap", ["0", "192", "256"])
+def test_block_two_sm_gemm_path(be, orc, synth, monkeypatch, T, E, TK, skew, swap):
     """Many rows per expert: the GEMMs in which a pair of SMs shares a tile
     (tokens as the MMA's M, 256 per pair).  Checked against the CPU checker and,
     bit for bit, against the one-SM kernels on the same inputs (a row's result
-    must not depend on the tiling).  gather: how the gate_up kernel gets its
-    token rows — 0 a permuted copy (default), 1 TMA gather4 from the block input,
-    2 the kernel's own gather warps (cp.async into the swizzled stage)."""
-    monkeypatch.setenv("APUS_CUDA_PAIR_GATHER", gather)
+    must not depend on the tiling).  swap: last chunks of fewer rows than this are
+    multiplied with the rows as N — 0 none, 192 the default, 256 all."""
+    monkeypatch.setenv("APUS_CUDA_PAIR_SWAP_BELOW", swap)
     cfg = dict(hidden=512, experts=E, moe_inter=128, shared_inter=128, top_k=TK)
     W = synth.host_weights(be, cfg, seed=60 + T, sigma=0.05)
     x = synth.host_x(be, T, cfg["hidden"], seed=60 + T)
@@ -353,7 +352,7 @@ def test_block_two_sm_gemm_path(be, orc, synth, monkeypatch, T, E, TK, skew, gat
         W, x = synth.apply_router_bias(W, x, synth.zipf_bias(cfg, seed=3, beta=0.6))
     exp = orc.moe_block(cfg, W, x)
     res = {}
-    monkeypatch.setenv("APUS_CUDA_PAIR_MIN_ROWS", "64")   # default: 192 rows per expert
+    monkeypatch.setenv("APUS_CUDA_PAIR_MIN_ROWS", "64")   # default: 136 rows per expert
     for pair in ("1", "0"):
         monkeypatch.setenv("APUS_CUDA_PAIR", pair)
         be.enable()

@@ -208,14 +208,15 @@ def test_graph_survives_workspace_growth(gpu, be, synth):
         assert "apus_cuda_reserve" in msg
 
 
-def test_host_call_in_two_halves_gives_the_same_bits(be, synth, monkeypatch):
-    """From 4096 tokens the host-pointer call runs as two half calls whose PCIe
-    copies overlap the other half's kernels (APUS_CUDA_HOST_SPLIT_T): every
-    output and trace array equals the single call bit for bit, odd token count
-    included."""
+@pytest.mark.parametrize("T", [4101, 6143, 6144, 7001])
+def test_host_call_in_parts_gives_the_same_bits(be, synth, monkeypatch, T):
+    """From 4096 tokens the host-pointer call runs as two part calls, from 6144 as
+    three, whose PCIe copies overlap the other parts' kernels
+    (APUS_CUDA_HOST_SPLIT_T): every output and trace array equals the single call
+    bit for bit, odd token counts included."""
     cfg = dict(hidden=512, experts=64, moe_inter=128, shared_inter=128, top_k=8)
     W = synth.host_weights(be, cfg, seed=41, sigma=0.05)
-    x = synth.host_x(be, 4101, cfg["hidden"], seed=41)
+    x = synth.host_x(be, T, cfg["hidden"], seed=41)
     res = {}
     for split in ("0", "4096"):
         monkeypatch.setenv("APUS_CUDA_HOST_SPLIT_T", split)
@@ -227,6 +228,39 @@ def test_host_call_in_two_halves_gives_the_same_bits(be, synth, monkeypatch):
             be.disable()
     for k in ("idx", "w", "shared", "routed", "out"):
         assert np.array_equal(res["0"][k], res["4096"][k]), k
+
+
+@pytest.mark.parametrize("T", [33, 4101, 6200])
+def test_host_call_on_page_locked_buffers(gpu, synth, T):
+    """Buffers that are page-locked already go to the copy engines as they are (33
+    rows of 512 are too few for that: they take the staging slots): same bits as from
+    plain memory, in one call, two parts and three, with and without a trace."""
+    import ctypes as C
+    import torch
+    from apus_b200 import backend
+    cfg = dict(hidden=512, experts=64, moe_inter=128, shared_inter=128, top_k=8)
+    W = synth.host_weights(gpu, cfg, seed=47, sigma=0.05)
+    x = synth.host_x(gpu, T, cfg["hidden"], seed=47)
+    want = gpu.moe_block(cfg, W, x)
+
+    def locked(a):
+        return torch.from_numpy(a.view(np.int32 if a.itemsize == 4 else np.int16)).pin_memory()
+
+    xp = locked(x)
+    c = backend.MoeCfg.from_dict(cfg)
+    w = backend.MoeW(*[W[k].ctypes.data for k in ("rtr_w", "exp_gu", "exp_d", "sh_g", "sh_u",
+                                                  "sh_d", "sh_gate")])
+    for trace in (True, False):
+        got = {k: locked(np.zeros_like(want[k])) for k in ("out", "idx", "w", "routed", "shared")}
+        tr = backend.MoeTrace(got["idx"].data_ptr(), got["w"].data_ptr(),
+                              got["routed"].data_ptr(), got["shared"].data_ptr(), None)
+        rc = gpu.lib.apus_cuda_moe_block(C.byref(c), C.byref(w),
+                                         C.cast(xp.data_ptr(), backend.u16p),
+                                         C.cast(got["out"].data_ptr(), backend.u16p), T,
+                                         C.byref(tr) if trace else None)
+        assert rc == 0 and gpu.last_block_status() == 0
+        for k in got if trace else ("out",):
+            assert np.array_equal(got[k].numpy().view(want[k].dtype), want[k]), (k, trace)
 
 
 def test_no_token_is_a_successful_no_op(gpu, be, synth):
