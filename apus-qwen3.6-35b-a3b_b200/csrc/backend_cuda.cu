@@ -2002,13 +2002,19 @@ extern "C" int apus_cuda_moe_block(const ApusCudaMoeCfg *cfg,
          * a call in parts gives the same bits; the PCIe copies of one part run
          * beside the kernels of another.  A part costs a pass over the weights
          * (~250 us) and saves the travel of its rows (~0.08 us a row and way): two
-         * halves from 4096 rows, a short first and last part from 6144. */
+         * halves from 4096 rows (1187 us in one call, 1148 in two; pageable 1740, 1467;
+         * 3072 rows 967, 1005).  Page-locked on both sides, a short first and last part
+         * from 7168 (halves 1611 us, edges of a quarter 1612, a fifth 1570, a sixth 1540;
+         * 8192: 1758, 1705, 1650, 1706; 6144: 1464, 1504, 1481, 1460).  Pageable rows are
+         * copied by the processor before and after, which a long middle part leaves less
+         * to hide behind: 8192 rows 2355 us in halves, 2545 with edges of a fifth. */
         if (!c->s_in) {
             CU_OK(cudaStreamCreateWithFlags(&c->s_in, cudaStreamNonBlocking));
             CU_OK(cudaStreamCreateWithFlags(&c->s_out, cudaStreamNonBlocking));
             for (auto &e : c->ev_io) CU_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
-        const int parts = T >= 6144 ? 3 : 2;
+        const int parts =
+            T >= 7168 && HostStage::page_locked(ln2) && HostStage::page_locked(moe_out) ? 3 : 2;
         const size_t edge = parts == 3 ? T / 5 : T / 2;
         const size_t cut[HOST_PARTS + 1] = {0, edge, parts == 3 ? T - edge : T, T};
         CU_OK(cudaEventRecord(c->ev_io[0], c->stream));       /* earlier work owns dx, dout */

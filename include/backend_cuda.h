@@ -151,9 +151,9 @@ typedef struct {
  * apus_cuda_register_layer_slabs).  Synchronous: moe_out and the trace rows are complete on
  * return.  T == 0 writes nothing and succeeds, as the engine's loops over T do.
  * From APUS_CUDA_HOST_SPLIT_T tokens (default 4096; 0: never) the call runs as
- * two half calls, from 6144 tokens as three (1/5, 3/5, 1/5), whose PCIe copies
- * overlap the other parts' kernels: the same bits, since a token's result does not
- * depend on its neighbours.
+ * two half calls, from 7168 tokens in page-locked buffers as three (1/5, 3/5, 1/5),
+ * whose PCIe copies overlap the other parts' kernels: the same bits, since a token's
+ * result does not depend on its neighbours.
  * Returns 0, or nonzero with apus_cuda_last_error() set. */
 int apus_cuda_moe_block(const ApusCudaMoeCfg *c, const ApusCudaMoeW *w,
                         const uint16_t *ln2, uint16_t *moe_out, size_t T,

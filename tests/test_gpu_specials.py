@@ -208,12 +208,12 @@ def test_graph_survives_workspace_growth(gpu, be, synth):
         assert "apus_cuda_reserve" in msg
 
 
-@pytest.mark.parametrize("T", [4101, 6143, 6144, 7001])
-def test_host_call_in_parts_gives_the_same_bits(be, synth, monkeypatch, T):
-    """From 4096 tokens the host-pointer call runs as two part calls, from 6144 as
-    three, whose PCIe copies overlap the other parts' kernels
-    (APUS_CUDA_HOST_SPLIT_T): every output and trace array equals the single call
-    bit for bit, odd token counts included."""
+@pytest.mark.parametrize("T", [4101, 7168])
+def test_host_call_in_two_halves_gives_the_same_bits(be, synth, monkeypatch, T):
+    """From 4096 tokens the host-pointer call runs as two half calls whose PCIe
+    copies overlap the other half's kernels (APUS_CUDA_HOST_SPLIT_T): every
+    output and trace array equals the single call bit for bit, odd token count
+    included."""
     cfg = dict(hidden=512, experts=64, moe_inter=128, shared_inter=128, top_k=8)
     W = synth.host_weights(be, cfg, seed=41, sigma=0.05)
     x = synth.host_x(be, T, cfg["hidden"], seed=41)
@@ -230,11 +230,11 @@ def test_host_call_in_parts_gives_the_same_bits(be, synth, monkeypatch, T):
         assert np.array_equal(res["0"][k], res["4096"][k]), k
 
 
-@pytest.mark.parametrize("T", [33, 4101, 6200])
+@pytest.mark.parametrize("T", [33, 4101, 7167, 7168, 7201])
 def test_host_call_on_page_locked_buffers(gpu, synth, T):
     """Buffers that are page-locked already go to the copy engines as they are (33
-    rows of 512 are too few for that: they take the staging slots): same bits as from
-    plain memory, in one call, two parts and three, with and without a trace."""
+    rows of 512 are too few for that: they take the staging slots), from 7168 rows in
+    three parts: same bits as from plain memory, with and without a trace."""
     import ctypes as C
     import torch
     from apus_b200 import backend
