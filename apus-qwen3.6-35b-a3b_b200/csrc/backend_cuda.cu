@@ -240,7 +240,7 @@ static int ctx_init() {
     g_pg_dynamic = (int)env_long("APUS_CUDA_GEMM_DYNAMIC", 3);
     g_pg_direct = (int)env_long("APUS_CUDA_GEMM_DIRECT", 1);
     g_pp_enable = (int)env_long("APUS_CUDA_PAIR", 1);
-    g_pp_min_rows = (int)env_long("APUS_CUDA_PAIR_MIN_ROWS", 136);
+    g_pp_min_rows = (int)env_long("APUS_CUDA_PAIR_MIN_ROWS", 120);
     g_pp_swap_below = (int)env_long("APUS_CUDA_PAIR_SWAP_BELOW", 192);
     c->host_split_t = env_long("APUS_CUDA_HOST_SPLIT_T", 4096);
     g_ctx = c;

@@ -563,12 +563,13 @@ pair_gemm_kernel(const __grid_constant__ PairMaps mapA,        /* xg | act   (to
 
 /* ---- host side ---------------------------------------------------------------- */
 inline int g_pp_enable = 1;          /* APUS_CUDA_PAIR=0: never take this path */
-/* Mean rows per resident expert from which it is taken.  us of the one-SM kernels against
- * these, block, even router (experts alone): 112 rows 501, 519 (397, 404); 128 543, 539
- * (431, 436); 144 615, 565 (488, 456); 160 672, 602.  Hidden 4096, width 768: 112 833, 825
- * (514, 561); 128 865, 816 (560, 620); 160 1017, 894 (629, 587).  A skewed router gains
- * earlier (112: 548, 522; 96: 493, 506). */
-inline int g_pp_min_rows = 136;
+/* Mean rows per resident expert from which it is taken.  us of the block with the one-SM
+ * kernels against these, even router: 104 rows 453, 463; 112 479, 490; 120 500, 500; 128
+ * 529, 512; 136 551, 533; 144 615, 565.  Skewed: 96 481, 482; 104 510, 499; 112 540, 523;
+ * 120 551, 536; 128 580, 564.  Hidden 4096, width 768, even: 112 833, 825; 128 865, 816; 160
+ * 1017, 894.  (The experts alone, as in expert parallelism, even: 112 397, 404; 128 431, 436;
+ * 144 488, 456.) */
+inline int g_pp_min_rows = 120;
 /* Last chunks of fewer rows are taken as N (APUS_CUDA_PAIR_SWAP_BELOW).  8192 skewed tokens:
  * never 912 us, below 64 911, 128 896, 160 891, 192 869, 224 860, 256 (always) 886; 144 rows
  * an expert, skewed: 655, 589, 571, 618, 603, 586, 625. */
