@@ -775,6 +775,10 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         ca.status = c->d_status;
         ca.stats = c->d_rc_stats;
         ca.lr = LaneRow(K);
+        /* Few tokens: an interval first costs more than the chains it saves (routing, even
+         * and skewed: 72 tokens 29.7 -> 27.2 us, 34.4 -> 31.6; 150 32.3 -> 29.4, 35.8 -> 33.3;
+         * 300 32.4 -> 29.8, 36.1 -> 34.9; 512 33.5 -> 33.6, 38.8 -> 39.3). */
+        ca.direct = T <= 2 * c->sm_count;
         /* One warp per token, two tokens a CTA where there are more tokens than SMs.  A
          * warp's ring of rows hides their latency where other warps do not: the deepest
          * with which all tokens still run at once, else two rows.  (1000 skewed tokens:

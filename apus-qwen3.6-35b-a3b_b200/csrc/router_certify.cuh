@@ -36,7 +36,8 @@
  * lanes' partial results meet in shared memory, where one lane per candidate adds
  * them up.  Candidate rows (4 KB each, from L2) arrive through a ring of D slots per
  * warp.  (A chain per candidate, one per lane, took 33 us at 512 tokens, 55 at 1999
- * and 148 at 8192.)
+ * and 148 at 8192; up to two tokens an SM it is what runs, one chain to a lane, since
+ * an interval costs more than the chains it saves there.)
  */
 #pragma once
 #include <climits>
@@ -70,6 +71,7 @@ struct CertifyArgs {
     int32_t *unit_hist;             /* [T / 256][E] += the selection (optional, place.cuh) */
     int *status;
     unsigned int *stats;            /* [0] += logits resolved exactly (optional) */
+    int direct;                     /* every candidate's chain, no intervals (LANES) */
     LaneRow lr;
 };
 
@@ -224,9 +226,39 @@ router_certify_kernel(const __grid_constant__ CertifyArgs a) {
     __syncwarp();
     mark(1);
 
-    /* ---- their intervals ---- */
+    /* ---- their chains, or intervals ---- */
     auto row_of = [&](int e) { return e == E ? a.extra_row : a.w + (size_t)e * K; };
+    auto xpiece = [&](int p) { return ldg16(a.x + (size_t)t * K + p * 8); };
+    auto token_f32 = [&](float *d) {
+        for (int p = lane; p < K / 8; p += 32) {
+            float f[8];
+            unpack8(xpiece(p), f);
+            float4 *d4 = reinterpret_cast<float4 *>(d + p * 8);
+            d4[0] = make_float4(f[0], f[1], f[2], f[3]);
+            d4[1] = make_float4(f[4], f[5], f[6], f[7]);
+        }
+        __syncwarp();
+    };
     int f_slot = 0;
+    /* Few tokens: a chain for every candidate at once, no intervals.  (Values large enough
+     * to overflow, or NaN, take the intervals, which leave those open.) */
+    const bool direct = LANES && a.direct && ok && (ok_extra || !a.extra_row) && bmax < 1e30f;
+    if (direct) {
+        float *xs = reinterpret_cast<float *>(slots);
+        token_f32(xs);
+#pragma unroll 1
+        for (int c0 = 0; c0 < n_eval; c0 += 32) {
+            const bool mine = c0 + lane < n_eval;
+            const int e = cand[mine ? c0 + lane : c0];       /* the others read along */
+            const float z = lane_chain<true>(row_of(e), xs, K);
+            if (mine) {
+                if (e < E && !(fabsf(z - __uint_as_float(cd[e])) <= cb * __ldg(&a.wnorm[e])))
+                    set_status(a.status, ST_BOUND_VIOLATED);
+                cd[e] = 0x10001u * bf16_bits(z);
+            }
+        }
+        __syncwarp();
+    }
     auto fetch = [&](int c) {
         if (c < n_eval)
             lane_row_fetch(slot0 + (uint32_t)(f_slot * row_bytes), row_of(cand[c]), lr, K, lane);
@@ -234,11 +266,12 @@ router_certify_kernel(const __grid_constant__ CertifyArgs a) {
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const uint16_t *xg = a.x + (size_t)t * K + (size_t)lane * lr.nu * 8;   /* NU == 0 */
+    if (!direct)
 #pragma unroll 1
-    for (int c = 0; c < D; c++) fetch(c);
+        for (int c = 0; c < D; c++) fetch(c);
     int slot = 0;
 #pragma unroll 1
-    for (int c0 = 0; c0 < n_eval; c0 += RC_BATCH) {
+    for (int c0 = direct ? n_eval : 0; c0 < n_eval; c0 += RC_BATCH) {
         const int n = min(RC_BATCH, n_eval - c0);
 #pragma unroll 1
         for (int c = 0; c < n; c++) {
@@ -312,16 +345,8 @@ router_certify_kernel(const __grid_constant__ CertifyArgs a) {
     Choice ch = rt_select(cd, E, TK, lane, sel);
     if (ch.any) {
         float *buf = reinterpret_cast<float *>(slots);
-        auto xpiece = [&](int p) { return ldg16(a.x + (size_t)t * K + p * 8); };
         if (LANES) {
-            for (int p = lane; p < K / 8; p += 32) {     /* the token in fp32 */
-                float f[8];
-                unpack8(xpiece(p), f);
-                float4 *d = reinterpret_cast<float4 *>(buf + p * 8);
-                d[0] = make_float4(f[0], f[1], f[2], f[3]);
-                d[1] = make_float4(f[4], f[5], f[6], f[7]);
-            }
-            __syncwarp();
+            token_f32(buf);
             resolve_lanes(cd, cand, n_eval, E, K, ch.kkey, ch.odd, lane, buf,
                           ok && (ok_extra || !a.extra_row), row_of);
         } else {

@@ -287,6 +287,27 @@ def test_router_certified_kernel_edges(gpu, orc, be, synth, T, E, K, kind):
     assert d.max() <= 1 and (d != 0).mean() <= 0.002
 
 
+@pytest.mark.parametrize("T,E,kind", [
+    (65, 256, "plain"), (296, 256, "bias"), (297, 256, "bias"), (65, 128, "ties"),
+    (66, 256, "ties"), (67, 256, "zero"), (68, 256, "subnormal"), (69, 256, "huge")])
+def test_router_certified_chains_without_intervals(gpu, orc, be, synth, T, E, kind):
+    """Up to two tokens an SM (296) every candidate gets its chain at once: both sides of
+    that line, more candidates than lanes, products that round and logits of 2^110 (whose
+    bound is out of this form's range)."""
+    if kind != "huge":
+        test_router_certified_kernel_edges(gpu, orc, be, synth, T, E, 2048, kind)
+        return
+    cfg = dict(hidden=2048, experts=E, moe_inter=128, shared_inter=128, top_k=8)
+    W = synth.host_weights(be, cfg, seed=T, sigma=0.05)
+    x = synth.host_x(be, T, 2048, seed=T)
+    W["rtr_w"][:] = synth.f32_to_bf16(synth.bf16_to_f32(W["rtr_w"]) * np.float32(2.0 ** 110))
+    idx, w = _route_dev(gpu, synth, cfg, W, x)
+    assert gpu.last_block_status() == 0
+    eidx, ew = orc.route_batch(x, W["rtr_w"], 8)
+    assert np.array_equal(idx, eidx)
+    assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
+
+
 @pytest.mark.parametrize("T,E,K,topk", [
     (9, 256, 2048, 8), (52, 256, 2048, 8), (53, 256, 2048, 8), (64, 257, 2048, 8),
     (61, 300, 1032, 5), (64, 1024, 512, 32), (33, 37, 24, 1)])
