@@ -2740,8 +2740,9 @@ extern "C" int apus_cuda_bf16_gemv_dev(const uint16_t *d_w, const uint16_t *d_x,
     }
     const size_t want = (groups * split + warps - 1) / warps;
     const unsigned grid = (unsigned)(want < sms ? want : sms);
+    const long round = 16L * grid * (warps / split);             /* rows of all teams */
     gemv_stream_kernel<<<grid, warps * 32, smem, st>>>(d_w, d_x, d_y, (int)M, (long)O, (int)K,
-                                                       split);
+                                                       split, ((long)O + round - 1) / round);
     LAUNCHED();
     return 0;
 }
