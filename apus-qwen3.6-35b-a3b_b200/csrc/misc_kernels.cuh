@@ -18,8 +18,29 @@ __device__ __forceinline__ float exact_dot(const uint16_t *__restrict__ wrow,
                                            const uint16_t *__restrict__ xrow,
                                            int K) {
     float acc = 0.0f;
-    for (int k = 0; k < K; k++)
-        acc = __fadd_rn(acc, __fmul_rn(bf16_f32(__ldg(wrow + k)), bf16_f32(__ldg(xrow + k))));
+    /* a lane's row and its own sequence of steps: the next sixteen operands are under way
+     * during the adds of these (M 40, O 333, K 1001, with both copies: 88 -> 66 us) */
+    constexpr int B = 16;
+    uint16_t wv[B], xv[B];
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+        wv[j] = j < K ? __ldg(wrow + j) : (uint16_t)0;
+        xv[j] = j < K ? __ldg(xrow + j) : (uint16_t)0;
+    }
+    int k = 0;
+#pragma unroll 1
+    for (; k + B <= K; k += B) {
+#pragma unroll
+        for (int j = 0; j < B; j++) {
+            acc = __fadd_rn(acc, __fmul_rn(bf16_f32(wv[j]), bf16_f32(xv[j])));
+            const int n = k + B + j;
+            wv[j] = n < K ? __ldg(wrow + n) : (uint16_t)0;
+            xv[j] = n < K ? __ldg(xrow + n) : (uint16_t)0;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < B; j++)
+        if (k + j < K) acc = __fadd_rn(acc, __fmul_rn(bf16_f32(wv[j]), bf16_f32(xv[j])));
     return acc;
 }
 
