@@ -74,7 +74,7 @@ exact_matvec_f32_kernel(const uint16_t *__restrict__ w,
  * slots ahead; mma.sync m16n8k16 multiplies them with all rows of x at once (columns past
  * M repeat the last row and are not stored), so eight rows cost what one does.  Scalar
  * multiply-adds on rows loaded straight into registers took 174 us for one row and 780 for
- * eight (O 248320, K 2048); this 174 and 182 (5.8 of 6.5 TB/s).
+ * eight (O 248320, K 2048); this 168 and 174 (6.0 of 6.5 TB/s).
  * mma.sync cuts off what its accumulator cannot hold, so two steps share one that starts
  * at zero and the rest is a tree: at K 2048 1.0e-4 of the results narrow to another BF16
  * value than 64-bit sums do, as in the scalar form (6e-4 with all 64 steps on one); at
