@@ -55,6 +55,14 @@ def test_hook_exact_order_kernels(gpu, orc, M, O, K, scale):
                               equal_nan=True)
 
 
+@pytest.mark.parametrize("K", [15, 17, 31, 34, 1001])
+@pytest.mark.parametrize("scale", ["plain", "underflow", "overflow"])
+def test_hook_rows_of_unaligned_pieces(gpu, orc, K, scale):
+    """K that is no multiple of eight, around the sixteen steps loaded ahead: bit for bit."""
+    test_hook_exact_order_kernels(gpu, orc, 3, 70, K, scale)
+    test_hook_exact_order_kernels(gpu, orc, 1, 70, K, scale)
+
+
 @pytest.mark.parametrize("M,O,K", [(4, 16000, 3008), (2, 14300, 6016)])
 def test_hook_rows_that_fill_shared_memory(gpu, orc, M, O, K):
     """Rows of x and the rings of four warps are 232448 bytes here, all that a CTA may have,
