@@ -566,7 +566,7 @@ def measure_output_head(env, steps, warmup, seed):
             "config": {"workload": "output head as a weight stream: y = W x, W 248320 x 2048 "
                                    "BF16, one token, device pointers", "tokens_per_step": 1,
                        "l2_policy": "inputs larger than L2 (1 GB of weights per step)"},
-            "roofline": {"bound": "hbm", "kernel": "gemv_stream_kernel<1>", "achieved": ach,
+            "roofline": {"bound": "hbm", "kernel": "gemv_stream_kernel", "achieved": ach,
                          "peak": pk["hbm_gbs"], "peak_source": pk["_source"], "unit": "GB/s",
                          "frac": ach / pk["hbm_gbs"], "traffic": None,
                          "algorithmic_bytes_per_launch": nbytes},
