@@ -55,12 +55,12 @@ def test_hook_exact_order_kernels(gpu, orc, M, O, K, scale):
                               equal_nan=True)
 
 
+@pytest.mark.parametrize("M", [1, 3])
 @pytest.mark.parametrize("K", [15, 17, 31, 34, 1001])
 @pytest.mark.parametrize("scale", ["plain", "underflow", "overflow"])
-def test_hook_rows_of_unaligned_pieces(gpu, orc, K, scale):
+def test_hook_rows_of_unaligned_pieces(gpu, orc, M, K, scale):
     """K that is no multiple of eight, around the sixteen steps loaded ahead: bit for bit."""
-    test_hook_exact_order_kernels(gpu, orc, 3, 70, K, scale)
-    test_hook_exact_order_kernels(gpu, orc, 1, 70, K, scale)
+    test_hook_exact_order_kernels(gpu, orc, M, 70, K, scale)
 
 
 @pytest.mark.parametrize("M,O,K", [(4, 16000, 3008), (2, 14300, 6016)])
