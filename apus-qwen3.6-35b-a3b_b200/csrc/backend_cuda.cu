@@ -722,9 +722,9 @@ static int launch_router_tt(Ctx *c, const uint16_t *dx, const uint16_t *dwr,
 struct RouterAux {
     const float *wnorm;     /* [E + 1] row norms of the router matrix */
     float wmax;             /* largest |w| */
-    float wmin_extra, wmax_extra, wnorm_extra;   /* the same of extra_row */
-    float *approx_ws;       /* fp32 workspace, at least T*E*4 bytes */
-    size_t approx_bytes;    /* its size: up to four [T, E] slabs are used */
+    float wmin_extra, wmax_extra;   /* the same of extra_row */
+    float *approx_ws;       /* workspace: one to four [T, E] slabs of fp32 and the lists */
+    size_t approx_bytes;    /* its size */
     /* [ceil(T / PL_UNIT)][E]: the selections counted per unit of tokens (optional) */
     int32_t *unit_hist = nullptr;
     bool counted = false;   /* out: they were */
@@ -739,17 +739,14 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         return fail("router: unsupported E=%d topk=%d K=%d", E, topk, K);
     /* many tokens: fast logits on the tensor cores, exact chains only for the
      * experts that can still reach the top_k (router_certify.cuh) */
+    const size_t list_words = rc_list_words((size_t)T, (size_t)E);
     if (c->router_certify && aux && aux->wnorm && aux->approx_ws && dlogits &&
-        T > ROUTER_SMALL_MAX_T && E % PG_BM == 0 && K % 256 == 0 &&
+        T > ROUTER_SMALL_MAX_T && (size_t)T < RC_MAX_T && E % PG_BM == 0 && K % 256 == 0 &&
         (((uintptr_t)dwr | (uintptr_t)dx | (uintptr_t)extra_row) & 15) == 0 &&
-        router_certify_smem(E, K, 6) * RC_WARPS + 2048 <= (size_t)c->smem_optin) {
+        ((size_t)T * E + list_words) * 4 <= aux->approx_bytes) {
         int ksplit = dense_logits_ksplit(c->sm_count, T, E, K);
-        while (ksplit > 1 && (size_t)ksplit * T * E * 4 > aux->approx_bytes) ksplit /= 2;
-        if (run_dense_logits(c->sm_count, c->smem_optin, dwr, dx, T, E, K, ksplit,
-                             aux->approx_ws, c->d_status, st, &c->last_block_launches,
-                             aux->unit_hist, (T + PL_UNIT - 1) / PL_UNIT * E))
-            return fail("%s", prefill_last_error());
-        c->launches++;
+        while (ksplit > 1 && ((size_t)ksplit * T * E + list_words) * 4 > aux->approx_bytes)
+            ksplit /= 2;
         CertifyArgs ca;
         memset((void *)&ca, 0, sizeof ca);
         ca.approx = aux->approx_ws;
@@ -758,7 +755,6 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         ca.w = dwr;
         ca.extra_row = extra_row;
         ca.wnorm = aux->wnorm;
-        ca.wnorm_extra = aux->wnorm_extra;
         ca.T = T; ca.E = E; ca.K = K; ca.topk = topk;
         ca.wmin = wmin;
         ca.wmax = aux->wmax;
@@ -767,6 +763,7 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         /* the sequential chain errs by at most (K-1)u times the sum of the
          * term magnitudes; the tensor cores are granted eight times that */
         ca.cbound = 9.1f * (float)K * 5.9604645e-8f;   /* = debug_fast_logits' *cbound */
+        rc_carve(ca, aux->approx_ws + (size_t)ksplit * T * E);
         ca.idx_out = didx;
         ca.w_out = dw;
         ca.extra_out = extra_out;
@@ -774,50 +771,45 @@ static int launch_router(Ctx *c, const uint16_t *dx, const uint16_t *dwr, int T,
         aux->counted = aux->unit_hist != nullptr;
         ca.status = c->d_status;
         ca.stats = c->d_rc_stats;
-        ca.lr = LaneRow(K);
-        /* Few tokens: an interval first costs more than the chains it saves (routing, even
-         * and skewed: 72 tokens 29.7 -> 27.2 us, 34.4 -> 31.6; 150 32.3 -> 29.4, 35.8 -> 33.3;
-         * 300 32.4 -> 29.8, 36.1 -> 34.9; 512 33.5 -> 33.6, 38.8 -> 39.3). */
-        ca.direct = T <= 2 * c->sm_count;
-        /* One warp per token, two tokens a CTA where there are more tokens than SMs.  A
-         * warp's ring of rows hides their latency where other warps do not: the deepest
-         * with which all tokens still run at once, else two rows.  (1000 skewed tokens:
-         * 48 us with two, 41 with four; 1500: 57 and, with three, 49; 888: 44 and, with
-         * six, 40; where a second wave begins the deeper ring loses, 8192: 166 and 174.)
-         * Likewise the chains, one to a lane where all tokens run at once (512: 44 -> 37
-         * us, 2000: 62 -> 57, skewed), with the warp's help else (3000: 90 -> 83). */
-        const int warps = T <= c->sm_count ? 1 : RC_WARPS;
-        auto at_once = [&](int slots) {
-            return T <= c->sm_count * RC_WARPS *
-                            (int)(c->smem_sm / (router_certify_smem(E, K, slots) * RC_WARPS + 1280));
-        };
-        int ring = 2;
-        if (K == 2048 && E <= 256)
-            for (int d : {3, 4, 6})
-                if (at_once(d)) ring = d;
-        void (*kern)(CertifyArgs) = E > 256       ? router_certify_kernel<32, 0, 2, false>
-                                    : K != 2048   ? router_certify_kernel<8, 0, 2, false>
-                                    : ring == 6   ? router_certify_kernel<8, 8, 6, true>
-                                    : ring == 4   ? router_certify_kernel<8, 8, 4, true>
-                                    : ring == 3   ? router_certify_kernel<8, 8, 3, true>
-                                    : at_once(2)  ? router_certify_kernel<8, 8, 2, true>
-                                                  : router_certify_kernel<8, 8, 2, false>;
-        const size_t smem = router_certify_smem(E, K, ring) * warps;
-        const size_t most = router_certify_smem(E, K, 6) * RC_WARPS;
-        static size_t set_smem = 0;
-        if (most > set_smem) {
-            for (auto k : {router_certify_kernel<32, 0, 2, false>,
-                           router_certify_kernel<8, 0, 2, false>,
-                           router_certify_kernel<8, 8, 2, false>,
-                           router_certify_kernel<8, 8, 2, true>,
-                           router_certify_kernel<8, 8, 3, true>,
-                           router_certify_kernel<8, 8, 4, true>,
-                           router_certify_kernel<8, 8, 6, true>})
-                CU_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)most));
-            set_smem = most;
+        const ZeroRanges zero = {{ca.counts, aux->unit_hist},
+                                 {E * RC_COUNT_STEP, (T + PL_UNIT - 1) / PL_UNIT * E}};
+        if (run_dense_logits(c->sm_count, c->smem_optin, dwr, dx, T, E, K, ksplit,
+                             aux->approx_ws, c->d_status, st, &c->last_block_launches, zero))
+            return fail("%s", prefill_last_error());
+        c->launches++;
+        /* Few tokens: a candidate list is short of a warp's 32 tokens and three kernels cost
+         * more than one (routing, one kernel / three, even and skewed: 72 tokens 27 / 34 us,
+         * 30 / 36; 297 29 / 35, 33 / 39; 512 33 / 36, 36 / 40; 700 38 / 37, 44 / 42; 1000
+         * 52 / 38, 59 / 44). */
+        auto direct = E > 256 ? router_direct_kernel<32> : router_direct_kernel<8>;
+        if (T <= 4 * c->sm_count &&
+            router_direct_smem(E, K) <= dynamic_smem_limit(c, (const void *)direct)) {
+            const size_t smem = router_direct_smem(E, K);
+            static size_t set_smem = 0;
+            if (smem > 40 * 1024 && smem > set_smem) {
+                for (auto k : {router_direct_kernel<32>, router_direct_kernel<8>})
+                    CU_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem));
+                set_smem = smem;
+            }
+            launch_k(direct, dim3(T), dim3(32), smem, st, ca);
+            LAUNCHED();
+            return 0;
         }
-        launch_k(kern, dim3((T + warps - 1) / warps), dim3(warps * 32), smem, st, ca);
+        const dim3 tokens((T + RC_WARPS - 1) / RC_WARPS);
+        launch_k(E > 256 ? router_candidates_kernel<32> : router_candidates_kernel<8>, tokens,
+                 dim3(RC_WARPS * 32), 0, st, ca);
+        LAUNCHED();
+        const size_t smem = router_chains_smem(E);
+        static size_t set_smem = 0;
+        if (smem > set_smem) {
+            CU_OK(cudaFuncSetAttribute(router_chains_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            set_smem = smem;
+        }
+        launch_k(router_chains_kernel, dim3(c->sm_count), dim3(CW_WARPS * 32), smem, st, ca);
+        LAUNCHED();
+        launch_k(router_choose_kernel, tokens, dim3(RC_WARPS * 32), router_choose_smem(E), st, ca);
         LAUNCHED();
         return 0;
     }
@@ -1311,6 +1303,7 @@ struct BlockBufs {
     int32_t *unit_hist;
     uint16_t *act, *sa, *eo, *sy, *xg;
     void *tiles;           /* prefill tile lists */
+    size_t eo_bytes;       /* eo is the router's workspace before it holds outputs */
     size_t total;
 };
 
@@ -1322,6 +1315,9 @@ static int block_layout(const ApusCudaMoeCfg &c, size_t T, Arena *a,
                         BlockBufs *b, bool prefill) {
     const size_t H = c.hidden, E = c.experts, I = c.moe_inter,
                  Is = c.shared_inter, TK = c.top_k, A = T * TK;
+    const size_t router = T > (size_t)ROUTER_SMALL_MAX_T && E * 4 <= TK * H * 2
+                              ? (T * E + rc_list_words(T, E)) * 4 : 0;
+    b->eo_bytes = A * H * 2 > router ? A * H * 2 : router;
     size_t sz[] = {
         A * 4,                         /* idx */
         A * 2,                         /* rw */
@@ -1330,7 +1326,7 @@ static int block_layout(const ApusCudaMoeCfg &c, size_t T, Arena *a,
         E * 4, (E + 1) * 4, A * 4, A * 4,            /* counts offsets perm pos */
         (A + E) * 4, (A + E) * 4, (A + E) * 4, 256,  /* groups, n_groups */
         dispatch_scratch_bytes(A, E),  /* unit_hist */
-        A * I * 2, T * Is * 2, A * H * 2, T * H * 2, /* act sa eo sy */
+        A * I * 2, T * Is * 2, b->eo_bytes, T * H * 2, /* act sa eo sy */
         prefill ? A * H * 2 : 0,       /* xg */
         prefill ? prefill_tiles_bytes_for(c, A, T) : 0,
     };
@@ -1637,8 +1633,8 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
     c->n_ev = 0;
     stage_mark(c, -1, st);
     /* the fast logits live in the combine buffer, which is written much later */
-    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate, L->wnorm_gate,
-                     reinterpret_cast<float *>(b.eo), (size_t)Ti * TK * H * 2};
+    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate,
+                     reinterpret_cast<float *>(b.eo), b.eo_bytes};
     if (prefill && Ti > PL_UNIT) aux.unit_hist = b.unit_hist;
     if (launch_router(c, d_ln2, L->rtr_w, Ti, E, H, TK, L->wmin, b.idx, b.rw,
                       b.logits, L->sh_gate, b.sgl, st,
@@ -2103,12 +2099,12 @@ extern "C" int apus_cuda_ep_route_dev(ApusCudaLayer *L, const uint16_t *d_x,
     Ordered ord(c, st);
     if (ord.rc) return 1;
     const size_t E = L->cfg.experts;
-    if (arena_reserve(c->ws, T * E * 18 + 8192)) return 1;
+    const size_t aux_bytes = T * E * 16 + rc_list_words(T, E) * 4;
+    if (arena_reserve(c->ws, T * E * 2 + aux_bytes + 8192)) return 1;
     c->ws.reset();
     uint16_t *logits = (uint16_t *)c->ws.take(T * E * 2);
-    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate, L->wnorm_gate,
-                     (float *)c->ws.take(T * E * 16),
-                     T * E * 16};
+    RouterAux aux = {L->d_wnorm, L->wmax, L->wmin_gate, L->wmax_gate,
+                     (float *)c->ws.take(aux_bytes), aux_bytes};
     return launch_router(c, d_x, L->rtr_w, (int)T, (int)E, (int)L->cfg.hidden,
                          (int)L->cfg.top_k, L->wmin, d_idx, d_w, logits,
                          L->sh_gate, d_sgl, st, &aux);
@@ -2664,10 +2660,11 @@ extern "C" int apus_cuda_route_dev(ApusCudaLayer *L, const uint16_t *d_x,
     Ordered ord(c, st);
     if (ord.rc) return 1;
     const size_t E = L->cfg.experts;
-    if (arena_reserve(c->ws, T * E * 18 + 8192)) return 1;
+    const size_t aux_bytes = T * E * 16 + rc_list_words(T, E) * 4;
+    if (arena_reserve(c->ws, T * E * 2 + aux_bytes + 8192)) return 1;
     c->ws.reset();
     uint16_t *logits = (uint16_t *)c->ws.take(T * E * 2);
-    RouterAux aux = {L->d_wnorm, L->wmax, 0.0f, 0.0f, 0.0f, (float *)c->ws.take(T * E * 16), T * E * 16};
+    RouterAux aux = {L->d_wnorm, L->wmax, 0.0f, 0.0f, (float *)c->ws.take(aux_bytes), aux_bytes};
     return launch_router(c, d_x, L->rtr_w, (int)T, (int)E, (int)L->cfg.hidden,
                          (int)L->cfg.top_k, L->wmin, d_idx, d_w, logits, nullptr,
                          nullptr, st, &aux);

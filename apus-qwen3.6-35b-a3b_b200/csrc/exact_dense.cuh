@@ -61,6 +61,27 @@ __device__ __forceinline__ void fold_range8(const uint4 &v, unsigned int &lo, un
         hi = max(hi, max(a, b));
     }
 }
+/* the same of many, two codes to an instruction: |code| - 1, where a zero is the largest */
+struct PackedRange {
+    uint32_t lo = 0xffffffffu, hi = 0;
+    __device__ __forceinline__ void fold8(const uint4 &v) {
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t m = w[q] & 0x7fff7fffu;
+            uint32_t less;
+            asm("add.u16x2 %0, %1, %2;" : "=r"(less) : "r"(m), "r"(0xffffffffu));
+            asm("min.u16x2 %0, %0, %1;" : "+r"(lo) : "r"(less));
+            asm("max.u16x2 %0, %0, %1;" : "+r"(hi) : "r"(m));
+        }
+    }
+    /* as fold_range8 has them */
+    __device__ __forceinline__ unsigned low() const {
+        const unsigned m = min(lo & 0xffffu, lo >> 16);
+        return m == 0xffffu ? 0x7f800000u : (m + 1u) << 16;
+    }
+    __device__ __forceinline__ unsigned high() const { return max(hi & 0xffffu, hi >> 16) << 16; }
+};
 /* every product of the two ranges is exact in fp32 (a NaN or an infinity on
  * either side fails the second test) */
 __device__ __forceinline__ bool products_exact(float wmin, float wmax, unsigned int xlo,

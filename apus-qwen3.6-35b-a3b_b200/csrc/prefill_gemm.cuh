@@ -271,6 +271,10 @@ gather_rows_peer_kernel(const unsigned long long *__restrict__ src, int cap,
 }
 
 /* ---- the grouped GEMM -------------------------------------------------------- */
+struct ZeroRanges {
+    int32_t *p[2];         /* null: none */
+    int n[2];
+};
 struct GemmParams {
     const int4 *tiles;
     const int *n_tiles;
@@ -319,8 +323,7 @@ struct GemmParams {
     int dense_T, dense_mt, dense_ntiles, dense_ksplit;
     float *out_f32;        /* [dense_ksplit][dense_T, ld_f32]: one slab per K slice */
     int ld_f32;
-    int32_t *zero;         /* cleared on the way, for the kernel that follows (optional) */
-    int zero_n;
+    ZeroRanges zero;       /* cleared on the way, for the kernels that follow */
 };
 
 /* the tile with this index: from the list, or (MODE 2) generated: token tile
@@ -402,8 +405,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
     if (!(MODE == 1 && p.done)) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (MODE != 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (MODE == 2)
-        for (int i = blockIdx.x * PG_THREADS + tid; i < p.zero_n; i += gridDim.x * PG_THREADS)
-            p.zero[i] = 0;
+#pragma unroll
+        for (int z = 0; z < 2; z++)
+            for (int i = blockIdx.x * PG_THREADS + tid; i < p.zero.n[z];
+                 i += gridDim.x * PG_THREADS)
+                p.zero.p[z][i] = 0;
     const int n_tiles = MODE == 2 ? p.dense_ntiles : *p.n_tiles;
     const int num_kb = p.K / PG_BK;
 
@@ -981,7 +987,7 @@ inline int dense_logits_ksplit(int sm_count, int T, int E, int K) {
 inline int run_dense_logits(int sm_count, int smem_optin, const uint16_t *w,
                             const uint16_t *x, int T, int E, int K, int ksplit,
                             float *out, int *status, cudaStream_t st, int *launches,
-                            int32_t *zero = nullptr, int zero_n = 0) {
+                            ZeroRanges zero = {}) {
     PFN_encodeTiled_local enc = tensor_map_encoder();
     if (!enc) return 1;
     const int smem = PG_STAGES * 2 * PG_TILE_BYTES + 1024 + 256;
@@ -1010,8 +1016,9 @@ inline int run_dense_logits(int sm_count, int smem_optin, const uint16_t *w,
     p.dense_ntiles = ((T + PG_BN_GU - 1) / PG_BN_GU) * p.dense_mt * ksplit;
     p.out_f32 = out;
     p.ld_f32 = E;
+    for (int z = 0; z < 2; z++)
+        if (!zero.p[z]) zero.n[z] = 0;
     p.zero = zero;
-    p.zero_n = zero ? zero_n : 0;
     p.status = status;
     const int grid = p.dense_ntiles < sm_count ? p.dense_ntiles : sm_count;
     launch_k(grouped_gemm_kernel<2>, dim3(grid), dim3(PG_THREADS), (size_t)smem, st,

@@ -258,58 +258,5 @@ __device__ __forceinline__ float lane_chain(const uint16_t *w, const float *xs, 
     }
     return acc;
 }
-/* Both resolve the logits that rt_needs names of list[0 .. n-1]: their codes become known.
- * row(e): weight row in global memory.  One chain to a lane; xs: the token in fp32, exact: no
- * product rounds. */
-template <typename Row>
-__device__ __forceinline__ void resolve_lanes(uint32_t *cd, const uint16_t *list, int n, int E,
-                                              int K, uint32_t kkey, bool odd, int lane,
-                                              const float *xs, bool exact, Row row) {
-#pragma unroll 1
-    for (int c0 = 0; c0 < n; c0 += 32) {
-        const int mine = c0 + lane < n ? list[c0 + lane] : E + 1;
-        const bool need = rt_needs(cd, mine, E, kkey, odd);
-        const unsigned m = __ballot_sync(0xffffffffu, need);
-        if (!m) continue;
-        /* the other lanes read along with the first */
-        const int first = __shfl_sync(0xffffffffu, mine, __ffs(m) - 1), e = need ? mine : first;
-        const float z = exact ? lane_chain<true>(row(e), xs, K) : lane_chain<false>(row(e), xs, K);
-        if (need) cd[e] = 0x10001u * bf16_bits(z);
-        __syncwarp();
-    }
-}
-/* The warp's help for up to CH_CHAINS at a time. */
-template <typename Row, typename XPiece>
-__device__ __forceinline__ void resolve_chains(uint32_t *cd, const uint16_t *list, int n, int E,
-                                               int K, uint32_t kkey, bool odd, int lane,
-                                               float *buf, Row row, XPiece xpiece) {
-#pragma unroll 1
-    for (int c0 = 0; c0 < n; c0 += 32) {
-        const int e = c0 + lane < n ? list[c0 + lane] : E + 1;
-        unsigned m = __ballot_sync(0xffffffffu, rt_needs(cd, e, E, kkey, odd));
-#pragma unroll 1
-        while (m) {
-            const int now = min(__popc(m), CH_CHAINS);
-            const int src = lane < now ? __fns(m, 0, lane + 1) : 0;
-            const int mine = __shfl_sync(0xffffffffu, e, src);
-            const float z = warp_chains<CH_CHAINS>(
-                now, K, lane, buf,
-                [&](int c) { return row(__shfl_sync(0xffffffffu, mine, c)); }, xpiece);
-            if (lane < now) cd[mine] = 0x10001u * bf16_bits(z);
-            __syncwarp();
-            m &= ~__reduce_or_sync(0xffffffffu, lane < now ? 1u << src : 0u);
-        }
-    }
-}
-/* a row of global memory into a LaneRow, by one warp (asynchronously; the caller
- * commits and waits) */
-__device__ __forceinline__ void lane_row_fetch(uint32_t dst, const uint16_t *src, const LaneRow lr,
-                                               int H, int lane) {
-    for (int c = lane; c < H / 8; c += 32) cp_async16_to(dst + (uint32_t)lr.at(c), src + c * 8);
-}
-__device__ __forceinline__ void cp_async_done() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
 
 }  // namespace apus

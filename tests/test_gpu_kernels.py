@@ -316,6 +316,29 @@ def test_router_certified_chains_without_intervals(gpu, orc, be, synth, T, E, ki
     assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
 
 
+@pytest.mark.parametrize("T,E,K,kind", [
+    (592, 256, 2048, "bias"), (593, 256, 2048, "bias"),        # one kernel, then lists
+    (593, 384, 768, "plain"), (600, 1024, 256, "bias"),        # more than 256 experts
+    (607, 128, 512, "ties"), (640, 128, 512, "zero"),          # every expert a candidate
+    (600, 128, 512, "subnormal"), (600, 128, 512, "huge"),     # products that round, overflow
+    (2049, 128, 256, "bias")])                                 # lists of many warps
+def test_router_candidate_lists(gpu, orc, be, synth, T, E, K, kind):
+    """Candidates' chains from lists per expert: both sides of four tokens an SM, lists that
+    end inside a warp's 32 tokens, tokens with more candidates than lanes beside others."""
+    if kind != "huge":
+        test_router_certified_kernel_edges(gpu, orc, be, synth, T, E, K, kind)
+        return
+    cfg = dict(hidden=K, experts=E, moe_inter=128, shared_inter=128, top_k=8)
+    W = synth.host_weights(be, cfg, seed=T, sigma=0.05)
+    x = synth.host_x(be, T, K, seed=T)
+    W["rtr_w"][:] = synth.f32_to_bf16(synth.bf16_to_f32(W["rtr_w"]) * np.float32(2.0 ** 110))
+    idx, w = _route_dev(gpu, synth, cfg, W, x)
+    assert gpu.last_block_status() == 0
+    eidx, ew = orc.route_batch(x, W["rtr_w"], 8)
+    assert np.array_equal(idx, eidx)
+    assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
+
+
 @pytest.mark.parametrize("T,E,K,topk", [
     (9, 256, 2048, 8), (52, 256, 2048, 8), (53, 256, 2048, 8), (64, 257, 2048, 8),
     (61, 300, 1032, 5), (64, 1024, 512, 32), (33, 37, 24, 1)])
