@@ -77,6 +77,15 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map,
         "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
 }
+/* the same with an L2 policy */
+__device__ __forceinline__ void tma_load_2d_policy(void *dst, const CUtensorMap *map, int x, int y,
+                                                   uint64_t *bar, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::"
+        "complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "l"(policy)
+        : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -480,6 +489,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
                     asm volatile("fence.proxy.async;" ::: "memory");
                 }
                 int claim = tile;
+                /* Routed weights are read once, and evicted first they leave rows, activations
+                 * and outputs of the call in L2 (T 9: 109 -> 99 us a layer, 61: 254 -> 238, 128:
+                 * 297 -> 276 a block, 512: 316 -> 305, 1999: 394 -> 385).  Every token tile
+                 * reads the shared expert's and the router's: those as usual (evicted first
+                 * too, T 128 took 281, T 512 302).  The two-SM kernels, where later chunks of
+                 * the expert read them again, lose (8192 tokens: 735 -> 790). */
+                const uint64_t policy = shared ? l2_read_again() : l2_read_once();
                 auto request = [&](int kb) -> bool {
                     const int s = kiter % STAGES;
                     const uint32_t ph = (kiter / STAGES) & 1u;
@@ -488,10 +504,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
                         return false;
                     unsigned char *st = smem + (size_t)s * STAGE_BYTES;
                     mbar_expect_tx(&full[s], (uint32_t)(B_OFF + brows * PG_BK * 2));
-                    tma_load_2d(st, ma, (kb0 + kb) * PG_BK, arow, &full[s]);
+                    tma_load_2d_policy(st, ma, (kb0 + kb) * PG_BK, arow, &full[s], policy);
                     if (GATE_UP)
-                        tma_load_2d(st + PG_TILE_BYTES, ma2, kb * PG_BK, arow2,
-                                    &full[s]);
+                        tma_load_2d_policy(st + PG_TILE_BYTES, ma2, kb * PG_BK, arow2, &full[s],
+                                           policy);
                     tma_load_2d(st + B_OFF, mb, (kb0 + kb) * PG_BK, brow, &full[s]);
                     kiter++;
                     return true;
