@@ -41,6 +41,7 @@
  */
 #pragma once
 #include <climits>
+#include <type_traits>
 
 #include "common.cuh"
 #include "decode_gemv.cuh"
@@ -207,11 +208,13 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     df_mark(a, 0);                          /* start */
     /* ---- this CTA's shares ---- */
     const int r_first = blockIdx.x, n_rr = r_first <= E ? (E - r_first) / G + 1 : 0;
-    const int sh_lo = (int)((long)Is * blockIdx.x / G),
-              sh_n = (int)((long)Is * (blockIdx.x + 1) / G) - sh_lo;
+    /* (in 32 bits, which the sizes that fused_supported admits leave room for: a 64-bit
+     * division takes half a microsecond) */
+    const unsigned b = blockIdx.x, g = gridDim.x;
+    const int sh_lo = (int)((unsigned)Is * b / g), sh_n = (int)((unsigned)Is * (b + 1) / g) - sh_lo;
     const int nS = (sh_n + DF_PAIRS - 1) / DF_PAIRS;   /* shared gate/up tiles */
-    const int h_lo = (int)((long)H * blockIdx.x / G);
-    const int ncols = (int)((long)H * (blockIdx.x + 1) / G) - h_lo;
+    const int h_lo = (int)((unsigned)H * b / g);
+    const int ncols = (int)((unsigned)H * (b + 1) / g) - h_lo;
     /* routed gate/up pairs and tiles, distinct experts: known after the selection */
     int gu_lo = 0, gu_n = 0, nR = 0, U = 0;
 
@@ -305,16 +308,22 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     };
     int i_tile = 0, i_slot = 0;             /* next gate/up tile of the phase, next slot */
     int i_unit = 0, i_ks = 0, n_unit = 0;   /* next down unit and k step in it */
-    bool i_sh = true;
     /* requests this warp's next tile if it is known; one commit group per call, so
-     * that a fixed number of groups stays ahead of the tile in use */
-    auto issue = [&]() {
+     * that a fixed number of groups stays ahead of the tile in use.  The callers say what it
+     * can be: the kernel waits for its instructions wherever they are new, so none of what a
+     * phase never requests lies in its way (a stack of four layers at 1 / 3 / 8 tokens 138 /
+     * 210 / 368 -> 136 / 202 / 361 us). */
+    constexpr int SHARED = 0, ROUTED = 1, DOWN = 2;
+    auto issue = [&](auto phase) {
+        constexpr int PHASE = decltype(phase)::value;
         const uint32_t slot = ring + (uint32_t)(i_slot * L.slot);
-        bool some = true;
-        if (i_tile < (i_sh ? nS : nR)) {
+        bool some = false;
+        if (PHASE != DOWN && i_tile < (PHASE == SHARED ? nS : nR)) {
             const int p0 = i_tile++ * DF_PAIRS;
-            fetch_pairs(slot, i_sh, p0, min(DF_PAIRS, (i_sh ? sh_n : gu_n) - p0));
-        } else if (i_unit < n_unit) {
+            fetch_pairs(slot, PHASE == SHARED, p0,
+                        min(DF_PAIRS, (PHASE == SHARED ? sh_n : gu_n) - p0));
+            some = true;
+        } else if (PHASE != SHARED && i_unit < n_unit) {
             const DownUnit d = down_unit(i_unit);
             fetch_down(slot, d, i_ks);
             i_ks += DF_KS;
@@ -322,24 +331,26 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
                 i_ks = 0;
                 i_unit++;
             }
-        } else {
-            some = false;
+            some = true;
         }
         if (some && ++i_slot == DF_DEPTH) i_slot = 0;
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (warp < DF_CW)
 #pragma unroll 1
-        for (int j = 0; j < DF_DEPTH; j++) issue();   /* constants: nothing to wait for */
+        for (int j = 0; j < DF_DEPTH; j++)   /* constants: nothing to wait for */
+            issue(std::integral_constant<int, SHARED>());
 
     unsigned int sync_at[2] = {0, 0};
     if (tid == 0) {
         s_dead = 0;
         s_open = 0;
         s_U = 0;
-        sync_at[0] = round_target(ld_acquire(&a.sync[0]));
-        sync_at[1] = round_target(ld_acquire(&a.sync[1]));
-        s_chain0 = ld_acquire(&a.sync[2]);
+        /* one round trip: nothing is read on the strength of these */
+        const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(a.sync));
+        sync_at[0] = round_target(v.x);
+        sync_at[1] = round_target(v.y);
+        s_chain0 = v.z;
     }
     if (tid < DF_MAX_T) {
         s_xlo[tid] = 0x7f800000u;
@@ -366,7 +377,10 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
             float rs = 1.0f;
             auto meet = [&] { asm volatile("bar.sync %0, 64;" ::"r"(3 + t) : "memory"); };
             if (a.res) {
-                const float ss = exact_sumsq(row, lr, lane, part, parts, &s_sum[t], meet);
+                const float ss =
+                    lr.nu / parts <= 4
+                        ? exact_sumsq<4>(row, lr, lane, part, parts, &s_sum[t], meet)
+                        : exact_sumsq<0>(row, lr, lane, part, parts, &s_sum[t], meet);
                 if (part) s_rs[t] = norm_scale(ss, H);
                 if (parts == 2) {
                     meet();
@@ -375,22 +389,23 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
                     rs = norm_scale(ss, H);
                 }
             }
-            unsigned int lo = 0x7f800000u, hi = 0;
+            PackedRange range;
             float sq = 0.0f;
+            /* (rolled: unrolled twice, a layer waited 1.2 us longer for instructions) */
 #pragma unroll 1
             for (int c = part * 32 + lane; c < cph; c += 32 * parts) {
                 uint4 *p = reinterpret_cast<uint4 *>(row + lr.at(c));
                 uint4 v = *p;
                 if (a.res) *p = v = norm8(v, gains[c], rs);
-                fold_range8(v, lo, hi);
+                range.fold8(v);
                 float f[8];
                 unpack8(v, f);
 #pragma unroll
                 for (int j = 0; j < 8; j++) sq = fmaf(f[j], f[j], sq);
             }
             sq = warp_sum(sq);
-            lo = __reduce_min_sync(0xffffffffu, lo);
-            hi = __reduce_max_sync(0xffffffffu, hi);
+            const unsigned lo = __reduce_min_sync(0xffffffffu, range.low()),
+                           hi = __reduce_max_sync(0xffffffffu, range.high());
             if (lane == 0) {
                 s_sq[part][t] = sq;
                 atomicMin(&s_xlo[t], lo);
@@ -448,7 +463,8 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     };
     /* gate/up tiles [0, n): the warps' partial sums meet in shared memory, four
      * warps in turn finish a tile while the others go on */
-    auto run_tiles = [&](int n, bool sh) {
+    auto run_tiles = [&](int n, auto phase) {
+        constexpr bool sh = decltype(phase)::value == SHARED;
 #pragma unroll 1
         for (int j = 0; j < n; j++) {
             float *buf = red + (j & 1) * (DF_CW * DF_ROWS * 8);
@@ -465,7 +481,7 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
             *reinterpret_cast<float2 *>(dst) = make_float2(c0[0] + c1[0], c0[1] + c1[1]);
             *reinterpret_cast<float2 *>(dst + 64) = make_float2(c0[2] + c1[2], c0[3] + c1[3]);
             __syncwarp();                       /* the slot is read out */
-            issue();
+            issue(phase);
             df_bar_compute();
             if ((warp >> 2) == (j & 3)) {
                 /* thread = row (2p gate, 2p + 1 up) x column */
@@ -490,7 +506,7 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
             }
         }
     };
-    if (warp < DF_CW) run_tiles(nS, true);
+    if (warp < DF_CW) run_tiles(nS, std::integral_constant<int, SHARED>());
     df_mark(a, 2);                          /* shared gate/up done */
     /* ---- routing ---- */
     if (tid == 0 && !spin_until(&a.sync[0], sync_at[0])) {
@@ -500,9 +516,19 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
     if (tid < 256) s_tmask[tid] = 0;
     __syncthreads();
     bool dead = s_dead != 0;
+    /* four requested before the first is stored: eight tokens' are four to a thread */
 #pragma unroll 1
-    for (int i = tid; i < T * (E + 1); i += DF_THREADS)
-        codes[i] = dead ? 0u : __ldcg(&a.code_ws[i]);
+    for (int i0 = tid; i0 < T * (E + 1); i0 += 4 * DF_THREADS) {
+        uint32_t v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int i = i0 + q * DF_THREADS;
+            v[q] = i < T * (E + 1) && !dead ? __ldcg(&a.code_ws[i]) : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (i0 + q * DF_THREADS < T * (E + 1)) codes[i0 + q * DF_THREADS] = v[q];
+    }
     __syncthreads();
     uint32_t kkey = 0;
     if (warp < T && !dead) {
@@ -678,8 +704,8 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
 
     /* ---- routed gate/up ---- */
     if (!dead) {
-        gu_lo = (int)((long)U * I * blockIdx.x / G);
-        gu_n = (int)((long)U * I * (blockIdx.x + 1) / G) - gu_lo;
+        gu_lo = (int)((unsigned)(U * I) * b / g);
+        gu_n = (int)((unsigned)(U * I) * (b + 1) / g) - gu_lo;
         nR = (gu_n + DF_PAIRS - 1) / DF_PAIRS;
         const int units = 2 * (U + 1);
         n_unit = warp < units ? (units - warp + DF_CW - 1) / DF_CW : 0;
@@ -689,10 +715,9 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
         }
     }
     i_tile = 0;
-    i_sh = false;
 #pragma unroll 1
-    for (int j = 0; j < DF_DEPTH; j++) issue();
-    run_tiles(nR, false);
+    for (int j = 0; j < DF_DEPTH; j++) issue(std::integral_constant<int, ROUTED>());
+    run_tiles(nR, std::integral_constant<int, ROUTED>());
     df_mark(a, 4);                      /* routed gate/up done */
     df_bar_compute();
     if (tid == 0) {
@@ -771,7 +796,7 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
                     for (int q = 0; q < 4; q++) ((s & 2) ? c1 : c0)[q] += p[q];
                 }
             __syncwarp();
-            issue();
+            issue(std::integral_constant<int, DOWN>());
             ks0 += DF_KS;
             ba += DF_KS * 32;
         } while (ks0 < d.nk);

@@ -81,10 +81,13 @@ __device__ __forceinline__ void square8(const unsigned char *p, float (&q)[8]) {
 /* Sum of squares of a LaneRow; the chain's value in every lane.  One warp (parts
  * == 1), or two with half of the row each (parts == 2, an even lr.nu): the second
  * prepares everything while the first walks, then takes the sum over from
- * `hand_over` in shared memory and goes on, `meet` being a barrier of the two.  The
- * loops stay rolled: at one row per launch the code runs once, and unrolled it
- * waits for its instructions. */
-template <typename Meet>
+ * `hand_over` in shared memory and goes on, `meet` being a barrier of the two.
+ *
+ * P > 0: a lane's chunk is at most P pieces, and its squares stay in registers.  What bounds
+ * a row is the walk over the lanes that leave a binade (about seven of 32 or 64), one
+ * addition after another: out of registers 150 cycles for 32 of them, out of shared memory
+ * twice that.  (P == 0: any chunk, rolled loops over shared memory.) */
+template <int P, typename Meet>
 __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const LaneRow lr, int lane,
                                              int part, int parts, float *hand_over, Meet meet) {
     /* chunk of this lane: of lr.nl * parts chunks in row order */
@@ -93,22 +96,46 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
     const int chunk = part * nl + (active ? lane : 0), l = chunk / parts;
     const unsigned char *mine = row + l * lr.pitch + (chunk - l * parts) * per * 16;
     const int nu = active ? per : 0;
+    float qr[P > 0 ? P : 1][8];
+    if (P > 0)
+#pragma unroll
+        for (int u = 0; u < P; u++) {
+            /* (adding zeros changes nothing) */
+            if (u < nu) square8(mine + u * 16, qr[u]);
+            else
+#pragma unroll
+                for (int j = 0; j < 8; j++) qr[u][j] = 0.0f;
+        }
+    auto each = [&](auto use) {                          /* use(eight squares), in order */
+        if (P > 0) {
+#pragma unroll
+            for (int u = 0; u < P; u++) use(qr[u]);
+        } else {
+#pragma unroll 1
+            for (int u = 0; u < nu; u++) {
+                float q[8];
+                square8(mine + u * 16, q);
+                use(q);
+            }
+        }
+    };
     /* where the sum will be, roughly: tree sums and a scan over the lanes */
-    auto rough = [&](const unsigned char *p) {
-        float t = 0.0f;
+    auto tree8 = [](const float (&q)[8]) {
+        return ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+    };
+    float tot = 0.0f;
+    each([&](const float (&q)[8]) { tot += tree8(q); });
+    float before = 0.0f;
+    if (part) {                                          /* the first half's */
+        const int c0 = active ? lane : 0, l0 = c0 / parts;
+        const unsigned char *p = row + l0 * lr.pitch + (c0 - l0 * parts) * per * 16;
 #pragma unroll 1
         for (int u = 0; u < nu; u++) {
             float q[8];
             square8(p + u * 16, q);
-            t += ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+            before += tree8(q);
         }
-        return t;
-    };
-    const float tot = rough(mine);
-    float before = 0.0f;
-    if (part) {                                          /* the first half's */
-        const int c0 = active ? lane : 0, l0 = c0 / parts;
-        before = warp_sum(rough(row + l0 * lr.pitch + (c0 - l0 * parts) * per * 16));
+        before = warp_sum(before);
     }
     float incl = tot;
 #pragma unroll
@@ -125,13 +152,10 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
     const float even = __uint_as_float((uint32_t)b0 << 23),
                 odd = __uint_as_float(((uint32_t)b0 << 23) + 1u);
     float fe = even, fo = odd;
-#pragma unroll 1
-    for (int u = 0; u < nu; u++) {
-        float q[8];
-        square8(mine + u * 16, q);
+    each([&](const float (&q)[8]) {
         fe = add8(fe, q);
         fo = add8(fo, q);
-    }
+    });
     ParityFn f;
     f.i0 = __float_as_int(fe) - __float_as_int(even);
     f.i1 = __float_as_int(fo) - __float_as_int(odd);
@@ -139,7 +163,7 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
     const int prev = __shfl_up_sync(0xffffffffu, key, 1);
     const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || key != prev);
     const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-#pragma unroll 1
+#pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         ParityFn g;
         g.i0 = __shfl_up_sync(0xffffffffu, f.i0, d);
@@ -171,15 +195,9 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
         }
 #pragma unroll 1
         for (; cur < end; cur++) {
-            if (lane == cur) {
-#pragma unroll 2
-                for (int u = 0; u < nu; u++) {
-                    float q[8];
-                    square8(mine + u * 16, q);
-                    s = add8(s, q);
-                }
-            }
-            s = __shfl_sync(0xffffffffu, s, cur);
+            float t = s;
+            each([&](const float (&q)[8]) { t = add8(t, q); });      /* its own lane's counts */
+            s = __shfl_sync(0xffffffffu, t, cur);
         }
     }
     if (parts == 2 && part == 0) {
@@ -188,9 +206,11 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
     }
     return s;
 }
+/* by one warp */
 __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const LaneRow lr,
                                              int lane) {
-    return exact_sumsq(row, lr, lane, 0, 1, nullptr, [] {});
+    return lr.nu <= 8 ? exact_sumsq<8>(row, lr, lane, 0, 1, nullptr, [] {})
+                      : exact_sumsq<0>(row, lr, lane, 0, 1, nullptr, [] {});
 }
 
 /* y = rnd((x * rs) * (1 + w)), eight values; w: the gain offsets */
@@ -211,8 +231,8 @@ __device__ __forceinline__ float norm_scale(float ss, int H) {
 
 /* RMSNorm with (1+w) gain (c/attn.h:175-186), rows of N % 8 == 0 values, 16-byte
  * aligned; one warp per row.  Bound: the latency of one row for few rows, and
- * instruction issue for many.  N 2048: 9.5 us for up to 64 rows (launch included;
- * the sequential chain took 12.6), 30 us for 8192 (65). */
+ * instruction issue for many.  N 2048: 11.1 us for up to 64 rows (launch included; 11.2 with the
+ * squares in shared memory), 10.6 for 1999 (16.1), 27.5 for 8192 (33.7). */
 constexpr int RN_WARPS = 4;
 __global__ void __launch_bounds__(RN_WARPS * 32)
 rmsnorm_rows_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ w,

@@ -99,3 +99,29 @@ def test_layer_at_the_real_dimensions_one_token(gpu, orc, be, synth):
     torch.cuda.synchronize()
     assert gpu.last_block_launches() == 1
     assert np.array_equal(d_out.cpu().numpy().view(np.uint16), out3)
+
+
+@pytest.mark.parametrize("H", [208, 512, 768, 1280, 1536, 2048])
+def test_one_kernel_norm_on_rows_made_to_go_wrong(gpu, be, synth, H):
+    """The one-kernel path's sum of squares, one warp or two to a row and lane chunks in
+    registers or not, against the row kernel's (which the checker's chain pins): sums on the
+    edge of a binade, ties in every add, a jump over binades, rising and falling terms."""
+    import torch
+    cfg = dict(hidden=H, experts=64, moe_inter=16, shared_inter=16, top_k=8)
+    layer = gpu.layer_create(cfg, synth.host_weights(be, cfg, seed=H, sigma=0.05))
+    rng = np.random.default_rng(H)
+    rows = [np.ones(H), np.full(H, 1.0 + 2 ** -7), rng.integers(1, 4, H) * 0.5,
+            np.where(np.arange(H) == H // 2, 1e3, rng.normal(0, 1, H)),
+            np.exp2(np.linspace(6, -12, H)), np.exp2(np.linspace(-12, 6, H)),
+            np.sign(rng.normal(0, 1, H)) * 181.0, rng.normal(0, 3, H)]
+    rows += [rng.normal(0, 2.0 ** s, H) for s in range(-4, 4)]
+    x = synth.f32_to_bf16(np.asarray(rows, np.float32))
+    for at, T in ((0, 8), (8, 8), (2, 1), (5, 3)):
+        d_res = _dev(torch, x[at:at + T])
+        _, expected = _three_calls(gpu, torch, layer, d_res, None, T, H)
+        d_out = torch.empty_like(d_res)
+        gpu.moe_layer_dev(layer, d_res.data_ptr(), None, d_out.data_ptr(), T)
+        torch.cuda.synchronize()
+        assert gpu.last_block_launches() == 1 and gpu.last_block_status() == 0
+        assert np.array_equal(d_out.cpu().numpy().view(np.uint16), expected)
+    gpu.layer_destroy(layer)
