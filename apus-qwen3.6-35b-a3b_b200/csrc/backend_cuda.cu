@@ -532,14 +532,14 @@ static const DevBuf *weight_buf(Ctx *c, const void *ptr, size_t bytes) {
  *    few warps per CTA as still put a CTA on every SM (a lane's chain takes the
  *    same time however many run beside it), at most eight;
  *  - more rows: by outputs per SM.  A wide warp tile widens fewer operands per
- *    multiply-add but leaves SMs idle when there are few outputs (M 64, O 1024:
- *    28 us with 2 x 32 per warp, 41 with 8 x 32; M 221, O 949: 68 us with 8 x 32,
- *    53 with 8 x 64; M 512, O 1024: 86 us with 8 x 64, 74 with 8 x 128);
+ *    multiply-add but leaves SMs idle when there are few outputs (calls, K 2048, in us, with
+ *    tiles of 2 x 128, 16 x 32, 16 x 64, 32 x 128: M 32, O 1024 54, 59, 63, 101; M 64 81, 71,
+ *    81, 119; M 128 135, 97, 94, 132; M 512 247, 196, 171, 201; O 2048 429, 283, 228, 234;
+ *    O 4096 762, 493, 365, 340);
  *  - K not a multiple of 8: rows are not made of aligned 16-byte pieces, the
  *    plain kernel.
  * M_all: rows of the whole call when a.M is one of the parts it runs in. */
 static int launch_exact(Ctx *c, const ExactArgs &a, int M_all, cudaStream_t st) {
-    const size_t optin = (size_t)c->smem_optin;
     auto allow = [&](const void *kern, size_t smem) {
         return smem <= 40 * 1024 ||        /* 48 KB with the static part */
                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -567,23 +567,15 @@ static int launch_exact(Ctx *c, const ExactArgs &a, int M_all, cudaStream_t st) 
         const long per_sm = (long)M_all * a.O / c->sm_count;
         auto launch = [&](auto tile, void (*kern)(ExactArgs)) -> int {
             using Tile = decltype(tile);
-            const long ot = (a.O + Tile::O - 1) / Tile::O,
-                       all = ((long)M_all + Tile::M - 1) / Tile::M * ot;
-            /* one wave: a CTA asks for more than half of an SM's shared memory, so
-             * that the parts of a call spread over the SMs instead of doubling up */
-            size_t smem = Tile::SMEM;
-            if (M_all > a.M && all <= c->sm_count && smem < optin / 2 + 1024)
-                smem = optin / 2 + 1024;
-            if (!allow((const void *)kern, smem)) return fail("exact tile: shared memory");
-            kern<<<dim3((unsigned)((a.M + Tile::M - 1) / Tile::M),
-                        (unsigned)(ot < 65535 ? ot : 65535)),
-                   Tile::THREADS, smem, st>>>(a);
+            const long all = ((long)a.M + Tile::M - 1) / Tile::M * ((a.O + Tile::O - 1) / Tile::O);
+            if (!allow((const void *)kern, Tile::SMEM)) return fail("exact tile: shared memory");
+            kern<<<(unsigned)(all < (1 << 30) ? all : 1 << 30), Tile::THREADS, Tile::SMEM, st>>>(a);
             return 0;
         };
-        const int rc = per_sm <= 512    ? launch(ExactTile<2, 1>(), exact_tile_kernel<2, 1>)
-                       : per_sm <= 1024 ? launch(ExactTile<4, 1>(), exact_tile_kernel<4, 1>)
-                       : per_sm <= 2048 ? launch(ExactTile<8, 2>(), exact_tile_kernel<8, 2>)
-                                        : launch(ExactTile<8, 4>(), exact_tile_kernel<8, 4>);
+        const int rc = per_sm <= 256    ? launch(ExactTile<2, 1, 1>(), exact_tile_kernel<2, 1, 1>)
+                       : per_sm <= 512  ? launch(ExactTile<4, 1, 4>(), exact_tile_kernel<4, 1, 4>)
+                       : per_sm <= 8192 ? launch(ExactTile<4, 2, 4>(), exact_tile_kernel<4, 2, 4>)
+                                        : launch(ExactTile<8, 4, 4>(), exact_tile_kernel<8, 4, 4>);
         if (rc) return 1;
     } else {
         const long total = (long)a.M * a.O;

@@ -243,27 +243,29 @@ exact_rows_kernel(ExactArgs a) {
 }
 
 /* ---- more rows -----------------------------------------------------------------
- * Bound: instruction issue.  A warp owns 32 * NO outputs (NO weight rows per lane)
- * x RM rows of x; the four warps of a CTA share the weight rows.
- * What the layout is for:
- *  - a shared-memory load delivers 128 bytes per cycle to the SM, broadcast or
- *    not.  fp32 operands under a 4 x 4 register tile cost 64 load cycles per k
- *    against 32 of multiply-adds (89 us at M 512, O 1024, K 2048), so operands
- *    stay BF16: a lane's 16 bytes are 8 k of its own weight row, or 8 k of one x
- *    row for the whole warp;
- *  - two chains per instruction (fma.rn.f32x2: the same fp32 pipes, half the issue
- *    slots) leave room for the shifts and masks that widen the operands.  The pair
- *    runs over two x rows; a weight is widened once and used for all RM of them.
- * M 512, O 1024, K 2048: 570 us as one thread per output reading global memory,
- * now 74 (fp32 pipes alone: 29; what is left is the widening, which the same pipes
- * do half of); M 64: 28, M 8, O 512: 28.
- * Rows arrive in blocks of 64 k (cp.async, eight lanes per row, pitch 144 bytes as
- * above), ET_STAGES - 1 blocks ahead; one barrier per block. */
+ * Bound: the fp32 pipes and the issue slots beside them.  A warp owns 32 * NO outputs (NO
+ * weight rows per lane) x RM rows of x; a CTA's four warps stand WM over rows of x and 4 / WM
+ * over outputs, and share what they read.  What the layout is for:
+ *  - two chains per instruction (fma.rn.f32x2: the same fp32 pipes, half the issue slots);
+ *    the pair runs over two x rows;
+ *  - widening takes as many instructions as multiplying if every operand is widened where it
+ *    is used.  x is the same for all lanes, so the CTA widens a block of it once, into pairs
+ *    of rows that a broadcast load puts where the multiply-add wants them; weights are a
+ *    lane's own, stay BF16 (sixteen bytes are eight k) and are widened once for all RM rows.
+ * Rows arrive in blocks of 64 k (cp.async, eight lanes per row; weights at pitch 144 bytes as
+ * above), ET_STAGES - 1 blocks ahead; one barrier per block.  Whether all products are exact
+ * is known when x has been read; where they are not, the CTA walks its chains again,
+ * literally.
+ * K 2048, a tile alone on its SM: 2 x 128 (rows x outputs) 31 us, 16 x 32 24, 16 x 64 30,
+ * 32 x 128 69.  (Both operands widened in the lanes, 32 x 128: 74, 8 x 32: 28.) */
 constexpr int ET_STAGES = 4;
-template <int RM, int NO>
+constexpr int ET_WARPS = 4;
+template <int RM, int NO, int WM>
 struct ExactTile {
-    static constexpr int M = 4 * RM, O = 32 * NO, THREADS = 128;
-    static constexpr int SMEM = ET_STAGES * (O + M) * ER_PITCH;
+    static constexpr int WO = ET_WARPS / WM, M = RM * WM, O = WO * 32 * NO,
+                         THREADS = ET_WARPS * 32;
+    static constexpr int W_STAGE = O * ER_PITCH, R_STAGE = M * ER_BK * 2, X_BUF = ER_BK * M * 4;
+    static constexpr int SMEM = ET_STAGES * (W_STAGE + R_STAGE) + 2 * X_BUF;
 };
 
 __device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
@@ -284,42 +286,77 @@ __device__ __forceinline__ void exact_step2(unsigned long long w, unsigned long 
     }
 }
 
-template <int RM, int NO, bool FMA>
+/* xlo, xhi: range of the magnitudes of the x values this thread has widened, |code| - 1 (a
+ * zero is the largest) and |code| */
+template <int RM, int NO, int WM, bool FMA>
 __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned char *smem, long o0,
-                                                int m0) {
-    using Tile = ExactTile<RM, NO>;
-    constexpr int WROWS = Tile::O, ROWS = WROWS + Tile::M, BUF = ROWS * ER_PITCH;
-    constexpr int STEP = Tile::THREADS / 8;             /* rows fetched side by side */
-    constexpr int NP = (ROWS + STEP - 1) / STEP;        /* 16-byte pieces per thread */
+                                                int m0, unsigned &xlo, unsigned &xhi) {
+    using Tile = ExactTile<RM, NO, WM>;
+    constexpr int STEP = Tile::THREADS / 8;
+    constexpr int XR = Tile::M * ER_BK / Tile::THREADS;  /* x rows that a thread widens */
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wm = warp % WM, wo = warp / WM;
     const int nkb = (a.K + ER_BK - 1) / ER_BK;
-    /* fetch side: piece fc of rows fr, fr + STEP, ... (rows of w, then rows of x) */
+    unsigned char *raw = smem + (size_t)ET_STAGES * Tile::W_STAGE;       /* x as it comes */
+    float *xs = reinterpret_cast<float *>(raw + ET_STAGES * Tile::R_STAGE);   /* [2][WM][k][RM] */
+    /* piece fc of rows fr, fr + STEP, ... */
     const int fc = tid & 7, fr = tid >> 3;
-    const uint16_t *src[NP];
-    uint32_t rok = 0;
-#pragma unroll
-    for (int i = 0; i < NP; i++) {
-        const int r = fr + i * STEP;
-        const bool ok = r < WROWS ? o0 + r < a.O : r < ROWS && m0 + r - WROWS < a.M;
-        src[i] = (r < WROWS ? a.w + (ok ? (o0 + r) * a.K : 0)
-                            : a.x + (ok ? (long)(m0 + r - WROWS) * a.K : 0)) + fc * 8;
-        rok |= (ok ? 1u : 0u) << i;
-    }
-    const uint32_t dst0 = smem_u32(smem) + (uint32_t)(fr * ER_PITCH + fc * 16);
+    const uint16_t *wsrc = a.w + (size_t)(o0 + fr) * a.K + fc * 8,
+                   *xsrc = a.x + (size_t)(m0 + fr) * a.K + fc * 8;
+    const uint32_t wdst = smem_u32(smem) + (uint32_t)(fr * ER_PITCH + fc * 16),
+                   xdst = smem_u32(raw) + (uint32_t)(tid * 16);
     int f_s = 0;
     auto fetch = [&](int kb) {
         if (kb < nkb) {
             const bool kok = kb * ER_BK + fc * 8 < a.K;
 #pragma unroll
-            for (int i = 0; i < NP; i++) {
-                const bool ok = kok && ((rok >> i) & 1u);
-                if (fr + i * STEP < ROWS)
-                    cp_async16_zfill(dst0 + (uint32_t)(f_s * BUF + i * STEP * ER_PITCH),
-                                     ok ? src[i] + (size_t)kb * ER_BK : a.w, ok);
+            for (int i = 0; i < Tile::O / STEP; i++) {
+                const bool ok = kok && o0 + fr + i * STEP < a.O;
+                cp_async16_zfill(wdst + (uint32_t)(f_s * Tile::W_STAGE + i * STEP * ER_PITCH),
+                                 ok ? wsrc + (size_t)(i * STEP) * a.K + kb * ER_BK : a.w, ok);
             }
+#pragma unroll
+            for (int i = 0; i < (Tile::M + STEP - 1) / STEP; i++)
+                if (fr + i * STEP < Tile::M) {
+                    const bool ok = kok && m0 + fr + i * STEP < a.M;
+                    cp_async16_zfill(
+                        xdst + (uint32_t)(f_s * Tile::R_STAGE + i * STEP * ER_BK * 2),
+                        ok ? xsrc + (size_t)(i * STEP) * a.K + kb * ER_BK : a.x, ok);
+                }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (++f_s == ET_STAGES) f_s = 0;
+    };
+    /* x: one k of XR rows */
+    const int xk = tid & (ER_BK - 1), xr0 = (tid / ER_BK) * XR;
+    int x_s = 0;
+    auto widen_x = [&](int kb) {
+        const uint16_t *src = reinterpret_cast<const uint16_t *>(raw + x_s * Tile::R_STAGE) +
+                              xr0 * ER_BK + xk;
+        if (++x_s == ET_STAGES) x_s = 0;
+        float f[XR];
+#pragma unroll
+        for (int r = 0; r < XR; r++) {
+            const unsigned v = src[r * ER_BK], m = v & 0x7fffu;
+            xlo = min(xlo, m - 1u);
+            xhi = max(xhi, m);
+            f[r] = __uint_as_float(v << 16);
+        }
+        float *d = xs + (kb & 1) * (ER_BK * Tile::M);
+        constexpr int V = XR < RM ? XR : RM < 4 ? RM : 4;    /* rows to a store, of one group */
+        static_assert(XR % V == 0 && RM % V == 0, "");
+#pragma unroll
+        for (int r = 0; r < XR; r += V) {
+            const int row = xr0 + r;
+            float *at = d + (row / RM * ER_BK + xk) * RM + row % RM;
+            if (V == 4)
+                *reinterpret_cast<float4 *>(at) =
+                    make_float4(f[r], f[(r + 1) % XR], f[(r + 2) % XR], f[(r + 3) % XR]);
+            else if (V == 2)
+                *reinterpret_cast<float2 *>(at) = make_float2(f[r], f[(r + 1) % XR]);
+            else
+                at[0] = f[r];
+        }
     };
     unsigned long long acc[NO][RM / 2];
 #pragma unroll
@@ -327,107 +364,129 @@ __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned cha
 #pragma unroll
         for (int j = 0; j < RM / 2; j++) acc[i][j] = 0ull;
     for (int kb = 0; kb < ET_STAGES - 1; kb++) fetch(kb);
+    asm volatile("cp.async.wait_group %0;" ::"n"(ET_STAGES - 2) : "memory");
+    __syncthreads();
+    widen_x(0);
     int s = 0;
 #pragma unroll 1
     for (int kb = 0; kb < nkb; kb++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(ET_STAGES - 2) : "memory");
-        __syncthreads();       /* block kb landed everywhere, block kb - 1 is used up */
+        asm volatile("cp.async.wait_group %0;" ::"n"(ET_STAGES - 3) : "memory");
+        __syncthreads();       /* block kb + 1 landed everywhere, block kb - 1 is used up */
         fetch(kb + ET_STAGES - 1);
-        const unsigned char *wb = smem + (size_t)s * BUF + (size_t)lane * ER_PITCH;
-        const unsigned char *xb = smem + (size_t)s * BUF + (size_t)(WROWS + warp * RM) * ER_PITCH;
-        uint4 wv[2][NO], xv[2][RM];
-        auto load = [&](int c, uint4 (&wq)[NO], uint4 (&xq)[RM]) {
+        if (kb + 1 < nkb) widen_x(kb + 1);
+        const unsigned char *wb =
+            smem + (size_t)s * Tile::W_STAGE + (size_t)(wo * 32 * NO + lane) * ER_PITCH;
+        const float *xb = xs + (kb & 1) * (ER_BK * Tile::M) + wm * (ER_BK * RM);
+        /* four k of x, eight of the weights: the next ones are requested before these are
+         * used */
+        uint4 wq[2][NO];
+        unsigned long long xp[2][4][RM / 2];
+        auto load_w = [&](int c, uint4 (&q)[NO]) {
 #pragma unroll
             for (int i = 0; i < NO; i++)
-                wq[i] = *reinterpret_cast<const uint4 *>(wb + i * 32 * ER_PITCH + c * 16);
-#pragma unroll
-            for (int m = 0; m < RM; m++)
-                xq[m] = *reinterpret_cast<const uint4 *>(xb + m * ER_PITCH + c * 16);
+                q[i] = *reinterpret_cast<const uint4 *>(wb + i * 32 * ER_PITCH + c * 16);
         };
-        auto use = [&](const uint4 (&wq)[NO], const uint4 (&xq)[RM]) {
+        auto load_p = [&](int c4, unsigned long long (&q)[4][RM / 2]) {
+            const float *at = xb + c4 * 4 * RM;
+            if (RM >= 4) {
 #pragma unroll
-            for (int h = 0; h < 8; h++) {
-                auto word = [&](const uint4 &v) {
-                    const uint32_t q = h < 2 ? v.x : h < 4 ? v.y : h < 6 ? v.z : v.w;
-                    return (h & 1) ? bf16hi(q) : bf16lo(q);
-                };
-                unsigned long long wp[NO];
+                for (int h = 0; h < 4; h++)
+#pragma unroll
+                    for (int j = 0; j < RM / 4; j++) {
+                        const ulonglong2 v =
+                            reinterpret_cast<const ulonglong2 *>(at + h * RM)[j];
+                        q[h][2 * j] = v.x;
+                        q[h][(2 * j + 1) % (RM / 2)] = v.y;
+                    }
+            } else {                       /* two k to a load */
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const ulonglong2 v = reinterpret_cast<const ulonglong2 *>(at)[h];
+                    q[2 * h][0] = v.x;
+                    q[2 * h + 1][0] = v.y;
+                }
+            }
+        };
+        auto use = [&](const uint4 (&wv)[NO], int half, const unsigned long long (&q)[4][RM / 2]) {
+#pragma unroll
+            for (int h = 0; h < 4; h++)
 #pragma unroll
                 for (int i = 0; i < NO; i++) {
-                    const float f = word(wq[i]);
-                    wp[i] = pack_f32x2(f, f);
-                }
+                    const uint32_t v = half ? (h < 2 ? wv[i].z : wv[i].w)
+                                            : (h < 2 ? wv[i].x : wv[i].y);
+                    const float f = (h & 1) ? bf16hi(v) : bf16lo(v);
+                    const unsigned long long wp = pack_f32x2(f, f);
 #pragma unroll
-                for (int j = 0; j < RM / 2; j++) {
-                    const unsigned long long xp = pack_f32x2(word(xq[2 * j]), word(xq[2 * j + 1]));
-#pragma unroll
-                    for (int i = 0; i < NO; i++) exact_step2<FMA>(wp[i], xp, acc[i][j]);
+                    for (int j = 0; j < RM / 2; j++) exact_step2<FMA>(wp, q[h][j], acc[i][j]);
                 }
-            }
         };
-        if (m0 + warp * RM < a.M) {
-            load(0, wv[0], xv[0]);
+        load_w(0, wq[0]);
+        load_p(0, xp[0]);
 #pragma unroll 1
-            for (int c = 0; c < ER_BK / 8; c += 2) {
-                load(c + 1, wv[1], xv[1]);
-                use(wv[0], xv[0]);
-                load(c + 2 < ER_BK / 8 ? c + 2 : 0, wv[0], xv[0]);
-                use(wv[1], xv[1]);
-            }
+        for (int c = 0; c < ER_BK / 8; c += 2) {
+            const int next = c + 2 < ER_BK / 8 ? c + 2 : 0;
+            load_p(2 * c + 1, xp[1]);
+            load_w(c + 1, wq[1]);
+            use(wq[0], 0, xp[0]);
+            load_p(2 * c + 2, xp[0]);
+            use(wq[0], 1, xp[1]);
+            load_p(2 * c + 3, xp[1]);
+            load_w(next, wq[0]);
+            use(wq[1], 0, xp[0]);
+            load_p(2 * next, xp[0]);
+            use(wq[1], 1, xp[1]);
         }
         if (++s == ET_STAGES) s = 0;
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < NO; i++) {
-        const long o = o0 + i * 32 + lane;
+        const long o = o0 + (wo * NO + i) * 32 + lane;
         if (o >= a.O) continue;
 #pragma unroll
         for (int j = 0; j < RM; j++) {
-            const int m = m0 + warp * RM + j;
+            const int m = m0 + wm * RM + j;
             if (m >= a.M) continue;
-            const float v =
-                __uint_as_float((uint32_t)(acc[i][j >> 1] >> ((j & 1) * 32)));
+            const float v = __uint_as_float((uint32_t)(acc[i][j >> 1] >> ((j & 1) * 32)));
+            const size_t at = (size_t)m * a.O + o;
             if (a.f32_out)
-                reinterpret_cast<float *>(a.y)[(size_t)m * a.O + o] = v;
+                reinterpret_cast<float *>(a.y)[at] = v;
             else
-                reinterpret_cast<uint16_t *>(a.y)[(size_t)m * a.O + o] = bf16_bits(v);
+                reinterpret_cast<uint16_t *>(a.y)[at] = bf16_bits(v);
         }
     }
 }
 
-/* grid: x over the row blocks (tiles that share weights run together), y over
- * the output blocks, taken in steps of gridDim.y */
-template <int RM, int NO>
-__global__ void __launch_bounds__(128)
+/* grid: one CTA per tile, or any number of them; tiles that share weights side by side */
+template <int RM, int NO, int WM>
+__global__ void __launch_bounds__(ET_WARPS * 32)
 exact_tile_kernel(ExactArgs a) {
-    using Tile = ExactTile<RM, NO>;
+    using Tile = ExactTile<RM, NO, WM>;
     extern __shared__ __align__(16) unsigned char et_smem[];
     __shared__ unsigned int s_lo, s_hi;
-    const int m0 = blockIdx.x * Tile::M, rows = min(Tile::M, a.M - m0);
-    if (threadIdx.x == 0) {
-        s_lo = 0x7f800000u;
-        s_hi = 0;
-    }
-    __syncthreads();
-    unsigned int lo = 0x7f800000u, hi = 0;
-    const uint16_t *x0 = a.x + (size_t)m0 * a.K;
-#pragma unroll 8
-    for (long i = threadIdx.x; i < (long)rows * (a.K / 8); i += Tile::THREADS)
-        fold_range8(ldg16(x0 + i * 8), lo, hi);
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&s_lo, lo);
-        atomicMax(&s_hi, hi);
-    }
-    __syncthreads();
-    const bool fma = products_exact(a.wmin, a.wmax, s_lo, s_hi);
-    for (long o0 = (long)blockIdx.y * Tile::O; o0 < a.O; o0 += (long)gridDim.y * Tile::O) {
-        if (fma)
-            exact_tile_body<RM, NO, true>(a, et_smem, o0, m0);
-        else
-            exact_tile_body<RM, NO, false>(a, et_smem, o0, m0);
+    const long mt = (a.M + Tile::M - 1) / Tile::M, tiles = mt * ((a.O + Tile::O - 1) / Tile::O);
+#pragma unroll 1
+    for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const long o0 = tile / mt * Tile::O;
+        const int m0 = (int)(tile - tile / mt * mt) * Tile::M;
+        if (threadIdx.x == 0) {
+            s_lo = 0xffffffffu;
+            s_hi = 0;
+        }
+        unsigned lo = 0xffffffffu, hi = 0;
+        exact_tile_body<RM, NO, WM, true>(a, et_smem, o0, m0, lo, hi);
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&s_lo, lo);
+            atomicMax(&s_hi, hi);
+        }
+        __syncthreads();
+        const unsigned xlo = s_lo == 0xffffffffu ? 0x7f800000u : (s_lo + 1u) << 16;
+        if (!products_exact(a.wmin, a.wmax, xlo, s_hi << 16))
+            exact_tile_body<RM, NO, WM, false>(a, et_smem, o0, m0, lo, hi);
+        __syncthreads();
     }
 }
 

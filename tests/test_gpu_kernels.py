@@ -55,6 +55,23 @@ def test_hook_exact_order_kernels(gpu, orc, M, O, K, scale):
                               equal_nan=True)
 
 
+@pytest.mark.parametrize("M,O,K", [
+    (5, 127, 64), (7, 129, 136),                       # tiles of 2 x 128
+    (65, 640, 200), (97, 481, 64),                     # 16 x 32
+    (67, 1217, 136), (130, 900, 72),                   # 16 x 64
+    (521, 2341, 72)])                                  # 32 x 128
+@pytest.mark.parametrize("scale", ["plain", "underflow"])
+def test_hook_exact_tiles_past_their_edges(gpu, orc, M, O, K, scale):
+    """The tiles of the product of many rows, rows, outputs and k blocks left over; one row of
+    underflowing products sends its tile, and only that, through the literal chain."""
+    rng = np.random.default_rng(M + O + K)
+    w, x = rng_codes(rng, (O, K), 0.5), rng_codes(rng, (M, K), 1.0)
+    if scale == "underflow":
+        w[::3] = rng_codes(rng, w[::3].shape, 1e-20)
+        x[M // 2] = rng_codes(rng, (K,), 1e-20)
+    assert np.array_equal(gpu.bf16_gemm(w, x), orc.gemm(w, x))
+
+
 @pytest.mark.parametrize("M", [1, 3])
 @pytest.mark.parametrize("K", [15, 17, 31, 34, 1001])
 @pytest.mark.parametrize("scale", ["plain", "underflow", "overflow"])
