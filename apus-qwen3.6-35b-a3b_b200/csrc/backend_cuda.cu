@@ -1437,7 +1437,8 @@ static int run_finalize(Ctx *c, const ApusCudaMoeCfg &cfg, int T,
                         const uint16_t *rw, const uint16_t *sy,
                         const uint16_t *sgl, uint16_t *d_out,
                         const ApusCudaMoeTrace *tr, cudaStream_t st,
-                        const uint16_t *res = nullptr, uint16_t *res_out = nullptr) {
+                        const uint16_t *res = nullptr, uint16_t *res_out = nullptr,
+                        bool eo_dead = false) {
     FinalizeArgs f;
     memset(&f, 0, sizeof f);
     f.res = res;
@@ -1454,6 +1455,7 @@ static int run_finalize(Ctx *c, const ApusCudaMoeCfg &cfg, int T,
     f.tr_routed = tr ? tr->moe_routed : nullptr;
     f.tr_shared = tr ? tr->moe_shared : nullptr;
     f.tr_out = tr ? tr->moe_out : nullptr;
+    f.eo_dead = eo_dead && !pos && cfg.hidden % 256 == 0 ? 1 : 0;
     long total = (long)T * (cfg.hidden / 8);
     int blocks = (int)((total + 255) / 256);
     if (blocks > c->sm_count * 8) blocks = c->sm_count * 8;
@@ -1700,7 +1702,7 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
         if (run_decode_experts(c, L, d_ln2, Ti, TK, 0, b, true, b.eo, st)) return 1;
     }
     if (run_finalize(c, cfg, Ti, b.eo, nullptr, b.rw, b.sy, b.sgl, d_out, d_tr, st,
-                     rz ? rz->res : nullptr, rz ? rz->res_out : nullptr))
+                     rz ? rz->res : nullptr, rz ? rz->res_out : nullptr, !pair))
         return 1;
     stage_mark(c, APUS_CUDA_STAGE_FINALIZE, st);
     if (d_tr && d_tr->rtr_idx)
