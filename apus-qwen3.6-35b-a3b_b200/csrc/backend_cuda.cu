@@ -1212,7 +1212,7 @@ extern "C" int apus_cuda_layer_load_slabs(ApusCudaLayer *L, const char *containe
     return 0;
 }
 
-/* ||x_t||_2 with the margin router_certify_kernel applies (one warp per row) */
+/* ||x_t||_2 with the margin TokenCandidates applies (one warp per row) */
 __global__ void __launch_bounds__(256)
 dbg_xnorm_kernel(const uint16_t *__restrict__ x, int T, int K, float *__restrict__ out) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;

@@ -13,7 +13,7 @@
  * The chain fixes the order inside an output, so the parallelism is outputs:
  *   exact_rows_kernel   up to four rows of x: one weight row per lane, weights
  *                       streamed through shared memory
- *   exact_tile_kernel   more rows: tiles of 8 x 32 to 32 x 128 (rows x outputs)
+ *   exact_tile_kernel   more rows: tiles of 2 x 128 to 32 x 128 (rows x outputs)
  * Both want K % 8 == 0 (16-byte pieces of a row); other K keep exact_gemm_kernel.
  */
 #pragma once

@@ -311,15 +311,14 @@ int apus_cuda_last_stage_ms(float *ms, int cap);
  * values written, or -1 if the last call did not take that path. */
 int apus_cuda_fused_timeline(unsigned long long *out, int cap);
 /* Diagnostic for the many-token router: it scores every expert with a fast
- * tensor-core product and resolves exactly (the code of the engine's sequential
- * chain, c/moe.h:289-291, from an interval or from the chain itself) only the
- * experts whose fast logit, widened by a proven error bound, can still reach the
+ * tensor-core product and walks the engine's sequential chain (c/moe.h:289-291)
+ * only for the experts whose fast logit, widened by a proven error bound, can still reach the
  * top_k.  Returns how many logits have been resolved since enable (256 per token
  * would be the plain exact router; the one-kernel path counts the chains it walks),
  * -1 when not enabled.  APUS_CUDA_ROUTER_CERTIFY=0 selects the plain exact router. */
 long apus_cuda_router_exact_chains(void);
 /* Diagnostic: phase boundaries of the many-token router's first CTA in its
- * last launch, out[0..3] = start, candidates known, selection known, end
+ * last launch, out[0..3] = start, candidates known, chains done, end
  * (nanoseconds, low 32 bits of the device's global timer), out[4] = logits
  * evaluated for its first token.  Returns 0, or -1 when not enabled. */
 int apus_cuda_router_timeline(unsigned int *out);
