@@ -380,10 +380,12 @@ router_chains_kernel(const __grid_constant__ CertifyArgs a) {
  * rt_weights do, with every code known, without shared memory.  Returned: code order decides,
  * and chosen is this lane's expert, if any.
  *
- * Code order decides (router_select.cuh) where every two different neighbours down to the
- * first that is not chosen are 2^-18 apart.  What is no candidate is far enough below if the
- * top_k-th is not small, or by the margin that it was left out with: one BF16 step at a
- * magnitude of at least bmax, 2^-7 bmax.  (Softmax for every token with a small top_k-th made
+ * Code order decides (router_select.cuh) where every two different neighbours are 2^-18 apart
+ * as the engine's exp takes them (less the largest logit, rounded), from the largest down to
+ * the first below the top_k-th code: any of its equals may be the chosen one, and what comes
+ * behind them must not have their probability.  What is no candidate is far enough below if the
+ * top_k-th is not small, or by the margin that it was left out with: 2^-6 bmax less the two
+ * roundings to BF16, 2^-17 and more.  (Softmax for every token with a small top_k-th made
  * a skewed batch wait 7 us for a few of them.) */
 __device__ __forceinline__ bool choose_narrow(int n, int e, uint32_t code, float bmax, int TK,
                                               int lane, int32_t *idx, uint16_t *wo,
@@ -404,10 +406,11 @@ __device__ __forceinline__ bool choose_narrow(int n, int e, uint32_t code, float
                 kval = key_value(kkey), v = bf16lo(code);
     const bool sel = on && rank < TK;
     const bool close = next && (next >> 16) != (key >> 16) &&
-                       !(v - key_value(next >> 16) >= 3.814697265625e-6f);
+                       !(__fsub_rn(v, top) - __fsub_rn(key_value(next >> 16), top) >=
+                         3.814697265625e-6f);
     const bool odd = !last || !(kval - top >= -80.0f) ||
                      (fabsf(kval) < 9.765625e-4f && bmax < 9.765625e-4f) ||
-                     (on && (key >> 16) >= kkey && !(fabsf(v) <= 32.0f)) || (sel && close);
+                     (on && (key >> 16) >= kkey && (close || !(fabsf(v) <= 32.0f)));
     if (__any_sync(0xffffffffu, odd)) return false;
     const float q = sel ? (float)exp((double)__fsub_rn(v, top)) : 0.0f;
     float sw = 0.0f;

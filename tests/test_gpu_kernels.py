@@ -492,6 +492,44 @@ def test_router_small_logits_in_any_company(gpu, orc, be, synth, path, T, E, K, 
     assert np.abs(gw.astype(np.int32) - ew.astype(np.int32)).max() <= 1
 
 
+@pytest.mark.parametrize("T,K", [(256, 256), (640, 768)])
+@pytest.mark.parametrize("seed", range(4))
+def test_router_small_logits_where_code_order_decides(gpu, orc, be, synth, T, K, seed):
+    """Logits around 2^-10 and far below, in both forms of the many-token router and with every
+    product exact, so that the choice is made on codes: ties at the last place chosen with a
+    neighbour below them that has their probability, zeros of either sign beside values that
+    nothing tells from them, and logits that only the subtraction of the largest makes equal."""
+    rng = np.random.default_rng(seed)
+    E, edge = 128, 2.0 ** -10
+    small = [0.0, -0.0, edge, -edge, edge * (1 + 2 ** -7), edge * (1 - 2 ** -8), 2 ** -11,
+             -edge * (1 - 2 ** -8), 1e-5, 1.01e-5, -1e-5, 3e-20, -3e-20]
+    z = rng.normal(-1.0, 1.0, (T, E))
+    z = np.where(z > -0.01, z - 3.0, z)
+    for t in range(T):
+        n, top = int(rng.integers(0, 8)), int(rng.integers(0, 9))
+        where = rng.permutation(E)
+        z[t, where[:top]] = rng.uniform(0.01, 2.0, top)
+        z[t, where[top:top + n]] = rng.choice(small, n)
+    z[:3] = -2.0
+    z[:3, 1:8] = np.linspace(0.5, 2.0, 7)
+    z[0, [85, 97, 48]] = 1.0073e-05, 1.0073e-05, 1.0013e-05
+    z[1, [60, 70, 9]] = 0.0, -0.0, -3e-20
+    z[2, [7, 100, 50]] = 32.0, -131 * 2.0 ** -19, -133 * 2.0 ** -19
+    z = synth.f32_to_bf16(z.astype(np.float32))
+    x = np.zeros((T, K), np.uint16)
+    x[np.arange(T), np.arange(T)] = 0x3f80
+    cfg = dict(hidden=K, experts=E, moe_inter=16, shared_inter=16, top_k=8)
+    W = synth.host_weights(be, cfg, seed=1, sigma=0.05)
+    W["rtr_w"] = np.zeros((E, K), np.uint16)
+    W["rtr_w"][:, :T] = z.T
+    eidx, ew = orc.route_batch(x, W["rtr_w"], 8)
+    assert eidx[:3, 7].tolist() == [48, 9, 50]           # the lowest number of its probability
+    idx, w = _route_dev(gpu, synth, cfg, W, x)
+    assert gpu.last_block_status() == 0
+    assert np.array_equal(idx, eidx)
+    assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
+
+
 def test_router_certified_can_be_switched_off(be, orc, synth, monkeypatch):
     monkeypatch.setenv("APUS_CUDA_ROUTER_CERTIFY", "0")
     be.enable()
