@@ -611,6 +611,7 @@ static int dense_op(const uint16_t *w, const uint16_t *x, void *y, size_t M,
     a.w = (const uint16_t *)wb->ptr;
     a.wmin = wb->wmin;
     a.wmax = wb->wmax;
+    a.codes = ExactCodes(wb->wmin, wb->wmax);
     uint16_t *dx = (uint16_t *)c->io.take(xb);
     a.x = dx;
     void *dy = c->io.take(yb);

@@ -7,8 +7,8 @@
  * most 16 significant bits, so it is exact in fp32 unless it underflows or
  * overflows; then fma(w, x, acc) is the same number as rn(rn(w*x) + acc).  Each
  * CTA checks (smallest nonzero |w|, largest |w|: found once when the weights
- * become resident) against those of its own rows of x and otherwise runs the
- * literal multiply-then-add chain.
+ * become resident) against those of its own rows of x, the kernel of many rows block by
+ * block, and otherwise runs the literal multiply-then-add chain.
  *
  * The chain fixes the order inside an output, so the parallelism is outputs:
  *   exact_rows_kernel   up to four rows of x: one weight row per lane, weights
@@ -17,19 +17,14 @@
  * Both want K % 8 == 0 (16-byte pieces of a row); other K keep exact_gemm_kernel.
  */
 #pragma once
+#include <cmath>
+#include <cstring>
+#include <type_traits>
+
 #include "common.cuh"
 #include "decode_gemv.cuh"
 
 namespace apus {
-
-struct ExactArgs {
-    const uint16_t *w, *x;      /* [O, K], [M, K] */
-    void *y;                    /* [M, O] BF16, or fp32 with f32_out */
-    int M, K;
-    long O;
-    float wmin, wmax;           /* smallest nonzero |w| (0: unknown), largest |w| */
-    int f32_out;
-};
 
 /* |code| range of n BF16 values: out[0] = min over the nonzero ones, out[1] =
  * max, as fp32 bits (the host initialises them to +inf and 0) */
@@ -90,6 +85,47 @@ __device__ __forceinline__ bool products_exact(float wmin, float wmax, unsigned 
            (double)wmin * (double)__uint_as_float(xlo) >= 7.52316384526264e-37 && /* 2^-120 */
            (double)wmax * (double)__uint_as_float(xhi) < 1.7e38;                  /* < 2^127 */
 }
+/* The |code|s with which that holds, |code| - 1 from `below` (a zero is the largest) and |code|
+ * up to `high`; wmin, wmax: of the other side.  They are found once per launch: the products
+ * above in every block of a tile took 2 us of its 24. */
+struct ExactCodes {
+    unsigned below;
+    int high;                   /* -1: no product is known to be exact */
+    ExactCodes() = default;
+    __host__ ExactCodes(float wmin, float wmax) {
+        const double lo = wmin, hi = wmax;
+        auto value = [](int code) {
+            float f;
+            const unsigned bits = (unsigned)code << 16;
+            memcpy(&f, &bits, 4);
+            return (double)f;
+        };
+        auto first = [](auto holds) {               /* code in 1 .. 0x7f80 */
+            int a = 1, b = 0x7f80;
+            while (a < b) {
+                const int mid = (a + b) / 2;
+                if (holds(mid)) b = mid; else a = mid + 1;
+            }
+            return a;
+        };
+        below = (unsigned)first([&](int c) { return lo * value(c) >= 7.52316384526264e-37; }) - 1u;
+        high = first([&](int c) { return !(hi * value(c) < 1.7e38); }) - 1;
+        if (!(lo > 0.0) || !(hi < INFINITY)) high = -1;
+    }
+    __device__ __forceinline__ bool hold(unsigned lo, unsigned hi) const {
+        return lo >= below && (int)hi <= high;
+    }
+};
+struct ExactArgs {
+    const uint16_t *w, *x;      /* [O, K], [M, K] */
+    void *y;                    /* [M, O] BF16, or fp32 with f32_out */
+    int M, K;
+    long O;
+    float wmin, wmax;           /* smallest nonzero |w| (0: unknown), largest |w| */
+    ExactCodes codes;           /* of x, for exact_tile_kernel */
+    int f32_out;
+};
+
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void *src, bool valid) {
     const int bytes = valid ? 16 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes)
@@ -253,9 +289,12 @@ exact_rows_kernel(ExactArgs a) {
  *    of rows that a broadcast load puts where the multiply-add wants them; weights are a
  *    lane's own, stay BF16 (sixteen bytes are eight k) and are widened once for all RM rows.
  * Rows arrive in blocks of 64 k (cp.async, eight lanes per row; weights at pitch 144 bytes as
- * above), ET_STAGES - 1 blocks ahead; one barrier per block.  Whether all products are exact
- * is known when x has been read; where they are not, the CTA walks its chains again,
- * literally.
+ * above), ET_STAGES - 1 blocks ahead; one barrier per block.  Whether a block's products are
+ * exact is known when its x has been widened, a block ahead: up to the first that holds one
+ * that may not be, both forms of the chain are the same, and from there on it is literal.
+ * (A weight of 1e-38 among 512 rows, K 2048, O 1024 / 4096: calls of 201 / 481 us; the whole
+ * chain again where it turns out inexact at its end 279 / 712, x read twice to know it before
+ * 258 / 514.)
  * K 2048, a tile alone on its SM: 2 x 128 (rows x outputs) 31 us, 16 x 32 24, 16 x 64 30,
  * 32 x 128 69.  (Both operands widened in the lanes, 32 x 128: 74, 8 x 32: 28.) */
 constexpr int ET_STAGES = 4;
@@ -286,11 +325,11 @@ __device__ __forceinline__ void exact_step2(unsigned long long w, unsigned long 
     }
 }
 
-/* xlo, xhi: range of the magnitudes of the x values this thread has widened, |code| - 1 (a
- * zero is the largest) and |code| */
-template <int RM, int NO, int WM, bool FMA>
+/* literal: two words of shared memory: products of an even, an odd block widened so far may
+ * round */
+template <int RM, int NO, int WM>
 __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned char *smem, long o0,
-                                                int m0, unsigned &xlo, unsigned &xhi) {
+                                                int m0, volatile int *literal) {
     using Tile = ExactTile<RM, NO, WM>;
     constexpr int STEP = Tile::THREADS / 8;
     constexpr int XR = Tile::M * ER_BK / Tile::THREADS;  /* x rows that a thread widens */
@@ -335,13 +374,15 @@ __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned cha
                               xr0 * ER_BK + xk;
         if (++x_s == ET_STAGES) x_s = 0;
         float f[XR];
+        unsigned lo = 0xffffffffu, hi = 0;
 #pragma unroll
         for (int r = 0; r < XR; r++) {
             const unsigned v = src[r * ER_BK], m = v & 0x7fffu;
-            xlo = min(xlo, m - 1u);
-            xhi = max(xhi, m);
+            lo = min(lo, m - 1u);
+            hi = max(hi, m);
             f[r] = __uint_as_float(v << 16);
         }
+        if (!a.codes.hold(lo, hi)) literal[kb & 1] = 1;
         float *d = xs + (kb & 1) * (ER_BK * Tile::M);
         constexpr int V = XR < RM ? XR : RM < 4 ? RM : 4;    /* rows to a store, of one group */
         static_assert(XR % V == 0 && RM % V == 0, "");
@@ -363,17 +404,21 @@ __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned cha
     for (int i = 0; i < NO; i++)
 #pragma unroll
         for (int j = 0; j < RM / 2; j++) acc[i][j] = 0ull;
+    if (tid < 2) literal[tid] = 0;
     for (int kb = 0; kb < ET_STAGES - 1; kb++) fetch(kb);
     asm volatile("cp.async.wait_group %0;" ::"n"(ET_STAGES - 2) : "memory");
     __syncthreads();
     widen_x(0);
     int s = 0;
-#pragma unroll 1
-    for (int kb = 0; kb < nkb; kb++) {
+    auto landed = [&] {        /* block kb + 1 everywhere; block kb - 1 is used up */
         asm volatile("cp.async.wait_group %0;" ::"n"(ET_STAGES - 3) : "memory");
-        __syncthreads();       /* block kb + 1 landed everywhere, block kb - 1 is used up */
+        __syncthreads();
+    };
+    auto ahead = [&](int kb) {
         fetch(kb + ET_STAGES - 1);
         if (kb + 1 < nkb) widen_x(kb + 1);
+    };
+    auto multiply = [&](int kb, auto fma) {
         const unsigned char *wb =
             smem + (size_t)s * Tile::W_STAGE + (size_t)(wo * 32 * NO + lane) * ER_PITCH;
         const float *xb = xs + (kb & 1) * (ER_BK * Tile::M) + wm * (ER_BK * RM);
@@ -417,7 +462,8 @@ __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned cha
                     const float f = (h & 1) ? bf16hi(v) : bf16lo(v);
                     const unsigned long long wp = pack_f32x2(f, f);
 #pragma unroll
-                    for (int j = 0; j < RM / 2; j++) exact_step2<FMA>(wp, q[h][j], acc[i][j]);
+                    for (int j = 0; j < RM / 2; j++)
+                        exact_step2<decltype(fma)::value>(wp, q[h][j], acc[i][j]);
                 }
         };
         load_w(0, wq[0]);
@@ -437,7 +483,25 @@ __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned cha
             use(wq[1], 1, xp[1]);
         }
         if (++s == ET_STAGES) s = 0;
+    };
+    int kb = 0;
+    bool lit = false;
+#pragma unroll 1
+    for (; kb < nkb; kb++) {
+        landed();
+        lit = literal[kb & 1] != 0;
+        ahead(kb);
+        if (lit) break;
+        multiply(kb, std::true_type());
     }
+    if (lit)
+#pragma unroll 1
+        for (;;) {
+            multiply(kb, std::false_type());
+            if (++kb == nkb) break;
+            landed();
+            ahead(kb);
+        }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 #pragma unroll
@@ -464,29 +528,13 @@ __global__ void __launch_bounds__(ET_WARPS * 32)
 exact_tile_kernel(ExactArgs a) {
     using Tile = ExactTile<RM, NO, WM>;
     extern __shared__ __align__(16) unsigned char et_smem[];
-    __shared__ unsigned int s_lo, s_hi;
+    __shared__ int s_literal[2];
     const long mt = (a.M + Tile::M - 1) / Tile::M, tiles = mt * ((a.O + Tile::O - 1) / Tile::O);
 #pragma unroll 1
     for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const long o0 = tile / mt * Tile::O;
-        const int m0 = (int)(tile - tile / mt * mt) * Tile::M;
-        if (threadIdx.x == 0) {
-            s_lo = 0xffffffffu;
-            s_hi = 0;
-        }
-        unsigned lo = 0xffffffffu, hi = 0;
-        exact_tile_body<RM, NO, WM, true>(a, et_smem, o0, m0, lo, hi);
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&s_lo, lo);
-            atomicMax(&s_hi, hi);
-        }
-        __syncthreads();
-        const unsigned xlo = s_lo == 0xffffffffu ? 0x7f800000u : (s_lo + 1u) << 16;
-        if (!products_exact(a.wmin, a.wmax, xlo, s_hi << 16))
-            exact_tile_body<RM, NO, WM, false>(a, et_smem, o0, m0, lo, hi);
-        __syncthreads();
+        const long ot = tile / mt;
+        exact_tile_body<RM, NO, WM>(a, et_smem, ot * Tile::O, (int)(tile - ot * mt) * Tile::M,
+                                    s_literal);
     }
 }
 

@@ -72,6 +72,22 @@ def test_hook_exact_tiles_past_their_edges(gpu, orc, M, O, K, scale):
     assert np.array_equal(gpu.bf16_gemm(w, x), orc.gemm(w, x))
 
 
+@pytest.mark.parametrize("M,O", [(5, 127), (97, 481), (130, 900), (521, 2341)])    # each tile
+@pytest.mark.parametrize("block", [0, 1, 2, 5])
+def test_hook_exact_tiles_turn_literal_on_the_way(gpu, orc, M, O, block):
+    """The first product that is not exact in some block of 64 k: from there on the sums are
+    the literal chain's, infinite past a product that overflows, where fused multiply-adds
+    (-3e38 + 4e38) stay finite."""
+    K, k = 328, 64 * block
+    rng = np.random.default_rng(M + block)
+    w, x = rng_codes(rng, (O, K), 0.5), rng_codes(rng, (M, K), 1.0)
+    w[:, k:k + 2] = x[:, k + 1] = 0x5f8b                 # 2e19
+    x[:, k] = 0xdf50                                     # -1.5e19
+    exp = orc.gemm(w, x)
+    assert np.isinf(f32(exp)).all()
+    assert np.array_equal(gpu.bf16_gemm(w, x), exp)
+
+
 @pytest.mark.parametrize("M", [1, 3])
 @pytest.mark.parametrize("K", [15, 17, 31, 34, 1001])
 @pytest.mark.parametrize("scale", ["plain", "underflow", "overflow"])
