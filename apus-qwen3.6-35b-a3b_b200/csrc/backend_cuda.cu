@@ -531,11 +531,18 @@ static const DevBuf *weight_buf(Ctx *c, const void *ptr, size_t bytes) {
  *  - up to ER_MAX_M rows: weights streamed row by row, one chain per lane.  As
  *    few warps per CTA as still put a CTA on every SM (a lane's chain takes the
  *    same time however many run beside it), at most eight;
- *  - more rows: by outputs per SM.  A wide warp tile widens fewer operands per
- *    multiply-add but leaves SMs idle when there are few outputs (calls, K 2048, in us, with
- *    tiles of 2 x 128, 16 x 32, 16 x 64, 32 x 128: M 32, O 1024 54, 59, 63, 101; M 64 81, 71,
- *    81, 119; M 128 135, 97, 94, 132; M 512 247, 196, 171, 201; O 2048 429, 283, 228, 234;
- *    O 4096 762, 493, 365, 340);
+ *  - more rows: by tiles, counted whole, edges and all (by outputs per SM, 100 x 700 took
+ *    154 tiles of 16 x 32 for 148 SMs and 102 us, 87 before that; now 80).  In us, K 2048, tiles
+ *    of 2 x 128, 8 x 64, 16 x 64, 32 x 128 (rows x outputs):
+ *      one wave of 2 x 128: 8 x 4096 50, 51, 59, 97; 16 x 2048 51, 53, 60, 98;
+ *      else one of 8 x 64: 9 x 4096 68, 57, 68, 105; 35 x 1032 72, 63, 74, 111; 64 x 518 75, 67,
+ *      75, 112; a call in parts, which run one behind the other, has up to three of them:
+ *      300 x 512 149, 141, 150, 186; 429 x 317 171, 157, 171, 204; 262 x 1324 (five) 164 with
+ *      8 x 64, 146 with 16 x 64;
+ *      else 16 x 64 or 32 x 128, a wave of which takes 3.1 times as long: 100 x 4018 231, 169, 141,
+ *      144 (3 waves and 1); 100 x 4096 229, 167, 156, 143 (4 and 1); 150 x 4096 348, 249, 226, 237
+ *      (5 and 2); 240 x 4096 473, 333, 284, 259 (7 and 2).  In parts 16 x 64 stays ahead for
+ *      longer: 512 x 2048 446, 282, 224, 233; 512 x 4096 793, 499, 368, 330;
  *  - K not a multiple of 8: rows are not made of aligned 16-byte pieces, the
  *    plain kernel.
  * M_all: rows of the whole call when a.M is one of the parts it runs in. */
@@ -564,7 +571,6 @@ static int launch_exact(Ctx *c, const ExactArgs &a, int M_all, cudaStream_t st) 
         if (!allow((const void *)kern, smem)) return fail("exact rows: shared memory");
         kern<<<(unsigned)grid, warps * 32, smem, st>>>(a);
     } else if (a.K % 8 == 0) {
-        const long per_sm = (long)M_all * a.O / c->sm_count;
         auto launch = [&](auto tile, void (*kern)(ExactArgs)) -> int {
             using Tile = decltype(tile);
             const long all = ((long)a.M + Tile::M - 1) / Tile::M * ((a.O + Tile::O - 1) / Tile::O);
@@ -572,10 +578,20 @@ static int launch_exact(Ctx *c, const ExactArgs &a, int M_all, cudaStream_t st) 
             kern<<<(unsigned)(all < (1 << 30) ? all : 1 << 30), Tile::THREADS, Tile::SMEM, st>>>(a);
             return 0;
         };
-        const int rc = per_sm <= 256    ? launch(ExactTile<2, 1, 1>(), exact_tile_kernel<2, 1, 1>)
-                       : per_sm <= 512  ? launch(ExactTile<4, 1, 4>(), exact_tile_kernel<4, 1, 4>)
-                       : per_sm <= 8192 ? launch(ExactTile<4, 2, 4>(), exact_tile_kernel<4, 2, 4>)
-                                        : launch(ExactTile<8, 4, 4>(), exact_tile_kernel<8, 4, 4>);
+        auto waves = [&](auto tile) {
+            using Tile = decltype(tile);
+            const long all = ((long)M_all + Tile::M - 1) / Tile::M * ((a.O + Tile::O - 1) / Tile::O);
+            return (all + c->sm_count - 1) / c->sm_count;
+        };
+        const bool parts = M_all > a.M;
+        const bool wide = parts ? (long)M_all * a.O / c->sm_count > 8192
+                                : 10 * waves(ExactTile<4, 2, 4>()) > 31 * waves(ExactTile<8, 4, 4>());
+        const int rc = waves(ExactTile<2, 1, 1>()) == 1
+                           ? launch(ExactTile<2, 1, 1>(), exact_tile_kernel<2, 1, 1>)
+                       : waves(ExactTile<4, 1, 2>()) <= (parts ? 3 : 1)
+                           ? launch(ExactTile<4, 1, 2>(), exact_tile_kernel<4, 1, 2>)
+                       : wide ? launch(ExactTile<8, 4, 4>(), exact_tile_kernel<8, 4, 4>)
+                              : launch(ExactTile<4, 2, 4>(), exact_tile_kernel<4, 2, 4>);
         if (rc) return 1;
     } else {
         const long total = (long)a.M * a.O;

@@ -295,8 +295,8 @@ exact_rows_kernel(ExactArgs a) {
  * (A weight of 1e-38 among 512 rows, K 2048, O 1024 / 4096: calls of 201 / 481 us; the whole
  * chain again where it turns out inexact at its end 279 / 712, x read twice to know it before
  * 258 / 514.)
- * K 2048, a tile alone on its SM: 2 x 128 (rows x outputs) 31 us, 16 x 32 24, 16 x 64 30,
- * 32 x 128 69.  (Both operands widened in the lanes, 32 x 128: 74, 8 x 32: 28.) */
+ * K 2048, a tile alone on its SM: 2 x 128 (rows x outputs) 24.5 us, 8 x 64 25.2, 16 x 64 31.5,
+ * 32 x 128 69.7.  (Both operands widened in the lanes, 32 x 128: 74, 8 x 32: 28.) */
 constexpr int ET_STAGES = 4;
 constexpr int ET_WARPS = 4;
 template <int RM, int NO, int WM>

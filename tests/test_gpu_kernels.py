@@ -33,9 +33,9 @@ def test_hook_gemm_bitwise(gpu, orc, M):
 
 @pytest.mark.parametrize("M,O,K", [
     (1, 31, 8), (1, 33, 64), (2, 32, 72), (3, 5000, 136), (4, 95, 2048),   # rows per lane
-    (5, 64, 8), (16, 65, 40), (17, 63, 96), (9, 130, 2048),                # 8-row tiles
-    (50, 2300, 72), (51, 4000, 136), (300, 1000, 104),                     # 16 and 32 rows
-    (129, 2560, 512), (513, 1500, 520)])                                   # 32 rows, in parts
+    (5, 64, 8), (16, 65, 40), (17, 63, 96), (9, 130, 2048),                # 2-row tiles
+    (50, 2300, 72), (51, 4000, 136), (300, 1000, 104),                     # 16-row tiles
+    (129, 2560, 512), (513, 1500, 520)])                                   # the same, in parts
 @pytest.mark.parametrize("scale", ["plain", "underflow", "overflow"])
 def test_hook_exact_order_kernels(gpu, orc, M, O, K, scale):
     """Each kernel of the exact-order product at the edges of its tiles, with
@@ -56,10 +56,11 @@ def test_hook_exact_order_kernels(gpu, orc, M, O, K, scale):
 
 
 @pytest.mark.parametrize("M,O,K", [
-    (5, 127, 64), (7, 129, 136),                       # tiles of 2 x 128
-    (65, 640, 200), (97, 481, 64),                     # 16 x 32
-    (67, 1217, 136), (130, 900, 72),                   # 16 x 64
-    (521, 2341, 72)])                                  # 32 x 128
+    (5, 127, 64), (7, 129, 136), (8, 4736, 64),        # tiles of 2 x 128
+    (65, 640, 200), (97, 481, 64), (9, 4736, 64),      # 8 x 64
+    (260, 300, 1016),                                  # the same in parts
+    (67, 1217, 136), (130, 900, 72), (521, 2341, 72),  # 16 x 64
+    (125, 3650, 72)])                                  # 32 x 128
 @pytest.mark.parametrize("scale", ["plain", "underflow"])
 def test_hook_exact_tiles_past_their_edges(gpu, orc, M, O, K, scale):
     """The tiles of the product of many rows, rows, outputs and k blocks left over; one row of
@@ -72,7 +73,7 @@ def test_hook_exact_tiles_past_their_edges(gpu, orc, M, O, K, scale):
     assert np.array_equal(gpu.bf16_gemm(w, x), orc.gemm(w, x))
 
 
-@pytest.mark.parametrize("M,O", [(5, 127), (97, 481), (130, 900), (521, 2341)])    # each tile
+@pytest.mark.parametrize("M,O", [(5, 127), (97, 481), (130, 900), (125, 3650)])    # each tile
 @pytest.mark.parametrize("block", [0, 1, 2, 5])
 def test_hook_exact_tiles_turn_literal_on_the_way(gpu, orc, M, O, block):
     """The first product that is not exact in some block of 64 k: from there on the sums are
