@@ -1594,7 +1594,12 @@ static int launch_rmsnorm(Ctx *c, const uint16_t *x, const uint16_t *w, uint16_t
     const bool enough = chunks >= 16 || (chunks == 8 && T <= 4 * c->sm_count);
     if (N >= 512 && N % 8 == 0 && enough && rows <= 40 * 1024 &&
         (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) == 0) {
-        launch_k(rmsnorm_rows_kernel, dim3((T + RN_WARPS - 1) / RN_WARPS), dim3(RN_WARPS * 32),
+        const int nu = LaneRow(N).nu;
+        auto kern = nu <= 2   ? rmsnorm_rows_kernel<2>
+                    : nu <= 4 ? rmsnorm_rows_kernel<4>
+                    : nu <= 8 ? rmsnorm_rows_kernel<8>
+                              : rmsnorm_rows_kernel<0>;
+        launch_k(kern, dim3((T + RN_WARPS - 1) / RN_WARPS), dim3(RN_WARPS * 32),
                  rows, st, x, w, y, T, N, LaneRow(N));
         LAUNCHED();
         return 0;

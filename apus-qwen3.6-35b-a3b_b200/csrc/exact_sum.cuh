@@ -196,7 +196,16 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
 #pragma unroll 1
         for (; cur < end; cur++) {
             float t = s;
-            each([&](const float (&q)[8]) { t = add8(t, q); });      /* its own lane's counts */
+            if (P > 0) {                                     /* its own lane's counts */
+                each([&](const float (&q)[8]) { t = add8(t, q); });
+            } else if (lane == cur) {                        /* one lane's way to its squares */
+#pragma unroll 2
+                for (int u = 0; u < nu; u++) {
+                    float q[8];
+                    square8(mine + u * 16, q);
+                    t = add8(t, q);
+                }
+            }
             s = __shfl_sync(0xffffffffu, t, cur);
         }
     }
@@ -205,12 +214,6 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
         meet();
     }
     return s;
-}
-/* by one warp */
-__device__ __forceinline__ float exact_sumsq(const unsigned char *row, const LaneRow lr,
-                                             int lane) {
-    return lr.nu <= 8 ? exact_sumsq<8>(row, lr, lane, 0, 1, nullptr, [] {})
-                      : exact_sumsq<0>(row, lr, lane, 0, 1, nullptr, [] {});
 }
 
 /* y = rnd((x * rs) * (1 + w)), eight values; w: the gain offsets */
@@ -230,10 +233,14 @@ __device__ __forceinline__ float norm_scale(float ss, int H) {
 }
 
 /* RMSNorm with (1+w) gain (c/attn.h:175-186), rows of N % 8 == 0 values, 16-byte
- * aligned; one warp per row.  Bound: the latency of one row for few rows, and
- * instruction issue for many.  N 2048: 11.1 us for up to 64 rows (launch included; 11.2 with the
- * squares in shared memory), 10.6 for 1999 (16.1), 27.5 for 8192 (33.7). */
+ * aligned; one warp per row.  Bound: the latency of one row for few rows, and instruction issue
+ * for many.  P as above, the smallest that holds lr.nu pieces (a lane adds the zeros of the
+ * others too, and every piece takes registers from the rows beside it): 2 from N 512, 4, 8 up
+ * to 2048; 0: longer rows and those of few lanes.  us, squares in shared memory -> as now (P 8
+ * or 0 for all): 8192 rows of N 512 21.1 -> 17.9 (24.2), 1024 26.2 -> 20.0 (26.9), 2048 35.7 ->
+ * 31.1, 2560 42.4 -> 42.5 (52.8), 4096 60.3 -> 61.2 (73.6); 33 rows of 2048 11.7 -> 10.3. */
 constexpr int RN_WARPS = 4;
+template <int P>
 __global__ void __launch_bounds__(RN_WARPS * 32)
 rmsnorm_rows_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ w,
                     uint16_t *__restrict__ y, int T, int N, LaneRow lr) {
@@ -265,7 +272,8 @@ rmsnorm_rows_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__
             *reinterpret_cast<uint4 *>(row + lr.at(c)) = __ldg(src + c);
     }
     __syncwarp();
-    const float rs = norm_scale(exact_sumsq(row, lr, lane), N);
+    const float rs =
+        norm_scale(exact_sumsq<P>(row, lr, lane, 0, 1, nullptr, [] {}), N);
     uint4 *dst = reinterpret_cast<uint4 *>(y + (size_t)t * N);
     if (N <= R * 256) {
 #pragma unroll

@@ -590,7 +590,8 @@ def test_rmsnorm_and_residual_add_bitwise(gpu, orc, be, synth, T, N):
     assert np.array_equal(d_y.cpu().numpy().view(np.uint16), orc.resadd(x, b))
 
 
-@pytest.mark.parametrize("N", [8, 128, 256, 768, 2048, 2560, 512, 576, 640, 1152, 1056, 4096])
+@pytest.mark.parametrize("N", [8, 128, 256, 768, 2048, 2560, 512, 576, 640, 1152, 1056, 4096,
+                               1024, 1280, 2304])
 def test_rmsnorm_sum_without_the_chain(gpu, orc, N):
     """The sum of squares composed from parity functions against the sequential
     chain, bit for bit, on rows made to go wrong: ties in every add, sums that sit
