@@ -62,7 +62,7 @@ SYMBOLS = [
     "apus_cuda_layer_destroy", "apus_cuda_layer_tensor",
     "apus_cuda_layer_refresh", "apus_cuda_layer_upload",
     "apus_cuda_layer_load_slabs", "apus_cuda_register_layer_slabs",
-    "apus_cuda_debug_fast_logits", "apus_cuda_moe_block_dev",
+    "apus_cuda_debug_fast_logits", "apus_cuda_debug_sumsq", "apus_cuda_moe_block_dev",
     "apus_cuda_moe_layer_dev", "apus_cuda_moe_stack_dev", "apus_cuda_reserve",
     "apus_cuda_last_block_launches", "apus_cuda_last_block_path",
     "apus_cuda_last_block_status",
@@ -136,6 +136,7 @@ class Backend:
                                                      C.c_char_p, C.c_int]
         L.apus_cuda_debug_fast_logits.argtypes = [u16p, u16p, sz, sz, sz, f32p,
                                                   f32p, f32p, f32p]
+        L.apus_cuda_debug_sumsq.argtypes = [u16p, sz, sz, C.c_int, C.c_int, f32p]
         L.apus_cuda_moe_block_dev.argtypes = [vp, vp, vp, sz,
                                               C.POINTER(MoeTrace), vp]
         L.apus_cuda_moe_layer_dev.argtypes = [vp, vp, vp, vp, sz, C.POINTER(MoeTrace), vp]
@@ -377,6 +378,15 @@ class Backend:
             _ptr(xn, f32p), _ptr(wn, f32p), _ptr(cb, f32p)),
             "apus_cuda_debug_fast_logits")
         return fast, xn, wn, float(cb[0])
+
+    def debug_sumsq(self, x, pieces, warps):
+        """The sums of squares of the rows, in a form of the norm kernels."""
+        x = _u16(x)
+        T, N = x.shape
+        out = np.zeros(T, np.float32)
+        self._check(self.lib.apus_cuda_debug_sumsq(_ptr(x, u16p), T, N, pieces, warps,
+                                                   _ptr(out, f32p)), "apus_cuda_debug_sumsq")
+        return out
 
     def reserve(self, cfg, T):
         c = MoeCfg.from_dict(cfg)

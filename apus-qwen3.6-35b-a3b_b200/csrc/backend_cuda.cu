@@ -1242,6 +1242,23 @@ dbg_xnorm_kernel(const uint16_t *__restrict__ x, int T, int K, float *__restrict
     ss = warp_sum(ss);
     if (lane == 0) out[warp] = sqrtf(ss) * 1.001f;
 }
+/* the sum of squares of a row (a CTA each) by one warp or two */
+template <int P>
+__global__ void __launch_bounds__(64)
+dbg_sumsq_kernel(const uint16_t *__restrict__ x, int N, LaneRow lr, int parts,
+                 float *__restrict__ out) {
+    extern __shared__ __align__(16) unsigned char dq_smem[];
+    __shared__ float s_sum;
+    const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint4 *src = reinterpret_cast<const uint4 *>(x + (size_t)blockIdx.x * N);
+    for (int c = threadIdx.x; c < N / 8; c += 64)
+        *reinterpret_cast<uint4 *>(dq_smem + lr.at(c)) = src[c];
+    __syncthreads();
+    if (part >= parts) return;
+    const float s = exact_sumsq<P>(dq_smem, lr, lane, part, parts, &s_sum,
+                                   [] { asm volatile("bar.sync 1, 64;" ::: "memory"); });
+    if (part == parts - 1 && lane == 31) out[blockIdx.x] = s;
+}
 __global__ void __launch_bounds__(256)
 dbg_sum_slabs_kernel(const float *__restrict__ slabs, int nslab, size_t n,
                      float *__restrict__ out) {
@@ -1298,6 +1315,36 @@ extern "C" int apus_cuda_debug_fast_logits(const uint16_t *x, const uint16_t *wg
     CU_OK(cudaStreamSynchronize(st));
     if (stw) return fail("debug_fast_logits: device status %d", stw);
     *cbound = 9.1f * (float)K * 5.9604645e-8f;
+    return 0;
+}
+
+extern "C" int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int pieces, int warps,
+                                     float *out) {
+    if (!x || !out || !T || !N || N % 8 || N > 16384 || T > 65535)
+        return fail("debug_sumsq: bad args");
+    const LaneRow lr((int)N);
+    const int per = warps > 0 ? lr.nu / warps : 0;
+    auto kern = pieces == 0   ? dbg_sumsq_kernel<0>
+                : pieces == 2 ? dbg_sumsq_kernel<2>
+                : pieces == 4 ? dbg_sumsq_kernel<4>
+                : pieces == 8 ? dbg_sumsq_kernel<8>
+                              : nullptr;
+    if (!kern || (warps != 1 && (warps != 2 || lr.nu % 2)) || (pieces && per > pieces))
+        return fail("debug_sumsq: %d pieces of %d, %d warps", pieces, lr.nu, warps);
+    std::lock_guard<std::recursive_mutex> lk(g_mu);
+    if (ctx_init()) return 1;
+    Ctx *c = g_ctx;
+    Ordered ord(c, c->stream);
+    if (ord.rc) return 1;
+    if (arena_reserve(c->io, T * N * 2 + T * 4 + 1024)) return 1;
+    c->io.reset();
+    uint16_t *dx = (uint16_t *)c->io.take(T * N * 2);
+    float *ds = (float *)c->io.take(T * 4);
+    CU_OK(cudaMemcpyAsync(dx, x, T * N * 2, cudaMemcpyHostToDevice, c->stream));
+    kern<<<(unsigned)T, 64, (size_t)lr.bytes(), c->stream>>>(dx, (int)N, lr, warps, ds);
+    LAUNCHED();
+    CU_OK(cudaMemcpyAsync(out, ds, T * 4, cudaMemcpyDeviceToHost, c->stream));
+    CU_OK(cudaStreamSynchronize(c->stream));
     return 0;
 }
 

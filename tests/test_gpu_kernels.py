@@ -617,6 +617,34 @@ def test_rmsnorm_sum_without_the_chain(gpu, orc, N):
     assert np.array_equal(d_y.cpu().numpy().view(np.uint16), orc.rmsnorm(x, None))
 
 
+@pytest.mark.parametrize("N,pieces,warps", [
+    (512, 2, 1), (768, 4, 1), (1024, 4, 1), (1280, 8, 1), (1792, 8, 1), (2048, 8, 1),
+    (1152, 0, 1), (2304, 0, 1), (2560, 0, 1), (208, 0, 1),          # rows of the row norm
+    (512, 4, 2), (1536, 4, 2), (2048, 4, 2), (2560, 0, 2), (144, 0, 1), (16, 4, 1), (1024, 4, 2)])
+def test_sum_of_squares_is_the_chains(gpu, N, pieces, warps):
+    """The fp32 sum itself, which a norm shows only through BF16, in every form that the row norm
+    and the one-kernel path use: ties in every add, sums on a binade's edge, jumps over binades
+    in either half of a row, falling and rising terms, subnormal squares, an overflow."""
+    rng = np.random.default_rng(N + pieces + warps)
+    at = np.arange(N)
+    rows = [np.ones(N), np.full(N, 1.5), np.full(N, 1.0 + 2 ** -7), np.zeros(N),
+            np.full(N, 1e20), np.sign(rng.normal(0, 1, N)) * 181.0, rng.integers(1, 4, N) * 0.5,
+            np.exp2(np.linspace(6, -12, N)), np.exp2(np.linspace(-12, 6, N)),
+            np.where(at % 64 == 0, 8.0, 0.0), rng.normal(0, 1e-18, N), rng.normal(0, 1e-22, N)]
+    rows += [np.where(at == p, 1e3, rng.normal(0, 1, N))
+             for p in (0, N // 4, N // 2 - 1, N // 2, N - 1)]
+    rows += [rng.normal(0, 2.0 ** rng.uniform(-4, 4), N) for _ in range(200)]
+    u = np.asarray(rows, np.float32).view(np.uint32).astype(np.uint64)
+    x = ((u + 0x7fff + ((u >> 16) & 1)) >> 16).astype(np.uint16)
+    with np.errstate(over="ignore", under="ignore"):
+        q = f32(x) * f32(x)
+        exp = np.zeros(len(rows), np.float32)
+        for k in range(N):
+            exp = exp + q[:, k]
+    got = gpu.debug_sumsq(x, pieces, warps)
+    assert np.array_equal(got.view(np.uint32), exp.view(np.uint32))
+
+
 # ---- the dense weight stream on device pointers --------------------------------
 
 @pytest.mark.parametrize("M,O,K,shift", [
