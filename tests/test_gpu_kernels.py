@@ -300,14 +300,13 @@ def test_router_certified_selection_is_exact(gpu, orc, be, synth, T, case):
 
 
 @pytest.mark.parametrize("T,E,K,kind", [
-    (148, 256, 2048, "bias"), (149, 256, 2048, "bias"),        # one token to a CTA, then two
-    (888, 256, 2048, "plain"), (889, 256, 2048, "bias"),       # deep rings, then shallow ones
+    (148, 256, 2048, "bias"), (149, 256, 2048, "bias"),        # a token to an SM, and one more
+    (888, 256, 2048, "plain"), (889, 256, 2048, "bias"),       # whole CTAs of tokens, a rest
     (65, 1024, 256, "plain"), (66, 128, 768, "bias"), (67, 384, 2304, "plain"),
     (65, 128, 512, "subnormal"), (65, 128, 512, "ties"), (65, 1024, 512, "zero")])
 def test_router_certified_kernel_edges(gpu, orc, be, synth, T, E, K, kind):
-    """The instances of the certifying kernel on both sides of the sizes that choose
-    between them; every logit on a chain of its own (products that round, ties of all
-    experts), more of them than one pass over the products takes, and tokens of zeros."""
+    """Both forms of the certifying router, up to 256 experts and more: selected logits that are
+    small beside their terms, products that round, ties of all experts, tokens of zeros."""
     cfg = dict(hidden=K, experts=E, moe_inter=128, shared_inter=128, top_k=8)
     W = synth.host_weights(be, cfg, seed=T + K, sigma=0.05)
     x = synth.host_x(be, T, K, seed=T + E)
@@ -333,9 +332,8 @@ def test_router_certified_kernel_edges(gpu, orc, be, synth, T, E, K, kind):
     (65, 256, "plain"), (296, 256, "bias"), (297, 256, "bias"), (65, 128, "ties"),
     (66, 256, "ties"), (67, 256, "zero"), (68, 256, "subnormal"), (69, 256, "huge")])
 def test_router_certified_chains_without_intervals(gpu, orc, be, synth, T, E, kind):
-    """Up to two tokens an SM (296) every candidate gets its chain at once: both sides of
-    that line, more candidates than lanes, products that round and logits of 2^110 (whose
-    bound is out of this form's range)."""
+    """The one-kernel form on one to three tokens an SM: more candidates than lanes, products
+    that round and logits of 2^110 (whose bound is out of the derivation's range)."""
     if kind != "huge":
         test_router_certified_kernel_edges(gpu, orc, be, synth, T, E, 2048, kind)
         return
@@ -413,8 +411,8 @@ def test_router_few_tokens_at_the_shared_memory_limit(gpu, orc, be, synth, T, E,
 
 @pytest.mark.parametrize("T", [1184, 1185, 1776, 1777, 2368, 2369])
 def test_router_certified_ring_and_chain_forms(gpu, orc, be, synth, T):
-    """Both sides of the token counts at which the ring of rows gets shallower (1184, 1776)
-    and the chains change their form (2368), with a router that leaves many logits open."""
+    """Candidate lists of eight to sixteen tokens an SM, tokens left over in the last CTA or
+    not, with a router whose logits lie close together."""
     cfg = dict(hidden=2048, experts=256, moe_inter=8, shared_inter=8, top_k=8)
     W = synth.host_weights(be, cfg, seed=T, sigma=0.02)
     x = synth.host_x(be, T, 2048, seed=T)
@@ -478,7 +476,8 @@ def test_router_few_tokens_weights_follow_the_engines_steps(gpu, orc, be, synth,
 def test_router_small_logits_in_any_company(gpu, orc, be, synth, path, T, E, K, seed):
     """Logits around 2^-10, below which two of them may have the same probability: one small
     competitor among others, several, beside zeros of either sign, as the last one chosen and
-    right below it.  One-hot tokens read the logits from the router matrix."""
+    right below it.  One-hot tokens read the logits from the router matrix.  (2e-38 makes
+    products round: above 64 tokens every token takes the softmax here.)"""
     rng = np.random.default_rng(seed)
     edge = 2.0 ** -10
     small = [0.0, -0.0, edge, -edge, edge * (1 + 2 ** -7), edge * (1 - 2 ** -8), 2 ** -11,
@@ -545,6 +544,43 @@ def test_router_small_logits_where_code_order_decides(gpu, orc, be, synth, T, K,
     assert gpu.last_block_status() == 0
     assert np.array_equal(idx, eidx)
     assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
+
+
+@pytest.mark.parametrize("T", [300, 640])                # one kernel, lists
+def test_router_candidates_and_gate_fill_a_warp(gpu, orc, be, synth, T):
+    """Tokens with 8 to 128 candidates side by side, the shared gate's chain the last that a
+    warp's lanes hold, the first beyond them, or far beyond: ids, weights and the gate's code."""
+    import torch
+    K, E = 768, 128
+    rng = np.random.default_rng(T)
+    counts = np.resize([8, 30, 31, 32, 33, 63, 64, 127, 128], T)
+    z = np.full((T, E), -1.0, np.float32)
+    for t in range(T):
+        z[t, rng.permutation(E)[:counts[t]]] = rng.choice([1.0, 1.0 + 2 ** -7], counts[t])
+    x = np.zeros((T, K), np.uint16)
+    x[np.arange(T), np.arange(T)] = 0x3f80               # each token reads its own column
+    cfg = dict(hidden=K, experts=E, moe_inter=128, shared_inter=128, top_k=8)
+    W = synth.host_weights(be, cfg, seed=1, sigma=0.05)
+    W["rtr_w"] = np.zeros((E, K), np.uint16)
+    W["rtr_w"][:, :T] = synth.f32_to_bf16(z).T
+    layer = gpu.layer_create(cfg, W)
+    d_x = torch.from_numpy(x.view(np.int16)).cuda()
+    d_idx = torch.full((T, 8), -1, dtype=torch.int32, device="cuda")
+    d_w = torch.zeros((T, 8), dtype=torch.int16, device="cuda")
+    d_gate = torch.zeros(T, dtype=torch.int16, device="cuda")
+    before = gpu.router_exact_chains()
+    gpu.ep_route_dev(layer, d_x.data_ptr(), T, d_idx.data_ptr(), d_w.data_ptr(),
+                     d_gate.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert gpu.last_block_status() == 0
+    assert gpu.router_exact_chains() - before == counts.sum() + T
+    eidx, ew = orc.route_batch(x, W["rtr_w"], 8)
+    w = d_w.cpu().numpy().view(np.uint16)
+    assert np.array_equal(d_idx.cpu().numpy(), eidx)
+    assert np.abs(w.astype(np.int32) - ew.astype(np.int32)).max() <= 1
+    gate = W["sh_gate"].reshape(-1)[:T]
+    assert np.array_equal(f32(d_gate.cpu().numpy().view(np.uint16)), f32(gate))
+    gpu.layer_destroy(layer)
 
 
 def test_router_certified_can_be_switched_off(be, orc, synth, monkeypatch):

@@ -103,9 +103,10 @@ def test_layer_at_the_real_dimensions_one_token(gpu, orc, be, synth):
 
 @pytest.mark.parametrize("H", [208, 512, 768, 1280, 1536, 2048])
 def test_one_kernel_norm_on_rows_made_to_go_wrong(gpu, be, synth, H):
-    """The one-kernel path's sum of squares, one warp or two to a row and lane chunks in
-    registers or not, against the row kernel's (which the checker's chain pins): sums on the
-    edge of a binade, ties in every add, a jump over binades, rising and falling terms."""
+    """The one-kernel path's norm, one warp or two to a row and lane chunks in registers or not,
+    against the row kernel's in the layer's output: sums on the edge of a binade, ties in every
+    add, a jump over binades, rising and falling terms.  (Last bits of the sum seldom show here:
+    test_sum_of_squares_is_the_chains compares them.)"""
     import torch
     cfg = dict(hidden=H, experts=64, moe_inter=16, shared_inter=16, top_k=8)
     layer = gpu.layer_create(cfg, synth.host_weights(be, cfg, seed=H, sigma=0.05))
