@@ -1243,7 +1243,7 @@ dbg_xnorm_kernel(const uint16_t *__restrict__ x, int T, int K, float *__restrict
     if (lane == 0) out[warp] = sqrtf(ss) * 1.001f;
 }
 /* the sum of squares of a row (a CTA each) by one warp or two */
-template <int P>
+template <int P, bool ALONE>
 __global__ void __launch_bounds__(64)
 dbg_sumsq_kernel(const uint16_t *__restrict__ x, int N, LaneRow lr, int parts,
                  float *__restrict__ out) {
@@ -1255,8 +1255,8 @@ dbg_sumsq_kernel(const uint16_t *__restrict__ x, int N, LaneRow lr, int parts,
         *reinterpret_cast<uint4 *>(dq_smem + lr.at(c)) = src[c];
     __syncthreads();
     if (part >= parts) return;
-    const float s = exact_sumsq<P>(dq_smem, lr, lane, part, parts, &s_sum,
-                                   [] { asm volatile("bar.sync 1, 64;" ::: "memory"); });
+    const float s = exact_sumsq<P, ALONE>(dq_smem, lr, lane, part, parts, &s_sum,
+                                          [] { asm volatile("bar.sync 1, 64;" ::: "memory"); });
     if (part == parts - 1 && lane == 31) out[blockIdx.x] = s;
 }
 __global__ void __launch_bounds__(256)
@@ -1324,12 +1324,13 @@ extern "C" int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int 
         return fail("debug_sumsq: bad args");
     const LaneRow lr((int)N);
     const int per = warps > 0 ? lr.nu / warps : 0;
-    auto kern = pieces == 0   ? dbg_sumsq_kernel<0>
-                : pieces == 2 ? dbg_sumsq_kernel<2>
-                : pieces == 4 ? dbg_sumsq_kernel<4>
-                : pieces == 8 ? dbg_sumsq_kernel<8>
+    auto kern = pieces == 0   ? dbg_sumsq_kernel<0, false>
+                : pieces == 2 ? dbg_sumsq_kernel<2, false>
+                : pieces == 4 ? dbg_sumsq_kernel<4, false>
+                : pieces == 8 ? dbg_sumsq_kernel<8, false>
+                : pieces < 0  ? dbg_sumsq_kernel<0, true>
                               : nullptr;
-    if (!kern || (warps != 1 && (warps != 2 || lr.nu % 2)) || (pieces && per > pieces))
+    if (!kern || (warps != 1 && (warps != 2 || lr.nu % 2)) || (pieces > 0 && per > pieces))
         return fail("debug_sumsq: %d pieces of %d, %d warps", pieces, lr.nu, warps);
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     if (ctx_init()) return 1;

@@ -379,8 +379,8 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
             if (a.res) {
                 const float ss =
                     lr.nu / parts <= 4
-                        ? exact_sumsq<4>(row, lr, lane, part, parts, &s_sum[t], meet)
-                        : exact_sumsq<0>(row, lr, lane, part, parts, &s_sum[t], meet);
+                        ? exact_sumsq<4, false>(row, lr, lane, part, parts, &s_sum[t], meet)
+                        : exact_sumsq<0, false>(row, lr, lane, part, parts, &s_sum[t], meet);
                 if (part) s_rs[t] = norm_scale(ss, H);
                 if (parts == 2) {
                     meet();

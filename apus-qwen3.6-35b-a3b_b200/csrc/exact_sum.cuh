@@ -86,8 +86,9 @@ __device__ __forceinline__ void square8(const unsigned char *p, float (&q)[8]) {
  * P > 0: a lane's chunk is at most P pieces, and its squares stay in registers.  What bounds
  * a row is the walk over the lanes that leave a binade (about seven of 32 or 64), one
  * addition after another: out of registers 150 cycles for 32 of them, out of shared memory
- * twice that.  (P == 0: any chunk, rolled loops over shared memory.) */
-template <int P, typename Meet>
+ * twice that.  (P == 0: any chunk, rolled loops over shared memory; ALONE: the walking lane
+ * reads alone, which an SM full of rows asks for.) */
+template <int P, bool ALONE, typename Meet>
 __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const LaneRow lr, int lane,
                                              int part, int parts, float *hand_over, Meet meet) {
     /* chunk of this lane: of lr.nl * parts chunks in row order */
@@ -196,9 +197,9 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
 #pragma unroll 1
         for (; cur < end; cur++) {
             float t = s;
-            if (P > 0) {                                     /* its own lane's counts */
+            if (!ALONE) {                                    /* its own lane's counts */
                 each([&](const float (&q)[8]) { t = add8(t, q); });
-            } else if (lane == cur) {                        /* one lane's way to its squares */
+            } else if (lane == cur) {
 #pragma unroll 2
                 for (int u = 0; u < nu; u++) {
                     float q[8];
@@ -273,7 +274,7 @@ rmsnorm_rows_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__
     }
     __syncwarp();
     const float rs =
-        norm_scale(exact_sumsq<P>(row, lr, lane, 0, 1, nullptr, [] {}), N);
+        norm_scale(exact_sumsq<P, P == 0>(row, lr, lane, 0, 1, nullptr, [] {}), N);
     uint4 *dst = reinterpret_cast<uint4 *>(y + (size_t)t * N);
     if (N <= R * 256) {
 #pragma unroll
