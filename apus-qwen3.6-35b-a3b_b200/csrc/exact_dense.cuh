@@ -295,8 +295,8 @@ exact_rows_kernel(ExactArgs a) {
  * (A weight of 1e-38 among 512 rows, K 2048, O 1024 / 4096: calls of 201 / 481 us; the whole
  * chain again where it turns out inexact at its end 279 / 712, x read twice to know it before
  * 258 / 514.)
- * K 2048, a tile alone on its SM: 2 x 128 (rows x outputs) 24.5 us, 8 x 64 25.2, 16 x 64 31.5,
- * 32 x 128 69.7.  (Both operands widened in the lanes, 32 x 128: 74, 8 x 32: 28.) */
+ * K 2048, a tile alone on its SM: 2 x 128 (rows x outputs) 24.3 us, 8 x 64 24.7, 16 x 64 29.9,
+ * 32 x 128 70.  (Both operands widened in the lanes, 32 x 128: 74, 8 x 32: 28.) */
 constexpr int ET_STAGES = 4;
 constexpr int ET_WARPS = 4;
 template <int RM, int NO, int WM>
@@ -476,7 +476,9 @@ __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned cha
                         exact_step2<decltype(fma)::value>(wp, q[h][j], acc[i][j]);
                 }
         };
-#pragma unroll 1
+        /* (unrolled, the products of a whole block are scheduled together: 16 x 64 31.6 -> 29.9 us,
+         * two of them on an SM 66.2 -> 62.4, 2 x 128 24.6 -> 24.3, 32 x 128 69.8 -> 70.0) */
+#pragma unroll
         for (int c = 0; c < ER_BK / 8; c += 2) {
             const int next = c + 2 < ER_BK / 8 ? c + 2 : 0;
             load_p(2 * c + 1, xp[1]);
