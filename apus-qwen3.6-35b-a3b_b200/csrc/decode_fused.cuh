@@ -575,7 +575,7 @@ decode_fused_kernel(const __grid_constant__ FusedArgs a) {
             const int t = amb[i] >> 11, e = amb[i] & 0x7ff;
             const uint16_t *w = e == E ? a.sh_gate : a.rtr_w + (size_t)e * H;
             const unsigned char *xr = xs + t * L.xrow;
-            const float z = warp_chains<4>(
+            const float z = warp_chains<CH_CHAINS>(
                 1, H, lane, reinterpret_cast<float *>(rr),
                 [&](int) { return w; },
                 [&](int p) { return *reinterpret_cast<const uint4 *>(xr + lr.at(p)); });

@@ -168,7 +168,7 @@ __device__ __forceinline__ bool rt_weights(const uint32_t *cd, const int *sel, i
  * wrow(c): weight row of chain c < n (called by all lanes together); xpiece(p): 16-byte
  * piece p of the token; buf: CH_ROW * G floats of shared memory, 16-byte aligned. */
 constexpr int CH_ROW = 256 + 4;          /* the rows of eight lanes in different banks */
-constexpr int CH_CHAINS = 8;
+constexpr int CH_CHAINS = 4;             /* G of the one-kernel path */
 constexpr int CH_BYTES = CH_CHAINS * CH_ROW * 4;
 template <int G, typename WRow, typename XPiece>
 __device__ __forceinline__ float warp_chains(int n, int K, int lane, float *buf, WRow wrow,
