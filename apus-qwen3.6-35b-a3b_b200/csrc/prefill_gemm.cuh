@@ -489,9 +489,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap mapA,     /* routed W */
                     asm volatile("fence.proxy.async;" ::: "memory");
                 }
                 int claim = tile;
-                /* Routed weights are read once, and evicted first they leave rows, activations
-                 * and outputs of the call in L2 (T 9: 109 -> 99 us a layer, 61: 254 -> 238, 128:
-                 * 297 -> 276 a block, 512: 316 -> 305, 1999: 394 -> 385).  Every token tile
+                /* Routed weights are read once, or by an expert's few token tiles side by side,
+                 * and evicted first they leave rows, activations and outputs of the call in L2
+                 * (T 9: 109 -> 99 us a layer, 61: 254 -> 238, 128: 297 -> 276 a block, 512: 316
+                 * -> 305, 1999: 394 -> 385; with a skewed router, whose hottest experts have up
+                 * to five tiles, 300: 321 -> 309, 1000: 357 -> 342, 1999: 396 -> 386, 3800: 506 ->
+                 * 503, and within 1 % of that where tiles with others behind them keep the
+                 * weights as usual).  Every token tile
                  * reads the shared expert's and the router's: those as usual (evicted first
                  * too, T 128 took 281, T 512 302).  The two-SM kernels, where later chunks of
                  * the expert read them again, lose (8192 tokens: 735 -> 790). */

@@ -21,8 +21,8 @@
  *      values further apart than it cannot round to the same code).  Any
  *      other expert's exact rounded logit is strictly below those of top_k
  *      experts, whatever the rounding did: it cannot be selected;
- *   4. every candidate (about top_k + 3 of 257 at the real dimensions, the
- *      shared-gate row included) gets its exact chain, and |a - z| <= B is checked on
+ *   4. every candidate (10.6 of 256 at the real dimensions, 12.7 with a skewed router) and
+ *      the shared-gate row get their exact chain, and |a - z| <= B is checked on
  *      every pair: ST_BOUND_VIOLATED is recorded if the assumption ever fails;
  *   5. selection and weights follow from the codes (router_select.cuh).
  *
@@ -76,7 +76,7 @@ struct CertifyArgs {
 constexpr int RC_NARROW = 32;
 constexpr int RC_SLOT_BITS = 11;    /* a slot is at most E <= 1024 */
 constexpr size_t RC_MAX_T = (size_t)1 << (32 - RC_SLOT_BITS);
-/* Counters that many tokens add to at once, one to a cache line: side by side, 96,000
+/* Counters that many tokens add to at once, one to a cache line: side by side, 87,000
  * additions to 256 counters took 10 of the candidates kernel's 38 us (8192 tokens). */
 constexpr int RC_COUNT_STEP = 32;
 inline int rc_code_pitch(int E) { return (E + 4) & ~3; }
@@ -247,8 +247,9 @@ router_candidates_kernel(const __grid_constant__ CertifyArgs a) {
  * arrive 64 k at a time (cp.async, eight lanes per row, pitch 144 bytes: a lane reads its
  * own row without bank conflicts, the weights as a broadcast), CW_STAGES - 1 blocks ahead.
  *
- * Bound: the rows' way from L2, 4 KB per chain (393 MB for 8192 tokens and an even router,
- * 460 for a skewed one): 45 us = 8.7 TB/s, and much the same with 8, 11, 12 and 15 warps of
+ * Bound: the rows' way from L2, 4 KB per chain (8192 tokens, gate included: 95,424 chains and
+ * 391 MB with an even router, 111,979 and 459 with a skewed one): 54 and 61 us by ncu, 7.2 and
+ * 7.5 TB/s, issue slots 57-60 % taken, and much the same with 8, 11, 12 and 15 warps of
  * 5, 4, 4 and 3 blocks each; blocks of 32 k 10-20 % slower.  Routing of 8192 tokens, even
  * and skewed: 92 and 100 us; with one warp per token, an interval around each chain (the same
  * rows) and a chain only where the interval left a code open: 126 and 174 (1999 tokens: 45 and

@@ -1,6 +1,7 @@
 /*
- * router_select.cuh — top-k selection on logit intervals (exact_sum.cuh), shared by
- * the one-kernel decode path and the many-token router (c/moe.h:321-371).
+ * router_select.cuh — top-k selection on the BF16 codes of logits (c/moe.h:321-371): intervals
+ * of them in the one-kernel decode path (exact_sum.cuh), known ones in the many-token router,
+ * where a token has more candidates than a warp has lanes, and in the few-token router.
  *
  * The engine takes the top-k of its softmax PROBABILITIES.  exp and the division keep
  * the order of the BF16 logits whenever the logits near the top differ by 2^-18 or
