@@ -292,7 +292,7 @@ exact_rows_kernel(ExactArgs a) {
  * above), ET_STAGES - 1 blocks ahead; one barrier per block.  Whether a block's products are
  * exact is known when its x has been widened, a block ahead: up to the first that holds one
  * that may not be, both forms of the chain are the same, and from there on it is literal.
- * (A weight of 1e-38 among 512 rows, K 2048, O 1024 / 4096: calls of 201 / 481 us; the whole
+ * (A weight of 1e-38 among 512 rows, K 2048, O 1024 / 4096: calls of 192 / 481 us; the whole
  * chain again where it turns out inexact at its end 279 / 712, x read twice to know it before
  * 258 / 514.)
  * K 2048, a tile alone on its SM: 2 x 128 (rows x outputs) 24.3 us, 8 x 64 24.7, 16 x 64 29.9,
@@ -476,9 +476,12 @@ __device__ __forceinline__ void exact_tile_body(const ExactArgs &a, unsigned cha
                         exact_step2<decltype(fma)::value>(wp, q[h][j], acc[i][j]);
                 }
         };
-        /* (unrolled, the products of a whole block are scheduled together: 16 x 64 31.6 -> 29.9 us,
-         * two of them on an SM 66.2 -> 62.4, 2 x 128 24.6 -> 24.3, 32 x 128 69.8 -> 70.0) */
-#pragma unroll
+        /* Unrolled, the products of a whole block are scheduled together: 16 x 64 31.6 -> 29.9 us,
+         * two of them on an SM 66.2 -> 62.4, 2 x 128 24.6 -> 24.3.  32 x 128 gains nothing (69.8,
+         * 70.0), and its literal form outgrows the instruction cache (calls of 512 x 4096 481 ->
+         * 600). */
+        constexpr int TURNS = RM * NO <= 8 ? ER_BK / 16 : 1;
+#pragma unroll TURNS
         for (int c = 0; c < ER_BK / 8; c += 2) {
             const int next = c + 2 < ER_BK / 8 ? c + 2 : 0;
             load_p(2 * c + 1, xp[1]);
