@@ -17,12 +17,11 @@
  * Both want K % 8 == 0 (16-byte pieces of a row); other K keep exact_gemm_kernel.
  */
 #pragma once
-#include <cmath>
-#include <cstring>
 #include <type_traits>
 
 #include "common.cuh"
 #include "decode_gemv.cuh"
+#include "exact_codes.h"
 
 namespace apus {
 
@@ -85,37 +84,6 @@ __device__ __forceinline__ bool products_exact(float wmin, float wmax, unsigned 
            (double)wmin * (double)__uint_as_float(xlo) >= 7.52316384526264e-37 && /* 2^-120 */
            (double)wmax * (double)__uint_as_float(xhi) < 1.7e38;                  /* < 2^127 */
 }
-/* The |code|s with which that holds, |code| - 1 from `below` (a zero is the largest) and |code|
- * up to `high`; wmin, wmax: of the other side.  They are found once per launch: the products
- * above in every block of a tile took 2 us of its 24. */
-struct ExactCodes {
-    unsigned below;
-    int high;                   /* -1: no product is known to be exact */
-    ExactCodes() = default;
-    __host__ ExactCodes(float wmin, float wmax) {
-        const double lo = wmin, hi = wmax;
-        auto value = [](int code) {
-            float f;
-            const unsigned bits = (unsigned)code << 16;
-            memcpy(&f, &bits, 4);
-            return (double)f;
-        };
-        auto first = [](auto holds) {               /* code in 1 .. 0x7f80 */
-            int a = 1, b = 0x7f80;
-            while (a < b) {
-                const int mid = (a + b) / 2;
-                if (holds(mid)) b = mid; else a = mid + 1;
-            }
-            return a;
-        };
-        below = (unsigned)first([&](int c) { return lo * value(c) >= 7.52316384526264e-37; }) - 1u;
-        high = first([&](int c) { return !(hi * value(c) < 1.7e38); }) - 1;
-        if (!(lo > 0.0) || !(hi < INFINITY)) high = -1;
-    }
-    __device__ __forceinline__ bool hold(unsigned lo, unsigned hi) const {
-        return lo >= below && (int)hi <= high;
-    }
-};
 struct ExactArgs {
     const uint16_t *w, *x;      /* [O, K], [M, K] */
     void *y;                    /* [M, O] BF16, or fp32 with f32_out */
