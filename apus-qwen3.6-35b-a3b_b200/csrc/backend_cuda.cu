@@ -23,6 +23,7 @@
 
 #include "common.cuh"
 #include "decode_fused.cuh"
+#include "decode_stack.cuh"
 #include "router_certify.cuh"
 #include "router_select.cuh"
 #include "router_small.cuh"
@@ -118,6 +119,7 @@ struct Ctx {
     uint16_t *d_df_chains = nullptr;             /* [DF_MAX_T * 1025] */
     uint16_t *d_df_act = nullptr, *d_df_sa = nullptr;
     unsigned int *d_df_sync = nullptr;
+    uint64_t *d_ds_codes = nullptr, *d_ds_chains = nullptr;     /* [DF_MAX_T][1025], tagged */
     unsigned long long *d_df_timeline = nullptr;   /* [sm_count][DF_MARKS] */
     bool df_timeline_valid = false;
     size_t df_act_elems = 0, df_sa_elems = 0;
@@ -231,6 +233,11 @@ static int ctx_init() {
     if (c->fused_max_t > DF_MAX_T) c->fused_max_t = DF_MAX_T;
     CU_OK(cudaMalloc(&c->d_df_codes, (size_t)DF_MAX_T * 1025 * sizeof(uint32_t)));
     CU_OK(cudaMalloc(&c->d_df_chains, (size_t)DF_MAX_T * 1025 * sizeof(uint16_t)));
+    const size_t ds_words = (size_t)DF_MAX_T * 1025 * sizeof(uint64_t);
+    CU_OK(cudaMalloc(&c->d_ds_codes, ds_words));
+    CU_OK(cudaMemset(c->d_ds_codes, 0, ds_words));      /* the tag of no launch */
+    CU_OK(cudaMalloc(&c->d_ds_chains, ds_words));
+    CU_OK(cudaMemset(c->d_ds_chains, 0, ds_words));
     CU_OK(cudaMalloc(&c->d_df_sync, 64));
     CU_OK(cudaMemset(c->d_df_sync, 0, 64));
     CU_OK(cudaMalloc(&c->d_df_timeline,
@@ -430,6 +437,8 @@ extern "C" void apus_cuda_disable(void) {
     if (c->d_df_codes) cudaFree(c->d_df_codes);
     if (c->d_df_chains) cudaFree(c->d_df_chains);
     if (c->d_df_sync) cudaFree(c->d_df_sync);
+    if (c->d_ds_codes) cudaFree(c->d_ds_codes);
+    if (c->d_ds_chains) cudaFree(c->d_ds_chains);
     if (c->d_df_timeline) cudaFree(c->d_df_timeline);
     if (c->d_df_act) cudaFree(c->d_df_act);
     if (c->d_df_sa) cudaFree(c->d_df_sa);
@@ -1243,6 +1252,20 @@ dbg_xnorm_kernel(const uint16_t *__restrict__ x, int T, int K, float *__restrict
     if (lane == 0) out[warp] = sqrtf(ss) * 1.001f;
 }
 /* the sum of squares of a row (a CTA each) by one warp or two */
+template <int W>
+__global__ void __launch_bounds__(W * 32)
+dbg_sumsq_wide_kernel(const uint16_t *__restrict__ x, int N, LaneRow lr, int,
+                      float *__restrict__ out) {
+    extern __shared__ __align__(16) unsigned char dq_smem[];
+    __shared__ SumShare share;
+    const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint4 *src = reinterpret_cast<const uint4 *>(x + (size_t)blockIdx.x * N);
+    for (int c = threadIdx.x; c < N / 8; c += W * 32)
+        *reinterpret_cast<uint4 *>(dq_smem + lr.at(c)) = src[c];
+    __syncthreads();
+    const float s = exact_sumsq_wide<W>(dq_smem, lr, lane, part, share, [] { __syncthreads(); });
+    if (part == W - 1 && lane == 31) out[blockIdx.x] = s;
+}
 template <int P, bool ALONE>
 __global__ void __launch_bounds__(64)
 dbg_sumsq_kernel(const uint16_t *__restrict__ x, int N, LaneRow lr, int parts,
@@ -1324,13 +1347,16 @@ extern "C" int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int 
         return fail("debug_sumsq: bad args");
     const LaneRow lr((int)N);
     const int per = warps > 0 ? lr.nu / warps : 0;
-    auto kern = pieces == 0   ? dbg_sumsq_kernel<0, false>
+    const bool wide = N == DS_H && ((pieces == 2 && warps == 4) || (pieces == 4 && warps == 2));
+    auto kern = wide          ? (warps == 4 ? dbg_sumsq_wide_kernel<4> : dbg_sumsq_wide_kernel<2>)
+                : pieces == 0 ? dbg_sumsq_kernel<0, false>
                 : pieces == 2 ? dbg_sumsq_kernel<2, false>
                 : pieces == 4 ? dbg_sumsq_kernel<4, false>
                 : pieces == 8 ? dbg_sumsq_kernel<8, false>
                 : pieces < 0  ? dbg_sumsq_kernel<0, true>
                               : nullptr;
-    if (!kern || (warps != 1 && (warps != 2 || lr.nu % 2)) || (pieces > 0 && per > pieces))
+    if (!kern || (warps != 1 && (warps != 2 || lr.nu % 2) && !wide) ||
+        (pieces > 0 && per > pieces))
         return fail("debug_sumsq: %d pieces of %d, %d warps", pieces, lr.nu, warps);
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     if (ctx_init()) return 1;
@@ -1342,7 +1368,7 @@ extern "C" int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int 
     uint16_t *dx = (uint16_t *)c->io.take(T * N * 2);
     float *ds = (float *)c->io.take(T * 4);
     CU_OK(cudaMemcpyAsync(dx, x, T * N * 2, cudaMemcpyHostToDevice, c->stream));
-    kern<<<(unsigned)T, 64, (size_t)lr.bytes(), c->stream>>>(dx, (int)N, lr, warps, ds);
+    kern<<<(unsigned)T, wide ? 32 * warps : 64, (size_t)lr.bytes(), c->stream>>>(dx, (int)N, lr, warps, ds);
     LAUNCHED();
     CU_OK(cudaMemcpyAsync(out, ds, T * 4, cudaMemcpyDeviceToHost, c->stream));
     CU_OK(cudaStreamSynchronize(c->stream));
@@ -1532,7 +1558,7 @@ static int run_finalize(Ctx *c, const ApusCudaMoeCfg &cfg, int T,
 
 /* scratch of the one-kernel path, sized by the layer shape */
 static int fused_scratch(Ctx *c, const ApusCudaMoeCfg &cfg) {
-    const size_t need_act = (size_t)DF_MAX_A * cfg.moe_inter,
+    const size_t need_act = (size_t)(DF_MAX_A + DF_MAX_T) * cfg.moe_inter,
                  need_sa = (size_t)DF_MAX_T * cfg.shared_inter;
     if (c->df_act_elems >= need_act && c->df_sa_elems >= need_sa) return 0;
     if (c->cur_capturing)
@@ -1630,6 +1656,84 @@ static bool fused_supported(Ctx *c, const ApusCudaMoeCfg &cfg, size_t T) {
     return (size_t)L.total <= dynamic_smem_limit(c, (const void *)decode_fused_kernel);
 }
 
+/* The same, and stacks of layers in one launch, for rows of DS_H values. */
+static int run_stack_decode(Ctx *c, ApusCudaLayer *const *layers, int n, const uint16_t *d_ln2,
+                            uint16_t *d_out, int T, const ApusCudaMoeTrace *tr, cudaStream_t st,
+                            const Residual *rz, const uint16_t *const *ln_w) {
+    const ApusCudaMoeCfg &cfg = layers[0]->cfg;
+    if (fused_scratch(c, cfg)) return 1;
+    StackArgs a;
+    memset((void *)&a, 0, sizeof a);
+    a.T = T; a.I = (int)cfg.moe_inter; a.E = (int)cfg.experts; a.TK = (int)cfg.top_k;
+    while (128 << a.slices_log2 < a.I) a.slices_log2++;
+    a.L = StackLayout(T, a.I, a.E, a.TK, c->sm_count);
+    const size_t smem = (size_t)a.L.total;
+    a.x = d_ln2;
+    if (rz) {
+        a.res = rz->res;
+        a.res_out = rz->res_out;
+    }
+    a.n_layers = n;
+    for (int l = 0; l < n; l++) {
+        const ApusCudaLayer *L = layers[l];
+        StackLayer &w = a.layer[l];
+        w.wmin = L->wmin; w.wmax = L->wmax;
+        w.wmin_gate = L->wmin_gate; w.wmax_gate = L->wmax_gate;
+        w.wnorm = L->d_wnorm;
+        w.wnorm_gate = L->wnorm_gate;
+        w.ln_w = ln_w ? ln_w[l] : nullptr;
+        w.rtr_w = L->rtr_w; w.exp_gu = L->exp_gu; w.exp_d = L->exp_d;
+        w.sh_g = L->sh_g; w.sh_u = L->sh_u; w.sh_d = L->sh_d; w.sh_gate = L->sh_gate;
+    }
+    a.code_ws = c->d_ds_codes; a.chain_ws = c->d_ds_chains;
+    a.act_ws = c->d_df_act;
+    a.sync = c->d_df_sync + 8;
+    a.out = d_out;
+    a.idx_out = tr ? tr->rtr_idx : nullptr;
+    a.w_out = tr ? tr->rtr_w : nullptr;
+    a.tr_routed = tr ? tr->moe_routed : nullptr;
+    a.tr_shared = tr ? tr->moe_shared : nullptr;
+    a.tr_out = tr ? tr->moe_out : nullptr;
+    a.status = c->d_status;
+    a.stats = c->d_rc_stats;
+    a.timeline = c->stage_timing ? c->d_df_timeline : nullptr;
+    c->df_timeline_valid = c->stage_timing;
+    static size_t set_smem = 0;
+    if (smem > set_smem) {
+        CU_OK(cudaFuncSetAttribute(decode_stack_kernel,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        set_smem = smem;
+    }
+    cudaLaunchConfig_t cfgl = {};
+    cfgl.gridDim = dim3(c->sm_count);
+    cfgl.blockDim = dim3(DS_THREADS);
+    cfgl.dynamicSmemBytes = smem;
+    cfgl.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfgl.attrs = attr;
+    cfgl.numAttrs = 1;
+    CU_OK(cudaLaunchKernelEx(&cfgl, decode_stack_kernel, a));
+    LAUNCHED();
+    return 0;
+}
+
+static bool stack_supported(Ctx *c, const ApusCudaMoeCfg &cfg, size_t T) {
+    if ((int)T > c->fused_max_t || T * cfg.top_k > DF_MAX_A) return false;
+    if (cfg.hidden != DS_H || cfg.moe_inter != cfg.shared_inter || cfg.experts > 256) return false;
+    const size_t I = cfg.moe_inter, G = (size_t)c->sm_count;
+    /* A down row of two or four slices: it fits a cell, and the sixteen warps' items span eight
+     * cells at most.  (With one slice a warp would wait for the landing after the next in a cell
+     * whose last one it has not seen, and a barrier's parity cannot tell the two apart.) */
+    if (I != 256 && I != 512) return false;
+    /* output columns of a CTA; its shared gate/up pairs, two tiles at most */
+    if ((DS_H + G - 1) / G > DF_MAX_COLS || G > DF_ROUND || (I + G - 1) / G > 2 * DS_PAIRS)
+        return false;
+    const StackLayout L((int)T, (int)I, (int)cfg.experts, (int)cfg.top_k, c->sm_count);
+    return (size_t)L.total <= dynamic_smem_limit(c, (const void *)decode_stack_kernel);
+}
+
 /* Rows of whole 16-byte pieces in enough lane chunks: one warp per row without the
  * sequential chain; others: the plain kernel.  N 1152 (16 chunks): 13.1 us at 2000 rows
  * against 13.4; N 1088 (8): 8.4 against 10.3 at 512 rows, 17 against 13 at 2000; N 2040 (1):
@@ -1674,6 +1778,11 @@ static int block_dev_locked(ApusCudaLayer *L, const uint16_t *d_ln2,
                     "expert-parallel entry points for a partial layer");
     c->last_block_launches = 0;
     c->df_timeline_valid = false;
+    if (stack_supported(c, cfg, T)) {
+        c->last_block_path = APUS_CUDA_PATH_FUSED;
+        return run_stack_decode(c, &L, 1, d_ln2, d_out, (int)T, d_tr, st, rz,
+                                rz ? &rz->ln_w : nullptr);
+    }
     if (fused_supported(c, cfg, T)) {
         c->last_block_path = APUS_CUDA_PATH_FUSED;
         return run_fused_decode(c, L, d_ln2, d_out, (int)T, d_tr, st, rz);
@@ -1841,6 +1950,12 @@ extern "C" int apus_cuda_moe_layer_dev(ApusCudaLayer *layer, const uint16_t *d_r
     return layer_dev(layer, d_res, d_ln_w, d_res_out, T, d_tr, st);
 }
 
+/* two layers that one launch may run one after another */
+static bool stackable(const ApusCudaLayer *a, const ApusCudaLayer *b) {
+    return !memcmp(&a->cfg, &b->cfg, sizeof a->cfg) && a->e_begin == 0 && b->e_begin == 0 &&
+           a->e_end == a->cfg.experts && b->e_end == b->cfg.experts;
+}
+
 extern "C" int apus_cuda_moe_stack_dev(ApusCudaLayer *const *layers,
                                        const uint16_t *const *d_ln_w, size_t n_layers,
                                        uint16_t *d_res, size_t T, void *stream) {
@@ -1853,6 +1968,23 @@ extern "C" int apus_cuda_moe_stack_dev(ApusCudaLayer *const *layers,
     int launches = 0;
     for (size_t l = 0; l < n_layers; l++) {
         if (!layers[l]) return fail("moe_stack_dev: layer %zu is null", l);
+        /* a run of layers of one shape in one launch */
+        size_t n = 1;
+        while (l + n < n_layers && n < DS_LAYERS && layers[l + n] &&
+               stackable(layers[l], layers[l + n]))
+            n++;
+        if (n > 1 && stack_supported(g_ctx, layers[l]->cfg, T)) {
+            Residual rz;
+            rz.res = rz.res_out = d_res;
+            g_ctx->last_block_launches = 0;
+            g_ctx->last_block_path = APUS_CUDA_PATH_FUSED;
+            if (run_stack_decode(g_ctx, layers + l, (int)n, nullptr, nullptr, (int)T, nullptr, st,
+                                 &rz, d_ln_w ? d_ln_w + l : nullptr))
+                return 1;
+            launches += g_ctx->last_block_launches;
+            l += n - 1;
+            continue;
+        }
         /* in place: a layer reads the stream's row (t, h) only in the thread
          * that then writes it, after everything else of the layer */
         if (layer_dev(layers[l], d_res, d_ln_w ? d_ln_w[l] : nullptr, d_res, T, nullptr, st))

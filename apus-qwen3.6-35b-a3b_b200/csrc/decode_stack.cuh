@@ -1,0 +1,813 @@
+/*
+ * decode_stack.cuh — the MoE block for one to eight tokens, and stacks of layers of it, in ONE
+ * cooperative kernel, for rows of 2048 values (decode_fused.cuh has the same steps for other
+ * shapes, one layer per launch; its head comment explains them: intervals for the logits, the
+ * selection on BF16 codes, mma.sync with the tokens as columns, one grid barrier).
+ *
+ * What bounds a layer at few tokens is not the 58 MB of weights (9 us) but instructions: each is
+ * fetched for the first time when it is needed, at about 8 cycles an instruction out of L2, 2.7
+ * once it is in the 128 KB that an SM keeps, 1 in the innermost 28 KB.  (decode_fused_kernel:
+ * 166 KB of code; 25 % of the warps' time waiting for instructions.)  So
+ *  - a stack of layers is a loop in the kernel: from the second layer on, the code is there, and
+ *    no launch lies between two layers, only a grid barrier;
+ *  - there is little code: the row length is a constant, loops are rolled where a phase runs once,
+ *    the shared and the routed gate/up rows go through the same loop, and so does a tile of down
+ *    rows through the same fragments;
+ *  - weights come by bulk copies that one warp requests (a tile of eight gate and eight up rows
+ *    is two requests of 32 KB, an expert's down rows one): the multiplying warps carry no
+ *    addresses.  (A request costs the copy engine 60 cycles, so rows of 1 KB one by one stream
+ *    at 4.4 TB/s and pieces of 2 KB and more at 7.0.)
+ *  - what a warp waits for comes with its own validity where it is small: logits and chains are
+ *    64-bit words that hold the launch's tag, so no counter, fence and second look.
+ *
+ * Copies are dense, so the rows of a fragment lie on the same banks; a lane's 16 bytes are four
+ * k steps of its row, and odd rows read the two halves of a 128-byte line the other way round.
+ */
+#pragma once
+#include "decode_fused.cuh"
+
+namespace apus {
+
+constexpr int DS_H = 2048;              /* values of a row */
+constexpr int DS_CW = 16;               /* multiplying warps; each has 128 k of a row */
+constexpr int DS_THREADS = (DS_CW + 2) * 32;    /* a requesting warp and a helper more */
+constexpr int DS_PAIRS = 8;             /* gate/up pairs of a tile */
+constexpr int DS_CELL = 16 * 1024;      /* down rows of an expert: at most 16 of 1 KB */
+constexpr int DS_CELLS = 8;
+constexpr int DS_TILE = 2 * DS_PAIRS * DS_H * 2;        /* 64 KB: four cells */
+constexpr int DS_LAYERS = 32;           /* layers of a launch, at most (parameter space) */
+static_assert(DS_CELL * DS_CELLS == 2 * DS_TILE, "two tiles or eight cells");
+
+struct StackLayout {
+    int xrow, rrows;
+    int off_x, off_rr, off_gain, off_share, off_code, off_tmask, off_amb, off_red, total;
+    StackLayout() = default;
+    StackLayout(int T, int I, int E, int TK, int G) {
+        const int A = T * TK;
+        xrow = LaneRow(DS_H).bytes();
+        rrows = (E + 1 + G - 1) / G;
+        off_x = 2 * DS_TILE;
+        off_rr = off_x + T * xrow;
+        off_gain = off_rr + (rrows * xrow > CH_BYTES ? rrows * xrow : CH_BYTES);
+        off_share = off_gain + DS_H * 2;
+        off_code = off_share + 8 * (int)sizeof(SumShare);
+        off_tmask = (off_code + T * (E + 1) * 4 + 7) & ~7;
+        off_amb = off_tmask + 1024;
+        off_red = (off_amb + T * (E + 1) * 2 + 127) & ~127;
+        /* partial sums of a tile [2][warps][rows][8]; later the down outputs
+         * [128-k slices][A + T][columns] */
+        const int r1 = 2 * DS_CW * 2 * DS_PAIRS * 8 * 4,
+                  r2 = I / 128 * (A + T) * DF_MAX_COLS * 4;
+        total = off_red + (r1 > r2 ? r1 : r2);
+    }
+};
+
+struct StackLayer {
+    float wmin, wmax;                   /* smallest nonzero and largest |w|: router matrix */
+    float wmin_gate, wmax_gate;         /* ... shared-gate row */
+    float wnorm_gate;
+    const float *wnorm;                 /* [E] row norms, rounded up */
+    const uint16_t *ln_w;
+    const uint16_t *rtr_w, *exp_gu, *exp_d, *sh_g, *sh_u, *sh_d, *sh_gate;
+};
+struct StackArgs {
+    int T, I, E, TK;
+    int slices_log2;                    /* 128-k slices of a down row: I = 128 << this, 1 or 2 */
+    int n_layers;                       /* > 1: in place on res_out == res */
+    const uint16_t *x;                  /* as in FusedArgs */
+    const uint16_t *res;
+    uint16_t *res_out;
+    uint64_t *code_ws;                  /* [DF_MAX_T][E + 1] logit code intervals, tag above */
+    uint64_t *chain_ws;                 /* [DF_MAX_T * (E + 1)] codes of the walked chains, tag */
+    uint16_t *act_ws;                   /* [DF_MAX_A + DF_MAX_T][I] */
+    unsigned int *sync;                 /* barrier */
+    uint16_t *out;
+    int32_t *idx_out;
+    uint16_t *w_out;
+    uint16_t *tr_routed, *tr_shared, *tr_out;
+    int *status;
+    unsigned int *stats;                /* [0] += chains walked */
+    unsigned long long *timeline;       /* of the last layer */
+    StackLayout L;
+    StackLayer layer[DS_LAYERS];
+};
+
+/* a word that carries its own validity: 64 bits are stored and loaded as one */
+__device__ __forceinline__ void st_tagged(uint64_t *p, uint32_t v, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v | ((uint64_t)tag << 32))
+                 : "memory");
+}
+__device__ __forceinline__ uint64_t ld_tagged(const uint64_t *p) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+/* (rolled: the compiler's unrolling of the waits alone was 40 KB) */
+__device__ __forceinline__ bool ds_wait(uint64_t *bar, uint32_t parity) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < APUS_WAIT_LIMIT; i++) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (i > 64) __nanosleep(64);
+    }
+    return false;
+}
+__device__ __forceinline__ bool ds_spin(const unsigned int *p, unsigned int target) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < (1u << 21); i++) {
+        if ((int)(ld_acquire(p) - target) >= 0) return true;
+        if (i > 64) __nanosleep(40);
+    }
+    return false;
+}
+
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+/* A lane's share of a row's 128-k slice: 16 bytes of each of its four 64-byte windows, which
+ * are the operands of two k steps each.  p: the row's slice + (lane & 3) * 16. */
+__device__ __forceinline__ void slice_pieces(const unsigned char *p, bool odd, uint4 (&f)[4]) {
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(p + l * 128 + (odd ? 64 : 0)),
+                    b = *reinterpret_cast<const uint4 *>(p + l * 128 + (odd ? 0 : 64));
+        f[2 * l] = odd ? b : a;
+        f[2 * l + 1] = odd ? a : b;
+    }
+}
+
+struct StackShared {
+    uint64_t tile_full[2], tile_free[2], cell_full[DS_CELLS], cell_free[DS_CELLS];
+    float gate[DF_MAX_T], sq[4][DF_MAX_T];
+    unsigned int xlo[DF_MAX_T], xhi[DF_MAX_T];
+    int sel[DF_MAX_A];                  /* selected experts, in provisional order */
+    int idx[DF_MAX_A], row[DF_MAX_A];   /* final order; down output of each */
+    int uexp[DF_MAX_A], ubase[DF_MAX_A];
+    int namb[DF_MAX_T], full[DF_MAX_T], open;
+    volatile int dead;
+    unsigned int tag;                   /* of this launch and layer */
+    uint16_t w[DF_MAX_A];
+    uint8_t umask[DF_MAX_A];
+};
+
+/* Parts of a layer that most CTAs or warps never run, or that nobody waits for, as functions:
+ * their code and registers stay out of the others' way. */
+
+/* The open logits of token t are experts amb[t][0 .. namb[t]); counted through all tokens, pair i
+ * is walked by CTA i % G.  This waits for that of pair k of token t, and puts it among the codes. */
+__device__ __forceinline__ bool take_chain(const StackArgs &a, StackShared &S, uint32_t *codes,
+                                           const uint16_t *amb, int t, int k) {
+    const int at = t * (a.E + 1);
+    uint64_t c = 0;
+    bool there = false;
+#pragma unroll 1
+    for (uint32_t n = 0; !there && n < (1u << 21); n++) {
+        c = ld_tagged(&a.chain_ws[at + k]);
+        there = (unsigned)(c >> 32) == S.tag;
+        if (!there && n > 64) __nanosleep(40);
+    }
+    codes[at + amb[at + k]] = (uint32_t)c | ((uint32_t)c << 16);
+    if (!there) set_status(a.status, ST_SCHED_TIMEOUT);
+    return there;
+}
+/* The helper warp: the products in the place of the router rows (rr). */
+__device__ __noinline__ void stack_walk_chains(const StackArgs &a, int layer, StackShared &S,
+                                               const uint16_t *amb, const unsigned char *xs,
+                                               unsigned char *rr) {
+    const StackLayer &W = a.layer[layer];
+    const LaneRow lr(DS_H);
+    const int lane = threadIdx.x & 31, E = a.E, G = gridDim.x;
+    int next = blockIdx.x, n = 0;       /* this CTA's next pair; pairs of the tokens so far */
+#pragma unroll 1
+    for (int t = 0; t < a.T; t++) {
+        const int at = t * (E + 1);
+#pragma unroll 1
+        for (; next < n + S.namb[t]; next += G) {
+            const int e = amb[at + next - n];
+            const uint16_t *w = e == E ? W.sh_gate : W.rtr_w + (size_t)e * DS_H;
+            const unsigned char *xr = xs + t * a.L.xrow;
+            const float z = warp_chains<CH_CHAINS>(
+                1, DS_H, lane, reinterpret_cast<float *>(rr), [&](int) { return w; },
+                [&](int p) { return *reinterpret_cast<const uint4 *>(xr + lr.at(p)); });
+            if (lane == 0) st_tagged(&a.chain_ws[at + next - n], bf16_bits(z), S.tag);
+        }
+        n += S.namb[t];
+    }
+    if (lane == 0 && a.stats && blockIdx.x == 0) atomicAdd(&a.stats[0], (unsigned)n);
+}
+/* A warp to a token, its chains known: the selection again, or the engine's softmax. */
+__device__ __noinline__ void stack_select_again(const StackArgs &a, StackShared &S, uint32_t *cd,
+                                                int t) {
+    const int lane = threadIdx.x & 31, E = a.E, TK = a.TK;
+    if (S.full[t]) {
+        float *p = reinterpret_cast<float *>(cd);
+#pragma unroll 1
+        for (int e = lane; e < E; e += 32) p[e] = bf16lo(cd[e]);
+        __syncwarp();
+        router_softmax_topk(p, E, TK, lane, S.idx + t * TK, S.w + t * TK);
+        __syncwarp();
+#pragma unroll 1
+        for (int i = lane; i < TK; i += 32) S.sel[t * TK + i] = S.idx[t * TK + i];
+    } else {
+        rt_select(cd, E, TK, lane, S.sel + t * TK);
+    }
+}
+/* The helper warp: final order, weights, shared gate, and where the down output of each slot
+ * will be. */
+__device__ __noinline__ void stack_weights(const StackArgs &a, StackShared &S, uint32_t *codes,
+                                           const uint16_t *amb, int U) {
+    const int lane = threadIdx.x & 31, T = a.T, E = a.E, TK = a.TK;
+    if (!S.open)
+#pragma unroll 1
+        for (int t = 0; t < T; t++)
+#pragma unroll 1
+            for (int k = lane; k < S.namb[t]; k += 32) take_chain(a, S, codes, amb, t, k);
+    __syncwarp();
+#pragma unroll 1
+    for (int t = 0; t < T; t++) {
+        if (!S.full[t])
+            rt_weights(codes + t * (E + 1), S.sel + t * TK, TK, lane, S.idx + t * TK, S.w + t * TK);
+        if (lane == 0) S.gate[t] = bf16_round(sigmoid_f32(bf16lo(codes[t * (E + 1) + E])));
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int i = lane; i < T * TK; i += 32) {
+        const int t = i / TK, e = S.idx[i];
+        int lo = 0, hi = U - 1;
+#pragma unroll 1
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (S.uexp[mid] < e) lo = mid + 1; else hi = mid;
+        }
+        S.row[i] = S.ubase[lo] + __popc(S.umask[lo] & ((1u << t) - 1u));
+        if (blockIdx.x == 0) {
+            if (a.idx_out) a.idx_out[i] = e;
+            if (a.w_out) a.w_out[i] = S.w[i];
+        }
+    }
+    __syncwarp();
+}
+
+/* One layer; tile0, item0: gate/up tiles and down items before it; sync_at: thread 0's target
+ * of the barrier. */
+__device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsigned int &sync_at,
+                                            int &tile0, int &item0) {
+    extern __shared__ __align__(128) unsigned char ds_smem[];
+    __shared__ StackShared S;
+
+    const bool first = layer == 0;
+    const StackLayer &W = a.layer[layer];
+    int tid = threadIdx.x, T = a.T, G = gridDim.x, cta = blockIdx.x;
+    /* (nothing of a layer's address arithmetic is kept over the loop) */
+    asm volatile("" : "+r"(tid), "+r"(T), "+r"(G), "+r"(cta));
+    const int I = a.I, E = a.E, TK = a.TK, A = T * TK;
+    const int lane = tid & 31, warp = tid >> 5;
+    const StackLayout &L = a.L;
+    const LaneRow lr(DS_H);
+    constexpr int PIECES = DS_H / 8;
+    unsigned char *xs = ds_smem + L.off_x, *rr = ds_smem + L.off_rr;
+    uint4 *gains = reinterpret_cast<uint4 *>(ds_smem + L.off_gain);
+    uint32_t *codes = reinterpret_cast<uint32_t *>(ds_smem + L.off_code);   /* [T][E + 1] */
+    uint16_t *amb = reinterpret_cast<uint16_t *>(ds_smem + L.off_amb);      /* t << 11 | e */
+    uint32_t *s_tmask = reinterpret_cast<uint32_t *>(ds_smem + L.off_tmask);   /* [256]: tokens of
+                                                        * each expert, a byte each */
+    float *red = reinterpret_cast<float *>(ds_smem + L.off_red);
+    const uint16_t *res = first ? a.res : a.res_out;
+
+    auto mark = [&](int k) {
+        if (a.timeline && tid == 0) {
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            a.timeline[(size_t)cta * DF_MARKS + k] = t;
+        }
+    };
+    auto give_up = [&] {
+        set_status(a.status, ST_SCHED_TIMEOUT);
+        S.dead = 1;
+    };
+    /* the k-th use of a place in the ring: copies landed, or warps done with it (both within
+     * this CTA, so that nothing is left in flight when another CTA's part never came) */
+    /* (by parity: whoever waits for the k-th has seen the one before it, or knows it to be over) */
+    auto landed = [&](uint64_t *bar, int k) {
+        if (!ds_wait(bar, (unsigned)k & 1u)) give_up();
+    };
+    mark(0);
+    /* ---- this CTA's shares ---- */
+    const int n_rr = cta <= E ? (E - cta) / G + 1 : 0;
+    const unsigned b = cta, g = G;
+    const int sh_lo = (int)((unsigned)I * b / g), sh_n = (int)((unsigned)I * (b + 1) / g) - sh_lo;
+    const int h_lo = (int)((unsigned)DS_H * b / g);
+    const int ncols = (int)((unsigned)DS_H * (b + 1) / g) - h_lo;
+
+    /* ---- what does not depend on the layer before: router rows, gains, first weights ---- */
+    if (first) {
+        if (tid == 0) {
+            S.dead = 0;
+            sync_at = round_target(__ldcg(a.sync));
+#pragma unroll 1
+            for (int i = 0; i < DS_CELLS; i++) {
+                mbar_init(&S.cell_full[i], 1);
+                mbar_init(&S.cell_free[i], 1u << a.slices_log2);
+                if (i < 2) {
+                    mbar_init(&S.tile_full[i], 1);
+                    mbar_init(&S.tile_free[i], DS_CW);
+                }
+            }
+            mbar_fence_init();
+        }
+        __syncthreads();
+    }
+    /* a tile of n pairs, the first k of one expert and the others of the next: lanes 0-3
+     * request a piece each */
+    auto request_tile = [&](int tile, const uint16_t *gate, const uint16_t *up, int k,
+                            const uint16_t *gate2, const uint16_t *up2, int n) {
+        if (tile >= 2) landed(&S.tile_free[tile & 1], (tile >> 1) + 1);
+        uint64_t *bar = &S.tile_full[tile & 1];
+        unsigned char *dst = ds_smem + (tile & 1) * DS_TILE;
+        if (lane == 0) mbar_expect_tx(bar, (uint32_t)(2 * n * DS_H * 2));
+        __syncwarp();
+        const int rows = lane & 2 ? n - k : k;
+        if (lane < 4 && rows > 0)
+            bulk_g2s(dst + ((lane & 1) * DS_PAIRS + (lane & 2 ? k : 0)) * DS_H * 2,
+                     lane & 2 ? (lane & 1 ? up2 : gate2) : lane & 1 ? up : gate,
+                     (uint32_t)(rows * DS_H * 2), bar);
+    };
+    const int n_sh = (sh_n + DS_PAIRS - 1) / DS_PAIRS;
+    if (warp == DS_CW)
+#pragma unroll 1
+        for (int j = 0; j < n_sh; j++) {        /* (two at most) */
+            const int n = min(DS_PAIRS, sh_n - j * DS_PAIRS);
+            const size_t at = (size_t)(sh_lo + j * DS_PAIRS) * DS_H;
+            request_tile(tile0 + j, W.sh_g + at, W.sh_u + at, n, nullptr, nullptr, n);
+        }
+    /* (the other two warps may be a phase ahead of these at a layer's end) */
+    if (warp < DS_CW)
+#pragma unroll 1
+        for (int c = tid; c < n_rr * PIECES; c += DS_CW * 32) {
+            const int r = c / PIECES, e = cta + r * G, p = c % PIECES;
+            *reinterpret_cast<uint4 *>(rr + r * L.xrow + lr.at(p)) =
+                ldg16((e == E ? W.sh_gate : W.rtr_w + (size_t)e * DS_H) + p * 8);
+        }
+    if (tid < PIECES)
+        gains[tid] = res && W.ln_w ? ldg16(W.ln_w + tid * 8) : make_uint4(0, 0, 0, 0);
+    if (tid < 256) s_tmask[tid] = 0;
+    if (tid < DF_MAX_T) {
+        S.xlo[tid] = 0x7f800000u;
+        S.xhi[tid] = 0;
+    }
+    if (tid == 0) {
+        S.open = 0;
+        /* the rows that the other CTAs' combines left: the end of the layer before */
+        if (!first) {
+            if (!S.dead && !ds_spin(a.sync, sync_at)) give_up();
+            sync_at += DF_ROUND;
+        }
+        S.tag = sync_at;
+    }
+    __syncthreads();
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(res ? res : a.x);
+#pragma unroll 1
+        for (int c = tid; c < T * PIECES; c += DS_THREADS)
+            *reinterpret_cast<uint4 *>(xs + c / PIECES * L.xrow + lr.at(c % PIECES)) =
+                __ldcg(src + c);
+    }
+    __syncthreads();
+    /* ---- norm (bit for bit the engine's) and the range of the tokens' values: four warps to a
+     * token, or two ---- */
+    const int parts = T <= 4 ? 4 : 2, t_norm = T <= 4 ? warp & 3 : warp & 7;
+    if (t_norm < T && warp < DS_CW) {
+        const int t = t_norm, part = T <= 4 ? warp >> 2 : warp >> 3;
+        unsigned char *row = xs + t * L.xrow;
+        float rs = 1.0f;
+        if (res) {
+            SumShare &share = reinterpret_cast<SumShare *>(ds_smem + L.off_share)[t];
+            auto meet = [&] {
+                asm volatile("bar.sync %0, %1;" ::"r"(3 + t), "r"(32 * parts) : "memory");
+            };
+            rs = norm_scale(parts == 4 ? exact_sumsq_wide<4>(row, lr, lane, part, share, meet)
+                                       : exact_sumsq_wide<2>(row, lr, lane, part, share, meet),
+                            DS_H);
+        }
+        PackedRange range;
+        float sq = 0.0f;
+#pragma unroll 1
+        for (int c = part * 32 + lane; c < PIECES; c += 32 * parts) {
+            uint4 *p = reinterpret_cast<uint4 *>(row + lr.at(c));
+            uint4 v = *p;
+            if (res) *p = v = norm8(v, gains[c], rs);
+            range.fold8(v);
+            float f[8];
+            unpack8(v, f);
+#pragma unroll
+            for (int j = 0; j < 8; j++) sq = fmaf(f[j], f[j], sq);
+        }
+        sq = warp_sum(sq);
+        const unsigned lo = __reduce_min_sync(0xffffffffu, range.low()),
+                       hi = __reduce_max_sync(0xffffffffu, range.high());
+        if (lane == 0) {
+            S.sq[part][t] = sq;
+            atomicMin(&S.xlo[t], lo);
+            atomicMax(&S.xhi[t], hi);
+        }
+    }
+    __syncthreads();
+
+    /* ---- router logits of this CTA's rows ---- */
+    if (warp < DS_CW)
+#pragma unroll 1
+        for (int p = warp; p < n_rr * T; p += DS_CW) {
+            const int r = p >= T ? p / T : 0, t = p - r * T, e = cta + r * G;
+            const bool gate = e == E;
+            uint32_t v = CODE_UNKNOWN;
+            if (products_exact(gate ? W.wmin_gate : W.wmin, gate ? W.wmax_gate : W.wmax, S.xlo[t],
+                               S.xhi[t])) {
+                const float sq = T <= 4 ? (S.sq[0][t] + S.sq[1][t]) + (S.sq[2][t] + S.sq[3][t])
+                                        : S.sq[0][t] + S.sq[1][t];
+                v = certified_logit(rr + r * L.xrow, xs + t * L.xrow, lr, lane,
+                                    (gate ? W.wnorm_gate : __ldg(&W.wnorm[e])) *
+                                        norm_above(sq, DS_H));
+            }
+            if (lane == 0) st_tagged(&a.code_ws[(size_t)t * (E + 1) + e], v, S.tag);
+        }
+    mark(1);                                /* own logits published */
+
+    const int fr = lane >> 2, fq = lane & 3;        /* row and piece of a fragment */
+    const bool odd = fr & 1;
+    int U = 0, gu_lo = 0, gu_n = 0, n_tiles = n_sh;
+    bool dead = false;
+    /* the shared expert's gate/up rows, for which nobody waits; then the routed ones */
+#pragma unroll 1
+    for (int phase = 0; phase < 2; phase++) {
+        if (phase == 1) {
+            mark(2);                        /* shared gate/up done */
+            /* ---- routing: a warp to a token; the others wait for all of them ---- */
+            auto mark_chosen = [&] {        /* the token's bit at its experts */
+                __syncwarp();
+#pragma unroll 1
+                for (int i = lane; i < TK; i += 32) {
+                    const int e = S.sel[warp * TK + i];
+                    atomicOr(&s_tmask[e >> 2], (1u << warp) << ((e & 3) * 8));
+                }
+            };
+            uint32_t *cd = codes + warp * (E + 1);
+            if (warp < T) {
+                /* its logits, as soon as this launch's are there, all under way at once */
+                constexpr int R = 9;
+                const uint64_t *src = a.code_ws + (size_t)warp * (E + 1) + lane;
+                const unsigned tag = S.tag;
+                uint64_t v[R];
+                bool all = false;
+#pragma unroll 1
+                for (uint32_t i = 0; !all && i < (1u << 21); i++) {
+                    all = true;
+#pragma unroll
+                    for (int q = 0; q < R; q++)
+                        v[q] = lane + q * 32 < E + 1 ? ld_tagged(src + q * 32)
+                                                     : (uint64_t)tag << 32;
+#pragma unroll
+                    for (int q = 0; q < R; q++) all &= (unsigned)(v[q] >> 32) == tag;
+                    all = __all_sync(0xffffffffu, all);
+                    if (!all && i > 64) __nanosleep(40);
+                }
+#pragma unroll
+                for (int q = 0; q < R; q++)
+                    if (lane + q * 32 < E + 1) cd[lane + q * 32] = (uint32_t)v[q];
+                __syncwarp();
+                if (all) {
+                    const Choice c = rt_select(cd, E, TK, lane, S.sel + warp * TK);
+                    int n = 0;              /* open logits: the same list in every CTA */
+                    if (c.any)
+#pragma unroll 1
+                        for (int e = lane; e - lane <= E; e += 32) {
+                            const bool need = rt_needs(cd, e, E, c.kkey, c.odd);
+                            const unsigned m = __ballot_sync(0xffffffffu, need);
+                            if (need)
+                                amb[warp * (E + 1) + n + __popc(m & ((1u << lane) - 1u))] =
+                                    (uint16_t)e;
+                            n += __popc(m);
+                        }
+                    if (lane == 0) {
+                        S.namb[warp] = n;
+                        S.full[warp] = c.odd;
+                        if (c.open || c.odd) S.open = 1;
+                    }
+                    mark_chosen();
+                } else if (lane == 0) {
+                    give_up();
+                }
+            }
+            __syncthreads();
+            dead = S.dead != 0;
+            int n_amb = 0;
+            if (!dead)
+#pragma unroll 1
+                for (int t = 0; t < T; t++) n_amb += S.namb[t];
+            if (n_amb > 0) {
+                if (warp == DS_CW + 1) stack_walk_chains(a, layer, S, amb, xs, rr);
+                if (S.open) {               /* the set itself waits for the chains */
+                    if (tid < 256) s_tmask[tid] = 0;
+#pragma unroll 1
+                    for (int t = warp; t < T; t += DS_THREADS / 32)
+#pragma unroll 1
+                        for (int k = lane; k < S.namb[t]; k += 32)
+                            if (!take_chain(a, S, codes, amb, t, k)) S.dead = 1;
+                    __syncthreads();
+                    dead = S.dead != 0;
+                    if (warp < T && !dead) {
+                        stack_select_again(a, S, cd, warp);
+                        mark_chosen();
+                    }
+                    __syncthreads();
+                }
+            }
+            /* ---- the distinct experts, ascending, and who uses them: every warp writes the
+             * whole list, and waits for nobody's ---- */
+            if (!dead) {
+                /* a lane has eight experts (E <= 256) */
+                const uint2 m = reinterpret_cast<const uint2 *>(s_tmask)[lane];
+                auto used = [](uint32_t v) {        /* 0x80 in each byte that is not zero */
+                    return (((v & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v) & 0x80808080u;
+                };
+                const int mine = __popc(used(m.x)) + __popc(used(m.y)) +
+                                 ((__popc(m.x) + __popc(m.y)) << 16);
+                int incl = mine;                    /* experts | assignments << 16 */
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += v;
+                }
+                int p = incl - mine;
+                U = __shfl_sync(0xffffffffu, incl, 31) & 0xffff;
+#pragma unroll 1
+                for (uint32_t h = 0, r = used(m.x); h < 2; h++, r = used(m.y))
+#pragma unroll 1
+                    for (; r; r &= r - 1) {
+                        const int k = __ffs(r) - 8;         /* first bit of the byte */
+                        const uint32_t who = ((h ? m.y : m.x) >> k) & 0xffu;
+                        const int u = p & 0xffff;
+                        S.uexp[u] = (lane * 2 + (int)h) * 4 + (k >> 3);
+                        S.umask[u] = (uint8_t)who;
+                        S.ubase[u] = p >> 16;
+                        p += 1 + (__popc(who) << 16);
+                    }
+                __syncwarp();
+            }
+            mark(3);                        /* selection known */
+            gu_lo = (int)((unsigned)(U * I) * b / g);
+            gu_n = (int)((unsigned)(U * I) * (b + 1) / g) - gu_lo;
+            n_tiles = (gu_n + DS_PAIRS - 1) / DS_PAIRS;
+            tile0 += n_sh;
+
+            if (warp == DS_CW) {
+                /* ---- the requesting warp: routed gate/up rows, then the down rows of this
+                 * CTA's columns (the shared expert's last), each as its place comes free ---- */
+#pragma unroll 1
+                for (int j = 0; j < n_tiles; j++) {
+                    const int it = gu_lo + j * DS_PAIRS, u = it / I, i = it - u * I;
+                    const int n = min(DS_PAIRS, gu_n - j * DS_PAIRS), k = min(n, I - i);
+                    const size_t half = (size_t)I * DS_H;
+                    const uint16_t *w = W.exp_gu + S.uexp[u] * 2 * half + (size_t)i * DS_H,
+                                   *w2 = W.exp_gu + S.uexp[k < n ? u + 1 : u] * 2 * half;
+                    request_tile(tile0 + j, w, w + half, k, w2, w2 + half, n);
+                }
+                tile0 += n_tiles;
+                /* a lane to a cell: it asks again as soon as its cell is free (one after another
+                 * they kept each other waiting: 25 us for the down rows of eight tokens) */
+                const uint32_t bytes = (uint32_t)(ncols * I * 2);
+                bool busy = lane < DS_CELLS && lane <= U;
+                int d = lane;
+                /* ... when the tile that lies there has been read, then its item before this */
+                uint64_t *free_bar = &S.tile_free[(tile0 + (lane >> 2)) & 1];
+                int use = (tile0 - 2 + (lane >> 2)) >> 1;
+#pragma unroll 1
+                for (uint32_t n = 0; __any_sync(0xffffffffu, busy) && n < APUS_WAIT_LIMIT; n++) {
+                    if (busy && mbar_test(free_bar, (unsigned)use & 1u)) {
+                        if (d <= U) {
+                            const int c = (item0 + d) & (DS_CELLS - 1);
+                            uint64_t *bar = &S.cell_full[c];
+                            mbar_expect_tx(bar, bytes);
+                            bulk_g2s(ds_smem + (((tile0 & 1) * 4 + d) & (DS_CELLS - 1)) * DS_CELL,
+                                     (d == U ? W.sh_d : W.exp_d + (size_t)S.uexp[d] * DS_H * I) +
+                                         (size_t)h_lo * I,
+                                     bytes, bar);
+                            free_bar = &S.cell_free[c];
+                            use = (item0 + d) >> 3;
+                            d += DS_CELLS;
+                        } else {
+                            busy = false;   /* and nothing is left in it: the next layer's first
+                                             * tiles may lie anywhere */
+                        }
+                    }
+                }
+                if (busy) give_up();
+                __syncwarp();
+                item0 += U + 1;
+                return;
+            }
+            if (warp > DS_CW) {
+                if (!dead) stack_weights(a, S, codes, amb, U);
+                asm volatile("bar.arrive 2, %0;" ::"n"(DS_CW * 32 + 32) : "memory");
+                tile0 += n_tiles;
+                item0 += U + 1;
+                return;
+            }
+        }
+        /* ---- gate/up tiles: the warps' partial sums meet in shared memory, four warps in
+         * turn finish a tile while the others go on ---- */
+        /* a warp's share of the tokens: column fr, 128 k */
+        uint4 xf[4];
+#pragma unroll
+        for (int w = 0; w < 4; w++)
+            xf[w] = *reinterpret_cast<const uint4 *>(xs + min(fr, T - 1) * L.xrow +
+                                                     lr.at((warp & 15) * 16 + w * 4 + fq));
+        if (warp < DS_CW)
+#pragma unroll 1
+            for (int j = 0; j < n_tiles; j++) {
+                const int tile = tile0 + j;
+                float *buf = red + (j & 1) * (DS_CW * 2 * DS_PAIRS * 8);
+                const unsigned char *p = ds_smem + (tile & 1) * DS_TILE + fr * (DS_H * 2) +
+                                         warp * 256 + fq * 16;
+                landed(&S.tile_full[tile & 1], tile >> 1);
+                uint4 gr[4], ur[4];
+                slice_pieces(p, odd, gr);
+                slice_pieces(p + DS_PAIRS * DS_H * 2, odd, ur);
+                float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int w = 0; w < 4; w++) {
+                    const uint32_t r0[4] = {gr[w].x, ur[w].x, gr[w].y, ur[w].y},
+                                   r1[4] = {gr[w].z, ur[w].z, gr[w].w, ur[w].w};
+                    mma_16x8(c0, r0, xf[w].x, xf[w].y);
+                    mma_16x8(c1, r1, xf[w].z, xf[w].w);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.tile_free[tile & 1]);
+                /* (gate and up of a pair side by side) */
+                float *dst = buf + (warp * 2 * DS_PAIRS + 2 * fr) * 8 + fq * 2;
+                *reinterpret_cast<float2 *>(dst) = make_float2(c0[0] + c1[0], c0[1] + c1[1]);
+                *reinterpret_cast<float2 *>(dst + 8) = make_float2(c0[2] + c1[2], c0[3] + c1[3]);
+                df_bar_compute();
+                if ((warp >> 2) == (j & 3)) {
+                    /* thread = row (2p gate, 2p + 1 up) x column */
+                    const int i = (warp & 3) * 32 + lane, col = i & 7,
+                              pi = j * DS_PAIRS + (i >> 4);
+                    float v = 0.0f;
+#pragma unroll
+                    for (int w = 0; w < DS_CW; w++) v += buf[w * (2 * DS_PAIRS * 8) + i];
+                    const float up = bf16_round(__shfl_xor_sync(0xffffffffu, v, 8));
+                    const float gate = bf16_round(v);
+                    if (!(i & 8) && pi < (phase ? gu_n : sh_n)) {
+                        int row = A + col, at = sh_lo + pi;
+                        bool mine = col < T;
+                        if (phase) {
+                            const int it = gu_lo + pi, u = it / I;
+                            const unsigned m = S.umask[u];
+                            mine = (m >> col) & 1u;
+                            row = S.ubase[u] + __popc(m & ((1u << col) - 1u));
+                            at = it - u * I;
+                        }
+                        /* silu_act_bits, silu_mul_bits */
+                        float y = __fmul_rn(gate, sigmoid_f32(gate));
+                        if (phase) y = bf16_round(y);
+                        if (mine) a.act_ws[(size_t)row * I + at] = bf16_bits(__fmul_rn(y, up));
+                    }
+                }
+            }
+    }
+    if (warp >= DS_CW) return;              /* (not reached: for the compiler) */
+    tile0 += n_tiles;
+    mark(4);                                /* routed gate/up done */
+    df_bar_compute();
+    if (tid == 0) {
+        round_arrive(a.sync);
+        if (!S.dead && !ds_spin(a.sync, sync_at)) give_up();
+        sync_at += DF_ROUND;                /* the layer's end */
+    }
+    df_bar_compute();
+    dead = S.dead != 0;
+    mark(5);                                /* barrier passed */
+    /* ---- down rows of this CTA's columns: a warp to 128 k of an expert.  Its activations are
+     * nobody else's here: they come straight from L2, the next unit's while this one is at work
+     * (all of them through shared memory first: 1.7 kcycles at one token, 6.6 at eight). ---- */
+    auto unit_rows = [&](int v, int &cnt, int &row0) {
+        const int d = v >> a.slices_log2;
+        cnt = d == U ? T : __popc(S.umask[d]);
+        row0 = d == U ? A : S.ubase[d];
+    };
+    auto unit_acts = [&](int v, uint4 (&x)[4]) {
+        int cnt, row0;
+        unit_rows(v, cnt, row0);
+        const uint4 *q = reinterpret_cast<const uint4 *>(
+            a.act_ws + (size_t)(row0 + min(fr, cnt - 1)) * I +   /* (extra columns are not used) */
+            (v & ((1 << a.slices_log2) - 1)) * 128 + fq * 8);
+#pragma unroll
+        for (int w = 0; w < 4; w++) x[w] = __ldcg(q + w * 4);
+    };
+    const int n_units = (U + 1) << a.slices_log2;
+    uint4 xn[4];
+    if (warp < n_units) unit_acts(warp, xn);
+#pragma unroll 1
+    for (int v = warp; v < n_units; v += DS_CW) {
+        uint4 xv[4];
+#pragma unroll
+        for (int w = 0; w < 4; w++) xv[w] = xn[w];
+        if (v + DS_CW < n_units) unit_acts(v + DS_CW, xn);
+        const int d = v >> a.slices_log2, slice = v & ((1 << a.slices_log2) - 1);
+        int cnt, row0;
+        unit_rows(v, cnt, row0);
+        const int item = item0 + d, cell = ((tile0 & 1) * 4 + d) & (DS_CELLS - 1);
+        const unsigned char *p = ds_smem + cell * DS_CELL + fr * (I * 2) + slice * 256 + fq * 16;
+        landed(&S.cell_full[item & (DS_CELLS - 1)], item >> 3);
+        uint4 lo[4], hi[4];
+        slice_pieces(p, odd, lo);
+        slice_pieces(p + 8 * I * 2, odd, hi);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.cell_free[item & (DS_CELLS - 1)]);
+        /* mma.sync cuts off what its accumulator cannot hold: two steps on one that starts at
+         * zero, sums of those rounded to nearest (decode_fused.cuh has the figures; the gate/up
+         * tiles end in a sum of sixteen warps and need no more than that). */
+        float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            const uint4 x = xv[w];
+            const uint32_t r0[4] = {lo[w].x, hi[w].x, lo[w].y, hi[w].y},
+                           r1[4] = {lo[w].z, hi[w].z, lo[w].w, hi[w].w};
+            float t[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_16x8(t, r0, x.x, x.y);
+            mma_16x8(t, r1, x.z, x.w);
+#pragma unroll
+            for (int k = 0; k < 4; k++) ((w & 1) ? c1 : c0)[k] += t[k];
+        }
+        const int col = fq * 2;
+        float *dst = red + ((size_t)slice * (A + T) + row0 + col) * DF_MAX_COLS + fr;
+        if (col < cnt) {
+            dst[0] = c0[0] + c1[0];
+            dst[8] = c0[2] + c1[2];
+        }
+        if (col + 1 < cnt) {
+            dst[DF_MAX_COLS] = c0[1] + c1[1];
+            dst[DF_MAX_COLS + 8] = c0[3] + c1[3];
+        }
+    }
+    item0 += U + 1;
+    df_bar_compute();
+    mark(6);                                /* down rows done */
+
+    /* ---- combine (c/layer.h:350,356-361), this CTA's columns: the slices' sums, then a thread
+     * to an output ---- */
+#pragma unroll 1
+    for (int i = tid; i < (A + T) * DF_MAX_COLS; i += DS_CW * 32) {
+        const int n = (A + T) * DF_MAX_COLS;
+        float y = red[i];
+        y += red[n + i];
+        if (a.slices_log2 > 1) y += red[2 * n + i] + red[3 * n + i];
+        red[i] = bf16_round(y);
+    }
+    /* the helper warp has been through as well */
+    asm volatile("bar.sync 2, %0;" ::"n"(DS_CW * 32 + 32) : "memory");
+    if (!dead && tid < T * ncols) {
+        const int t = tid / ncols, h = tid - t * ncols;
+        float acc = 0.0f;
+#pragma unroll 2
+        for (int s = 0; s < TK; s++)
+            acc = __fadd_rn(acc, __fmul_rn(bf16_f32(S.w[t * TK + s]),
+                                           red[S.row[t * TK + s] * DF_MAX_COLS + h]));
+        const float routed = bf16_round(acc);
+        const float shared = bf16_round(__fmul_rn(red[(A + t) * DF_MAX_COLS + h], S.gate[t]));
+        const uint16_t v = bf16_bits(__fadd_rn(routed, shared));
+        const size_t at = (size_t)t * DS_H + h_lo + h;
+        if (a.out) a.out[at] = v;
+        if (a.res_out)                          /* c/layer.h:230-234,388 */
+            a.res_out[at] = bf16_bits(__fadd_rn(bf16_f32(__ldcg(res + at)), bf16_f32(v)));
+        if (a.tr_out) a.tr_out[at] = v;
+        if (a.tr_routed) a.tr_routed[at] = bf16_bits(routed);
+        if (a.tr_shared) a.tr_shared[at] = bf16_bits(shared);
+    }
+    mark(7);                                /* combine done */
+    if (layer + 1 < a.n_layers) {
+        df_bar_compute();
+        if (tid == 0) round_arrive(a.sync);
+    }
+}
+
+__global__ void __launch_bounds__(DS_THREADS, 1)
+decode_stack_kernel(const __grid_constant__ StackArgs a) {
+    unsigned int sync_at = 0;
+    int tile0 = 0, item0 = 0;
+#pragma unroll 1
+    for (int layer = 0; layer < a.n_layers; layer++)
+        stack_layer(a, layer, sync_at, tile0, item0);
+}
+
+}  // namespace apus

@@ -217,6 +217,188 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
     return s;
 }
 
+/* The same sum of a row of 2048 values by W warps, four or two: what the one-kernel path waits
+ * for before anything else.  A lane has 64 / W terms, and a binade's end costs
+ * one addition instead of a chunk's: the tree sums say at which term the sum passes it, so a lane
+ * there has a parity function for the terms before, the term itself with the neighbour that
+ * lies nearer to the edge (the chain's sum may pass one term earlier or later than the tree's),
+ * and a function for the terms behind.  The functions are joined from one such place to the
+ * next, and every lane of the W warps walks the few joined runs and the terms between them.  A run must start
+ * and end in the binade it was composed for, as above; otherwise everything is added in order.
+ * Cycles of a row, instructions at hand: 2590 by four warps, 3310 by two, against 4000 to 4900
+ * by two of the form above. */
+constexpr int SUM_RUNS = 16;             /* runs of a warp, at most; one more ends them */
+struct SumShare {
+    float total[4];                      /* the warps' tree sums */
+    float start;                         /* the sum of the row's first two chunks */
+    int n[4];                            /* runs of each warp; < 0: add in order */
+    /* x: function of an even sum | binade << 24, y: of an odd one; z, w: the terms behind it */
+    int4 run[4][SUM_RUNS];
+};
+template <int W, typename Meet>
+__device__ __forceinline__ float exact_sumsq_wide(const unsigned char *row, const LaneRow lr,
+                                                  int lane, int part, SumShare &sh, Meet meet) {
+    constexpr int P = 8 / W, N = P * 8;         /* 16-byte pieces and terms of a lane */
+    const int chunk = part * 32 + lane, l = chunk / W;
+    const unsigned char *mine = row + l * lr.pitch + (chunk - l * W) * P * 16;
+    float q[N];
+#pragma unroll
+    for (int u = 0; u < P; u++) {
+        float f[8];
+        unpack8(*reinterpret_cast<const uint4 *>(mine + u * 16), f);
+#pragma unroll
+        for (int j = 0; j < 8; j++) q[u * 8 + j] = __fmul_rn(f[j], f[j]);
+    }
+    /* tree sums: of the lane, of the lanes before it, of the warps before that */
+    float tot = 0.0f;
+#pragma unroll
+    for (int u = 0; u < P; u++)
+        tot += ((q[u * 8] + q[u * 8 + 1]) + (q[u * 8 + 2] + q[u * 8 + 3])) +
+               ((q[u * 8 + 4] + q[u * 8 + 5]) + (q[u * 8 + 6] + q[u * 8 + 7]));
+    float incl = tot;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+    }
+    if (lane == 31) sh.total[part] = incl;
+    meet();
+    float before = 0.0f;
+#pragma unroll
+    for (int w = 0; w < W - 1; w++)
+        if (w < part) before += sh.total[w];
+    const float first = before + (incl - tot);
+    /* Binades, taken from the sums at the lanes' ends so that neighbours agree on them.  The
+     * row's first two chunks, where the sum doubles fast, are simply added up. */
+    const bool head = chunk < 2;
+    const int b1 = binade(before + incl);
+    int b0 = __shfl_up_sync(0xffffffffu, b1, 1);
+    if (lane == 0) b0 = binade(before);
+    const bool cross = !head && b1 != b0;
+    bool bad = b1 < b0 || b0 > 250;
+    /* terms [0, j0) before the edge, j0 and j1 on it */
+    const float edge = __uint_as_float((uint32_t)(b0 + 1) << 23);
+    int j0 = N, j1 = N;
+    if (cross) {
+        float p = first, below = first, above = INFINITY;
+        j0 = 0;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            p += q[i];
+            const bool under = p < edge;
+            j0 += under;
+            if (under) below = p;
+            else above = fminf(above, p);
+        }
+        j0 = min(j0, N - 1);
+        j1 = j0;
+        if (edge - below < above - edge) j0 = max(j0 - 1, 0);
+        else j1 = min(j1 + 1, N - 1);
+    }
+    /* what the terms do to the smallest even and odd sum of their binade */
+    const int e0 = head ? 0 : b0 << 23, e1 = b1 << 23;
+    float fe = __int_as_float(e0), fo = __int_as_float(e0 + 1);
+    float q0 = 0.0f, q1 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const float t = i < j0 ? q[i] : 0.0f;
+        fe = __fadd_rn(fe, t);
+        fo = __fadd_rn(fo, t);
+    }
+    auto square_at = [&](int i) {
+        const float v = bf16_f32(reinterpret_cast<const uint16_t *>(mine)[i]);
+        return __fmul_rn(v, v);
+    };
+    if (cross) {
+        q0 = square_at(j0);
+        if (j1 > j0) q1 = square_at(j1);
+    }
+    ParityFn pre;
+    pre.i0 = __float_as_int(fe) - e0;
+    pre.i1 = __float_as_int(fo) - (e0 + 1);
+    if (part == 0) {
+        float s = __shfl_sync(0xffffffffu, fe, 0);
+#pragma unroll
+        for (int i = 0; i < N; i++) s = __fadd_rn(s, q[i]);
+        if (lane == 1) sh.start = s;
+        if (head) pre.i0 = pre.i1 = 0;
+    }
+    ParityFn f = pre;
+    if (__any_sync(0xffffffffu, cross)) {
+        fe = __int_as_float(e1);
+        fo = __int_as_float(e1 + 1);
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const float t = i > j1 ? q[i] : 0.0f;
+            fe = __fadd_rn(fe, t);
+            fo = __fadd_rn(fo, t);
+        }
+        if (cross) {
+            f.i0 = __float_as_int(fe) - e1;
+            f.i1 = __float_as_int(fo) - (e1 + 1);
+        }
+    }
+    /* joined from one edge to the next; the run that ends at a lane's edge is what the lanes
+     * before it left and its own terms before the edge */
+    const unsigned edges = __ballot_sync(0xffffffffu, cross);
+    const int from = 31 - __clz((edges | 1u) & (0xffffffffu >> (31 - lane)));
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        ParityFn g;
+        g.i0 = __shfl_up_sync(0xffffffffu, f.i0, d);
+        g.i1 = __shfl_up_sync(0xffffffffu, f.i1, d);
+        if (lane - d >= from) f = compose(g, f);
+    }
+    ParityFn run;
+    run.i0 = __shfl_up_sync(0xffffffffu, f.i0, 1);
+    run.i1 = __shfl_up_sync(0xffffffffu, f.i1, 1);
+    run = lane > 0 ? compose(run, pre) : pre;
+    bad = __any_sync(0xffffffffu, bad) || __popc(edges) >= SUM_RUNS;
+    if (cross && !bad)
+        sh.run[part][__popc(edges & ((1u << lane) - 1u))] =
+            make_int4(run.i0 | (b0 << 24), run.i1, __float_as_int(q0), __float_as_int(q1));
+    if (lane == 31) {
+        const int n = __popc(edges);
+        if (!bad) sh.run[part][n] = make_int4(f.i0 | (b1 << 24), f.i1, 0, 0);
+        sh.n[part] = bad ? -1 : n + 1;
+    }
+    meet();
+    float s = sh.start;
+    int n[W];
+    int4 r[W];
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+        n[w] = sh.n[w];
+        r[w] = sh.run[w][0];
+    }
+    bool ok = true;
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+        ok &= n[w] > 0;
+#pragma unroll 1
+        for (int i = 1;; i++) {
+            const int4 next = sh.run[w][min(i, SUM_RUNS - 1)];
+            const int at = __float_as_int(s), to = at + ((at & 1) ? r[w].y : r[w].x & 0xffffff);
+            ok &= (at >> 23) == (int)((unsigned)r[w].x >> 24) && (to >> 23) == (at >> 23);
+            s = __fadd_rn(__fadd_rn(__int_as_float(to), __int_as_float(r[w].z)),
+                          __int_as_float(r[w].w));
+            if (i >= n[w]) break;
+            r[w] = next;
+        }
+    }
+    if (!ok) {
+        s = 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < lr.nl * lr.nu; c++) {
+            float t[8];
+            square8(row + lr.at(c), t);
+            s = add8(s, t);
+        }
+        meet();                              /* the caller may write over the row */
+    }
+    return s;
+}
+
 /* y = rnd((x * rs) * (1 + w)), eight values; w: the gain offsets */
 __device__ __forceinline__ uint4 norm8(const uint4 v, const uint4 g, float rs) {
     const uint32_t xw[4] = {v.x, v.y, v.z, v.w}, gw[4] = {g.x, g.y, g.z, g.w};

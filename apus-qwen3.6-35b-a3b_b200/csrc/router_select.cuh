@@ -45,80 +45,89 @@ __device__ __forceinline__ Choice rt_select(const uint32_t *cd, int E, int TK, i
     /* keys: low code, then lowest index first; all different.  Up to 256 experts
      * they stay in registers. */
     constexpr int R = 8;
-    uint32_t kr[R], best = 0, kth = 0;
+    uint32_t kr[R], best = 0, kth = 0, mine = 0;
+    uint32_t far = 0;                       /* largest high key of those that are not known */
     const bool regs = E <= 32 * R;
-    auto key_of = [&](int e) { return (code_key(cd[e]) << 16) | (0xffffu - (uint32_t)e); };
+    auto key_of = [&](uint32_t c, int e) { return (code_key(c) << 16) | (0xffffu - (uint32_t)e); };
+    auto far_of = [&](uint32_t c) { return code_known(c) ? 0u : code_key(c >> 16) + 1u; };
     if (regs) {
 #pragma unroll
         for (int i = 0; i < R; i++) {
-            kr[i] = lane + 32 * i < E ? key_of(lane + 32 * i) : 0u;
+            const uint32_t c = lane + 32 * i < E ? cd[lane + 32 * i] : CODE_NEVER;
+            kr[i] = lane + 32 * i < E ? key_of(c, lane + 32 * i) : 0u;
             best = max(best, kr[i]);
+            far = max(far, far_of(c));
         }
     } else {
 #pragma unroll 1
-        for (int e = lane; e < E; e += 32) best = max(best, key_of(e));
+        for (int e = lane; e < E; e += 32) {
+            best = max(best, key_of(cd[e], e));
+            far = max(far, far_of(cd[e]));
+        }
     }
+    uint32_t first = 0;
 #pragma unroll 1
     for (int i = 0; i < TK; i++) {
         kth = __reduce_max_sync(0xffffffffu, best);
-        if (lane == 0) sel[i] = (int)(0xffffu - (kth & 0xffffu));
+        if (lane == (i & 31)) mine = kth;
+        if ((i & 31) == 31) {
+            if (i == 31) first = __shfl_sync(0xffffffffu, mine, 0);
+            sel[i - 31 + lane] = (int)(0xffffu - (mine & 0xffffu));
+        }
         if (regs) {
-            best = 0;
+            uint32_t b[R];
 #pragma unroll
-            for (int j = 0; j < R; j++)
-                if (kr[j] < kth) best = max(best, kr[j]);
+            for (int j = 0; j < R; j++) b[j] = kr[j] < kth ? kr[j] : 0u;
+            best = max(max(max(b[0], b[1]), max(b[2], b[3])), max(max(b[4], b[5]), max(b[6], b[7])));
         } else if (best == kth) {                        /* this lane's next one */
             best = 0;
+#pragma unroll 1
             for (int e = lane; e < E; e += 32) {
-                const uint32_t k = key_of(e);
+                const uint32_t k = key_of(cd[e], e);
                 if (k < kth) best = max(best, k);
             }
         }
     }
+    if (lane < (TK & 31)) sel[(TK & ~31) + lane] = (int)(0xffffu - (mine & 0xffffu));
+    if (TK < 32) first = __shfl_sync(0xffffffffu, mine, 0);
     Choice c;
     c.kkey = kth >> 16;
-    bool open = false, odd = false, any = false;
-    int small = 0, zeros = 0;                            /* below 2^-10: nonzero, zero */
-    float top = -INFINITY;
-    uint32_t reach = 0;                                  /* bit i: expert lane + 32 i competes */
-    if (regs) {
-#pragma unroll
-        for (int i = 0; i < R; i++)
-            if (lane + 32 * i < E && code_key(cd[lane + 32 * i] >> 16) >= c.kkey) reach |= 1u << i;
-    } else {
-        for (int e = lane, i = 0; e < E; e += 32, i++)
-            if (code_key(cd[e] >> 16) >= c.kkey) reach |= 1u << i;
-    }
-    for (; reach; reach &= reach - 1) {
-        const int e = lane + 32 * (__ffs(reach) - 1);
-        const uint32_t v = cd[e];
-        const bool known = code_known(v);
-        any |= !known;
-        if (!known && key_of(e) < kth) open = true;      /* not among the chosen */
-        const float lo = bf16lo(v), hi = bf16hi(v);
-        const bool plain = fabsf(lo) >= 9.765625e-4f && fabsf(hi) >= 9.765625e-4f &&
-                           (lo < 0.0f) == (hi < 0.0f);
-        if (!(fabsf(lo) <= 32.0f && fabsf(hi) <= 32.0f)) odd = true;      /* or a NaN */
-        if (known && (v & 0x7fffu) == 0)
-            zeros++;
-        else if (!plain)                                 /* an interval around zero counts */
-            small++;
-        top = fmaxf(top, hi);
-    }
-    __syncwarp();
-    /* order-preserving integer of a float, for the integer reduction */
-    const int ti = __float_as_int(top);
-    const int tm = __reduce_max_sync(0xffffffffu, ti >= 0 ? ti : ti ^ 0x7fffffff);
-    top = __int_as_float(tm >= 0 ? tm : tm ^ 0x7fffffff);
     const float kval = key_value(c.kkey);
-    if (!(kval - top >= -80.0f) || fabsf(kval) < 9.765625e-4f) odd = true;
+    /* Nearly always: every logit that reaches that far is known, so the chosen ones alone do,
+     * and they lie between two values that leave nothing to doubt. */
+    if (!__any_sync(0xffffffffu, far > c.kkey) && kval >= 9.765625e-4f &&
+        key_value(first >> 16) <= 32.0f) {
+        c.open = c.odd = false;
+        c.any = !code_known(cd[E]);
+        return c;
+    }
+    /* every expert whose high code reaches that far, without a branch: a lane's last one would
+     * keep the others waiting */
+    constexpr uint32_t SMALL = 0x3a80u, FAR = 0x4200u;   /* 2^-10 and 32 */
+    uint32_t flags = 0, count = 0, topk = 0;     /* 1 any, 2 open, 4 odd; small ones, zeros << 16 */
+    auto judge = [&](uint32_t w, uint32_t key) {
+        const uint32_t hk = code_key(w >> 16), lm = w & 0x7fffu, hm = (w >> 16) & 0x7fffu;
+        const bool in = hk >= c.kkey, known = code_known(w);
+        topk = max(topk, hk);
+        if (in && !known) flags |= key < kth ? 3u : 1u;  /* open: not among the chosen */
+        if (in && max(lm, hm) > FAR) flags |= 4u;        /* or a NaN */
+        const bool plain = min(lm, hm) >= SMALL && !((w ^ (w >> 16)) & 0x8000u);
+        /* (an interval around zero counts as small) */
+        if (in && !plain) count += known && lm == 0 ? 0x10000u : 1u;
+    };
+#pragma unroll 1
+    for (int e = lane; e < E; e += 32) judge(cd[e], key_of(cd[e], e));
+    __syncwarp();
+    flags = __reduce_or_sync(0xffffffffu, flags);
+    count = __reduce_add_sync(0xffffffffu, count);
+    const float top = key_value(__reduce_max_sync(0xffffffffu, topk));
+    if (!(kval - top >= -80.0f) || fabsf(kval) < 9.765625e-4f) flags |= 4u;
     /* equal zeros tie, as their probabilities do; beside another small one they may not */
-    small = (int)__reduce_add_sync(0xffffffffu, (unsigned)small);
-    zeros = (int)__reduce_add_sync(0xffffffffu, (unsigned)zeros);
-    if (small > 1 || (small > 0 && zeros > 0)) odd = true;
-    c.odd = __any_sync(0xffffffffu, odd);
-    c.open = __any_sync(0xffffffffu, open);
-    c.any = __any_sync(0xffffffffu, any) || c.odd || !code_known(cd[E]);
+    const uint32_t small = count & 0xffffu, zeros = count >> 16;
+    if (small > 1 || (small > 0 && zeros > 0)) flags |= 4u;
+    c.odd = flags & 4u;
+    c.open = flags & 2u;
+    c.any = (flags & 5u) || !code_known(cd[E]);
     return c;
 }
 /* the logits that need their chain: competitors whose code is open (all of them if
@@ -141,10 +150,12 @@ __device__ __forceinline__ bool rt_weights(const uint32_t *cd, const int *sel, i
     const uint32_t c = cd[e] & 0xffffu;
     const uint32_t key = on ? (code_key(c) << 16) | (0xffffu - (uint32_t)e) : 0u;
     int rank = 0;
+#pragma unroll 1
     for (int i = 0; i < TK; i++) rank += __shfl_sync(0xffffffffu, key, i) > key;
     const float m = key_value(__reduce_max_sync(0xffffffffu, key) >> 16);
     const float q = on ? (float)exp((double)__fsub_rn(bf16lo(c), m)) : 0.0f;
     float sw = 0.0f;
+#pragma unroll 1
     for (int i = 0; i < TK; i++) {
         const int src = __ffs(__ballot_sync(0xffffffffu, on && rank == i)) - 1;
         sw = __fadd_rn(sw, __shfl_sync(0xffffffffu, q, src));

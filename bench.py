@@ -463,11 +463,11 @@ def measure_stack(env, layers, T, chain, steps, warmup, sustain_s, seed,
     one_pass(trace_uniq=uniq)
     torch.cuda.synchronize()
     fused = be.last_block_launches() == 1
-    launches_per_layer = be.last_block_launches() + (2 if chain else 0)
+    launches_per_step = be.last_block_launches() * L
     if chain:
         one_pass()
         torch.cuda.synchronize()
-        launches_per_layer = be.last_block_launches() // L
+        launches_per_step = be.last_block_launches()      # of the whole stack
     step, mode = capture(torch, stream, one_pass, env["no_graph"])
     for _ in range(max(3, warmup)):
         step()
@@ -487,13 +487,13 @@ def measure_stack(env, layers, T, chain, steps, warmup, sustain_s, seed,
     res = {"ms_per_step": ms, "token_layers_per_s": tok_layers / (ms * 1e-3),
            "us_per_token_layer": ms * 1e3 / tok_layers, "layers": L,
            "tokens_per_layer": T, "chained": bool(chain), "launch": mode,
-           "clocks": clocks, "launches_per_step": launches_per_layer * L,
+           "clocks": clocks, "launches_per_step": launches_per_step,
            "unique_experts_mean": sum(uniq) / L, "stage_ms_per_layer": stage_ms,
            "device_status": status,
            "l2_policy": f"inputs larger than L2: one pass reads "
                         f"{bytes_pass / 1e6:.0f} MB of weights across {L} layers",
            "roofline": {"bound": "hbm",
-                        "kernel": "decode_fused_kernel" if fused else
+                        "kernel": "decode_stack_kernel" if fused else
                                   "whole layer (all kernels of the block)",
                         "achieved": bytes_pass / L / (kms * 1e-3) / 1e9 if kms else None,
                         "peak": pk["hbm_gbs"], "peak_source": pk["_source"],

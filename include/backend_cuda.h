@@ -278,8 +278,8 @@ int apus_cuda_moe_stack_dev(ApusCudaLayer *const *layers, const uint16_t *const 
 /* Grow the workspace arena for blocks of up to T tokens of this shape (and
  * allocate the one-kernel path's scratch for it). */
 int apus_cuda_reserve(const ApusCudaMoeCfg *c, size_t T);
-/* Kernels one apus_cuda_moe_block_dev call launched last time (for the
- * benchmark's launch count). */
+/* Kernels the last call of a block, layer or stack launched (for the benchmark's launch count;
+ * a stack of few tokens runs up to 32 layers in one). */
 int apus_cuda_last_block_launches(void);
 /* Which kernels the last apus_cuda_moe_block[_dev] call took (-1: none yet). */
 enum {
@@ -334,7 +334,7 @@ int apus_cuda_debug_fast_logits(const uint16_t *x, const uint16_t *wg, size_t T,
                                 float *wnorm, float *cbound);
 /* Diagnostic of the norms (host pointers, synchronous): the fp32 sum of squares of each row
  * of x [T,N], N % 8 == 0, as the sequential chain gives it (c/attn.h:175-186), by one warp to
- * a row or two; pieces: the 16-byte pieces whose squares a lane keeps in registers (2, 4, 8; 0:
+ * a row or two (N 2048: four with 2 pieces, two with 4, the one-kernel path's form); pieces: the 16-byte pieces whose squares a lane keeps in registers (2, 4, 8; 0:
  * none; -1: none, and lanes read them one at a time).  Refused where a row does not fit the form. */
 int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int pieces, int warps,
                           float *out);

@@ -656,7 +656,8 @@ def test_rmsnorm_sum_without_the_chain(gpu, orc, N):
 @pytest.mark.parametrize("N,pieces,warps", [
     (512, 2, 1), (768, 4, 1), (1024, 4, 1), (1280, 8, 1), (1792, 8, 1), (2048, 8, 1),
     (1152, -1, 1), (2304, -1, 1), (2560, -1, 1),                    # rows of the row norm
-    (512, 4, 2), (1536, 4, 2), (2048, 4, 2), (2560, 0, 2), (208, 0, 1), (144, 0, 1), (16, 4, 1), (1024, 4, 2)])
+    (512, 4, 2), (1536, 4, 2), (2048, 4, 2), (2560, 0, 2), (208, 0, 1), (144, 0, 1), (16, 4, 1), (1024, 4, 2),
+    (2048, 2, 4)])
 def test_sum_of_squares_is_the_chains(gpu, N, pieces, warps):
     """The fp32 sum itself, which a norm shows only through BF16, in every form that the row norm
     and the one-kernel path use: ties in every add, sums on a binade's edge, jumps over binades

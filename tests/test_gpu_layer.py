@@ -85,6 +85,37 @@ def test_stack_in_place_equals_the_chain_of_calls(gpu, be, synth, T):
         assert gpu.last_block_launches() == L          # one kernel per layer
 
 
+@pytest.mark.parametrize("T,E,I,TK,L", [
+    (1, 64, 256, 8, 3), (8, 37, 256, 8, 2), (4, 256, 512, 8, 2), (5, 256, 256, 8, 3),
+    (3, 8, 256, 8, 35), (8, 16, 512, 1, 2), (2, 5, 256, 3, 4)])
+def test_stack_of_wide_rows_in_one_launch(gpu, be, synth, T, E, I, TK, L):
+    """Layers of 2048 values, up to 32 to a launch: the bits of a call per step and layer.  Few
+    and many experts a token shares, two and four slices of a down row, more items than places in
+    the ring and fewer, a second launch for the layers left over."""
+    import torch
+    cfg = dict(hidden=2048, experts=E, moe_inter=I, shared_inter=I, top_k=TK)
+    some = [gpu.layer_create(cfg, synth.host_weights(be, cfg, seed=82, layer=l, sigma=0.02))
+            for l in range(min(L, 3))]
+    layers = [some[l % len(some)] for l in range(L)]
+    H = cfg["hidden"]
+    gains = [_dev(torch, synth.f32_to_bf16(np.random.default_rng(l).normal(0, 0.1, H)
+                                           .astype(np.float32))) for l in range(L)]
+    ref = _dev(torch, synth.host_x(be, T, H, seed=82 + T))
+    d = ref.clone()
+    for lay, g in zip(layers, gains):
+        _, out = _three_calls(gpu, torch, lay, ref, g, T, H)
+        ref = _dev(torch, out)
+    for _ in range(2):                       # the second call finds the first one's words
+        x = d.clone()
+        gpu.moe_stack_dev(layers, x.data_ptr(), T, d_ln_w=[g.data_ptr() for g in gains])
+        torch.cuda.synchronize()
+        assert gpu.last_block_status() == 0
+        assert gpu.last_block_launches() == (L + 31) // 32
+        assert np.array_equal(x.cpu().numpy(), ref.cpu().numpy())
+    for lay in some:
+        gpu.layer_destroy(lay)
+
+
 def test_layer_at_the_real_dimensions_one_token(gpu, orc, be, synth):
     import torch
     cfg = synth.QWEN_CFG
