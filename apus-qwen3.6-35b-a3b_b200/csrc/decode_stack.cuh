@@ -103,6 +103,13 @@ __device__ __forceinline__ uint64_t ld_tagged(const uint64_t *p) {
     return v;
 }
 
+/* both codes of an interval, a zero always the positive one (the order of the codes as integers
+ * is then that of the values, but for the sign) */
+__device__ __forceinline__ uint32_t no_negative_zero(uint32_t v) {
+    if ((v & 0xffffu) == 0x8000u) v &= 0xffff0000u;
+    if ((v >> 16) == 0x8000u) v &= 0xffffu;
+    return v;
+}
 /* (rolled: the compiler's unrolling of the waits alone was 40 KB) */
 __device__ __forceinline__ bool ds_wait(uint64_t *bar, uint32_t parity) {
 #pragma unroll 1
@@ -200,11 +207,89 @@ __device__ __noinline__ void stack_walk_chains(const StackArgs &a, int layer, St
             const float z = warp_chains<CH_CHAINS>(
                 1, DS_H, lane, reinterpret_cast<float *>(rr), [&](int) { return w; },
                 [&](int p) { return *reinterpret_cast<const uint4 *>(xr + lr.at(p)); });
-            if (lane == 0) st_tagged(&a.chain_ws[at + next - n], bf16_bits(z), S.tag);
+            if (lane == 0)
+                st_tagged(&a.chain_ws[at + next - n], no_negative_zero(bf16_bits(z)), S.tag);
         }
         n += S.namb[t];
     }
     if (lane == 0 && a.stats && blockIdx.x == 0) atomicAdd(&a.stats[0], (unsigned)n);
+}
+/* The selection where stack_select leaves something to look at: the whole of rt_select, and the
+ * list of what is open.  Returned: open | odd << 1 | entries of the list << 2. */
+__device__ __noinline__ int stack_select_slow(const uint32_t *cd, int E, int TK, int *sel,
+                                              uint16_t *amb) {
+    const int lane = threadIdx.x & 31;
+    const Choice c = rt_select(cd, E, TK, lane, sel);
+    int n = 0;
+    if (c.any)
+#pragma unroll 1
+        for (int e = lane; e - lane <= E; e += 32) {
+            const bool need = rt_needs(cd, e, E, c.kkey, c.odd);
+            const unsigned m = __ballot_sync(0xffffffffu, need);
+            if (need) amb[n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)e;
+            n += __popc(m);
+        }
+    return (c.open ? 1 : 0) | (c.odd ? 2 : 0) | (n << 2);
+}
+/* rt_select on the codes as they arrive (v[q]: expert lane + 32 q; no negative zeros; E <= 256),
+ * and the list of what is open, the same one in every CTA.  What is left out of it is what hardly
+ * ever is: a chosen logit, or one that may be, below 2^-10 or above 32.  A warp alone waits for
+ * each of its instructions, so the keys are made two at a time and the competitors that are not
+ * known are all that is looked at again.  (Cycles at one token / where a token of three or eight
+ * had one open: 3460 -> 2900, 6500 -> 3900.) */
+__device__ __forceinline__ int stack_select(const uint64_t (&v)[9], const uint32_t *cd, int E,
+                                            int TK, int lane, int *sel, uint16_t *amb) {
+    constexpr uint32_t SMALL = 0x3a80u | 0x8000u, FAR = 0x4200u | 0x8000u;  /* keys of 2^-10, 32 */
+    auto keys_of = [](uint32_t w) {                      /* code_key of both halves */
+        return w ^ (((w >> 15) & 0x00010001u) * 0xffffu | 0x80008000u);
+    };
+    uint32_t kr[8], unk = 0, kth = 0, mine = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int e = lane + 32 * q;
+        const uint32_t k = keys_of((uint32_t)v[q]);
+        kr[q] = e < E ? (k << 16) | (0xffffu - (uint32_t)e) : 0u;
+        if (e < E && (k & 0xffffu) != k >> 16) unk |= 1u << q;
+    }
+    uint32_t best = max(max(max(kr[0], kr[1]), max(kr[2], kr[3])),
+                        max(max(kr[4], kr[5]), max(kr[6], kr[7])));
+#pragma unroll 1
+    for (int i = 0; i < TK; i++) {
+        kth = __reduce_max_sync(0xffffffffu, best);
+        if (lane == (i & 31)) mine = kth;
+        if (i == 31) sel[lane] = (int)(0xffffu - (mine & 0xffffu));
+        uint32_t b[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) b[j] = kr[j] < kth ? kr[j] : 0u;
+        best = max(max(max(b[0], b[1]), max(b[2], b[3])), max(max(b[4], b[5]), max(b[6], b[7])));
+    }
+    if (lane < (TK & 31)) sel[(TK & ~31) + lane] = (int)(0xffffu - (mine & 0xffffu));
+    const uint32_t kkey = kth >> 16;
+    bool open = false, other = false;
+    int n = 0;
+#pragma unroll 1
+    while (__any_sync(0xffffffffu, unk != 0)) {
+        const int e = lane + 32 * (__ffs(unk) - 1);
+        bool need = false;
+        if (unk) {
+            const uint32_t k = keys_of(cd[e]);
+            need = k >> 16 >= kkey;
+            open |= need && ((k << 16) | (0xffffu - (uint32_t)e)) < kth;
+            other |= need && ((k & 0xffffu) < SMALL || k >> 16 > FAR);
+            unk &= unk - 1;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, need);
+        if (need) amb[n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)e;
+        n += __popc(m);
+    }
+    /* the largest: the first one's low code, or what the loop looked at */
+    other |= kkey < SMALL || (lane == 0 && (TK < 32 ? mine >> 16 > FAR : true));
+    if (__any_sync(0xffffffffu, other)) return stack_select_slow(cd, E, TK, sel, amb);
+    if (!code_known(cd[E])) {
+        if (lane == 0) amb[n] = (uint16_t)E;
+        n++;
+    }
+    return (__any_sync(0xffffffffu, open) ? 1 : 0) | (n << 2);
 }
 /* A warp to a token, its chains known: the selection again, or the engine's softmax. */
 __device__ __noinline__ void stack_select_again(const StackArgs &a, StackShared &S, uint32_t *cd,
@@ -396,9 +481,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
             auto meet = [&] {
                 asm volatile("bar.sync %0, %1;" ::"r"(3 + t), "r"(32 * parts) : "memory");
             };
-            rs = norm_scale(parts == 4 ? exact_sumsq_wide<4>(row, lr, lane, part, share, meet)
-                                       : exact_sumsq_wide<2>(row, lr, lane, part, share, meet),
-                            DS_H);
+            const float sum = parts == 4 ? exact_sumsq_wide<4>(row, lr, lane, part, share, meet)
+                                         : exact_sumsq_wide<2>(row, lr, lane, part, share, meet);
+            /* norm_scale; a quotient by a power of two is the product */
+            rs = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(sum, 1.0f / DS_H), 1e-6f)));
         }
         PackedRange range;
         float sq = 0.0f;
@@ -439,7 +525,8 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                                     (gate ? W.wnorm_gate : __ldg(&W.wnorm[e])) *
                                         norm_above(sq, DS_H));
             }
-            if (lane == 0) st_tagged(&a.code_ws[(size_t)t * (E + 1) + e], v, S.tag);
+            if (lane == 0)
+                st_tagged(&a.code_ws[(size_t)t * (E + 1) + e], no_negative_zero(v), S.tag);
         }
     mark(1);                                /* own logits published */
 
@@ -486,22 +573,12 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                     if (lane + q * 32 < E + 1) cd[lane + q * 32] = (uint32_t)v[q];
                 __syncwarp();
                 if (all) {
-                    const Choice c = rt_select(cd, E, TK, lane, S.sel + warp * TK);
-                    int n = 0;              /* open logits: the same list in every CTA */
-                    if (c.any)
-#pragma unroll 1
-                        for (int e = lane; e - lane <= E; e += 32) {
-                            const bool need = rt_needs(cd, e, E, c.kkey, c.odd);
-                            const unsigned m = __ballot_sync(0xffffffffu, need);
-                            if (need)
-                                amb[warp * (E + 1) + n + __popc(m & ((1u << lane) - 1u))] =
-                                    (uint16_t)e;
-                            n += __popc(m);
-                        }
+                    const int r = stack_select(v, cd, E, TK, lane, S.sel + warp * TK,
+                                               amb + warp * (E + 1));
                     if (lane == 0) {
-                        S.namb[warp] = n;
-                        S.full[warp] = c.odd;
-                        if (c.open || c.odd) S.open = 1;
+                        S.namb[warp] = r >> 2;
+                        S.full[warp] = (r >> 1) & 1;
+                        if (r & 3) S.open = 1;
                     }
                     mark_chosen();
                 } else if (lane == 0) {
@@ -715,6 +792,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
         for (int w = 0; w < 4; w++) x[w] = __ldcg(q + w * 4);
     };
     const int n_units = (U + 1) << a.slices_log2;
+    /* the combine's output of this thread, and what it is added to */
+    const int out_t = tid / ncols, out_at = out_t * DS_H + h_lo + (tid - out_t * ncols);
+    uint16_t out_res = 0;
+    if (a.res_out && out_t < T) out_res = __ldcg(res + out_at);
     uint4 xn[4];
     if (warp < n_units) unit_acts(warp, xn);
 #pragma unroll 1
@@ -776,8 +857,8 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     }
     /* the helper warp has been through as well */
     asm volatile("bar.sync 2, %0;" ::"n"(DS_CW * 32 + 32) : "memory");
-    if (!dead && tid < T * ncols) {
-        const int t = tid / ncols, h = tid - t * ncols;
+    if (!dead && out_t < T) {
+        const int t = out_t, h = out_at - t * DS_H - h_lo;
         float acc = 0.0f;
 #pragma unroll 2
         for (int s = 0; s < TK; s++)
@@ -786,10 +867,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
         const float routed = bf16_round(acc);
         const float shared = bf16_round(__fmul_rn(red[(A + t) * DF_MAX_COLS + h], S.gate[t]));
         const uint16_t v = bf16_bits(__fadd_rn(routed, shared));
-        const size_t at = (size_t)t * DS_H + h_lo + h;
+        const size_t at = out_at;
         if (a.out) a.out[at] = v;
         if (a.res_out)                          /* c/layer.h:230-234,388 */
-            a.res_out[at] = bf16_bits(__fadd_rn(bf16_f32(__ldcg(res + at)), bf16_f32(v)));
+            a.res_out[at] = bf16_bits(__fadd_rn(bf16_f32(out_res), bf16_f32(v)));
         if (a.tr_out) a.tr_out[at] = v;
         if (a.tr_routed) a.tr_routed[at] = bf16_bits(routed);
         if (a.tr_shared) a.tr_shared[at] = bf16_bits(shared);
