@@ -36,6 +36,7 @@ constexpr int DS_CELL = 16 * 1024;      /* down rows of an expert: at most 16 of
 constexpr int DS_CELLS = 8;
 constexpr int DS_TILE = 2 * DS_PAIRS * DS_H * 2;        /* 64 KB: four cells */
 constexpr int DS_LAYERS = 32;           /* layers of a launch, at most (parameter space) */
+static_assert(CH_BYTES <= 8 * sizeof(SumShare), "a chain's products in the place of the sums'");
 static_assert(DS_CELL * DS_CELLS == 2 * DS_TILE, "two tiles or eight cells");
 
 struct StackLayout {
@@ -48,7 +49,7 @@ struct StackLayout {
         rrows = (E + 1 + G - 1) / G;
         off_x = 2 * DS_TILE;
         off_rr = off_x + T * xrow;
-        off_gain = off_rr + (rrows * xrow > CH_BYTES ? rrows * xrow : CH_BYTES);
+        off_gain = off_rr + rrows * xrow;
         off_share = off_gain + DS_H * 2;
         off_code = off_share + 8 * (int)sizeof(SumShare);
         off_tmask = (off_code + T * (E + 1) * 4 + 7) & ~7;
@@ -157,6 +158,7 @@ __device__ __forceinline__ void slice_pieces(const unsigned char *p, bool odd, u
 struct StackShared {
     uint64_t tile_full[2], tile_free[2], cell_full[DS_CELLS], cell_free[DS_CELLS];
     float gate[DF_MAX_T], sq[4][DF_MAX_T];
+    float part[2][DS_CW];               /* a logit's parts: sums, error terms */
     unsigned int xlo[DF_MAX_T], xhi[DF_MAX_T];
     int sel[DF_MAX_A];                  /* selected experts, in provisional order */
     int idx[DF_MAX_A], row[DF_MAX_A];   /* final order; down output of each */
@@ -188,10 +190,10 @@ __device__ __forceinline__ bool take_chain(const StackArgs &a, StackShared &S, u
     if (!there) set_status(a.status, ST_SCHED_TIMEOUT);
     return there;
 }
-/* The helper warp: the products in the place of the router rows (rr). */
+/* The helper warp; buf: CH_BYTES of shared memory for the products. */
 __device__ __noinline__ void stack_walk_chains(const StackArgs &a, int layer, StackShared &S,
                                                const uint16_t *amb, const unsigned char *xs,
-                                               unsigned char *rr) {
+                                               unsigned char *buf) {
     const StackLayer &W = a.layer[layer];
     const LaneRow lr(DS_H);
     const int lane = threadIdx.x & 31, E = a.E, G = gridDim.x;
@@ -205,14 +207,14 @@ __device__ __noinline__ void stack_walk_chains(const StackArgs &a, int layer, St
             const uint16_t *w = e == E ? W.sh_gate : W.rtr_w + (size_t)e * DS_H;
             const unsigned char *xr = xs + t * a.L.xrow;
             const float z = warp_chains<CH_CHAINS>(
-                1, DS_H, lane, reinterpret_cast<float *>(rr), [&](int) { return w; },
+                1, DS_H, lane, reinterpret_cast<float *>(buf), [&](int) { return w; },
                 [&](int p) { return *reinterpret_cast<const uint4 *>(xr + lr.at(p)); });
             if (lane == 0)
                 st_tagged(&a.chain_ws[at + next - n], no_negative_zero(bf16_bits(z)), S.tag);
         }
         n += S.namb[t];
     }
-    if (lane == 0 && a.stats && blockIdx.x == 0) atomicAdd(&a.stats[0], (unsigned)n);
+    if (lane == 0 && n > 0 && a.stats && blockIdx.x == 0) atomicAdd(&a.stats[0], (unsigned)n);
 }
 /* The selection where stack_select leaves something to look at: the whole of rt_select, and the
  * list of what is open.  Returned: open | odd << 1 | entries of the list << 2. */
@@ -436,16 +438,21 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
             const size_t at = (size_t)(sh_lo + j * DS_PAIRS) * DS_H;
             request_tile(tile0 + j, W.sh_g + at, W.sh_u + at, n, nullptr, nullptr, n);
         }
-    /* (the other two warps may be a phase ahead of these at a layer's end) */
-    if (warp < DS_CW)
+    /* (the requesting warp has asked for a later layer's in the layer before) */
+    auto fetch_rows = [&](const StackLayer &w, int at, int step) {
 #pragma unroll 1
-        for (int c = tid; c < n_rr * PIECES; c += DS_CW * 32) {
+        for (int c = at; c < (n_rr + 1) * PIECES; c += step) {
             const int r = c / PIECES, e = cta + r * G, p = c % PIECES;
-            *reinterpret_cast<uint4 *>(rr + r * L.xrow + lr.at(p)) =
-                ldg16((e == E ? W.sh_gate : W.rtr_w + (size_t)e * DS_H) + p * 8);
+            if (r < n_rr)
+                cp_async16_to(smem_u32(rr + r * L.xrow + lr.at(p)),
+                              (e == E ? w.sh_gate : w.rtr_w + (size_t)e * DS_H) + p * 8);
+            else if (a.res && w.ln_w)
+                cp_async16_to(smem_u32(gains + p), w.ln_w + p * 8);
+            else
+                gains[p] = make_uint4(0, 0, 0, 0);
         }
-    if (tid < PIECES)
-        gains[tid] = res && W.ln_w ? ldg16(W.ln_w + tid * 8) : make_uint4(0, 0, 0, 0);
+    };
+    if (first && warp < DS_CW) fetch_rows(W, tid, DS_CW * 32);
     if (tid < 256) s_tmask[tid] = 0;
     if (tid < DF_MAX_T) {
         S.xlo[tid] = 0x7f800000u;
@@ -460,6 +467,7 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
         }
         S.tag = sync_at;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(res ? res : a.x);
@@ -510,23 +518,71 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     }
     __syncthreads();
 
-    /* ---- router logits of this CTA's rows ---- */
+    /* ---- router logits of this CTA's rows: up to two tokens four warps to one, up to four two
+     * (certified_logit, the rows cut across the warps like the norm's) ---- */
+    const int lg = L.rrows > 2 || T > 4 ? 0 : T > 2 ? 1 : 2, per = 1 << lg;
     if (warp < DS_CW)
 #pragma unroll 1
-        for (int p = warp; p < n_rr * T; p += DS_CW) {
-            const int r = p >= T ? p / T : 0, t = p - r * T, e = cta + r * G;
+        for (int p = warp >> lg; p < n_rr * T; p += DS_CW >> lg) {
+            const int r = p >= T ? p / T : 0, t = p - r * T, e = cta + r * G,
+                      part = warp & (per - 1);
             const bool gate = e == E;
-            uint32_t v = CODE_UNKNOWN;
-            if (products_exact(gate ? W.wmin_gate : W.wmin, gate ? W.wmax_gate : W.wmax, S.xlo[t],
-                               S.xhi[t])) {
+            const bool exact = products_exact(gate ? W.wmin_gate : W.wmin,
+                                              gate ? W.wmax_gate : W.wmax, S.xlo[t], S.xhi[t]);
+            const int chunk = part * 32 + lane, nu = 8 >> lg;
+            const int off = (chunk >> lg) * lr.pitch + (chunk & (per - 1)) * nu * 16;
+            const unsigned char *wp = rr + r * L.xrow + off, *xp = xs + t * L.xrow + off;
+            float run = 0.0f, err = 0.0f;
+#pragma unroll 2
+            for (int i = 0; i < nu; i++) {
+                float wf[8], xf[8];
+                unpack8(*reinterpret_cast<const uint4 *>(wp + i * 16), wf);
+                unpack8(*reinterpret_cast<const uint4 *>(xp + i * 16), xf);
+                float s0 = __fmul_rn(wf[0], xf[0]), s1 = __fmul_rn(wf[4], xf[4]);
+#pragma unroll
+                for (int j = 1; j < 4; j++) {
+                    s0 = __fmaf_rn(wf[j], xf[j], s0);
+                    s1 = __fmaf_rn(wf[4 + j], xf[4 + j], s1);
+                }
+                err += fabsf(run);
+                run += s0 + s1;
+            }
+            float sum = run;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const float v = __shfl_up_sync(0xffffffffu, sum, d);
+                if (lane >= d) sum += v;
+            }
+            float tot = __shfl_sync(0xffffffffu, sum, 31);
+            auto meet = [&] {
+                asm volatile("bar.sync %0, %1;" ::"r"(3 + (warp >> lg)), "r"(32 << lg) : "memory");
+            };
+            if (per > 1) {
+                if (lane == 0) S.part[0][warp] = tot;
+                meet();
+                float before = 0.0f;
+                for (int i = 0; i < part; i++) before += S.part[0][warp - part + i];
+                sum += before;
+                tot += before;              /* (the last part's: the whole) */
+            }
+            err = warp_sum(8.0f * nu * fabsf(sum - run) + 9.0f * err + 8.0f * fabsf(run));
+            if (per > 1) {
+                if (lane == 0) S.part[1][warp] = err;
+                meet();
+                err = 0.0f;
+                for (int i = 0; i < per; i++) err += S.part[1][warp - part + i];
+            }
+            if (part == per - 1 && lane == 0) {
                 const float sq = T <= 4 ? (S.sq[0][t] + S.sq[1][t]) + (S.sq[2][t] + S.sq[3][t])
                                         : S.sq[0][t] + S.sq[1][t];
-                v = certified_logit(rr + r * L.xrow, xs + t * L.xrow, lr, lane,
-                                    (gate ? W.wnorm_gate : __ldg(&W.wnorm[e])) *
-                                        norm_above(sq, DS_H));
-            }
-            if (lane == 0)
+                const float cs = (gate ? W.wnorm_gate : __ldg(&W.wnorm[e])) * norm_above(sq, DS_H);
+                err = (err + 12.0f * cs) * (1.05f * 5.9604645e-8f);
+                const float lo = __fadd_rd(tot, -err), hi = __fadd_ru(tot, err);
+                const uint32_t v = exact && lo <= hi
+                                       ? (uint32_t)bf16_bits(lo) | ((uint32_t)bf16_bits(hi) << 16)
+                                       : CODE_UNKNOWN;
                 st_tagged(&a.code_ws[(size_t)t * (E + 1) + e], no_negative_zero(v), S.tag);
+            }
         }
     mark(1);                                /* own logits published */
 
@@ -587,27 +643,22 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
             }
             __syncthreads();
             dead = S.dead != 0;
-            int n_amb = 0;
-            if (!dead)
+            if (warp == DS_CW + 1 && !dead)
+                stack_walk_chains(a, layer, S, amb, xs, ds_smem + L.off_share);
+            if (S.open && !dead) {          /* the set itself waits for the chains */
+                if (tid < 256) s_tmask[tid] = 0;
 #pragma unroll 1
-                for (int t = 0; t < T; t++) n_amb += S.namb[t];
-            if (n_amb > 0) {
-                if (warp == DS_CW + 1) stack_walk_chains(a, layer, S, amb, xs, rr);
-                if (S.open) {               /* the set itself waits for the chains */
-                    if (tid < 256) s_tmask[tid] = 0;
+                for (int t = warp; t < T; t += DS_THREADS / 32)
 #pragma unroll 1
-                    for (int t = warp; t < T; t += DS_THREADS / 32)
-#pragma unroll 1
-                        for (int k = lane; k < S.namb[t]; k += 32)
-                            if (!take_chain(a, S, codes, amb, t, k)) S.dead = 1;
-                    __syncthreads();
-                    dead = S.dead != 0;
-                    if (warp < T && !dead) {
-                        stack_select_again(a, S, cd, warp);
-                        mark_chosen();
-                    }
-                    __syncthreads();
+                    for (int k = lane; k < S.namb[t]; k += 32)
+                        if (!take_chain(a, S, codes, amb, t, k)) S.dead = 1;
+                __syncthreads();
+                dead = S.dead != 0;
+                if (warp < T && !dead) {
+                    stack_select_again(a, S, cd, warp);
+                    mark_chosen();
                 }
+                __syncthreads();
             }
             /* ---- the distinct experts, ascending, and who uses them: every warp writes the
              * whole list, and waits for nobody's ---- */
@@ -627,18 +678,19 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                 }
                 int p = incl - mine;
                 U = __shfl_sync(0xffffffffu, incl, 31) & 0xffff;
+                /* bit i: expert 8 lane + i */
+                uint32_t r = (((used(m.x) >> 7) * 0x01020408u) >> 24 & 15u) |
+                             (((used(m.y) >> 7) * 0x01020408u) >> 20 & 0xf0u);
 #pragma unroll 1
-                for (uint32_t h = 0, r = used(m.x); h < 2; h++, r = used(m.y))
-#pragma unroll 1
-                    for (; r; r &= r - 1) {
-                        const int k = __ffs(r) - 8;         /* first bit of the byte */
-                        const uint32_t who = ((h ? m.y : m.x) >> k) & 0xffu;
-                        const int u = p & 0xffff;
-                        S.uexp[u] = (lane * 2 + (int)h) * 4 + (k >> 3);
-                        S.umask[u] = (uint8_t)who;
-                        S.ubase[u] = p >> 16;
-                        p += 1 + (__popc(who) << 16);
-                    }
+                for (; r; r &= r - 1) {
+                    const int k = __ffs(r) - 1;
+                    const uint32_t who = ((k & 4 ? m.y : m.x) >> ((k & 3) * 8)) & 0xffu;
+                    const int u = p & 0xffff;
+                    S.uexp[u] = lane * 8 + k;
+                    S.umask[u] = (uint8_t)who;
+                    S.ubase[u] = p >> 16;
+                    p += 1 + (__popc(who) << 16);
+                }
                 __syncwarp();
             }
             mark(3);                        /* selection known */
@@ -660,6 +712,8 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                     request_tile(tile0 + j, w, w + half, k, w2, w2 + half, n);
                 }
                 tile0 += n_tiles;
+                /* (nobody looks at this layer's any more) */
+                if (layer + 1 < a.n_layers) fetch_rows(a.layer[layer + 1], lane, 32);
                 /* a lane to a cell: it asks again as soon as its cell is free (one after another
                  * they kept each other waiting: 25 us for the down rows of eight tokens) */
                 const uint32_t bytes = (uint32_t)(ncols * I * 2);
