@@ -1746,6 +1746,11 @@ static int launch_rmsnorm(Ctx *c, const uint16_t *x, const uint16_t *w, uint16_t
     const bool enough = chunks >= 16 || (chunks == 8 && T <= 4 * c->sm_count);
     if (N >= 512 && N % 8 == 0 && enough && rows <= 40 * 1024 &&
         (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) == 0) {
+        if (N == 2048 && T <= c->sm_count) {
+            launch_k(rmsnorm_wide_kernel, dim3(T), dim3(128), 0, st, x, w, y);
+            LAUNCHED();
+            return 0;
+        }
         const int nu = LaneRow(N).nu;
         auto kern = nu <= 2   ? rmsnorm_rows_kernel<2>
                     : nu <= 4 ? rmsnorm_rows_kernel<4>

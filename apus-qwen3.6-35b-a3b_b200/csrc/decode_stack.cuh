@@ -294,8 +294,8 @@ __device__ __forceinline__ int stack_select(const uint64_t (&v)[9], const uint32
     return (__any_sync(0xffffffffu, open) ? 1 : 0) | (n << 2);
 }
 /* A warp to a token, its chains known: the selection again, or the engine's softmax. */
-__device__ __noinline__ void stack_select_again(const StackArgs &a, StackShared &S, uint32_t *cd,
-                                                int t) {
+__device__ __forceinline__ void stack_select_again(const StackArgs &a, StackShared &S,
+                                                   uint32_t *cd, int t) {
     const int lane = threadIdx.x & 31, E = a.E, TK = a.TK;
     if (S.full[t]) {
         float *p = reinterpret_cast<float *>(cd);
@@ -354,10 +354,15 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     __shared__ StackShared S;
 
     const bool first = layer == 0;
-    const StackLayer &W = a.layer[layer];
-    int tid = threadIdx.x, T = a.T, G = gridDim.x, cta = blockIdx.x;
-    /* (nothing of a layer's address arithmetic is kept over the loop) */
-    asm volatile("" : "+r"(tid), "+r"(T), "+r"(G), "+r"(cta));
+    /* What is computed from these is computed again in every layer, and below in both phases,
+     * instead of being kept in registers over the loops: 96 of them are all that eighteen warps
+     * can have (four layers at 1 / 3 / 8 tokens 114 / 178 / 341 us without any of it). */
+    int wl = layer;
+    asm volatile("" : "+r"(wl));
+    const StackLayer &W = a.layer[wl];
+    int tid = threadIdx.x;
+    const int T = a.T, G = gridDim.x, cta = blockIdx.x;
+    asm volatile("" : "+r"(tid));
     const int I = a.I, E = a.E, TK = a.TK, A = T * TK;
     const int lane = tid & 31, warp = tid >> 5;
     const StackLayout &L = a.L;
@@ -593,6 +598,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     /* the shared expert's gate/up rows, for which nobody waits; then the routed ones */
 #pragma unroll 1
     for (int phase = 0; phase < 2; phase++) {
+        int lane = tid & 31, warp = tid >> 5;
+        asm volatile("" : "+r"(lane), "+r"(warp));
+        const int fr = lane >> 2, fq = lane & 3;
+        const bool odd = fr & 1;
         if (phase == 1) {
             mark(2);                        /* shared gate/up done */
             /* ---- routing: a warp to a token; the others wait for all of them ---- */
@@ -829,8 +838,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     dead = S.dead != 0;
     mark(5);                                /* barrier passed */
     /* ---- down rows of this CTA's columns: a warp to 128 k of an expert.  Its activations are
-     * nobody else's here: they come straight from L2, the next unit's while this one is at work
-     * (all of them through shared memory first: 1.7 kcycles at one token, 6.6 at eight). ---- */
+     * nobody else's here: they come straight from L2, beside the wait for the rows (all of them
+     * through shared memory first: 1.7 kcycles at one token, 6.6 at eight; those of the next unit
+     * while this one is at work cost sixteen registers, and with what they spilled 3 to 5 % of
+     * four layers). ---- */
     auto unit_rows = [&](int v, int &cnt, int &row0) {
         const int d = v >> a.slices_log2;
         cnt = d == U ? T : __popc(S.umask[d]);
@@ -850,14 +861,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     const int out_t = tid / ncols, out_at = out_t * DS_H + h_lo + (tid - out_t * ncols);
     uint16_t out_res = 0;
     if (a.res_out && out_t < T) out_res = __ldcg(res + out_at);
-    uint4 xn[4];
-    if (warp < n_units) unit_acts(warp, xn);
 #pragma unroll 1
     for (int v = warp; v < n_units; v += DS_CW) {
         uint4 xv[4];
-#pragma unroll
-        for (int w = 0; w < 4; w++) xv[w] = xn[w];
-        if (v + DS_CW < n_units) unit_acts(v + DS_CW, xn);
+        unit_acts(v, xv);
         const int d = v >> a.slices_log2, slice = v & ((1 << a.slices_log2) - 1);
         int cnt, row0;
         unit_rows(v, cnt, row0);

@@ -230,7 +230,7 @@ __device__ __forceinline__ float exact_sumsq(const unsigned char *row, const Lan
 constexpr int SUM_RUNS = 16;             /* runs of a warp, at most; one more ends them */
 struct SumShare {
     float total[4];                      /* the warps' tree sums */
-    float start;                         /* the sum of the row's first two chunks */
+    float start;                         /* the sum of the row's first chunks */
     int n[4];                            /* runs of each warp; < 0: add in order */
     /* x: function of an even sum | binade << 24, y: of an odd one; z, w: the terms behind it */
     int4 run[4][SUM_RUNS];
@@ -239,6 +239,9 @@ template <int W, typename Meet>
 __device__ __forceinline__ float exact_sumsq_wide(const unsigned char *row, const LaneRow lr,
                                                   int lane, int part, SumShare &sh, Meet meet) {
     constexpr int P = 8 / W, N = P * 8;         /* 16-byte pieces and terms of a lane */
+    /* The row's first chunks, where a chunk may pass two edges, are simply added up: with two of
+     * 16 terms 11 of 1600 normal rows had to be added in order, with three none. */
+    constexpr int HEAD = W == 4 ? 3 : 2;
     const int chunk = part * 32 + lane, l = chunk / W;
     const unsigned char *mine = row + l * lr.pitch + (chunk - l * W) * P * 16;
     float q[N];
@@ -268,9 +271,8 @@ __device__ __forceinline__ float exact_sumsq_wide(const unsigned char *row, cons
     for (int w = 0; w < W - 1; w++)
         if (w < part) before += sh.total[w];
     const float first = before + (incl - tot);
-    /* Binades, taken from the sums at the lanes' ends so that neighbours agree on them.  The
-     * row's first two chunks, where the sum doubles fast, are simply added up. */
-    const bool head = chunk < 2;
+    /* Binades, taken from the sums at the lanes' ends so that neighbours agree on them. */
+    const bool head = chunk < HEAD;
     const int b1 = binade(before + incl);
     int b0 = __shfl_up_sync(0xffffffffu, b1, 1);
     if (lane == 0) b0 = binade(before);
@@ -317,10 +319,14 @@ __device__ __forceinline__ float exact_sumsq_wide(const unsigned char *row, cons
     pre.i0 = __float_as_int(fe) - e0;
     pre.i1 = __float_as_int(fo) - (e0 + 1);
     if (part == 0) {
-        float s = __shfl_sync(0xffffffffu, fe, 0);
+        float s = fe;
 #pragma unroll
-        for (int i = 0; i < N; i++) s = __fadd_rn(s, q[i]);
-        if (lane == 1) sh.start = s;
+        for (int c = 1; c < HEAD; c++) {
+            s = __shfl_sync(0xffffffffu, s, c - 1);
+#pragma unroll
+            for (int i = 0; i < N; i++) s = __fadd_rn(s, q[i]);
+        }
+        if (lane == HEAD - 1) sh.start = s;
         if (head) pre.i0 = pre.i1 = 0;
     }
     ParityFn f = pre;
@@ -386,7 +392,7 @@ __device__ __forceinline__ float exact_sumsq_wide(const unsigned char *row, cons
             r[w] = next;
         }
     }
-    if (!ok) {
+    if (!ok) {                               /* (inline: a call cost 1 % of a decode layer) */
         s = 0.0f;
 #pragma unroll 1
         for (int c = 0; c < lr.nl * lr.nu; c++) {
@@ -470,6 +476,37 @@ rmsnorm_rows_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__
             dst[c] = norm8(*reinterpret_cast<const uint4 *>(row + lr.at(c)),
                            w ? __ldg(gsrc + c) : make_uint4(0, 0, 0, 0), rs);
     }
+}
+
+/* The same for rows of 2048 values, at most one to an SM: the latency of one row is all that is
+ * waited for, so four warps share it.  One CTA per row.  61 rows back to back 5.1 -> 4.3 us, 148 the
+ * same; from 300 on one of them often needs the sum in order (9.3 against 5.5): those stay with
+ * the form above. */
+__global__ void __launch_bounds__(128)
+rmsnorm_wide_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ w,
+                    uint16_t *__restrict__ y) {
+    constexpr int N = 2048;
+    __shared__ __align__(16) unsigned char row[32 * (N / 16 + 16)];
+    __shared__ SumShare share;
+    const LaneRow lr(N);
+    const int tid = threadIdx.x;
+    const uint4 *src = reinterpret_cast<const uint4 *>(x + (size_t)blockIdx.x * N),
+                *gsrc = reinterpret_cast<const uint4 *>(w);
+    uint4 g[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)}, v[2];
+    if (w)                                   /* (not the kernel's before) */
+#pragma unroll
+        for (int i = 0; i < 2; i++) g[i] = __ldg(gsrc + tid + 128 * i);
+    pdl_enter();
+#pragma unroll
+    for (int i = 0; i < 2; i++) v[i] = __ldg(src + tid + 128 * i);
+#pragma unroll
+    for (int i = 0; i < 2; i++) *reinterpret_cast<uint4 *>(row + lr.at(tid + 128 * i)) = v[i];
+    __syncthreads();
+    const float rs = norm_scale(
+        exact_sumsq_wide<4>(row, lr, tid & 31, tid >> 5, share, [] { __syncthreads(); }), N);
+    uint4 *dst = reinterpret_cast<uint4 *>(y + (size_t)blockIdx.x * N);
+#pragma unroll
+    for (int i = 0; i < 2; i++) dst[tid + 128 * i] = norm8(v[i], g[i], rs);
 }
 
 /* A logit as far as it is known: the BF16 codes between which the chain's rounded
