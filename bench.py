@@ -328,7 +328,7 @@ def measure_layer(env, layer, x_host, T, skew, steps, warmup, sustain_s,
     tc_ideal = flops(cfg, T) / (pk["bf16_tflops"] * 1e12)
     if launches_per_step == 1:
         kms = sum(stage_ms.values())
-        roof = {"bound": "hbm", "kernel": "decode_fused_kernel",
+        roof = {"bound": "hbm", "kernel": "decode_stack_kernel",
                 "achieved": block_bytes / (kms * 1e-3) / 1e9 if kms else None,
                 "peak": pk["hbm_gbs"], "unit": "GB/s", "traffic": None,
                 "algorithmic_bytes_per_launch": block_bytes}
