@@ -6,6 +6,8 @@ checked against the CPU checker; and the CPU checker's chain directly."""
 import numpy as np
 import pytest
 
+from test_gpu_block import check_block
+
 pytestmark = pytest.mark.gpu
 
 MID = dict(hidden=512, experts=64, moe_inter=128, shared_inter=128, top_k=8)
@@ -114,6 +116,23 @@ def test_stack_of_wide_rows_in_one_launch(gpu, be, synth, T, E, I, TK, L):
         assert np.array_equal(x.cpu().numpy(), ref.cpu().numpy())
     for lay in some:
         gpu.layer_destroy(lay)
+
+
+@pytest.mark.parametrize("T,E,I,TK", [(1, 64, 256, 8), (8, 37, 256, 8), (5, 256, 256, 8),
+                                      (3, 8, 256, 8), (8, 16, 512, 1), (2, 5, 256, 3)])
+def test_stack_kernels_block_is_the_checkers(gpu, orc, be, synth, T, E, I, TK):
+    """The comparison above is with block calls that run the same kernel at these shapes: here
+    against the CPU checker, two calls in a row.  (Outputs stay below 4, where one BF16 step,
+    2^-6, is below the largest difference allowed.)"""
+    cfg = dict(hidden=2048, experts=E, moe_inter=I, shared_inter=I, top_k=TK)
+    W = synth.host_weights(be, cfg, seed=82, sigma=0.02)
+    for seed in (21, 22):
+        x = synth.host_x(be, T, 2048, seed=seed)
+        exp = orc.moe_block(cfg, W, x)
+        assert np.abs(f32(exp["out"])).max() < 4
+        got = gpu.moe_block(cfg, W, x)
+        assert gpu.last_block_status() == 0 and gpu.last_block_launches() == 1
+        check_block(got, exp, f"T={T} E={E} I={I}")
 
 
 def test_layer_at_the_real_dimensions_one_token(gpu, orc, be, synth):
