@@ -214,11 +214,14 @@ __device__ __forceinline__ uint4 ldg16(const void *p) {
     return __ldg(reinterpret_cast<const uint4 *>(p));
 }
 
-/* Programmatic dependent launch: every kernel of the block begins with
- * pdl_enter(): it lets the next kernel in the stream be scheduled early (its
- * own prologue then overlaps this kernel's tail) and waits until the previous
- * kernel's memory is complete and visible.  Without the launch attribute both
- * instructions are no-ops. */
+/* Programmatic dependent launch: a kernel of the block begins with pdl_enter()
+ * or with its two instructions apart: the first lets the next kernel in the
+ * stream be scheduled early (its own prologue then overlaps this kernel's tail),
+ * the second waits until the previous kernel's memory is complete and visible.
+ * Only what a resident layer holds, and what was complete before the previous
+ * kernel let go, is read before that wait; all else that a call brings, the
+ * norm's gains included, may be the previous kernel's output.
+ * Without the launch attribute both instructions are no-ops. */
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

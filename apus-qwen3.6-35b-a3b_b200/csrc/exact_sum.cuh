@@ -479,9 +479,10 @@ rmsnorm_rows_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__
 }
 
 /* The same for rows of 2048 values, at most one to an SM: the latency of one row is all that is
- * waited for, so four warps share it.  One CTA per row.  61 rows back to back 5.1 -> 4.3 us, 148 the
- * same; from 300 on one of them often needs the sum in order (9.3 against 5.5): those stay with
- * the form above. */
+ * waited for, so four warps share it.  One CTA per row.  Back to back, us, the form above -> this:
+ * 9 rows 4.8 -> 2.3, 61 rows 4.9 -> 2.4, 148 rows 4.9 -> 2.4; four layers of 9 tokens 389 -> 376,
+ * of 32 731 -> 718, of 148 1101 -> 1097.  From 300 rows on one of them often needs the sum in
+ * order (9.3 against 5.5): those stay with the form above. */
 __global__ void __launch_bounds__(128)
 rmsnorm_wide_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ w,
                     uint16_t *__restrict__ y) {
@@ -493,10 +494,10 @@ rmsnorm_wide_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__
     const uint4 *src = reinterpret_cast<const uint4 *>(x + (size_t)blockIdx.x * N),
                 *gsrc = reinterpret_cast<const uint4 *>(w);
     uint4 g[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)}, v[2];
-    if (w)                                   /* (not the kernel's before) */
+    pdl_enter();                             /* the gains too may be the kernel's before */
+    if (w)
 #pragma unroll
         for (int i = 0; i < 2; i++) g[i] = __ldg(gsrc + tid + 128 * i);
-    pdl_enter();
 #pragma unroll
     for (int i = 0; i < 2; i++) v[i] = __ldg(src + tid + 128 * i);
 #pragma unroll

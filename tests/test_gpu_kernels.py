@@ -653,6 +653,30 @@ def test_rmsnorm_sum_without_the_chain(gpu, orc, N):
     assert np.array_equal(d_y.cpu().numpy().view(np.uint16), orc.rmsnorm(x, None))
 
 
+@pytest.mark.parametrize("T,N", [(148, 2048), (9, 2048), (149, 2048), (148, 512)])
+def test_rmsnorm_gains_from_the_kernel_before(gpu, orc, T, N):
+    """A norm whose gains are a row of the norm in front of it: each kernel releases its successor
+    early, so it has to wait for the gains as for the rows.  Buffers of their own for every link,
+    so that a read too early finds zeros."""
+    import torch
+    rng = np.random.default_rng(T + N)
+    links = 24
+    x = rng_codes(rng, (links, T, N), 1.0)
+    d_x = torch.from_numpy(x.view(np.int16)).cuda()
+    d_y = torch.zeros_like(d_x)
+    sp = torch.cuda.current_stream().cuda_stream
+    torch.cuda.synchronize()
+    for i in range(links):
+        gpu.rmsnorm_dev(d_x[i].data_ptr(), d_y[i - 1, T - 1].data_ptr() if i else None,
+                        d_y[i].data_ptr(), T, N, stream=sp)
+    torch.cuda.synchronize()
+    gains = None
+    for i in range(links):
+        y = orc.rmsnorm(x[i], gains)
+        assert np.array_equal(d_y[i].cpu().numpy().view(np.uint16), y), i
+        gains = y[T - 1]
+
+
 @pytest.mark.parametrize("N,pieces,warps", [
     (512, 2, 1), (768, 4, 1), (1024, 4, 1), (1280, 8, 1), (1792, 8, 1), (2048, 8, 1),
     (1152, -1, 1), (2304, -1, 1), (2560, -1, 1),                    # rows of the row norm
