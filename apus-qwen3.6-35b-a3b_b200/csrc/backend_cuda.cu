@@ -92,6 +92,7 @@ struct ApusCudaLayer {
     PrefillMaps *maps = nullptr; /* tensor maps for the tcgen05 path */
 };
 
+constexpr int DS_SYNC = 8;               /* 32 bytes from the other counters */
 struct Ctx {
     int device = 0;
     int sm_count = 0;
@@ -118,8 +119,8 @@ struct Ctx {
     uint32_t *d_df_codes = nullptr;              /* [DF_MAX_T][1025] */
     uint16_t *d_df_chains = nullptr;             /* [DF_MAX_T * 1025] */
     uint16_t *d_df_act = nullptr, *d_df_sa = nullptr;
-    unsigned int *d_df_sync = nullptr;
-    uint64_t *d_ds_codes = nullptr, *d_ds_chains = nullptr;     /* [DF_MAX_T][1025], tagged */
+    unsigned int *d_df_sync = nullptr;           /* decode_fused_kernel's; from DS_SYNC on: stacks */
+    uint64_t *d_ds_codes = nullptr, *d_ds_chains = nullptr;     /* [DS_WORDS], tagged */
     unsigned long long *d_df_timeline = nullptr;   /* [sm_count][DF_MARKS] */
     bool df_timeline_valid = false;
     size_t df_act_elems = 0, df_sa_elems = 0;
@@ -233,9 +234,9 @@ static int ctx_init() {
     if (c->fused_max_t > DF_MAX_T) c->fused_max_t = DF_MAX_T;
     CU_OK(cudaMalloc(&c->d_df_codes, (size_t)DF_MAX_T * 1025 * sizeof(uint32_t)));
     CU_OK(cudaMalloc(&c->d_df_chains, (size_t)DF_MAX_T * 1025 * sizeof(uint16_t)));
-    const size_t ds_words = (size_t)DF_MAX_T * 1025 * sizeof(uint64_t);
+    const size_t ds_words = (size_t)DS_WORDS * sizeof(uint64_t);
     CU_OK(cudaMalloc(&c->d_ds_codes, ds_words));
-    CU_OK(cudaMemset(c->d_ds_codes, 0, ds_words));      /* the tag of no launch */
+    CU_OK(cudaMemset(c->d_ds_codes, 0, ds_words));      /* the tag of no layer */
     CU_OK(cudaMalloc(&c->d_ds_chains, ds_words));
     CU_OK(cudaMemset(c->d_ds_chains, 0, ds_words));
     CU_OK(cudaMalloc(&c->d_df_sync, 64));
@@ -1341,6 +1342,14 @@ extern "C" int apus_cuda_debug_fast_logits(const uint16_t *x, const uint16_t *wg
     return 0;
 }
 
+extern "C" int apus_cuda_debug_decode_rounds(uint32_t rounds) {
+    std::lock_guard<std::recursive_mutex> lk(g_mu);
+    if (ctx_init()) return 1;
+    CU_OK(cudaDeviceSynchronize());
+    const unsigned at = rounds * DF_ROUND;
+    CU_OK(cudaMemcpy(g_ctx->d_df_sync + DS_SYNC, &at, sizeof at, cudaMemcpyHostToDevice));
+    return 0;
+}
 extern "C" int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int pieces, int warps,
                                      float *out) {
     if (!x || !out || !T || !N || N % 8 || N > 16384 || T > 65535)
@@ -1687,7 +1696,7 @@ static int run_stack_decode(Ctx *c, ApusCudaLayer *const *layers, int n, const u
     }
     a.code_ws = c->d_ds_codes; a.chain_ws = c->d_ds_chains;
     a.act_ws = c->d_df_act;
-    a.sync = c->d_df_sync + 8;
+    a.sync = c->d_df_sync + DS_SYNC;
     a.out = d_out;
     a.idx_out = tr ? tr->rtr_idx : nullptr;
     a.w_out = tr ? tr->rtr_w : nullptr;

@@ -45,6 +45,7 @@
 
 #include "common.cuh"
 #include "decode_gemv.cuh"
+#include "decode_tags.h"
 #include "exact_dense.cuh"
 #include "exact_sum.cuh"
 #include "router_select.cuh"
@@ -150,7 +151,6 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
 __device__ __forceinline__ void red_release_add(unsigned int *p, unsigned int v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-constexpr unsigned DF_ROUND = 256;      /* >= the number of CTAs, a power of two */
 /* the value a round counter reaches when every CTA of this launch has arrived; v was
  * read before this CTA arrived */
 __device__ __forceinline__ unsigned int round_target(unsigned int v) {

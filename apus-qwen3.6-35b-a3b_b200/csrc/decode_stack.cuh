@@ -18,7 +18,8 @@
  *    addresses.  (A request costs the copy engine 60 cycles, so rows of 1 KB one by one stream
  *    at 4.4 TB/s and pieces of 2 KB and more at 7.0.)
  *  - what a warp waits for comes with its own validity where it is small: logits and chains are
- *    64-bit words that hold the launch's tag, so no counter, fence and second look.
+ *    64-bit words that hold the layer's tag (decode_tags.h), so no counter, fence and second
+ *    look.
  *
  * Copies are dense, so the rows of a fragment lie on the same banks; a lane's 16 bytes are four
  * k steps of its row, and odd rows read the two halves of a 128-byte line the other way round.
@@ -35,7 +36,7 @@ constexpr int DS_PAIRS = 8;             /* gate/up pairs of a tile */
 constexpr int DS_CELL = 16 * 1024;      /* down rows of an expert: at most 16 of 1 KB */
 constexpr int DS_CELLS = 8;
 constexpr int DS_TILE = 2 * DS_PAIRS * DS_H * 2;        /* 64 KB: four cells */
-constexpr int DS_LAYERS = 32;           /* layers of a launch, at most (parameter space) */
+constexpr int DS_WORDS = DF_MAX_T * 1025;       /* tagged words of logits, and of chains */
 static_assert(CH_BYTES <= 8 * sizeof(SumShare), "a chain's products in the place of the sums'");
 static_assert(DS_CELL * DS_CELLS == 2 * DS_TILE, "two tiles or eight cells");
 
@@ -78,8 +79,9 @@ struct StackArgs {
     const uint16_t *x;                  /* as in FusedArgs */
     const uint16_t *res;
     uint16_t *res_out;
-    uint64_t *code_ws;                  /* [DF_MAX_T][E + 1] logit code intervals, tag above */
-    uint64_t *chain_ws;                 /* [DF_MAX_T * (E + 1)] codes of the walked chains, tag */
+    uint64_t *code_ws;                  /* [T][E + 1] logit code intervals, tag above */
+    uint64_t *chain_ws;                 /* [T * (E + 1)] codes of the walked chains, tag; both
+                                         * of DS_WORDS */
     uint16_t *act_ws;                   /* [DF_MAX_A + DF_MAX_T][I] */
     unsigned int *sync;                 /* barrier */
     uint16_t *out;
@@ -172,6 +174,25 @@ struct StackShared {
 
 /* Parts of a layer that most CTAs or warps never run, or that nobody waits for, as functions:
  * their code and registers stay out of the others' way. */
+
+/* All words lose their tags, before any CTA writes this launch's first ones; target: thread 0's
+ * of a round of its own. */
+__device__ __noinline__ void stack_clear_words(const StackArgs &a, StackShared &S,
+                                               unsigned int target) {
+#pragma unroll 1
+    for (int i = blockIdx.x * DS_THREADS + threadIdx.x; i < DS_WORDS; i += gridDim.x * DS_THREADS) {
+        st_tagged(&a.code_ws[i], 0, 0);
+        st_tagged(&a.chain_ws[i], 0, 0);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        round_arrive(a.sync);
+        if (!ds_spin(a.sync, target)) {
+            set_status(a.status, ST_SCHED_TIMEOUT);
+            S.dead = 1;
+        }
+    }
+}
 
 /* The open logits of token t are experts amb[t][0 .. namb[t]); counted through all tokens, pair i
  * is walked by CTA i % G.  This waits for that of pair k of token t, and puts it among the codes. */
@@ -406,7 +427,7 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     if (first) {
         if (tid == 0) {
             S.dead = 0;
-            sync_at = round_target(__ldcg(a.sync));
+            S.tag = sync_at = round_target(__ldcg(a.sync));
 #pragma unroll 1
             for (int i = 0; i < DS_CELLS; i++) {
                 mbar_init(&S.cell_full[i], 1);
@@ -419,6 +440,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
             mbar_fence_init();
         }
         __syncthreads();
+        if (stack_clears(S.tag)) {
+            stack_clear_words(a, S, sync_at);
+            sync_at += DF_ROUND;
+        }
     }
     /* a tile of n pairs, the first k of one expert and the others of the next: lanes 0-3
      * request a piece each */
@@ -470,7 +495,7 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
             if (!S.dead && !ds_spin(a.sync, sync_at)) give_up();
             sync_at += DF_ROUND;
         }
-        S.tag = sync_at;
+        S.tag = stack_tag(sync_at);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();

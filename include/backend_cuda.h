@@ -339,6 +339,10 @@ int apus_cuda_debug_fast_logits(const uint16_t *x, const uint16_t *wg, size_t T,
  * and lanes read them one at a time).  Refused where a row does not fit the form. */
 int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int pieces, int warps,
                           float *out);
+/* Diagnostic of the one-kernel decode (synchronous): its round counter as after this many rounds
+ * (modulo 2^24; a launch of n layers takes 2 n - 1), so that a test can see it wrap.  To be set
+ * ahead only, and not past the end of its range without a launch in the last 512 rounds before. */
+int apus_cuda_debug_decode_rounds(uint32_t rounds);
 
 /* Device-side status word of the last block call: 0 = ok; nonzero = a
  * bounded wait inside a kernel gave up (the context stays usable). */

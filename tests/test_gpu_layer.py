@@ -135,6 +135,44 @@ def test_stack_kernels_block_is_the_checkers(gpu, orc, be, synth, T, E, I, TK):
         check_block(got, exp, f"T={T} E={E} I={I}")
 
 
+def test_stack_at_the_end_of_the_round_counter(gpu, be, synth):
+    """The words that CTAs exchange carry the round counter as their tag, and the counter wraps:
+    what eight tokens left there a turn ago is not this call's, in no row and at no place of the
+    lists of chains.  (The middle layer's products underflow: all its logits are chains.)"""
+    import torch
+    T, H, L, END = 8, 2048, 3, 1 << 24
+    cfg = dict(hidden=H, experts=64, moe_inter=256, shared_inter=256, top_k=8)
+    layers = []
+    for l in range(L):
+        W = synth.host_weights(be, cfg, seed=83, layer=l, sigma=0.02)
+        if l == 1:
+            W["rtr_w"][:] = synth.f32_to_bf16(synth.bf16_to_f32(W["rtr_w"]) * 1e-36)
+        layers.append(gpu.layer_create(cfg, W))
+
+    def run(x, T, stack=layers):
+        y = x.clone()
+        gpu.moe_stack_dev(stack, y.data_ptr(), T)
+        torch.cuda.synchronize()
+        assert gpu.last_block_status() == 0
+        return y
+
+    a, b = (_dev(torch, synth.host_x(be, T, H, seed=s)) for s in (83, 84))
+    want_a, want_b, want_1, want_32 = run(a, T), run(b, T), run(a, 1), run(b, 3, layers[::2] * 16)
+    gpu.debug_decode_rounds(1000)
+    assert torch.equal(run(a, T), want_a)
+    gpu.debug_decode_rounds(END - 530)          # a launch of three layers takes five rounds
+    for i in range(60):
+        assert torch.equal(run(a, 1), want_1), i
+    assert torch.equal(run(b, T), want_b)
+    gpu.debug_decode_rounds(END - 30)
+    assert torch.equal(run(b, 3, layers[::2] * 16), want_32)    # its tags on both sides
+    assert torch.equal(run(a, 1), want_1)
+    gpu.debug_decode_rounds(1000)
+    assert torch.equal(run(b, T), want_b)       # the rounds, so the tags, of `a` above
+    for lay in layers:
+        gpu.layer_destroy(lay)
+
+
 def test_layer_at_the_real_dimensions_one_token(gpu, orc, be, synth):
     import torch
     cfg = synth.QWEN_CFG
