@@ -549,7 +549,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     __syncthreads();
 
     /* ---- router logits of this CTA's rows: up to two tokens four warps to one, up to four two
-     * (certified_logit, the rows cut across the warps like the norm's) ---- */
+     * (certified_logit, the rows cut across the warps like the norm's).  Its error terms hold
+     * with one factor larger: of u |lane sum| there are one for the lane's last addition, five for
+     * the scan and, where four warps share a row, up to three more, two in `before` and one in
+     * `tot`: nine, and ten are taken. ---- */
     const int lg = L.rrows > 2 || T > 4 ? 0 : T > 2 ? 1 : 2, per = 1 << lg;
     if (warp < DS_CW)
 #pragma unroll 1
@@ -595,7 +598,7 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                 sum += before;
                 tot += before;              /* (the last part's: the whole) */
             }
-            err = warp_sum(8.0f * nu * fabsf(sum - run) + 9.0f * err + 8.0f * fabsf(run));
+            err = warp_sum(8.0f * nu * fabsf(sum - run) + 9.0f * err + 10.0f * fabsf(run));
             if (per > 1) {
                 if (lane == 0) S.part[1][warp] = err;
                 meet();

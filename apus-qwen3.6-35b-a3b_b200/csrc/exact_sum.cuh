@@ -531,7 +531,8 @@ __device__ __forceinline__ float norm_above(float ss, int n) {
  *     eight is at most |sum before the lane| + |running sum before the eight| + the
  *     eight's sum of magnitudes;
  *   this sum against the true one:  4 u of the magnitudes, u |running sum| per eight,
- *     u |lane sum| per level of the scan.
+ *     u |lane sum| per level of the scan (five; six with the lane's last running sum, and
+ *     eight are taken).
  * The magnitudes of all eights together are at most cs = ||w|| ||x|| (Cauchy-Schwarz).
  * The factors below round up (second-order terms, and the fp32 sums that the bound
  * itself is built from). */

@@ -98,7 +98,10 @@ def test_block_one_kernel_path(gpu, orc, be, synth, qwen_weights, cfgname, T):
 
 
 @pytest.mark.parametrize("T,H,E,I,Is,TK", [
-    (5, 2048, 256, 512, 512, 8), (8, 2048, 256, 512, 512, 8), (7, 208, 37, 48, 16, 3),
+    (5, 2048, 256, 512, 512, 8), (8, 2048, 256, 512, 512, 8),
+    # rows of 2048: a logit's row cut over four warps (one and two tokens) and over two
+    (1, 2048, 256, 256, 256, 8), (2, 2048, 256, 512, 512, 8), (3, 2048, 256, 256, 256, 8),
+    (4, 2048, 256, 256, 256, 8), (4, 2048, 16, 256, 256, 4), (7, 208, 37, 48, 16, 3),
     (8, 1040, 300, 272, 144, 8), (3, 512, 1024, 128, 256, 2), (8, 16, 8, 16, 16, 8),
     (1, 128, 16, 32, 32, 1)])
 @pytest.mark.parametrize("case", ["plain", "tied_rows", "tiny_logits", "opposite", "underflow"])
@@ -179,6 +182,24 @@ def test_block_on_a_few_sms(be, orc, synth, monkeypatch, sms, T):
         got = be.moe_block(cfg, W, x)
         assert be.last_block_status() == 0
         check_block(got, orc.moe_block(cfg, W, x), f"T={T} on {sms} SMs")
+    finally:
+        be.disable()
+
+
+@pytest.mark.parametrize("T", [1, 3, 4, 8])
+def test_block_one_kernel_on_fewer_sms(be, orc, synth, monkeypatch, T):
+    """128 SMs have three router rows each, which warps then take one by one, and columns of
+    the down rows without a remainder."""
+    cfg = dict(hidden=2048, experts=256, moe_inter=256, shared_inter=256, top_k=8)
+    W = synth.host_weights(be, cfg, seed=78, sigma=0.02)
+    W["rtr_w"][1::2] = W["rtr_w"][0::2]
+    x = synth.host_x(be, T, cfg["hidden"], seed=T)
+    monkeypatch.setenv("APUS_CUDA_SMS", "128")
+    be.enable()
+    try:
+        got = be.moe_block(cfg, W, x)
+        assert be.last_block_status() == 0 and be.last_block_launches() == 1
+        check_block(got, orc.moe_block(cfg, W, x), f"T={T} on 128 SMs")
     finally:
         be.disable()
 
