@@ -63,7 +63,7 @@ SYMBOLS = [
     "apus_cuda_layer_refresh", "apus_cuda_layer_upload",
     "apus_cuda_layer_load_slabs", "apus_cuda_register_layer_slabs",
     "apus_cuda_debug_fast_logits", "apus_cuda_debug_sumsq", "apus_cuda_debug_decode_rounds",
-    "apus_cuda_moe_block_dev",
+    "apus_cuda_debug_decode_absent", "apus_cuda_moe_block_dev",
     "apus_cuda_moe_layer_dev", "apus_cuda_moe_stack_dev", "apus_cuda_reserve",
     "apus_cuda_last_block_launches", "apus_cuda_last_block_path",
     "apus_cuda_last_block_status",
@@ -139,6 +139,7 @@ class Backend:
                                                   f32p, f32p, f32p]
         L.apus_cuda_debug_sumsq.argtypes = [u16p, sz, sz, C.c_int, C.c_int, f32p]
         L.apus_cuda_debug_decode_rounds.argtypes = [C.c_uint32]
+        L.apus_cuda_debug_decode_absent.argtypes = [C.c_int]
         L.apus_cuda_moe_block_dev.argtypes = [vp, vp, vp, sz,
                                               C.POINTER(MoeTrace), vp]
         L.apus_cuda_moe_layer_dev.argtypes = [vp, vp, vp, vp, sz, C.POINTER(MoeTrace), vp]
@@ -394,6 +395,11 @@ class Backend:
         """The round counter of the one-kernel decode, set ahead."""
         self._check(self.lib.apus_cuda_debug_decode_rounds(rounds),
                     "apus_cuda_debug_decode_rounds")
+
+    def debug_decode_absent(self, cta):
+        """The next launch of the one-kernel decode does without this CTA, and times out."""
+        self._check(self.lib.apus_cuda_debug_decode_absent(cta),
+                    "apus_cuda_debug_decode_absent")
 
     def reserve(self, cfg, T):
         c = MoeCfg.from_dict(cfg)

@@ -123,6 +123,7 @@ struct Ctx {
     uint64_t *d_ds_codes = nullptr, *d_ds_chains = nullptr;     /* [DS_WORDS], tagged */
     unsigned long long *d_df_timeline = nullptr;   /* [sm_count][DF_MARKS] */
     bool df_timeline_valid = false;
+    int ds_absent = -1;
     size_t df_act_elems = 0, df_sa_elems = 0;
     int last_block_launches = 0;
     int last_block_path = 0;
@@ -1350,6 +1351,12 @@ extern "C" int apus_cuda_debug_decode_rounds(uint32_t rounds) {
     CU_OK(cudaMemcpy(g_ctx->d_df_sync + DS_SYNC, &at, sizeof at, cudaMemcpyHostToDevice));
     return 0;
 }
+extern "C" int apus_cuda_debug_decode_absent(int cta) {
+    std::lock_guard<std::recursive_mutex> lk(g_mu);
+    if (ctx_init()) return 1;
+    g_ctx->ds_absent = cta;
+    return 0;
+}
 extern "C" int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int pieces, int warps,
                                      float *out) {
     if (!x || !out || !T || !N || N % 8 || N > 16384 || T > 65535)
@@ -1697,6 +1704,8 @@ static int run_stack_decode(Ctx *c, ApusCudaLayer *const *layers, int n, const u
     a.code_ws = c->d_ds_codes; a.chain_ws = c->d_ds_chains;
     a.act_ws = c->d_df_act;
     a.sync = c->d_df_sync + DS_SYNC;
+    a.absent = c->ds_absent;
+    c->ds_absent = -1;
     a.out = d_out;
     a.idx_out = tr ? tr->rtr_idx : nullptr;
     a.w_out = tr ? tr->rtr_w : nullptr;

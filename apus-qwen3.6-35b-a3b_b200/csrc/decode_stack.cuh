@@ -84,6 +84,7 @@ struct StackArgs {
                                          * of DS_WORDS */
     uint16_t *act_ws;                   /* [DF_MAX_A + DF_MAX_T][I] */
     unsigned int *sync;                 /* barrier */
+    int absent;                         /* a CTA that leaves at once (a test's), or -1 */
     uint16_t *out;
     int32_t *idx_out;
     uint16_t *w_out;
@@ -113,20 +114,29 @@ __device__ __forceinline__ uint32_t no_negative_zero(uint32_t v) {
     if ((v >> 16) == 0x8000u) v &= 0xffffu;
     return v;
 }
-/* (rolled: the compiler's unrolling of the waits alone was 40 KB) */
-__device__ __forceinline__ bool ds_wait(uint64_t *bar, uint32_t parity) {
+/* Waits end when what they wait for is there, at their limit, or when the CTA has given up
+ * elsewhere (`dead`), so that one limit is waited for and not one for every piece that is missing.
+ * (rolled: the compiler's unrolling of the waits alone was 40 KB) */
+__device__ __forceinline__ bool ds_wait(uint64_t *bar, uint32_t parity, const volatile int &dead) {
 #pragma unroll 1
     for (uint32_t i = 0; i < APUS_WAIT_LIMIT; i++) {
         if (mbar_try_wait(bar, parity)) return true;
-        if (i > 64) __nanosleep(64);
+        if (i > 64) {
+            if (dead) return false;
+            __nanosleep(64);
+        }
     }
     return false;
 }
-__device__ __forceinline__ bool ds_spin(const unsigned int *p, unsigned int target) {
+__device__ __forceinline__ bool ds_spin(const unsigned int *p, unsigned int target,
+                                        const volatile int &dead) {
 #pragma unroll 1
     for (uint32_t i = 0; i < (1u << 21); i++) {
         if ((int)(ld_acquire(p) - target) >= 0) return true;
-        if (i > 64) __nanosleep(40);
+        if (i > 64) {
+            if (dead) return false;
+            __nanosleep(40);
+        }
     }
     return false;
 }
@@ -166,7 +176,8 @@ struct StackShared {
     int idx[DF_MAX_A], row[DF_MAX_A];   /* final order; down output of each */
     int uexp[DF_MAX_A], ubase[DF_MAX_A];
     int namb[DF_MAX_T], full[DF_MAX_T], open;
-    volatile int dead;
+    int asked[2 + DS_CELLS];            /* copies requested of each place of tiles, of cells */
+    volatile int dead;                  /* this CTA has given up: a wait ran out */
     unsigned int tag;                   /* of this launch and layer */
     uint16_t w[DF_MAX_A];
     uint8_t umask[DF_MAX_A];
@@ -187,11 +198,21 @@ __device__ __noinline__ void stack_clear_words(const StackArgs &a, StackShared &
     __syncthreads();
     if (threadIdx.x == 0) {
         round_arrive(a.sync);
-        if (!ds_spin(a.sync, target)) {
+        if (!ds_spin(a.sync, target, S.dead)) {
             set_status(a.status, ST_SCHED_TIMEOUT);
             S.dead = 1;
         }
     }
+}
+/* The first warp of a CTA that has given up, the others being through: its copies must have landed
+ * before the shared memory is another's. */
+__device__ __noinline__ void stack_drain(StackShared &S) {
+    const volatile int never = 0;
+    const int i = threadIdx.x;
+    if (i < 2 + DS_CELLS && S.asked[i] > 0)
+        ds_wait(i < 2 ? &S.tile_full[i] : &S.cell_full[i - 2], (unsigned)(S.asked[i] - 1) & 1u,
+                never);
+    __syncwarp();
 }
 
 /* The open logits of token t are experts amb[t][0 .. namb[t]); counted through all tokens, pair i
@@ -205,7 +226,10 @@ __device__ __forceinline__ bool take_chain(const StackArgs &a, StackShared &S, u
     for (uint32_t n = 0; !there && n < (1u << 21); n++) {
         c = ld_tagged(&a.chain_ws[at + k]);
         there = (unsigned)(c >> 32) == S.tag;
-        if (!there && n > 64) __nanosleep(40);
+        if (!there && n > 64) {
+            if (S.dead) break;
+            __nanosleep(40);
+        }
     }
     codes[at + amb[at + k]] = (uint32_t)c | ((uint32_t)c << 16);
     if (!there) set_status(a.status, ST_SCHED_TIMEOUT);
@@ -340,7 +364,8 @@ __device__ __noinline__ void stack_weights(const StackArgs &a, StackShared &S, u
 #pragma unroll 1
         for (int t = 0; t < T; t++)
 #pragma unroll 1
-            for (int k = lane; k < S.namb[t]; k += 32) take_chain(a, S, codes, amb, t, k);
+            for (int k = lane; k < S.namb[t]; k += 32)
+                if (!take_chain(a, S, codes, amb, t, k)) S.dead = 1;
     __syncwarp();
 #pragma unroll 1
     for (int t = 0; t < T; t++) {
@@ -367,12 +392,28 @@ __device__ __noinline__ void stack_weights(const StackArgs &a, StackShared &S, u
     __syncwarp();
 }
 
+/* A CTA that has given up leaves the launch before a layer's first barrier: the others' rounds, and
+ * the launches to come, count on its arrivals. */
+__device__ __noinline__ bool stack_leave(const StackArgs &a, int layer) {
+    if (threadIdx.x == 0) {
+        set_status(a.status, ST_SCHED_TIMEOUT);
+        red_release_add(a.sync, (2u * (a.n_layers - layer) - 1u) *
+                                    (blockIdx.x == 0 ? DF_ROUND - gridDim.x + 1u : 1u));
+    }
+    return false;
+}
+
 /* One layer; tile0, item0: gate/up tiles and down items before it; sync_at: thread 0's target
- * of the barrier. */
-__device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsigned int &sync_at,
-                                            int &tile0, int &item0) {
+ * of the barrier.  False: given up, in all warps.
+ *
+ * Where a wait runs out, S.dead is set and the status recorded.  The CTA's own barriers need all of
+ * its warps, so it goes on without waiting for anything, on whatever is there, to where the next
+ * selection would be, and leaves.  (There S.dead is read anyway; asking where a layer begins cost
+ * a quarter of a microsecond a layer.)  It is read between two barriers, between which nobody can
+ * be who may set it, so all warps agree. */
+__device__ __forceinline__ bool stack_layer(const StackArgs &a, StackShared &S, int layer,
+                                            unsigned int &sync_at, int &tile0, int &item0) {
     extern __shared__ __align__(128) unsigned char ds_smem[];
-    __shared__ StackShared S;
 
     const bool first = layer == 0;
     /* What is computed from these is computed again in every layer, and below in both phases,
@@ -413,7 +454,9 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
      * this CTA, so that nothing is left in flight when another CTA's part never came) */
     /* (by parity: whoever waits for the k-th has seen the one before it, or knows it to be over) */
     auto landed = [&](uint64_t *bar, int k) {
-        if (!ds_wait(bar, (unsigned)k & 1u)) give_up();
+        const bool ok = ds_wait(bar, (unsigned)k & 1u, S.dead);
+        if (!ok) give_up();
+        return ok;
     };
     mark(0);
     /* ---- this CTA's shares ---- */
@@ -430,6 +473,7 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
             S.tag = sync_at = round_target(__ldcg(a.sync));
 #pragma unroll 1
             for (int i = 0; i < DS_CELLS; i++) {
+                S.asked[i] = S.asked[2 + i] = 0;
                 mbar_init(&S.cell_full[i], 1);
                 mbar_init(&S.cell_free[i], 1u << a.slices_log2);
                 if (i < 2) {
@@ -444,15 +488,20 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
             stack_clear_words(a, S, sync_at);
             sync_at += DF_ROUND;
         }
+        if (cta == a.absent) return stack_leave(a, layer);
     }
     /* a tile of n pairs, the first k of one expert and the others of the next: lanes 0-3
      * request a piece each */
     auto request_tile = [&](int tile, const uint16_t *gate, const uint16_t *up, int k,
                             const uint16_t *gate2, const uint16_t *up2, int n) {
-        if (tile >= 2) landed(&S.tile_free[tile & 1], (tile >> 1) + 1);
+        const bool free = tile < 2 || landed(&S.tile_free[tile & 1], (tile >> 1) + 1);
+        if (!__all_sync(0xffffffffu, free)) return;
         uint64_t *bar = &S.tile_full[tile & 1];
         unsigned char *dst = ds_smem + (tile & 1) * DS_TILE;
-        if (lane == 0) mbar_expect_tx(bar, (uint32_t)(2 * n * DS_H * 2));
+        if (lane == 0) {
+            S.asked[tile & 1] = (tile >> 1) + 1;
+            mbar_expect_tx(bar, (uint32_t)(2 * n * DS_H * 2));
+        }
         __syncwarp();
         const int rows = lane & 2 ? n - k : k;
         if (lane < 4 && rows > 0)
@@ -492,7 +541,7 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
         S.open = 0;
         /* the rows that the other CTAs' combines left: the end of the layer before */
         if (!first) {
-            if (!S.dead && !ds_spin(a.sync, sync_at)) give_up();
+            if (!S.dead && !ds_spin(a.sync, sync_at, S.dead)) give_up();
             sync_at += DF_ROUND;
         }
         S.tag = stack_tag(sync_at);
@@ -622,7 +671,6 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
     const int fr = lane >> 2, fq = lane & 3;        /* row and piece of a fragment */
     const bool odd = fr & 1;
     int U = 0, gu_lo = 0, gu_n = 0, n_tiles = n_sh;
-    bool dead = false;
     /* the shared expert's gate/up rows, for which nobody waits; then the routed ones */
 #pragma unroll 1
     for (int phase = 0; phase < 2; phase++) {
@@ -659,7 +707,10 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
 #pragma unroll
                     for (int q = 0; q < R; q++) all &= (unsigned)(v[q] >> 32) == tag;
                     all = __all_sync(0xffffffffu, all);
-                    if (!all && i > 64) __nanosleep(40);
+                    if (!all && i > 64) {
+                        if (__any_sync(0xffffffffu, S.dead)) break;
+                        __nanosleep(40);
+                    }
                 }
 #pragma unroll
                 for (int q = 0; q < R; q++)
@@ -679,19 +730,20 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                 }
             }
             __syncthreads();
-            dead = S.dead != 0;
-            if (warp == DS_CW + 1 && !dead)
+            if (S.dead) return stack_leave(a, layer);
+            if (warp == DS_CW + 1)
                 stack_walk_chains(a, layer, S, amb, xs, ds_smem + L.off_share);
-            if (S.open && !dead) {          /* the set itself waits for the chains */
+            if (S.open) {                   /* the set itself waits for the chains */
                 if (tid < 256) s_tmask[tid] = 0;
+                __syncthreads();            /* (all have seen that S.dead is not set) */
 #pragma unroll 1
                 for (int t = warp; t < T; t += DS_THREADS / 32)
 #pragma unroll 1
                     for (int k = lane; k < S.namb[t]; k += 32)
                         if (!take_chain(a, S, codes, amb, t, k)) S.dead = 1;
                 __syncthreads();
-                dead = S.dead != 0;
-                if (warp < T && !dead) {
+                if (S.dead) return stack_leave(a, layer);
+                if (warp < T) {
                     stack_select_again(a, S, cd, warp);
                     mark_chosen();
                 }
@@ -699,7 +751,7 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
             }
             /* ---- the distinct experts, ascending, and who uses them: every warp writes the
              * whole list, and waits for nobody's ---- */
-            if (!dead) {
+            {
                 /* a lane has eight experts (E <= 256) */
                 const uint2 m = reinterpret_cast<const uint2 *>(s_tmask)[lane];
                 auto used = [](uint32_t v) {        /* 0x80 in each byte that is not zero */
@@ -759,12 +811,19 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                 /* ... when the tile that lies there has been read, then its item before this */
                 uint64_t *free_bar = &S.tile_free[(tile0 + (lane >> 2)) & 1];
                 int use = (tile0 - 2 + (lane >> 2)) >> 1;
+                /* (a limit behind the barrier's: what frees a cell may wait for that) */
 #pragma unroll 1
-                for (uint32_t n = 0; __any_sync(0xffffffffu, busy) && n < APUS_WAIT_LIMIT; n++) {
+                for (uint32_t n = 0; __any_sync(0xffffffffu, busy); n++) {
+                    if (n > 256) {
+                        if (n > 8 * APUS_WAIT_LIMIT) give_up();
+                        if (__any_sync(0xffffffffu, S.dead)) break;
+                        __nanosleep(20);
+                    }
                     if (busy && mbar_test(free_bar, (unsigned)use & 1u)) {
                         if (d <= U) {
                             const int c = (item0 + d) & (DS_CELLS - 1);
                             uint64_t *bar = &S.cell_full[c];
+                            S.asked[2 + c] = ((item0 + d) >> 3) + 1;
                             mbar_expect_tx(bar, bytes);
                             bulk_g2s(ds_smem + (((tile0 & 1) * 4 + d) & (DS_CELLS - 1)) * DS_CELL,
                                      (d == U ? W.sh_d : W.exp_d + (size_t)S.uexp[d] * DS_H * I) +
@@ -779,17 +838,16 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                         }
                     }
                 }
-                if (busy) give_up();
                 __syncwarp();
                 item0 += U + 1;
-                return;
+                return true;
             }
             if (warp > DS_CW) {
-                if (!dead) stack_weights(a, S, codes, amb, U);
+                stack_weights(a, S, codes, amb, U);
                 asm volatile("bar.arrive 2, %0;" ::"n"(DS_CW * 32 + 32) : "memory");
                 tile0 += n_tiles;
                 item0 += U + 1;
-                return;
+                return true;
             }
         }
         /* ---- gate/up tiles: the warps' partial sums meet in shared memory, four warps in
@@ -853,17 +911,17 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
                 }
             }
     }
-    if (warp >= DS_CW) return;              /* (not reached: for the compiler) */
+    if (warp >= DS_CW) return true;         /* (not reached: for the compiler) */
     tile0 += n_tiles;
     mark(4);                                /* routed gate/up done */
     df_bar_compute();
     if (tid == 0) {
         round_arrive(a.sync);
-        if (!S.dead && !ds_spin(a.sync, sync_at)) give_up();
+        if (!S.dead && !ds_spin(a.sync, sync_at, S.dead)) give_up();
         sync_at += DF_ROUND;                /* the layer's end */
     }
     df_bar_compute();
-    dead = S.dead != 0;
+    const bool dead = S.dead != 0;
     mark(5);                                /* barrier passed */
     /* ---- down rows of this CTA's columns: a warp to 128 k of an expert.  Its activations are
      * nobody else's here: they come straight from L2, beside the wait for the rows (all of them
@@ -969,15 +1027,19 @@ __device__ __forceinline__ void stack_layer(const StackArgs &a, int layer, unsig
         df_bar_compute();
         if (tid == 0) round_arrive(a.sync);
     }
+    return true;
 }
 
 __global__ void __launch_bounds__(DS_THREADS, 1)
 decode_stack_kernel(const __grid_constant__ StackArgs a) {
+    __shared__ StackShared S;
     unsigned int sync_at = 0;
     int tile0 = 0, item0 = 0;
 #pragma unroll 1
     for (int layer = 0; layer < a.n_layers; layer++)
-        stack_layer(a, layer, sync_at, tile0, item0);
+        if (!stack_layer(a, S, layer, sync_at, tile0, item0)) break;
+    __syncthreads();                        /* nobody requests or waits any more */
+    if (S.dead && threadIdx.x < 32) stack_drain(S);
 }
 
 }  // namespace apus

@@ -343,6 +343,10 @@ int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int pieces, int
  * (modulo 2^24; a launch of n layers takes 2 n - 1), so that a test can see it wrap.  To be set
  * ahead only, and not past the end of its range without a launch in the last 512 rounds before. */
 int apus_cuda_debug_decode_rounds(uint32_t rounds);
+/* ... and of what it does when a part never comes: in the next launch for rows of 2048 values this
+ * CTA takes no part.  The others' waits for it run out (one limit, about a second, for the whole
+ * launch), the status is 4, the results are not valid, and later calls are as ever. */
+int apus_cuda_debug_decode_absent(int cta);
 
 /* Device-side status word of the last block call: 0 = ok; nonzero = a
  * bounded wait inside a kernel gave up (the context stays usable). */

@@ -173,6 +173,38 @@ def test_stack_at_the_end_of_the_round_counter(gpu, be, synth):
         gpu.layer_destroy(lay)
 
 
+@pytest.mark.parametrize("T,L,cta", [(1, 1, 0), (3, 6, 5), (8, 32, 64), (8, 3, 147)])
+def test_stack_with_a_part_that_never_comes(gpu, be, synth, T, L, cta):
+    """A CTA that leaves at once, with router rows of its own (up to 64 here) and without: the
+    others' waits for its logits run out, once for the whole launch, whatever its layers, tiles
+    and cells; the status says so, and the next calls are right."""
+    import time
+    import torch
+    H = 2048
+    cfg = dict(hidden=H, experts=64, moe_inter=512, shared_inter=512, top_k=8)
+    layer = gpu.layer_create(cfg, synth.host_weights(be, cfg, seed=85, sigma=0.02))
+    d = _dev(torch, synth.host_x(be, T, H, seed=85))
+
+    def run():
+        y = d.clone()
+        torch.cuda.synchronize()
+        t = time.monotonic()
+        gpu.moe_stack_dev([layer] * L, y.data_ptr(), T)
+        torch.cuda.synchronize()
+        return y, time.monotonic() - t
+
+    want, _ = run()
+    assert gpu.last_block_status() == 0
+    gpu.debug_decode_absent(cta)
+    _, took = run()
+    assert gpu.last_block_status() == 4
+    assert took < 10, took                   # 32 layers would wait for 32 and more
+    for _ in range(3):
+        got, _ = run()
+        assert gpu.last_block_status() == 0 and torch.equal(got, want)
+    gpu.layer_destroy(layer)
+
+
 def test_layer_at_the_real_dimensions_one_token(gpu, orc, be, synth):
     import torch
     cfg = synth.QWEN_CFG
