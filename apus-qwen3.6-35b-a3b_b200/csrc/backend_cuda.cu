@@ -1253,7 +1253,7 @@ dbg_xnorm_kernel(const uint16_t *__restrict__ x, int T, int K, float *__restrict
     ss = warp_sum(ss);
     if (lane == 0) out[warp] = sqrtf(ss) * 1.001f;
 }
-/* the sum of squares of a row (a CTA each) by one warp or two */
+/* the sum of squares of a row (a CTA each) by four warps or two, the wide rows' form */
 template <int W>
 __global__ void __launch_bounds__(W * 32)
 dbg_sumsq_wide_kernel(const uint16_t *__restrict__ x, int N, LaneRow lr, int,
@@ -1268,6 +1268,7 @@ dbg_sumsq_wide_kernel(const uint16_t *__restrict__ x, int N, LaneRow lr, int,
     const float s = exact_sumsq_wide<W>(dq_smem, lr, lane, part, share, [] { __syncthreads(); });
     if (part == W - 1 && lane == 31) out[blockIdx.x] = s;
 }
+/* ... by one warp or two */
 template <int P, bool ALONE>
 __global__ void __launch_bounds__(64)
 dbg_sumsq_kernel(const uint16_t *__restrict__ x, int N, LaneRow lr, int parts,
@@ -1363,14 +1364,15 @@ extern "C" int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int 
         return fail("debug_sumsq: bad args");
     const LaneRow lr((int)N);
     const int per = warps > 0 ? lr.nu / warps : 0;
-    const bool wide = N == DS_H && ((pieces == 2 && warps == 4) || (pieces == 4 && warps == 2));
-    auto kern = wide          ? (warps == 4 ? dbg_sumsq_wide_kernel<4> : dbg_sumsq_wide_kernel<2>)
-                : pieces == 0 ? dbg_sumsq_kernel<0, false>
-                : pieces == 2 ? dbg_sumsq_kernel<2, false>
-                : pieces == 4 ? dbg_sumsq_kernel<4, false>
-                : pieces == 8 ? dbg_sumsq_kernel<8, false>
-                : pieces < 0  ? dbg_sumsq_kernel<0, true>
-                              : nullptr;
+    const bool wide = N == DS_H && ((pieces == -2 && (warps == 2 || warps == 4)) ||
+                                    (pieces == 2 && warps == 4));   /* (has one form only) */
+    auto kern = wide           ? (warps == 4 ? dbg_sumsq_wide_kernel<4> : dbg_sumsq_wide_kernel<2>)
+                : pieces == 0  ? dbg_sumsq_kernel<0, false>
+                : pieces == 2  ? dbg_sumsq_kernel<2, false>
+                : pieces == 4  ? dbg_sumsq_kernel<4, false>
+                : pieces == 8  ? dbg_sumsq_kernel<8, false>
+                : pieces == -1 ? dbg_sumsq_kernel<0, true>
+                               : nullptr;
     if (!kern || (warps != 1 && (warps != 2 || lr.nu % 2) && !wide) ||
         (pieces > 0 && per > pieces))
         return fail("debug_sumsq: %d pieces of %d, %d warps", pieces, lr.nu, warps);
@@ -1384,7 +1386,8 @@ extern "C" int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int 
     uint16_t *dx = (uint16_t *)c->io.take(T * N * 2);
     float *ds = (float *)c->io.take(T * 4);
     CU_OK(cudaMemcpyAsync(dx, x, T * N * 2, cudaMemcpyHostToDevice, c->stream));
-    kern<<<(unsigned)T, wide ? 32 * warps : 64, (size_t)lr.bytes(), c->stream>>>(dx, (int)N, lr, warps, ds);
+    kern<<<(unsigned)T, wide ? 32 * warps : 64, (size_t)lr.bytes(), c->stream>>>(dx, (int)N, lr,
+                                                                               warps, ds);
     LAUNCHED();
     CU_OK(cudaMemcpyAsync(out, ds, T * 4, cudaMemcpyDeviceToHost, c->stream));
     CU_OK(cudaStreamSynchronize(c->stream));

@@ -334,9 +334,10 @@ int apus_cuda_debug_fast_logits(const uint16_t *x, const uint16_t *wg, size_t T,
                                 float *wnorm, float *cbound);
 /* Diagnostic of the norms (host pointers, synchronous): the fp32 sum of squares of each row
  * of x [T,N], N % 8 == 0, as the sequential chain gives it (c/attn.h:175-186), by one warp to
- * a row or two (N 2048: four with 2 pieces and two with 4 are the one-kernel path's form);
- * pieces: the 16-byte pieces whose squares a lane keeps in registers (2, 4, 8; 0: none; -1: none,
- * and lanes read them one at a time).  Refused where a row does not fit the form. */
+ * a row or two; pieces: the 16-byte pieces whose squares a lane keeps in registers (2, 4, 8; 0:
+ * none; -1: none, and lanes read them one at a time; -2: the form for rows of 2048 values by two
+ * warps or four, which 2 pieces by four warps is as well).  Refused where a row does not fit
+ * the form. */
 int apus_cuda_debug_sumsq(const uint16_t *x, size_t T, size_t N, int pieces, int warps,
                           float *out);
 /* Diagnostic of the one-kernel decode (synchronous): its round counter as after this many rounds

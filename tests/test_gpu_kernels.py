@@ -600,7 +600,7 @@ def test_router_certified_can_be_switched_off(be, orc, synth, monkeypatch):
 
 
 # --- the callers either side of the block: rmsnorm before, residual add after ---
-@pytest.mark.parametrize("T,N", [(1, 2048), (5, 2048), (33, 512), (3, 130), (2, 24)])
+@pytest.mark.parametrize("T,N", [(1, 2048), (5, 2048), (149, 2048), (33, 512), (3, 130), (2, 24)])
 def test_rmsnorm_and_residual_add_bitwise(gpu, orc, be, synth, T, N):
     """apus_cuda_rmsnorm_dev / apus_cuda_resadd_dev against the checker
     (c/attn.h:175-186 with its sequential sum of squares; c/layer.h:230-234):
@@ -681,7 +681,7 @@ def test_rmsnorm_gains_from_the_kernel_before(gpu, orc, T, N):
     (512, 2, 1), (768, 4, 1), (1024, 4, 1), (1280, 8, 1), (1792, 8, 1), (2048, 8, 1),
     (1152, -1, 1), (2304, -1, 1), (2560, -1, 1),                    # rows of the row norm
     (512, 4, 2), (1536, 4, 2), (2048, 4, 2), (2560, 0, 2), (208, 0, 1), (144, 0, 1), (16, 4, 1), (1024, 4, 2),
-    (2048, 2, 4)])
+    (2048, 2, 4), (2048, -2, 2), (2048, -2, 4)])
 def test_sum_of_squares_is_the_chains(gpu, N, pieces, warps):
     """The fp32 sum itself, which a norm shows only through BF16, in every form that the row norm
     and the one-kernel path use: ties in every add, sums on a binade's edge, jumps over binades
