@@ -135,6 +135,79 @@ def test_stack_kernels_block_is_the_checkers(gpu, orc, be, synth, T, E, I, TK):
         check_block(got, exp, f"T={T} E={E} I={I}")
 
 
+@pytest.fixture(scope="module")
+def loud_weights(be, synth):
+    """Three layers of a shape, made once: down rows four times as large as the others."""
+    made = {}
+
+    def get(E, I):
+        if (E, I) not in made:
+            cfg = dict(hidden=2048, experts=E, moe_inter=I, shared_inter=I, top_k=8)
+            made.clear()
+            made[E, I] = cfg, [synth.host_weights(be, cfg, seed=86, layer=l, sigma=0.02)
+                               for l in range(3)]
+            for W in made[E, I][1]:
+                for name in ("exp_d", "sh_d"):
+                    W[name] += np.where(W[name] & 0x7f80, 0x100, 0).astype(np.uint16)
+        return made[E, I]
+    return get
+
+
+@pytest.mark.parametrize("T,E,I", [(1, 64, 256), (2, 160, 256), (3, 32, 512), (4, 48, 256),
+                                   (8, 64, 256)])
+@pytest.mark.parametrize("case", ["tied_rows", "tiny_logits", "opposite", "underflow"])
+def test_stack_of_hard_routers_is_the_checkers(gpu, orc, be, synth, loud_weights, T, E, I, case):
+    """Routers that leave the selection open, in the first layer of a launch and the ones behind it,
+    which find the lists, masks and chains of the layer before.  The stack of n layers starts from
+    what the stack of n - 1 gave, bit for bit, so each layer is checked by itself.
+
+    The block's norm is 0.2 of the stream's and more here (asserted), of which each side's last
+    narrowing is 2^-9 / sqrt(3) at most, 0.6 % of the block; with the block's own tolerance of 1 %
+    2e-2 bounds the difference.  One of a token's experts left out is 0.08 of the block and more
+    (the checker, these inputs), another in its place 1.4 times that."""
+    import torch
+    H, L = 2048, 3
+    cfg, base = loud_weights(E, I)
+    layers, weights = [], []
+    for l in range(L):
+        W = dict(base[l], rtr_w=base[l]["rtr_w"].copy())
+        rtr = W["rtr_w"]
+        if case == "tied_rows":
+            rtr[1::2] = rtr[0::2]
+        elif case == "tiny_logits":
+            rtr[:] = synth.f32_to_bf16(synth.bf16_to_f32(rtr) * 2.0 ** -14)
+        elif case == "opposite":            # the stream stays in pairs, so that every sum cancels
+            rtr[:, 1::2] = rtr[:, 0::2] ^ 0x8000
+            W["exp_d"] = np.repeat(W["exp_d"].reshape(E, H, I)[:, 0::2], 2, axis=1)
+            W["sh_d"] = np.repeat(W["sh_d"].reshape(H, I)[0::2], 2, axis=0)
+        else:
+            rtr[:] = synth.f32_to_bf16(synth.bf16_to_f32(rtr) * 1e-36)
+        weights.append(W)
+        layers.append(gpu.layer_create(cfg, W))
+    first = synth.host_x(be, T, H, seed=86 + T)
+    if case == "opposite":
+        first[:, 1::2] = first[:, 0::2]
+    res = first
+    for n in range(1, L + 1):
+        y = _dev(torch, first)
+        before = gpu.router_exact_chains()
+        gpu.moe_stack_dev(layers[:n], y.data_ptr(), T)
+        torch.cuda.synchronize()
+        if case in ("opposite", "underflow"):       # (half of them at least, in every layer)
+            assert gpu.router_exact_chains() - before >= n * T * E // (
+                1 if case == "underflow" else 2)
+        assert gpu.last_block_status() == 0 and gpu.last_block_launches() == 1
+        got = y.cpu().numpy().view(np.uint16)
+        exp = orc.resadd(res, orc.moe_block(cfg, weights[n - 1], orc.rmsnorm(res, None))["out"])
+        diff = np.linalg.norm(f32(got) - f32(exp), axis=1)
+        block = np.linalg.norm(f32(exp) - f32(res), axis=1)
+        assert (block >= 0.2 * np.linalg.norm(f32(res), axis=1)).all()
+        assert (diff <= 2e-2 * block).all(), (n, diff / block)
+        res = got
+    for lay in layers:
+        gpu.layer_destroy(lay)
+
+
 def test_stack_at_the_end_of_the_round_counter(gpu, be, synth):
     """The words that CTAs exchange carry the round counter as their tag, and the counter wraps:
     what eight tokens left there a turn ago is not this call's, in no row and at no place of the
@@ -221,14 +294,15 @@ def test_layer_at_the_real_dimensions_one_token(gpu, orc, be, synth):
     assert np.array_equal(d_out.cpu().numpy().view(np.uint16), out3)
 
 
-@pytest.mark.parametrize("H", [208, 512, 768, 1280, 1536, 2048])
-def test_one_kernel_norm_on_rows_made_to_go_wrong(gpu, be, synth, H):
+@pytest.mark.parametrize("H,I", [(208, 16), (512, 16), (768, 16), (1280, 16), (1536, 16),
+                                 (2048, 16), (2048, 256)])
+def test_one_kernel_norm_on_rows_made_to_go_wrong(gpu, be, synth, H, I):
     """The one-kernel path's norm, one warp or two to a row and lane chunks in registers or not,
     against the row kernel's in the layer's output: sums on the edge of a binade, ties in every
     add, a jump over binades, rising and falling terms.  (Last bits of the sum seldom show here:
     test_sum_of_squares_is_the_chains compares them.)"""
     import torch
-    cfg = dict(hidden=H, experts=64, moe_inter=16, shared_inter=16, top_k=8)
+    cfg = dict(hidden=H, experts=64, moe_inter=I, shared_inter=I, top_k=8)
     layer = gpu.layer_create(cfg, synth.host_weights(be, cfg, seed=H, sigma=0.05))
     rng = np.random.default_rng(H)
     rows = [np.ones(H), np.full(H, 1.0 + 2 ** -7), rng.integers(1, 4, H) * 0.5,
