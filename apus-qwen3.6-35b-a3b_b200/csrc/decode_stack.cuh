@@ -7,7 +7,8 @@
  * What bounds a layer at few tokens is not the 58 MB of weights (9 us) but instructions: each is
  * fetched for the first time when it is needed, at about 8 cycles an instruction out of L2, 2.7
  * once it is in the 128 KB that an SM keeps, 1 in the innermost 28 KB.  (decode_fused_kernel:
- * 166 KB of code; 25 % of the warps' time waiting for instructions.)  So
+ * 176 KB of code; 25 % of the warps' time waiting for instructions.  Here: 111 KB, and 29 in
+ * functions beside a layer's way.)  So
  *  - a stack of layers is a loop in the kernel: from the second layer on, the code is there, and
  *    no launch lies between two layers, only a grid barrier;
  *  - there is little code: the row length is a constant, loops are rolled where a phase runs once,
@@ -433,9 +434,10 @@ __device__ __forceinline__ bool stack_layer(const StackArgs &a, StackShared &S, 
     unsigned char *xs = ds_smem + L.off_x, *rr = ds_smem + L.off_rr;
     uint4 *gains = reinterpret_cast<uint4 *>(ds_smem + L.off_gain);
     uint32_t *codes = reinterpret_cast<uint32_t *>(ds_smem + L.off_code);   /* [T][E + 1] */
-    uint16_t *amb = reinterpret_cast<uint16_t *>(ds_smem + L.off_amb);      /* t << 11 | e */
-    uint32_t *s_tmask = reinterpret_cast<uint32_t *>(ds_smem + L.off_tmask);   /* [256]: tokens of
-                                                        * each expert, a byte each */
+    uint16_t *amb = reinterpret_cast<uint16_t *>(ds_smem + L.off_amb);      /* [T][E + 1]: a
+                                                        * token's open logits, S.namb of them */
+    uint32_t *s_tmask = reinterpret_cast<uint32_t *>(ds_smem + L.off_tmask);   /* tokens of each
+                                                        * expert, a byte each (64 words in use) */
     float *red = reinterpret_cast<float *>(ds_smem + L.off_red);
     const uint16_t *res = first ? a.res : a.res_out;
 
